@@ -93,3 +93,38 @@ def test_bin_edges_follow_numpy():
         out = post.zenith_brf(w, rec, n_bins)
     ref = np.histogram(theta, bins=n_bins, range=(0., np.pi / 2))[0]
     assert np.array_equal(out['counts'][0], ref)
+
+
+@pytest.mark.parametrize('n,n_bins,n_cfg,order,dtype', [
+    (1, 137, 1, 'sorted', 'RECORD32'), (31, 1, 2, 'sorted', 'RECORD32'), (257, 18, 3, 'mixed', 'RECORD32'),
+    (70001, 2048, 5, 'sorted', 'RECORD32P'), (70001, 2049, 5, 'mixed', 'RECORD32'),
+    (70001, 137, 300, 'sorted', 'RECORD64'), (70001, 90, 300, 'mixed', 'RECORD64P')])
+def test_records_in_any_order_match_numpy(walker, n, n_bins, n_cfg, order, dtype):
+    """Block and warp remainders, configs in runs and in no order, bins within and past the
+    shared-memory histogram, angles outside [0, pi/2] and undefined, unused conditions."""
+    rng = np.random.default_rng(n + n_bins)
+    rec = np.zeros(n + 1, getattr(_abi, dtype))[1:]
+    rec['condition'] = rng.integers(0, 7, n)
+    rec['n_scat'] = rng.integers(0, 2000, n)
+    rec['wvn'] = rng.uniform(0.5, 1.2, n)
+    rec['theta_n'] = rng.uniform(-0.1, 1.7, n)
+    rec['theta_n'][::17] = np.nan
+    rec['path_length'] = rng.exponential(0.1, n)
+    rec['config'] = rng.integers(0, n_cfg + 1, n)          # one config past the asked ones
+    if order == 'sorted':
+        rec['config'] = np.sort(rec['config'])
+    out = post.zenith_brf(walker, rec, n_bins, n_cfg)
+    edges = np.linspace(0., np.pi / 2, n_bins + 1)
+    used = (rec['condition'] >= 1) & (rec['condition'] <= 5)
+    for c in range(n_cfg):
+        at = used & (rec['config'] == c)
+        up = at & (rec['condition'] == 1) & np.isfinite(rec['theta_n'])
+        theta, wvn = rec['theta_n'][up].astype(np.float64), rec['wvn'].astype(np.float64)
+        assert np.array_equal(out['counts'][c], np.histogram(theta, edges)[0])
+        assert np.allclose(out['hist'][c], np.histogram(theta, edges, weights=wvn[up])[0], rtol=1e-9, atol=0)
+        assert np.array_equal(out['n_cond'][c][1:], [np.sum(at & (rec['condition'] == k)) for k in range(1, 6)])
+        assert np.isclose(out['q_down'][c], wvn[at].sum(), rtol=1e-9, atol=0)
+        if at.any():
+            assert np.isclose(out['mean_wavelength'][c], np.mean(1 / wvn[at]), rtol=1e-12, atol=0)
+            assert np.isclose(out['mean_path_length'][c], rec['path_length'][at].astype(np.float64).mean(), rtol=1e-12, atol=0)
+            assert out['mean_n_scat'][c] == rec['n_scat'][at].astype(np.int64).sum() / at.sum()
