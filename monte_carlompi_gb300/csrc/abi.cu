@@ -356,7 +356,7 @@ int make_plan(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, int32_t mode,
 }
 
 struct Shape {
-    int grid, block, chunk, bps;
+    int grid, block, chunk, bps, lanes;
 };
 
 Shape pick_shape(const mcw_ctx *ctx, const mcw_launch &l, const Plan &plan) {
@@ -367,10 +367,9 @@ Shape pick_shape(const mcw_ctx *ctx, const mcw_launch &l, const Plan &plan) {
     if (occ <= 0) occ = 1;
     s.bps = (l.blocks_per_sm > 0) ? std::min(l.blocks_per_sm, occ) : occ;
     s.chunk = l.regen_chunk;
-    int64_t grid = (int64_t)ctx->sm_count * s.bps;
-    const int64_t needed = (total + s.block - 1) / s.block;
-    grid = std::max<int64_t>(1, std::min(grid, needed));
-    s.grid = (int)grid;
+    const WalkSpread spread = spread_walk(total, (int64_t)ctx->sm_count * s.bps, s.block);
+    s.grid = spread.grid;
+    s.lanes = spread.lanes;
     return s;
 }
 
@@ -435,7 +434,7 @@ LutArgs lut_args(const mcw_ctx *ctx, const Plan &plan, DevBuf &cfgs, DevBuf &lut
 }
 
 WalkArgs walk_args(const mcw_ctx *ctx, const Plan &plan, DevBuf &cfgs, DevBuf &lut, DevBuf &tallies,
-                   DevBuf &counters, mcw_record32 *records, int chunk, uint64_t seed) {
+                   DevBuf &counters, mcw_record32 *records, int chunk, int lanes, uint64_t seed) {
     WalkArgs wa{};
     wa.cfgs = (const DevConfig *)cfgs.p;
     wa.prefix = (const int64_t *)((const char *)cfgs.p + prefix_offset(plan.cfgs.size()));
@@ -444,6 +443,7 @@ WalkArgs walk_args(const mcw_ctx *ctx, const Plan &plan, DevBuf &cfgs, DevBuf &l
     wa.lut = (const LutEntry *)lut.p;
     wa.n_cfg = (int32_t)plan.cfgs.size();
     wa.regen_chunk = chunk;
+    wa.lanes = lanes;
     wa.total = plan.total;
     Counters *cn = (Counters *)counters.p;
     wa.work = &cn->work;
@@ -458,6 +458,8 @@ WalkArgs walk_args(const mcw_ctx *ctx, const Plan &plan, DevBuf &cfgs, DevBuf &l
     return wa;
 }
 
+constexpr int32_t kDrainSpread = 512;
+
 // Attach the drain queue (one slot per thread of the walk grid) when handover is on.
 int attach_drain(mcw_ctx *ctx, WalkArgs &wa, DevBuf &drain, const Shape &shape) {
     wa.drain = nullptr;
@@ -467,6 +469,11 @@ int attach_drain(mcw_ctx *ctx, WalkArgs &wa, DevBuf &drain, const Shape &shape) 
     wa.drain = (float4 *)drain.p;
     wa.drain_cap = (uint32_t)((size_t)shape.grid * shape.block);
     wa.drain_from = ctx->launch.drain_from;
+    // a launch whose photons all start at once is as long as its longest walk: a photon goes to
+    // a block of its own early.  Deep snow, kernel time handing over past 256 / 512 / 4096 steps:
+    // 1,000 photons 103 / 105 / 134 us, 10,000 238 / 255 / 298, 60,000 537 / 515 / 629; walks of
+    // 40 steps (few reach it) 46 / 44 / 44, 62 / 60 / 58, 93 / 91 / 87
+    if (shape.lanes < 32) wa.drain_from = std::min(wa.drain_from, kDrainSpread);
     return MCW_OK;
 }
 
@@ -830,7 +837,7 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
     }
     // the launch shape first (occupancy queries, allocations): once the copies and
     // kernels below are queued, nothing on the host stands between them
-    Shape shape{0, 0, 0, 0};
+    Shape shape{0, 0, 0, 0, 32};
     if (mode == MCW_MODE_F32) shape = pick_shape(ctx, ctx->launch, plan);
     uint64_t h2d = 0;
     // a call on the configs and tables of the previous F32 / POL32 call finds their
@@ -864,7 +871,7 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
     };
     if (mode == MCW_MODE_F32) {
         WalkArgs wa = walk_args(ctx, plan, ctx->cfgs, ctx->lut, ctx->tallies, ctx->counters,
-                                (mcw_record32 *)dev_records, shape.chunk, seed);
+                                (mcw_record32 *)dev_records, shape.chunk, shape.lanes, seed);
         rc = attach_drain(ctx, wa, ctx->drain, shape);
         if (rc) return rc;
         // the lookup-table kernel also clears the counters and tallies
@@ -877,7 +884,7 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
         // the lookup-table kernel also clears the counters and tallies
         if ((rc = lut_launch())) return rc;
         WalkArgs wa = walk_args(ctx, plan, ctx->cfgs, ctx->lut, ctx->tallies, ctx->counters,
-                                (mcw_record32 *)dev_records, 1, seed);
+                                (mcw_record32 *)dev_records, 1, 32, seed);
         wa.phase = (const DevPhase32 *)ctx->phase_tables32.p;
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, st));
         CUDA_TRY(ctx, launch_walk_pol32(wa, ctx->sm_count, st));
@@ -1109,7 +1116,7 @@ int mcw_graph_create(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, mcw_re
     const Shape shape = pick_shape(ctx, ctx->launch, plan);
     g->grid = shape.grid;
     g->block = shape.block;
-    g->args = walk_args(ctx, plan, g->cfgs, g->lut, g->tallies, g->counters, device_records, shape.chunk, 0);
+    g->args = walk_args(ctx, plan, g->cfgs, g->lut, g->tallies, g->counters, device_records, shape.chunk, shape.lanes, 0);
     rc = attach_drain(ctx, g->args, g->drain, shape);
     if (rc) return fail(rc);
     const LutArgs la = lut_args(ctx, plan, g->cfgs, g->lut, g->tallies, g->counters);

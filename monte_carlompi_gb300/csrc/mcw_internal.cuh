@@ -124,6 +124,9 @@ struct WalkArgs {
     const LutEntry *lut;
     int32_t n_cfg;
     int32_t regen_chunk;
+    // photons a warp walks at once (1 to 32).  Below 32 the launch holds every photon in its
+    // warps' first claims (lanes * warps >= total), so no warp claims a second time.
+    int32_t lanes;
     int64_t total;               // photons over all configs
     unsigned long long *work;    // next unclaimed global photon id
     unsigned int *status;
@@ -183,6 +186,24 @@ struct LutArgs {
 
 // Why a config is invalid (nullptr when valid); n_ice = number of ice tables.
 const char *config_problem(const mcw_config &c, int32_t n_ice);
+
+// How a walk of `total` photons is spread over at most max_grid blocks of `block` threads: the
+// photons a warp walks at once (WalkArgs::lanes), as few as hold every photon, and the blocks
+// that then have one.  A warp with few photons computes their draws across its idle lanes
+// (sparse rounds) and walks fewer block passes one after another: 1,000 photons of deep snow on
+// 4 full blocks took 345 us (walk and drain kernels), on 125 blocks of one photon per warp
+// 134 us.
+struct WalkSpread {
+    int grid, lanes;
+};
+inline WalkSpread spread_walk(int64_t total, int64_t max_grid, int block) {
+    const int64_t warps = block / 32, slots = max_grid * warps;
+    int64_t lanes = (total + slots - 1) / slots;
+    lanes = lanes < 1 ? 1 : (lanes > 32 ? 32 : lanes);
+    int64_t grid = (total + warps * lanes - 1) / (warps * lanes);
+    grid = grid < 1 ? 1 : (grid > max_grid ? max_grid : grid);
+    return {(int)grid, (int)lanes};
+}
 
 // Kernel launchers (defined in the .cu files).
 // recs: n records of `stride` bytes starting with an mcw_record64 (f64) or mcw_record32.

@@ -233,10 +233,9 @@ extern "C" int mcw_walk_noalloc(const mcw_config *cfg, const mcw_ssp_table *ice_
         const bool impurity = c.imp_cnc > 0;
         int bps = walk_f32_max_blocks_per_sm(256, 1, impurity);
         if (bps < 1) bps = 1;
-        int64_t grid = (int64_t)sms * bps;
-        const int64_t needed = (c.n_photon + 255) / 256;
-        if (grid > needed) grid = needed;
-        if (launch_walk_f32(wa, impurity, (int)grid, 256, sms, st) != cudaSuccess) return MCW_ERR_CUDA;
+        const WalkSpread spread = spread_walk(c.n_photon, (int64_t)sms * bps, 256);
+        wa.lanes = spread.lanes;
+        if (launch_walk_f32(wa, impurity, spread.grid, 256, sms, st) != cudaSuccess) return MCW_ERR_CUDA;
     }
     NoAllocCounters h;
     if (cudaMemcpyAsync(&h, &s->counters, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess) return MCW_ERR_CUDA;

@@ -1187,13 +1187,13 @@ __global__ void __launch_bounds__(256, 2) walk_f32_kernel(const WalkArgs a) {
         if (nidle > 0 && (nidle >= a.regen_chunk || nidle == 32) && !(exhausted && n_birth == 0)) {
             int cnt = n_birth;
             if (cnt < nidle && !exhausted) {
-                const int want = 32 - cnt;
+                const int want = a.lanes - cnt;
                 unsigned long long base = 0;
                 if (lane == 0) base = atomicAdd(a.work, (unsigned long long)want);
                 base = __shfl_sync(0xffffffffu, base, 0);
                 const int64_t left = a.total - (int64_t)base;
                 const int valid = (int)max((int64_t)0, min((int64_t)want, left));
-                if (left <= want) exhausted = true;
+                if (left <= want || a.lanes < 32) exhausted = true;
                 if (lane < valid) {
                     const int64_t g = (int64_t)base + lane;
                     const int k = find_config(claim, a.n_cfg, g);

@@ -349,6 +349,18 @@ def test_f32_sparse_rounds_same_records(walker, n):
         assert np.array_equal(small.records, big.records[:n]), case
 
 
+@pytest.mark.parametrize('n', [40, 2431, 2433, 19457, 77823, 77825])
+def test_f32_records_independent_of_spread(walker, n):
+    """Photons spread over the warps of the grid, from one a warp to full warps and past the
+    grid's lanes (152 SMs x 16 warps = 2,432 warps): the first n records of a larger run."""
+    cfg, ice, imp = cfg2_geometry(90000)
+    walker.set_tables([ice], imp)
+    big = walker.walk([cfg], 17, mode='f32')
+    small = walker.walk([dataclasses.replace(cfg, n_photon=n)], 17, mode='f32')
+    assert np.array_equal(small.records, big.records[:n])
+    assert int(small.tallies['n_cond'][0].sum()) == n
+
+
 def test_f32_long_walks_same_records_with_and_without_drain(walker):
     """Weakly absorbing, deep snow (lambda 1.0 um, r_eff 50 um, tau ~1000: walks of
     thousands of steps): the walks that leave for the drain queue, whose block passes a
