@@ -186,15 +186,23 @@ __device__ __forceinline__ bool try_wait(uint64_t *bar, uint32_t parity) {
 // Bounded wait on the phase of the given parity.  With an abort flag the wait also
 // gives up as soon as another role has given up, and a timeout raises the flag.
 __device__ __forceinline__ bool wait_bar(uint64_t *bar, uint32_t parity, volatile int *abort) {
-    const unsigned long long t0 = now_ns();
-    while (!try_wait(bar, parity)) {
+    unsigned long long t0 = 0;
+    for (unsigned tries = 1; !try_wait(bar, parity); ++tries) {
+        if (tries & 63u) continue;
         if (abort && *abort) return false;
-        if (now_ns() - t0 > kWaitNs) {
+        const unsigned long long t = now_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > kWaitNs) {
             if (abort) *abort = 1;
             return false;
         }
     }
     return true;
+}
+
+// The same by a whole warp, with one verdict.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile int *abort) {
+    return __all_sync(0xffffffffu, wait_bar(bar, parity, abort));
 }
 
 __device__ __forceinline__ void arrive(uint64_t *bar) {
@@ -212,26 +220,43 @@ __device__ __forceinline__ void load_chunk(void *dst, const void *src, uint32_t 
                  : "memory");
 }
 
+// One lane of the converged warp, the same each time (its MMAs and commits are one sequence).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t yes;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(yes));
+    return yes != 0;
+}
+
 __device__ __forceinline__ void commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
                  :: "r"(smem_u32(bar)));
 }
 
-// `steps` MMAs of K = 16: A k-steps a_step0 .. from a tile with rows of a_kdim,
-// B k-steps 0 .. from a tile with rows of b_kdim.
-__device__ __forceinline__ void mma_steps(uint32_t tmem, uint32_t a_base, int a_kdim, int a_step0, uint32_t b_base,
-                                          int b_kdim, int steps, uint32_t id, bool accumulate_first) {
-#pragma unroll 1
-    for (int t = 0; t < steps; ++t) {
-        const uint64_t da = smem_desc(a_base + (uint32_t)(a_step0 + t) * 256, 128, (uint32_t)(a_kdim / 8) * 128);
-        const uint64_t db = smem_desc(b_base + (uint32_t)t * 256, 128, (uint32_t)(b_kdim / 8) * 128);
-        const uint32_t acc = (accumulate_first || t > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-            :: "r"(tmem), "l"(da), "l"(db), "r"(id), "r"(acc));
+// kSteps MMAs of K = 16: A k-steps a_step0 .. from a tile with rows of kAk, B k-steps 0 .. from
+// a tile with rows of kBk.  Called by the whole warp, one elected lane issues: the descriptors
+// then are computed in uniform registers (under `lane == 0` each MMA took about 200 cycles to
+// issue, 13 us of a tile's 129; 65,536 rows of five members 313 us, now 287).
+template <int kAk, int kBk, int kSteps>
+__device__ __forceinline__ void mma_steps(uint32_t tmem, uint32_t a_base, int a_step0, uint32_t b_base, uint32_t id,
+                                          bool accumulate_first) {
+    if (elect_one()) {
+#pragma unroll
+        for (int t = 0; t < kSteps; ++t) {
+            const uint64_t da = smem_desc(a_base + (uint32_t)(a_step0 + t) * 256, 128, (uint32_t)(kAk / 8) * 128);
+            const uint64_t db = smem_desc(b_base + (uint32_t)t * 256, 128, (uint32_t)(kBk / 8) * 128);
+            const uint32_t acc = (accumulate_first || t > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                :: "r"(tmem), "l"(da), "l"(db), "r"(id), "r"(acc));
+        }
     }
+    __syncwarp();
 }
 
 // 32 consecutive accumulator columns of this warp's 32 lanes: issue, then wait.  The
@@ -538,7 +563,7 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     volatile int *abort = &abort_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // networks of an ensemble: CTA blockIdx.x carries tile (blockIdx.x % tiles) of member
     // (blockIdx.x / tiles), whose biases lie bias_stride floats and whose packed weights
     // blob_stride bytes after the previous member's, its output rows m * ldy after them
@@ -569,19 +594,21 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
     asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n");
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
     if (warp == kProducerWarp) {
-        if (lane == 0) {
+        {
             int issued = 0;
             for (int i = 0; i < kSeqChunks; ++i) {
                 const int slot = i % kSlots;
-                if (i >= kSlots && !wait_bar(&bars.empty[slot], (uint32_t)(i / kSlots - 1) & 1u, abort)) break;
+                if (i >= kSlots && !warp_wait(&bars.empty[slot], (uint32_t)(i / kSlots - 1) & 1u, abort)) break;
                 const int c = chunk_at(i);
-                load_chunk(ring + slot * kChunkBytes,
-                           blob + (kEnsemble ? (size_t)((int)blockIdx.x / tiles) * (size_t)blob_stride : 0) +
-                               chunk_offset(c),
-                           chunk_bytes(c), &bars.full[slot]);
+                if (elect_one())
+                    load_chunk(ring + slot * kChunkBytes,
+                               blob + (kEnsemble ? (size_t)((int)blockIdx.x / tiles) * (size_t)blob_stride : 0) +
+                                   chunk_offset(c),
+                               chunk_bytes(c), &bars.full[slot]);
+                __syncwarp();
                 issued = i + 1;
             }
             // the last copy into each slot has landed before the CTA can leave
@@ -589,7 +616,7 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
                 wait_bar(&bars.full[i % kSlots], (uint32_t)(i / kSlots) & 1u, nullptr);
         }
     } else if (warp == kMmaWarp) {
-        if (lane == 0) {
+        {
             const uint32_t ring_a = smem_u32(ring);
             int chunk = 0;
             uint32_t act_phase[kTiles];
@@ -597,16 +624,21 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
             bool ok = true;
             auto take = [&](void) -> uint32_t {      // wait for the next chunk; its shared address
                 const int slot = chunk % kSlots;
-                ok = ok && wait_bar(&bars.full[slot], (uint32_t)(chunk / kSlots) & 1u, abort);
+                ok = ok && warp_wait(&bars.full[slot], (uint32_t)(chunk / kSlots) & 1u, abort);
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
                 return ring_a + (uint32_t)slot * kChunkBytes;
             };
             auto release = [&](void) {               // chunk's MMAs issued: free its slot when they finish
-                commit(&bars.empty[chunk % kSlots]);
+                if (elect_one()) commit(&bars.empty[chunk % kSlots]);
+                __syncwarp();
                 ++chunk;
             };
+            auto done = [&](uint64_t *bar) {         // arrive when the MMAs issued so far are complete
+                if (elect_one()) commit(bar);
+                __syncwarp();
+            };
             auto wait_act = [&](int t) {             // tile t's input / activations written
-                ok = ok && wait_bar(&bars.act[t], act_phase[t], abort);
+                ok = ok && warp_wait(&bars.act[t], act_phase[t], abort);
                 act_phase[t] ^= 1u;
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
             };
@@ -616,9 +648,9 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
                 if (!ok) break;
                 const uint32_t w = take();
                 if (!ok) break;
-                mma_steps(tmem + (uint32_t)(t * 256), smem_u32(xt0 + t * kXBytes), FK1, 0, w, FK1, 1, idesc(FH), false);
+                mma_steps<FK1, FK1, 1>(tmem + (uint32_t)(t * 256), smem_u32(xt0 + t * kXBytes), 0, w, idesc(FH), false);
                 release();
-                commit(&bars.accf[t][0]);
+                done(&bars.accf[t][0]);
             }
             // layers 2 and 3: eight chunks of 32 k each, tile by tile (one tile's MMAs run
             // while the other's epilogue writes its activations)
@@ -629,11 +661,11 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
                     for (int c = 0; c < kHidChunks && ok; ++c) {
                         const uint32_t w = take();
                         if (!ok) break;
-                        mma_steps(tmem + (uint32_t)(t * 256), act_a, FH, c * (kHidK / 16), w, kHidK, kHidK / 16,
-                                  idesc(FH), c > 0);
+                        mma_steps<FH, kHidK, kHidK / 16>(tmem + (uint32_t)(t * 256), act_a, c * (kHidK / 16), w,
+                                                         idesc(FH), c > 0);
                         release();
                     }
-                    if (ok) commit(&bars.accf[t][0]);
+                    if (ok) done(&bars.accf[t][0]);
                 }
             }
             // output layer: six 128-column blocks per tile alternating between the halves
@@ -644,22 +676,22 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
                 for (int j = 0; j < kOutBlocks && ok; ++j) {
                     const int h = j & 1;
                     if (j >= 2) {
-                        ok = wait_bar(&bars.acce[t][h], (uint32_t)((j >> 1) - 1) & 1u, abort);
+                        ok = warp_wait(&bars.acce[t][h], (uint32_t)((j >> 1) - 1) & 1u, abort);
                         asm volatile("tcgen05.fence::after_thread_sync;\n");
                         if (!ok) break;
                     }
                     for (int c = 0; c < kOutChunks && ok; ++c) {
                         const uint32_t w = take();
                         if (!ok) break;
-                        mma_steps(tmem + (uint32_t)(t * 256 + h * kOutN), act_a, FH, c * (kOutK / 16), w, kOutK,
-                                  kOutK / 16, idesc(kOutN), c > 0);
+                        mma_steps<FH, kOutK, kOutK / 16>(tmem + (uint32_t)(t * 256 + h * kOutN), act_a,
+                                                         c * (kOutK / 16), w, idesc(kOutN), c > 0);
                         release();
                     }
-                    if (ok) commit(&bars.accf[t][h]);
+                    if (ok) done(&bars.accf[t][h]);
                 }
             }
             // every MMA issued by this thread has completed before the memory is freed
-            commit(&bars.fin);
+            done(&bars.fin);
             wait_bar(&bars.fin, 0, nullptr);
         }
     } else {
