@@ -30,6 +30,8 @@ extern "C" {
 #define MCW_EPI_BIAS_F32 1   /* c (f32) = acc + bias (bias may be NULL) */
 #define MCW_EPI_BIAS_SILU 2  /* c2 (f32, optional) = z = acc + bias; c (bf16) = silu(z) */
 #define MCW_EPI_DSILU 3      /* g = acc * silu'(aux); c (bf16) = g; c2 (f32, optional) = g */
+#define MCW_EPI_LOSS 4       /* y = acc + bias, d = y - aux; *loss += sum w d^2 / (m n); c (bf16) and c2 (f32,
+                                optional) = 2 w d / (m n) (mcw_mlp_gemm_batch only) */
 
 /* C[m, n] = sum_k A(m, k) B(n, k) on BF16 tensor cores with FP32 accumulation.
  * A is bf16 stored [m, k] (trans_a = 0) or [k, m] (trans_a = 1), leading
@@ -75,6 +77,13 @@ int mcw_mlp_status(int32_t clear, uint32_t *flags);
 
 /* y (bf16) = x (f32), n elements. */
 int mcw_mlp_cast_bf16(const float *x, void *y, int64_t n, void *stream);
+
+/* dst (bf16, rows ld_dst apart, columns cols .. ld_dst - 1 set to zero) = src (f32, or bf16 with
+ * src_bf16 != 0; rows ld_src apart); colsum (optional, f32 src): the column sums of src over every
+ * 128 rows, colsum[(row / 128) * ld_colsum + j].  Rows of 16 bytes are what the TMA-fed products
+ * read. */
+int mcw_mlp_cast_rows(const void *src, int32_t src_bf16, int64_t rows, int32_t cols, int64_t ld_src, void *dst,
+                      int64_t ld_dst, float *colsum, int64_t ld_colsum, void *stream);
 
 /* Fused inference of the whole network MCW_MLP_IN -> 3 x MCW_MLP_HIDDEN (SiLU) -> MCW_MLP_OUT. */
 #define MCW_MLP_IN 4
@@ -150,6 +159,48 @@ typedef struct {
 } McwGemmGrouped;
 
 int mcw_mlp_gemm_grouped(const McwGemmGrouped *p, void *stream);
+
+/* Up to MCW_GEMM_BATCH_MAX such problems of one epilogue and one pair of operand layouts in one
+ * launch.  trans_a / trans_b: the operand is stored [k, m] / [k, n], lda / ldb its row pitch (the
+ * same rules; both with MCW_EPI_F32, trans_b also with MCW_EPI_DSILU).  Beside
+ * mcw_mlp_gemm_grouped:
+ *  - MCW_EPI_LOSS (weights per column or NULL, loss per group);
+ *  - colsum of MCW_EPI_DSILU / MCW_EPI_LOSS (optional): the column sums of the f32 result over
+ *    every 128 rows, colsum[g * stride_colsum + (row / 128) * ld_colsum + j];
+ *  - of MCW_EPI_F32 with colsum_in: colsum[g * stride_bias + i] = sum over q < colsum_chunks of
+ *    colsum_in[g * stride_colsum + q * ld_colsum + i], i < m (a bias gradient beside its weight
+ *    gradient). */
+#define MCW_GEMM_BATCH_MAX 4
+typedef struct {
+    int32_t m, n, k;
+    int32_t groups;
+    int32_t splits;
+    int32_t epilogue;
+    const void *a;
+    int64_t lda, stride_a;
+    const void *b;
+    int64_t ldb, stride_b;
+    const float *bias;
+    int64_t stride_bias;
+    const float *aux;
+    int64_t ldaux, stride_aux;
+    void *c;
+    int64_t ldc, stride_c, stride_split;
+    void *c2;
+    int64_t ldc2, stride_c2;
+    void *ct;
+    int64_t ldct, stride_ct;
+    float *colsum;
+    const float *colsum_in;
+    int64_t stride_colsum, ld_colsum;
+    const float *weights;
+    float *loss;
+    int32_t colsum_chunks;
+    int32_t trans_a, trans_b;
+    int32_t pad;
+} McwGemmProblem;
+
+int mcw_mlp_gemm_batch(const McwGemmProblem *p, int32_t n, void *stream);
 
 /* dst[g][i][j] = sum over s < splits of src[s * stride_split + g * stride_src + i * ld_src + j]. */
 int mcw_mlp_reduce_splits(const float *src, int64_t stride_split, int64_t stride_src, int64_t ld_src, float *dst,

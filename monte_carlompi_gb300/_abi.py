@@ -116,6 +116,15 @@ class GemmGroupedC(ctypes.Structure):
                 ('ct', ctypes.c_void_p), ('ldct', ctypes.c_int64), ('stride_ct', ctypes.c_int64)]
 
 
+class GemmProblemC(ctypes.Structure):
+    """McwGemmProblem of include/mcw_mlp.h."""
+    _fields_ = GemmGroupedC._fields_ + [
+        ('colsum', ctypes.c_void_p), ('colsum_in', ctypes.c_void_p), ('stride_colsum', ctypes.c_int64),
+        ('ld_colsum', ctypes.c_int64), ('weights', ctypes.c_void_p), ('loss', ctypes.c_void_p),
+        ('colsum_chunks', ctypes.c_int32), ('trans_a', ctypes.c_int32), ('trans_b', ctypes.c_int32),
+        ('pad', ctypes.c_int32)]
+
+
 class ColsumLayerC(ctypes.Structure):
     """McwColsumLayer of include/mcw_mlp.h."""
     _fields_ = [('g', ctypes.c_void_p), ('ld', ctypes.c_int64), ('stride', ctypes.c_int64),
@@ -128,14 +137,16 @@ class TransposeBlockC(ctypes.Structure):
                 ('rows', ctypes.c_int32), ('cols', ctypes.c_int32)]
 
 
-EPI_F32, EPI_BIAS_F32, EPI_BIAS_SILU, EPI_DSILU = 0, 1, 2, 3
+EPI_F32, EPI_BIAS_F32, EPI_BIAS_SILU, EPI_DSILU, EPI_LOSS = 0, 1, 2, 3, 4
+GEMM_BATCH_MAX = 4
 ENGINE_MMA_SYNC, ENGINE_TCGEN05 = 0, 1
 
 # entry points of include/mcw_mlp.h
 MLP_EXPORTS = ['mcw_mlp_gemm', 'mcw_mlp_colsum', 'mcw_mlp_loss', 'mcw_mlp_adam', 'mcw_mlp_cast_bf16',
                'mcw_mlp_status', 'mcw_mlp_pack', 'mcw_mlp_forward', 'mcw_mlp_forward_f16',
                'mcw_mlp_forward_ensemble_f16',
-               'mcw_mlp_gemm_grouped', 'mcw_mlp_reduce_splits', 'mcw_mlp_loss_grouped',
+               'mcw_mlp_gemm_grouped', 'mcw_mlp_gemm_batch', 'mcw_mlp_cast_rows', 'mcw_mlp_reduce_splits',
+               'mcw_mlp_loss_grouped',
                'mcw_mlp_colsum_grouped', 'mcw_mlp_adam_grouped', 'mcw_mlp_gather', 'mcw_mlp_advance']
 MLP_PACK_BYTES = 5 * 256 * 256 * 2 + 256 * 16 * 2
 MLP_BIAS_FLOATS = 3 * 256 + 649
@@ -220,6 +231,8 @@ def load(path=None):
         'mcw_mlp_forward_f16': ([vp, i32, vp, vp, vp, vp, vp, vp, i32, vp], ctypes.c_int),
         'mcw_mlp_forward_ensemble_f16': ([vp, i32, i32, vp, vp, vp, i32, vp], ctypes.c_int),
         'mcw_mlp_gemm_grouped': ([ctypes.POINTER(GemmGroupedC), vp], ctypes.c_int),
+        'mcw_mlp_gemm_batch': ([ctypes.POINTER(GemmProblemC), i32, vp], ctypes.c_int),
+        'mcw_mlp_cast_rows': ([vp, i32, i64, i32, i64, vp, i64, vp, i64, vp], ctypes.c_int),
         'mcw_mlp_reduce_splits': ([vp, i64, i64, i64, vp, i64, i64, i32, i32, i32, i32, vp], ctypes.c_int),
         'mcw_mlp_loss_grouped': ([vp, i64, i64, vp, i64, i64, vp, i32, i32, i32, vp, i64, i64, vp, i64,
                                   vp, i64, i64, vp, vp], ctypes.c_int),

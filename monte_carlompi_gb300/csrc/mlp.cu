@@ -231,8 +231,51 @@ __global__ void cast_kernel(const float *x, __nv_bfloat16 *y, int n) {
     if (i < n) y[i] = __float2bfloat16(x[i]);
 }
 
+// Rows of src as bf16 rows of ld_dst, zero past cols: a block takes 128 rows x 64 columns, a lane
+// two neighbouring columns of 16 rows, so stores are 128-byte runs; the block's column sums are
+// the lanes' running sums, combined in warp order.  Bound: HBM (6 bytes per value).
+template <bool kBf16>
+__global__ void __launch_bounds__(256) cast_rows_kernel(const void *src, long long rows, int cols, long long ld_src,
+                                                        __nv_bfloat16 *dst, long long ld_dst, float *colsum,
+                                                        long long ld_colsum) {
+    __shared__ float part[8][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c = blockIdx.y * 64 + 2 * lane;
+    const long long r0 = (long long)blockIdx.x * 128 + warp * 16;
+    float v[16][2];
+#pragma unroll
+    for (int r = 0; r < 16; ++r)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const bool in = r0 + r < rows && c + e < cols;
+            const size_t at = (size_t)(r0 + r) * ld_src + c + e;
+            if (kBf16) v[r][e] = in ? __bfloat162float(static_cast<const __nv_bfloat16 *>(src)[at]) : 0.f;
+            else v[r][e] = in ? __ldg(static_cast<const float *>(src) + at) : 0.f;
+        }
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        s0 += v[r][0];
+        s1 += v[r][1];
+        if (r0 + r < rows && c < ld_dst)         // ld_dst is even
+            *reinterpret_cast<__nv_bfloat162 *>(dst + (size_t)(r0 + r) * ld_dst + c) =
+                __floats2bfloat162_rn(v[r][0], v[r][1]);
+    }
+    if (!colsum) return;
+    part[warp][2 * lane] = s0;
+    part[warp][2 * lane + 1] = s1;
+    __syncthreads();
+    if (threadIdx.x < 64 && blockIdx.y * 64 + threadIdx.x < cols) {
+        float s = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += part[q][threadIdx.x];
+        colsum[(size_t)blockIdx.x * ld_colsum + blockIdx.y * 64 + threadIdx.x] = s;
+    }
+}
+
 }  // namespace
 
+bool gemm_by_tma(const McwGemm &p, cudaStream_t s, int *rc);
 cudaError_t launch_gemm_tc(const McwGemm &p, unsigned int *err, cudaStream_t s);
 unsigned int *tc_err_flag();
 
@@ -251,6 +294,8 @@ int mcw_mlp_gemm(const McwGemm *p, void *stream) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cudaError_t e;
     if (p->engine == MCW_ENGINE_TCGEN05) {
+        int rc;
+        if (gemm_by_tma(*p, s, &rc)) return rc;
         unsigned int *err = tc_err_flag();
         if (!err) return MCW_MLP_ERR_CUDA;
         e = launch_gemm_tc(*p, err, s);
@@ -309,6 +354,22 @@ int mcw_mlp_cast_bf16(const float *x, void *y, int64_t n, void *stream) {
     if (n == 0) return 0;
     cast_kernel<<<(int)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         x, static_cast<__nv_bfloat16 *>(y), (int)n);
+    return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
+}
+
+int mcw_mlp_cast_rows(const void *src, int32_t src_bf16, int64_t rows, int32_t cols, int64_t ld_src, void *dst,
+                      int64_t ld_dst, float *colsum, int64_t ld_colsum, void *stream) {
+    if (!src || !dst || rows < 0 || cols < 0 || ld_src < cols || ld_dst < cols || (ld_dst & 7) ||
+        (reinterpret_cast<uintptr_t>(dst) & 15) || (colsum && (src_bf16 || ld_colsum < cols)))
+        return MCW_MLP_ERR_ARG;
+    if (rows == 0 || ld_dst == 0) return 0;
+    const long long by = (ld_dst + 63) / 64, bx = (rows + 127) / 128;
+    if (bx > 0x7fffffffLL || by > 65535) return MCW_MLP_ERR_ARG;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    __nv_bfloat16 *d = static_cast<__nv_bfloat16 *>(dst);
+    const dim3 grid((unsigned)bx, (unsigned)by);
+    if (src_bf16) cast_rows_kernel<true><<<grid, 256, 0, s>>>(src, rows, cols, ld_src, d, ld_dst, nullptr, 0);
+    else cast_rows_kernel<false><<<grid, 256, 0, s>>>(src, rows, cols, ld_src, d, ld_dst, colsum, ld_colsum);
     return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
 }
 

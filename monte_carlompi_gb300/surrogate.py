@@ -157,18 +157,38 @@ def forward_ensemble(torch, x, blob, bias, members):
     return y[:, :, :DIMS[-1]]
 
 
+def _cast_rows(torch, t, colsum=None):
+    """t [m, n] (f32 or bf16) as bf16 rows of a whole number of 16 bytes, zero past n (what the
+    TMA-fed products read): [m, n rounded up to 8].  colsum: [ceil(m / 128), n] f32 for the column
+    sums of t over every 128 rows."""
+    t = t.contiguous()
+    m, n = t.shape
+    out = torch.empty((m, _align8(n)), dtype=torch.bfloat16, device=t.device)
+    rc = _abi.load().mcw_mlp_cast_rows(_ptr(t), int(t.dtype == torch.bfloat16), m, n, n, _ptr(out), out.shape[1],
+                                       _ptr(colsum), n, _stream(torch))
+    if rc:
+        raise _abi.McwError(rc, 'mcw_mlp_cast_rows failed')
+    return out
+
+
+def _rows16(torch, t):
+    """t (bf16) itself when its rows are whole 16-byte runs, else padded."""
+    return t if t.shape[1] % 8 == 0 and t.is_contiguous() and t.data_ptr() % 16 == 0 else _cast_rows(torch, t)
+
+
 def forward_cached(torch, x16, w16, biases, keep=True):
     """Forward pass on the tensor-core kernels; returns (y fp32, cache for backward).
     keep=False (inference) skips storing the FP32 pre-activations."""
     m = x16.shape[0]
-    a = x16
-    zs, acts = [], [x16]
+    a = _rows16(torch, x16)
+    zs, acts = [], [a]
     for layer in range(3):
         n, k = w16[layer].shape
+        w = _rows16(torch, w16[layer])
         z = torch.empty((m, n), dtype=torch.float32, device=x16.device) if keep else None
         nxt = torch.empty((m, n), dtype=torch.bfloat16, device=x16.device)
-        _gemm(torch, _abi.EPI_BIAS_SILU, m, n, k, a, k, w16[layer], k, nxt, n, bias=biases[layer],
-              c2=z, ldc2=n, engine=TRAIN_ENGINE)
+        _gemm(torch, _abi.EPI_BIAS_SILU, m, n, min(k, DIMS[layer]), a, a.shape[1], w, w.shape[1], nxt, n,
+              bias=biases[layer], c2=z, ldc2=n, engine=TRAIN_ENGINE)
         zs.append(z)
         acts.append(nxt)
         a = nxt
@@ -179,34 +199,54 @@ def forward_cached(torch, x16, w16, biases, keep=True):
 
 
 def backward_cached(torch, gy, w16, cache, need_dx=True):
-    """Backward pass: gradients of the weights, biases and (optionally) the input."""
+    """Backward pass: gradients of the weights, biases and (optionally) the input.  Three products
+    down the layers, whose epilogues leave the column sums of every 128 rows, then the four weight
+    gradients in one launch, which also adds up the bias gradients: the operands are read where
+    they lie, transposed by the tensor core."""
     zs, acts = cache
     m = gy.shape[0]
-    g32 = gy.contiguous().float()
-    g16 = _cast(torch, g32)
-    dws, dbs = [None] * 4, [None] * 4
-    for layer in (3, 2, 1, 0):
-        n_out, k_in = w16[layer].shape
-        a_in = acts[layer]
-        dw = torch.empty((n_out, k_in), dtype=torch.float32, device=gy.device)
-        # dW[o, i] = sum_b G[b, o] A[b, i]
-        _gemm(torch, _abi.EPI_F32, n_out, k_in, m, g16, n_out, a_in, k_in, dw, k_in, trans_a=1, trans_b=1,
-              engine=TRAIN_ENGINE)
-        dws[layer] = dw
-        dbs[layer] = _colsum(torch, g32)
-        if layer == 0:
-            if not need_dx:
-                return None, dws, dbs
-            dx = torch.empty((m, k_in), dtype=torch.float32, device=gy.device)
-            _gemm(torch, _abi.EPI_F32, m, k_in, n_out, g16, n_out, w16[layer], k_in, dx, k_in, trans_b=1,
-                  engine=TRAIN_ENGINE)
-            return dx, dws, dbs
+    dev = gy.device
+    blocks = (m + 127) // 128
+    f32 = torch.float32
+    sums = [torch.empty((blocks, w.shape[0]), dtype=f32, device=dev) for w in w16]
+    g16 = [None] * 3 + [_cast_rows(torch, gy.float(), colsum=sums[3])]
+    st = _stream(torch)
+    L = _abi.load()
+    for layer in (3, 2, 1):
         # G_prev[b, i] = (sum_o G[b, o] W[o, i]) * silu'(Z_prev[b, i])
-        g16_prev = torch.empty((m, k_in), dtype=torch.bfloat16, device=gy.device)
-        g32_prev = torch.empty((m, k_in), dtype=torch.float32, device=gy.device)
-        _gemm(torch, _abi.EPI_DSILU, m, k_in, n_out, g16, n_out, w16[layer], k_in, g16_prev, k_in,
-              trans_b=1, aux=zs[layer - 1], ldaux=k_in, c2=g32_prev, ldc2=k_in, engine=TRAIN_ENGINE)
-        g16, g32 = g16_prev, g32_prev
+        n_out, k_in = w16[layer].shape
+        g = g16[layer]
+        prev = torch.empty((m, k_in), dtype=torch.bfloat16, device=dev)
+        q = _abi.GemmProblemC(m=m, n=k_in, k=n_out, groups=1, splits=1, epilogue=_abi.EPI_DSILU, a=g.data_ptr(),
+                              lda=g.shape[1], b=w16[layer].data_ptr(), ldb=k_in, trans_b=1,
+                              aux=zs[layer - 1].data_ptr(), ldaux=k_in, c=prev.data_ptr(), ldc=k_in,
+                              colsum=sums[layer - 1].data_ptr(), ld_colsum=k_in)
+        rc = L.mcw_mlp_gemm_batch(ctypes.byref(q), 1, st)
+        if rc:
+            raise _abi.McwError(rc, 'backward product failed (layer %d)' % layer)
+        g16[layer - 1] = prev
+    dx = None
+    if need_dx:
+        n_out, k_in = w16[0].shape
+        w = _rows16(torch, w16[0])
+        dx = torch.empty((m, DIMS[0]), dtype=f32, device=dev)
+        _gemm(torch, _abi.EPI_F32, m, DIMS[0], n_out, g16[0], n_out, w, w.shape[1], dx, DIMS[0], trans_b=1,
+              engine=TRAIN_ENGINE)
+    # dW[o, i] = sum_b G[b, o] A[b, i], db[o] = sum_b G[b, o]
+    dws = [torch.empty((w.shape[0], DIMS[layer]), dtype=f32, device=dev) for layer, w in enumerate(w16)]
+    dbs = [torch.empty(w.shape[0], dtype=f32, device=dev) for w in w16]
+    calls = (_abi.GemmProblemC * 4)()
+    for layer, w in enumerate(w16):
+        n_out, k_in = dws[layer].shape
+        calls[layer] = _abi.GemmProblemC(
+            m=n_out, n=k_in, k=m, groups=1, splits=1, epilogue=_abi.EPI_F32, a=g16[layer].data_ptr(),
+            lda=g16[layer].shape[1], b=acts[layer].data_ptr(), ldb=acts[layer].shape[1], trans_a=1, trans_b=1,
+            c=dws[layer].data_ptr(), ldc=k_in, colsum=dbs[layer].data_ptr(), colsum_in=sums[layer].data_ptr(),
+            ld_colsum=n_out, colsum_chunks=blocks)
+    rc = L.mcw_mlp_gemm_batch(calls, 4, st)
+    if rc:
+        raise _abi.McwError(rc, 'weight gradients failed (m=%d)' % m)
+    return dx, dws, dbs
 
 
 def forward_tangent(torch, x16, xdot16, w16, biases):
@@ -215,17 +255,19 @@ def forward_tangent(torch, x16, xdot16, w16, biases):
     backward pass per output).  x16, xdot16 bf16 [n, 4]; returns (y, ydot) fp32 [n, 649].
     Per layer: hdot_l = (hdot_{l-1} W_l^T) * silu'(z_l), the SiLU' epilogue of the backward
     GEMMs with the pre-activations z_l of the forward pass; ydot = hdot_3 W_4^T."""
+    w16 = [_rows16(torch, w) for w in w16]
     y, (zs, _) = forward_cached(torch, x16, w16, biases, keep=True)
     m = x16.shape[0]
-    t = xdot16
+    t = _rows16(torch, xdot16)
     for layer in range(3):
         n, k = w16[layer].shape
         nxt = torch.empty((m, n), dtype=torch.bfloat16, device=x16.device)
-        _gemm(torch, _abi.EPI_DSILU, m, n, k, t, k, w16[layer], k, nxt, n, aux=zs[layer], ldaux=n)
+        _gemm(torch, _abi.EPI_DSILU, m, n, min(k, DIMS[layer]), t, t.shape[1], w16[layer], k, nxt, n, aux=zs[layer],
+              ldaux=n, engine=TRAIN_ENGINE)
         t = nxt
     n, k = w16[3].shape
     ydot = torch.empty((m, n), dtype=torch.float32, device=x16.device)
-    _gemm(torch, _abi.EPI_F32, m, n, k, t, k, w16[3], k, ydot, n)
+    _gemm(torch, _abi.EPI_F32, m, n, k, t, k, w16[3], k, ydot, n, engine=TRAIN_ENGINE)
     return y, ydot
 
 

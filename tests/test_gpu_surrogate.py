@@ -302,3 +302,21 @@ def test_forward_tangent_matches_cpu_jvp():
     rel = (ydot - ref).norm(dim=1) / ref.norm(dim=1)
     assert torch.isfinite(ydot).all()
     assert rel.median().item() < 0.02 and rel.max().item() < 0.08, (rel.median().item(), rel.max().item())
+
+
+@pytest.mark.parametrize('rows', [1, 129, 3000])
+def test_autograd_gradients_at_odd_row_counts(rows):
+    """Value, input and parameter gradients over row counts that leave remainders of the products'
+    tiles and of the 128-row sums, a broadcast upstream gradient among them."""
+    net = surrogate.SurrogateMLP(seed=3)
+    g = torch.Generator().manual_seed(rows)
+    x = torch.rand(rows, 4, generator=g) * 2 - 1
+    params = [p.detach().clone().requires_grad_(True) for p in net.params]
+    xg = x.cuda().requires_grad_(True)
+    surrogate.mlp_apply(xg, params).sum().backward()
+    cparams = [p.detach().cpu().double().requires_grad_(True) for p in net.params]
+    xc = x.double().requires_grad_(True)
+    _reference_mlp(xc, cparams).sum().backward()
+    for got, ref in [(xg.grad, xc.grad)] + [(p.grad, c.grad) for p, c in zip(params, cparams)]:
+        got, ref = got.cpu().double().flatten(), ref.flatten()
+        assert (got - ref).norm() < 3e-2 * ref.norm()

@@ -242,3 +242,99 @@ def test_ensemble_training_fits_a_smooth_map():
         pred = net.predict_std(xt, half=False)
         err = ((pred - torch.from_numpy(y[:512]).cuda()) ** 2).mean().item()
         assert err < 0.05, err
+
+
+def _problem(epi, m, n, k, a, b, c, ta, tb, groups=1, **more):
+    f = dict(m=m, n=n, k=k, groups=groups, splits=1, epilogue=epi, trans_a=ta, trans_b=tb, a=a.data_ptr(),
+             lda=a.shape[-1], stride_a=a.shape[-2] * a.shape[-1], b=b.data_ptr(), ldb=b.shape[-1],
+             stride_b=b.shape[-2] * b.shape[-1], c=c.data_ptr(), ldc=c.shape[-1],
+             stride_c=c.shape[-2] * c.shape[-1])
+    f.update(more)
+    return _abi.GemmProblemC(**f)
+
+
+@pytest.mark.parametrize('ta,tb', [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize('m,n,k', [(1, 1, 1), (129, 33, 63), (128, 64, 65), (40000, 65, 17), (255, 4, 1000)])
+def test_gemm_batch_layouts_match_float64(ta, tb, m, n, k):
+    """Operands stored along either dimension, remainders of every tile, two groups, and two
+    problems of different sizes in one launch."""
+    g = torch.Generator().manual_seed(m + 7 * n + 11 * k + ta + 2 * tb)
+    r8 = lambda v: (v + 7) // 8 * 8  # noqa: E731
+    calls = (_abi.GemmProblemC * 2)()
+    keep = []
+    for i, (mm, nn, kk) in enumerate(((m, n, k), (n, m if m < 3000 else 9, k + 5))):
+        a = torch.randn((2, kk, r8(mm)) if ta else (2, mm, r8(kk)), generator=g).to(torch.bfloat16).cuda()
+        b = (torch.randn((2, kk, r8(nn)) if tb else (2, nn, r8(kk)), generator=g) * 0.1).to(torch.bfloat16).cuda()
+        c = torch.full((2, mm + 1, nn + 1), 7.0, device='cuda')        # a row and a column that stay
+        calls[i] = _problem(_abi.EPI_F32, mm, nn, kk, a, b, c, ta, tb, groups=2)
+        keep.append((a, b, c, mm, nn, kk))
+    _status_clear()
+    assert _abi.load().mcw_mlp_gemm_batch(calls, 2, _stream()) == 0
+    torch.cuda.synchronize()
+    _status_ok()
+    for a, b, c, mm, nn, kk in keep:
+        A = (a[:, :, :mm].transpose(1, 2) if ta else a[:, :, :kk]).cpu().double()
+        B = (b[:, :, :nn] if tb else b[:, :, :kk].transpose(1, 2)).cpu().double()
+        ref = A @ B
+        err = (c[:, :mm, :nn].cpu().double() - ref).abs().max().item()
+        assert err <= 1e-4 * max(1.0, ref.abs().max().item()) + 1e-5 * math.sqrt(kk), err
+        assert (c[:, mm] == 7).all() and (c[:, :, nn] == 7).all()
+
+
+@pytest.mark.parametrize('m,n', [(1, 649), (130, 40), (700, 256)])
+def test_gemm_batch_loss_and_column_sums(m, n):
+    """The loss epilogue, the column sums of SiLU' and loss results over every 128 rows, their
+    total beside a plain product, and rows cast to padded bf16 with their column sums."""
+    G, k = 2, 256
+    g = torch.Generator().manual_seed(m + n)
+    a = torch.randn(G, m, k, generator=g).to(torch.bfloat16).cuda()
+    b = (torch.randn(G, n, k, generator=g) * 0.1).to(torch.bfloat16).cuda()
+    aux = torch.randn(G, m, n, generator=g).cuda()
+    bias, w = torch.randn(G, n, generator=g).cuda(), torch.rand(n, generator=g).cuda()
+    blocks = (m + 127) // 128
+    acc = a.cpu().double() @ b.cpu().double().transpose(1, 2)
+    for epi in (_abi.EPI_LOSS, _abi.EPI_DSILU):
+        out16 = torch.zeros(G, m, n, dtype=torch.bfloat16, device='cuda')
+        out32 = torch.zeros(G, m, n, device='cuda')
+        sums = torch.zeros(G, blocks, n, device='cuda')
+        loss = torch.zeros(G, device='cuda')
+        q = _problem(epi, m, n, k, a, b, out16, 0, 0, groups=G, aux=aux.data_ptr(), ldaux=n, stride_aux=m * n,
+                     bias=bias.data_ptr(), stride_bias=n, c2=out32.data_ptr(), ldc2=n, stride_c2=m * n,
+                     colsum=sums.data_ptr(), ld_colsum=n, stride_colsum=blocks * n, weights=w.data_ptr(),
+                     loss=loss.data_ptr())
+        assert _abi.load().mcw_mlp_gemm_batch(ctypes.byref(q), 1, _stream()) == 0
+        torch.cuda.synchronize()
+        x = aux.cpu().double()
+        if epi == _abi.EPI_LOSS:
+            d = acc + bias.cpu().double()[:, None] - x
+            ref = 2 * w.cpu().double() * d / (m * n)
+            lref = (w.cpu().double() * d * d).sum((1, 2)) / (m * n)
+            assert ((loss.cpu().double() - lref).abs() < 1e-5 * lref).all()
+        else:
+            s = torch.sigmoid(x)
+            ref = acc * s * (1 + x * (1 - s))
+        assert (out32.cpu().double() - ref).abs().max() < 1e-4 * ref.abs().max()
+        assert torch.equal(out16, out32.to(torch.bfloat16))
+        for q0 in range(blocks):
+            part = out32[:, 128 * q0:128 * q0 + 128].double().sum(1)
+            assert (sums[:, q0].double() - part).abs().max() < 1e-5 * part.abs().max() + 1e-12
+    # the total of the last sums beside the product it is the bias gradient of
+    gt = torch.zeros(G, m, (n + 7) // 8 * 8, dtype=torch.bfloat16, device='cuda')
+    gt[:, :, :n] = out16
+    dw, db = torch.zeros(G, n, k, device='cuda'), torch.zeros(G, n, device='cuda')
+    q = _problem(_abi.EPI_F32, n, k, m, gt, a, dw, 1, 1, groups=G, colsum=db.data_ptr(), stride_bias=n,
+                 colsum_in=sums.data_ptr(), ld_colsum=n, stride_colsum=blocks * n, colsum_chunks=blocks)
+    assert _abi.load().mcw_mlp_gemm_batch(ctypes.byref(q), 1, _stream()) == 0
+    torch.cuda.synchronize()
+    assert (db.double() - out32.double().sum(1)).abs().max() < 1e-5 * out32.double().sum(1).abs().max() + 1e-12
+    ref = out16.cpu().double().transpose(1, 2) @ a.cpu().double()
+    assert (dw.cpu().double() - ref).abs().max() < 1e-4 * ref.abs().max()
+    # padded rows
+    src = out32[0].contiguous()
+    dst = torch.full((m, (n + 7) // 8 * 8), 5.0, dtype=torch.bfloat16, device='cuda')
+    cs = torch.zeros(blocks, n, device='cuda')
+    rc = _abi.load().mcw_mlp_cast_rows(src.data_ptr(), 0, m, n, n, dst.data_ptr(), dst.shape[1], cs.data_ptr(), n,
+                                       _stream())
+    torch.cuda.synchronize()
+    assert rc == 0 and torch.equal(dst[:, :n], src.to(torch.bfloat16)) and (dst[:, n:] == 0).all()
+    assert (cs.double().sum(0) - src.double().sum(0)).abs().max() < 1e-5 * src.double().sum(0).abs().max() + 1e-12
