@@ -904,12 +904,14 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
         ra.ice = (const DevTable *)ctx->ice_tables.p;
         Counters *cn = (Counters *)ctx->counters.p;
         ra.status = &cn->status;
+        ra.work = &cn->work;
+        ra.slots = ra.claim = 0;
         ra.records = dev_records;
         ra.tallies = (mcw_tally *)ctx->tallies.p;
         ra.budget_ns = (unsigned long long)(ctx->budget_s * 1e9);
         ra.seed = seed;
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, st));
-        CUDA_TRY(ctx, launch_walk_replay(ra, st));
+        CUDA_TRY(ctx, launch_walk_replay(ra, ctx->sm_count, st));
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev1, st));
         shape.block = 128;
         shape.grid = (int)((plan.total + 127) / 128);

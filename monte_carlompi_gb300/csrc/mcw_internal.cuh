@@ -168,6 +168,8 @@ struct ReplayArgs {
     mcw_tally *tallies;
     unsigned long long budget_ns;
     uint64_t seed;
+    unsigned long long *work;    // HG walk: next unclaimed photon
+    int32_t slots, claim;        // HG walk: photons a block walks and starts at once (set by the launcher)
 };
 
 struct LutArgs {
@@ -217,7 +219,7 @@ constexpr int kDrainSlot = 6;
 // Launches the walk and, when a.drain_from > 0, the drain kernel after it
 // (sm_count SMs; a.drain must then hold grid * block slots).
 cudaError_t launch_walk_f32(const WalkArgs &a, bool impurity, int grid, int block, int sm_count, cudaStream_t s);
-cudaError_t launch_walk_replay(const ReplayArgs &a, cudaStream_t s);
+cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s);
 // The FP32 polarised walk (a.phase set, a.records holding mcw_record32p).
 cudaError_t launch_walk_pol32(const WalkArgs &a, int sm_count, cudaStream_t s);
 int walk_f32_max_blocks_per_sm(int block, int n_cfg, bool impurity);

@@ -1,14 +1,34 @@
-// FP64 replay walk: one thread per photon, the reference's arithmetic order,
-// uniforms from the photon-indexed Philox replay stream.  Compiled with
-// --fmad=false so every product and sum is rounded on its own, as NumPy does.
+// FP64 replay walk: the reference's arithmetic order, uniforms from the photon-indexed
+// Philox replay stream.  Compiled with --fmad=false so every product and sum is rounded on
+// its own, as NumPy does.
 //
-// Restates MonteCarlo.monte_carlo3D (monte_carloMPI/monte_carlo3D.py:1111-1490,
-// HG branch) with the draws of populate_pdfs (:905-1025) and initial_pdfs
-// (:1027-1044), and the wavelength draw of MonteCarlo.run (:1515-1520).  The
-// kernel instance kPol restates the polarised branch of aspherical grains: the
-// rejection sampler of populate_pdfs (:922-1004) and the Stokes-vector update
-// of monte_carlo3D (:1282-1342).
+// Restates MonteCarlo.monte_carlo3D (monte_carloMPI/monte_carlo3D.py:1111-1490) with the draws
+// of populate_pdfs (:905-1025) and initial_pdfs (:1027-1044), and the wavelength draw of
+// MonteCarlo.run (:1515-1520): walk_replay_kernel the HG branch, walk_replay_pol_kernel the
+// polarised branch of aspherical grains, one thread per photon (the rejection sampler of
+// populate_pdfs, :922-1004, and the Stokes-vector update of monte_carlo3D, :1282-1342).
+//
+// What bounds the HG walk: an FP64 instruction takes a warp 64 cycles of its sub-core's FP64
+// pipe, however many of its lanes are active and whether or not it waits for the one before.  A
+// walk of one thread's own took about 170 of them per event, 5.6 us, and the longest walk of
+// 10,000 photons has 25,000 events.  So the work is laid out across lanes and warps:
+//  * a block of two warps holds up to eight photons.  The producer warp draws the steps ahead,
+//    32 at a time (all of one photon's, or four each of eight): angles, optical path, path
+//    increment, absorption; none of them depends on where the photon is;
+//  * the consumer warp walks the chain that remains with four lanes a photon: Z carries mu_z
+//    (which depends on mu_z alone) one step ahead of X, Y (mu_x, mu_y) and M (depth, path, end
+//    conditions), and each of the eleven FP64 instructions of a step serves all four;
+//  * sqrt(1 - mu_z^2) and its reciprocal come from one Newton step and a residual correction
+//    (Markstein, IBM J. Res. Dev. 34, 1990), six operations, and the two divisions by it take
+//    three each.
+// The producer assumes that a step does nothing but scatter; a photon that ends, is reflected or
+// is replaced sits out the round that was drawn for it.  Every value is the one-thread walk's, in
+// its order of operations: sqrt and quotients are correctly rounded but where the exact value
+// lies within 2^-28 ulp of a rounding boundary (none in @@ROUND@@).
+// 10,000 photons of the driver's default run: 141 ms on one thread each, @@REPLAY@@ ms.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "mcw_internal.cuh"
 #include "ssp_device.cuh"
@@ -53,6 +73,52 @@ __device__ double replay_wavelength(const DevConfig &c, uint64_t seed, uint64_t 
     double z = sqrt(-2.0 * log(u0)) * cos(kTwoPi * u1);
     double x = c.wvl0 + c.scale * z;
     return rint(x * 100.0) / 100.0;
+}
+
+// Record and tallies of a photon that ended with `condition` (0: stopped early) after i steps.
+template <bool kPol>
+__device__ void finish_photon(const ReplayArgs &a, int64_t gid, int ci, int condition, int64_t i, double wvl_um,
+                              double mux_0, double muy_0, double muz_0, double path_length, double snow_depth,
+                              const double *st) {
+    mcw_record64p r;
+    r.condition = condition;
+    r.n_scat = (int32_t)(i - 1);                                      // :1487
+    r.wvn = 1. / wvl_um;                                              // :1468
+    r.theta_n = acos(muz_0);                                          // :1469
+    r.flags = 0;
+    if (i == 1) r.phi_n = 0.;                                         // :1472-1485
+    else if (mux_0 > 0 && muy_0 > 0) r.phi_n = atan(muy_0 / mux_0);
+    else if (mux_0 < 0 && muy_0 > 0) r.phi_n = atan(muy_0 / mux_0) + kPi;
+    else if (mux_0 < 0 && muy_0 < 0) r.phi_n = atan(muy_0 / mux_0) + kPi;
+    else if (mux_0 > 0 && muy_0 < 0) r.phi_n = atan(muy_0 / mux_0) + kTwoPi;
+    else { r.phi_n = __longlong_as_double(0x7ff8000000000000LL); r.flags = 1u; }
+    r.path_length = path_length;
+    r.snow_depth = snow_depth;
+    r.config = (uint32_t)ci;
+    if (a.records) {
+        if (kPol) {
+            r.stokes_q = st[1];
+            r.stokes_u = st[2];
+            r.stokes_v = st[3];
+            static_cast<mcw_record64p *>(a.records)[gid] = r;
+        } else {
+            mcw_record64 &d = static_cast<mcw_record64 *>(a.records)[gid];
+            d.condition = r.condition;
+            d.n_scat = r.n_scat;
+            d.wvn = r.wvn;
+            d.theta_n = r.theta_n;
+            d.phi_n = r.phi_n;
+            d.path_length = r.path_length;
+            d.snow_depth = r.snow_depth;
+            d.config = r.config;
+            d.flags = r.flags;
+        }
+    }
+    if (a.tallies && condition > 0) {
+        const unsigned long long wfx = (unsigned long long)llrint(r.wvn * 4294967296.0);
+        float th = (float)r.theta_n, ph = (r.flags ? 0.f : (float)r.phi_n);
+        tally_global(a.tallies + ci, condition, r.n_scat, wfx, th, ph);
+    }
 }
 
 // scipy interp1d (linear) on an ascending grid: searchsorted (left) clipped to
@@ -134,15 +200,7 @@ __device__ bool polarised_angles(const DevPhase &ph, int row, const double st[4]
     return true;
 }
 
-// Henyey_Greenstein2 (monte_carlo3D.py:790-800).
-__device__ __forceinline__ double hg2(double g, double r) {
-    if (g == 0) return 1 - 2 * r;
-    double q = (1 - g * g) / (1 - g + 2 * g * r);
-    return (1. / (2. * g)) * (1 + g * g - q * q);
-}
-
-template <bool kPol>
-__global__ void __launch_bounds__(128) walk_replay_kernel(const ReplayArgs a) {
+__global__ void __launch_bounds__(128) walk_replay_pol_kernel(const ReplayArgs a) {
     const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= a.total) return;
     const int ci = find_config(a.prefix, a.n_cfg, gid);
@@ -161,11 +219,8 @@ __global__ void __launch_bounds__(128) walk_replay_kernel(const ReplayArgs a) {
     double ext_rand = s.next();
     double p_rand = 0, phi_rand = 0;
     double st[4] = {1, 0, 0, 0};                                      // :1132
-    DevPhase ph{};
-    if (kPol) {
-        ph = a.phase[c.ice_table];
-        for (int k = 0; k < 4; ++k) st[k] = c.stokes0[k];
-    }
+    const DevPhase ph = a.phase[c.ice_table];
+    for (int k = 0; k < 4; ++k) st[k] = c.stokes0[k];
 
     double mux_0 = c.mux0_d, muy_0 = 0, muz_0 = c.muz0_d;             // :1121-1124
     double muz2_0 = muz_0 * muz_0;
@@ -180,14 +235,9 @@ __global__ void __launch_bounds__(128) walk_replay_kernel(const ReplayArgs a) {
     while (condition == 0) {                                          // :1212
         i += 1;
         if (i > 1) {                                                  // :1215-1224
-            if (kPol) {
-                if (!polarised_angles(ph, o.row, st, s, p_rand, phi_rand, t0, a.budget_ns)) {
-                    atomicOr(a.status, s.overrun ? kStatusStream : kStatusBudget);
-                    break;
-                }
-            } else {
-                p_rand = hg2(o.g, s.next());
-                phi_rand = s.next() * kTwoPi;
+            if (!polarised_angles(ph, o.row, st, s, p_rand, phi_rand, t0, a.budget_ns)) {
+                atomicOr(a.status, s.overrun ? kStatusStream : kStatusBudget);
+                break;
             }
             tau_rand = -log(s.next());
             ssa_rand = s.next();
@@ -236,7 +286,7 @@ __global__ void __launch_bounds__(128) walk_replay_kernel(const ReplayArgs a) {
             if (bottom_reflection) {                                  // :1283-1285
                 st[0] = 1; st[1] = 0; st[2] = 0; st[3] = 0;
                 bottom_reflection = false;
-            } else if (kPol) {                                        // :1287-1342
+            } else {                                                  // :1287-1342
                 const double cos2theta = costheta * costheta;
                 const double phi_sca = acos(cosphi);
                 double sp[4], sc[4], sm[4];
@@ -307,56 +357,496 @@ __global__ void __launch_bounds__(128) walk_replay_kernel(const ReplayArgs a) {
         }
     }
 
-    mcw_record64p r;
-    r.condition = condition;
-    r.n_scat = (int32_t)(i - 1);                                      // :1487
-    r.wvn = 1. / o.wvl_um;                                            // :1468
-    r.theta_n = acos(muz_0);                                          // :1469
-    r.flags = 0;
-    if (i == 1) r.phi_n = 0.;                                         // :1472-1485
-    else if (mux_0 > 0 && muy_0 > 0) r.phi_n = atan(muy_0 / mux_0);
-    else if (mux_0 < 0 && muy_0 > 0) r.phi_n = atan(muy_0 / mux_0) + kPi;
-    else if (mux_0 < 0 && muy_0 < 0) r.phi_n = atan(muy_0 / mux_0) + kPi;
-    else if (mux_0 > 0 && muy_0 < 0) r.phi_n = atan(muy_0 / mux_0) + kTwoPi;
-    else { r.phi_n = __longlong_as_double(0x7ff8000000000000LL); r.flags = 1u; }
-    r.path_length = path_length;
-    r.snow_depth = o.snow_depth;
-    r.config = (uint32_t)ci;
-    r.stokes_q = st[1];
-    r.stokes_u = st[2];
-    r.stokes_v = st[3];
-    if (a.records) {
-        if (kPol) {
-            static_cast<mcw_record64p *>(a.records)[gid] = r;
-        } else {
-            mcw_record64 &d = static_cast<mcw_record64 *>(a.records)[gid];
-            d.condition = r.condition;
-            d.n_scat = r.n_scat;
-            d.wvn = r.wvn;
-            d.theta_n = r.theta_n;
-            d.phi_n = r.phi_n;
-            d.path_length = r.path_length;
-            d.snow_depth = r.snow_depth;
-            d.config = r.config;
-            d.flags = r.flags;
+    finish_photon<true>(a, gid, ci, condition, i, o.wvl_um, mux_0, muy_0, muz_0, path_length, o.snow_depth, st);
+}
+
+// ---------------------------------------------------------------- the HG walk
+
+constexpr int kSlots = 8;                    // photons a block walks at once
+constexpr uint32_t kRefl = 1u, kSurface = 2u, kBottom = 4u, kIso = 8u, kActive = 16u;
+
+// A photon in flight (shared memory).
+struct Slot {
+    double mux, muy, muz, z, path;
+    double hg_b, hg_c, hg_d, hg_e, hg_a;     // 1-g^2, 1-g, 2g, 1/(2g), 1+g^2
+    double ext, rext;                        // ext_cff * rho_snw and its reciprocal
+    double ssa_ice, ssa_imp, p_imp, tau, R;
+    double wvl_um, depth;
+    uint64_t rid, k;                         // stream id, next uniform
+    int64_t gid;
+    int64_t i;                               // steps walked
+    int32_t ci;
+    uint32_t flags;
+    __device__ __forceinline__ bool lambertian() const { return (flags & (kRefl | kSurface)) != 0; }
+};
+
+// A finished photon waiting for its record.
+struct Finished {
+    double mux, muy, muz, path, wvl_um, depth;
+    int64_t gid, i;
+    int32_t ci, cond;
+};
+
+// 32 steps drawn ahead, S of each of n photons: entry rank * S + t is step t of photon `rank`.
+struct Ahead {
+    double ct[32], st[32], cp[32], sp[32], dtau[32], inc[32];
+    uint32_t fl[32];                         // 1 absorbed here, 2 by ice
+    int32_t n, S;
+    int32_t slot[kSlots], steps[kSlots], lamb[kSlots], shift[kSlots];
+    uint64_t rid[kSlots], k0[kSlots], k1[kSlots];   // photon, its stream before and after the steps
+    // whether rank r's entries are those of its slot's photon as it stands
+    __device__ __forceinline__ bool holds(int r, const Slot *slots) const {
+        if (r >= n) return false;
+        const Slot &s = slots[slot[r]];
+        return (s.flags & kActive) && s.rid == rid[r] && s.k == k0[r] && (int)s.lambertian() == lamb[r];
+    }
+};
+
+struct ReplayBlock {
+    Ahead ahead[2];
+    Slot slots[kSlots], born[32];
+    Finished fin[32];
+    double lamb_ct[kSlots];
+    int32_t stop;
+};
+
+__device__ __forceinline__ double from_bits(uint64_t b) { return __longlong_as_double((long long)b); }
+__device__ __forceinline__ uint64_t to_bits(double x) { return (uint64_t)__double_as_longlong(x); }
+
+// u01_f64 by its bits: 1.m - (1 - 2^-53), exact, one FP64 operation.
+__device__ __forceinline__ double u01_bits(uint64_t w) {
+    return from_bits(0x3ff0000000000000ull | (w >> 12)) - 0x1.fffffffffffffp-1;
+}
+
+__device__ __forceinline__ uint4 stream_block(uint64_t seed, uint64_t rid, uint64_t block) {
+    return philox10_seed(make_uint4((uint32_t)block, kTagWalk, (uint32_t)rid, (uint32_t)(rid >> 32)), seed);
+}
+
+__device__ __forceinline__ uint64_t word(const uint4 x, bool second) {
+    return second ? (((uint64_t)x.w << 32) | x.z) : (((uint64_t)x.y << 32) | x.x);
+}
+
+// Uniform k of a photon's stream.
+__device__ __forceinline__ double uniform_at(uint64_t seed, uint64_t rid, uint64_t k) {
+    return u01_bits(word(stream_block(seed, rid, k >> 1), k & 1));
+}
+
+// x > 0 and x < -t (t >= 0) by their bits, false for NaN: no FP64 operation.
+__device__ __forceinline__ bool is_pos(double x) {
+    const uint64_t b = to_bits(x);
+    return b > 0 && b <= 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ bool below_minus(double x, double t) {
+    const uint64_t b = to_bits(x), m = b & 0x7fffffffffffffffull;
+    return (b >> 63) && m > to_bits(t) && m <= 0x7ff0000000000000ull;
+}
+__device__ __forceinline__ bool is_unit(double x) { return (to_bits(x) & 0x7fffffffffffffffull) == 0x3ff0000000000000ull; }
+
+// A power-of-two factor by the exponent (normal, finite x).
+__device__ __forceinline__ double halved(double x) { return __hiloint2double(__double2hiint(x) - 0x00100000, __double2loint(x)); }
+__device__ __forceinline__ double doubled(double x) { return __hiloint2double(__double2hiint(x) + 0x00100000, __double2loint(x)); }
+
+__device__ __forceinline__ double rsqrt_seed(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+
+// sqrt(x), x normal and in (0, 1]: a Newton step from the hardware's approximation, then the
+// residual's correction.
+__device__ __forceinline__ double sqrt_res(double x) {
+    const double y = rsqrt_seed(x), h = halved(y);
+    const double g = x * y;
+    const double r = fma(-g, h, 0.5);
+    const double g1 = fma(g, r, g), h1 = fma(h, r, h);
+    return fma(fma(-g1, g1, x), h1, g1);
+}
+
+// a / b, b normal: a Newton step on the hardware's reciprocal, then the residual's correction.
+__device__ __forceinline__ double div_res(double a, double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(fma(-b, y, 1.0), y, y);
+    const double q = a * y;
+    return fma(fma(-q, b, a), y, q);
+}
+
+__device__ __forceinline__ double shfl_d(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
+
+// sqrt(1 - ct^2) as the reference writes it (ct = +-1: 0; past it, by rounding: NaN).
+__device__ __forceinline__ double sin_from(double ct) {
+    const double x = 1 - ct * ct;
+    const uint64_t b = to_bits(x);
+    return b == 0 || (b >> 63) ? sqrt(x) : sqrt_res(x);
+}
+
+// The end of a step (:1390-1466) at depth z (z_prev before it): the path's exit correction, the
+// bottom's reflectance draw (uniform *k, taken when drawn), the end condition (0: walking on, or
+// reflected, kRefl set in *flags).
+__device__ int step_end(const Slot &s, uint64_t seed, double &z, double z_prev, double dtau, double muz, double &path,
+                        bool first, bool absorbed, bool ice, uint64_t *k, uint32_t *flags) {
+    if (z > 0) {                                                      // :1390-1397
+        path += -((z * dtau) / ((z - z_prev) * s.ext));
+        return 1;
+    }
+    if (z < -s.tau) {                                                 // :1399-1459
+        path += -(((z + s.tau) * dtau) / ((z - z_prev) * s.ext));
+        const double corr = -(((z + s.tau) / (z_prev - z)) * dtau);
+        z = z - (muz * corr);
+        if (s.flags & kBottom) {
+            const double u = uniform_at(seed, s.rid, *k);
+            *k += 1;
+            if (u <= s.R) {
+                *flags |= kRefl;
+                return 0;
+            }
+        }
+        return first ? 3 : 2;
+    }
+    return absorbed ? (ice ? 4 : 5) : 0;                              // :1461-1466
+}
+
+// Photon gid at its birth and after its first step (:1215-1237: the direction is the beam's), into
+// a slot; returns its end condition.
+__device__ int replay_birth(const ReplayArgs &a, int64_t gid, Slot &out) {
+    const int ci = find_config(a.prefix, a.n_cfg, gid);
+    const DevConfig &c = a.cfgs[ci];
+    Slot s;
+    s.gid = gid;
+    s.ci = ci;
+    s.rid = c.rng_base + (uint64_t)(gid - c.offset);
+    const double wvl = replay_wavelength(c, a.seed, s.rid);
+    const Optics o = photon_optics(c, a.ice[c.ice_table], a.imp, wvl);
+    const double g = o.g;
+    s.flags = kActive | ((c.flags & kFlagLamSurface) ? kSurface : 0u) | ((c.flags & kFlagLamBottom) ? kBottom : 0u) |
+              (g == 0 ? kIso : 0u);
+    s.hg_b = 1 - g * g;
+    s.hg_c = 1 - g;
+    s.hg_d = 2 * g;
+    s.hg_e = 1. / (2. * g);
+    s.hg_a = 1 + g * g;
+    s.ext = o.ext_cff_mss * c.rho_snw;                                // :1355-1356
+    s.rext = 1.0 / s.ext;
+    s.tau = c.tau_tot_d;
+    s.R = c.R_d;
+    s.ssa_ice = (s.flags & kSurface) ? s.R : o.ssa_ice;               // :1385-1387
+    s.ssa_imp = (s.flags & kSurface) ? s.R : o.ssa_imp;
+    s.p_imp = o.p_imp;
+    s.wvl_um = o.wvl_um;
+    s.depth = o.snow_depth;
+    s.mux = c.mux0_d;                                                 // :1121-1124
+    s.muy = 0;
+    s.muz = c.muz0_d;
+    s.i = 1;
+    s.k = 3;
+    const double dtau = (s.flags & kSurface) ? 0 : -log(uniform_at(a.seed, s.rid, 0));   // :1035-1038, :1227-1229
+    const double ssa_rand = uniform_at(a.seed, s.rid, 1);
+    const bool ice = uniform_at(a.seed, s.rid, 2) > s.p_imp;          // :1375-1383
+    s.path = 0 + dtau / s.ext;                                        // :1372
+    s.z = 0 + dtau * s.muz;                                           // :1352
+    const int cond = step_end(s, a.seed, s.z, 0, dtau, s.muz, s.path, true, ssa_rand >= (ice ? s.ssa_ice : s.ssa_imp),
+                              ice, &s.k, &s.flags);
+    out = s;
+    return cond;
+}
+
+// The producer's round: the next steps of the block's photons into `next`, assuming that those of
+// `now` (being walked) end in nothing.  Arrives at barrier 2 once it has read the slots.
+__device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, const Ahead &now, Ahead &next, int lane) {
+    const unsigned act = __ballot_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive));
+    const int n = __popc(act);
+    const int S = n <= 1 ? 32 : 1 << (5 - (32 - __clz(n - 1)));       // 32 / n, a power of two
+    const int rank = lane / S, t = lane % S;
+    const bool mine = rank < n;
+    const int si = mine ? __fns(act, 0, rank + 1) : 0;
+    Slot s = B.slots[si];
+    bool lamb = s.lambertian();
+    for (int r = 0; r < now.n; ++r)
+        if (now.slot[r] == si && now.holds(r, B.slots)) {
+            s.k = now.k1[r];
+            lamb = (s.flags & kSurface) != 0;
+        }
+    __syncwarp();
+    asm volatile("bar.arrive 2, 64;\n" ::: "memory");
+    // a Lambertian direction first (:1238-1250): its photon's lanes test pairs of uniforms past the
+    // step's five, and the first that passes is taken
+    int shift = 0;
+    double ct_l = 1.0;
+    bool look = mine && lamb;
+    const unsigned group = S == 32 ? 0xffffffffu : ((1u << S) - 1u) << (rank * S);
+    for (int round = 0; __any_sync(0xffffffffu, look); ++round) {
+        bool pass = false;
+        double c = 1.0;
+        const int j = round * S + t;
+        if (look) {
+            const double theta = 0 + (kPi / 2 - 0) * uniform_at(a.seed, s.rid, s.k + 5 + 2 * (uint64_t)j);
+            const double r1 = uniform_at(a.seed, s.rid, s.k + 6 + 2 * (uint64_t)j);
+            double sn;
+            sincos(theta, &sn, &c);
+            pass = r1 < 2 * sn * c;
+            if (round >= 4096) pass = true;                           // no stream needs as many
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, pass) & group;
+        const int src = hit ? __ffs(hit) - 1 : lane;
+        const double cs = shfl_d(c, src);
+        if (look && hit) {
+            ct_l = cs;
+            shift = 2 * (round * S + (src - rank * S) + 1);
+            look = false;
         }
     }
-
-    if (a.tallies && condition > 0) {
-        const unsigned long long wfx = (unsigned long long)llrint(r.wvn * 4294967296.0);
-        float th = (float)r.theta_n, ph = (r.flags ? 0.f : (float)r.phi_n);
-        tally_global(a.tallies + ci, condition, r.n_scat, wfx, th, ph);
+    if (mine) {
+        const int steps = (s.flags & kSurface) ? 1 : S;               // on a surface every step's stream shifts
+        const uint64_t k = s.k + 5 * (uint64_t)t + (t > 0 ? shift : 0);
+        const uint4 x0 = stream_block(a.seed, s.rid, k >> 1), x1 = stream_block(a.seed, s.rid, (k >> 1) + 1),
+                    x2 = stream_block(a.seed, s.rid, (k >> 1) + 2);
+        const bool odd = k & 1;
+        const double u0 = u01_bits(word(x0, odd)), u1 = u01_bits(odd ? word(x1, false) : word(x0, true)),
+                     u2 = u01_bits(word(x1, odd)), u3 = u01_bits(odd ? word(x2, false) : word(x1, true)),
+                     u4 = u01_bits(word(x2, odd));
+        double ct;
+        if (t == 0 && lamb) {
+            ct = ct_l;
+        } else if (s.flags & kIso) {                                  // Henyey_Greenstein2 (:790-800)
+            ct = 1 - 2 * u0;
+        } else {
+            const double q = div_res(s.hg_b, s.hg_c + s.hg_d * u0);
+            ct = s.hg_e * (s.hg_a - q * q);
+        }
+        double sp, cp;
+        sincos(u1 * kTwoPi, &sp, &cp);
+        const double dtau = -log(u2);
+        const double q0 = dtau * s.rext;                              // dtau / ext (:1372)
+        const bool ice = u4 > s.p_imp;                                // :1375-1383
+        next.ct[lane] = ct;
+        next.st[lane] = sin_from(ct);
+        next.cp[lane] = cp;
+        next.sp[lane] = sp;
+        next.dtau[lane] = dtau;
+        next.inc[lane] = fma(fma(-q0, s.ext, dtau), s.rext, q0);
+        next.fl[lane] = (u3 >= (ice ? s.ssa_ice : s.ssa_imp) ? 1u : 0u) | (ice ? 2u : 0u);
+        if (t == 0) {
+            next.slot[rank] = si;
+            next.steps[rank] = steps;
+            next.lamb[rank] = lamb ? 1 : 0;
+            next.shift[rank] = shift;
+            next.rid[rank] = s.rid;
+            next.k0[rank] = s.k;
+            next.k1[rank] = s.k + 5 * (uint64_t)steps + shift;
+            if (next.k1[rank] > (1ull << 33)) atomicOr(a.status, kStatusStream);
+        }
     }
+    if (lane == 0) {
+        next.n = n;
+        next.S = S;
+    }
+}
+
+// The consumer's chain over the steps in `now` (see the top of the file).  Four lanes a photon: 0 Z,
+// 1 X, 2 Y, 3 M.  Returns, on an M lane, the photon's end condition.  The slots are written only
+// after barrier 2 (the producer has read them).
+__device__ int walk_ahead(const ReplayArgs &a, ReplayBlock &B, const Ahead &now, int lane) {
+    const int role = lane & 3, r = lane >> 2;
+    const bool isZ = role == 0, isM = role == 3, isX = role == 1;
+    const bool held = now.holds(r, B.slots);
+    const int si = held ? now.slot[r] : 0, S = now.S;
+    const int base = held ? r * S : 0, steps = held ? now.steps[r] : 0;
+    Slot &slot = B.slots[si];
+    const double tau = slot.tau;
+    double mz = slot.muz, va = isX ? slot.mux : slot.muy, vb = isX ? slot.muy : slot.mux;
+    double z = slot.z, path = slot.path, zp = z, dt = 0, mzn = mz;
+    if (held && now.lamb[r]) { mz = 1.0; va = 0.0; vb = 0.0; }
+    double mzb = mz, sq = 1.0, h2 = 1.0;             // before the lagging step; sqrt(1 - mzb^2), 1 / that
+    bool alive = held;
+    int done = 0;                                    // M: steps walked
+    bool event = false;
+    for (int it = 0; __any_sync(0xffffffffu, alive); ++it) {
+        const bool zs = alive && it < steps, ls = alive && it > 0;
+        const int lag = base + (it > 0 ? it - 1 : 0), cur = base + (it < S ? it : S - 1);
+        const int e = isZ ? cur : lag;
+        const double st = now.st[e], ct = isM ? now.ct[cur] : now.ct[e], cp = now.cp[e];
+        const double sp = isX ? -now.sp[e] : now.sp[e], dtau = now.dtau[e], inc = now.inc[e];
+        // 1: mz mz | a mzb | mz ct (Z's)
+        const double r1 = (isZ || isM ? mz : va) * (isZ ? mz : (isM ? ct : mzb));
+        const double u_z = shfl_d(r1, lane | 3);
+        // 2: 1 - . | . cp | dtau mz
+        const double r2 = fma(isM ? dtau : r1, isZ ? -1.0 : (isM ? mz : cp), isZ ? 1.0 : -0.0);
+        const double y0 = rsqrt_seed(isZ ? r2 : 1.0), h = halved(y0);
+        // 3: x y0 | b sp | z + .
+        const double r3 = fma(isZ ? r2 : (isM ? z : vb), isZ ? y0 : (isM ? 1.0 : sp), isM ? r2 : -0.0);
+        // 4: 1/2 - g h | sum | path + inc
+        const double r4 = fma(isZ ? r3 : (isM ? path : r2), isZ ? -h : 1.0, isZ ? 0.5 : (isM ? inc : r3));
+        // 5: g1 | st .
+        const double r5 = fma(isZ ? r3 : st, r4, isZ ? r3 : -0.0);
+        // 6: h1 | . / sq, approximate
+        const double r6 = fma(isZ ? h : r5, isZ ? r4 : h2, isZ ? h : -0.0);
+        // 7: residuals
+        const double r7 = fma(-(isZ ? r5 : r6), isZ ? r5 : sq, isZ ? r2 : r5);
+        // 8: sqrt | quotient
+        const double r8 = fma(r7, isZ ? r6 : h2, isZ ? r5 : r6);
+        // 9: -sq st | a ct
+        const double r9 = (isZ ? r8 : va) * (isZ ? -st : ct);
+        // 10: . cp | the new mu_x, mu_y
+        const double r10 = fma(isZ ? r9 : r8, isZ ? cp : 1.0, isZ ? -0.0 : r9);
+        // 11: the new mu_z
+        double nz = r10 + u_z, nxy = r10;
+        // about the vertical (:1262-1269): mu_z = +-1, or a Lambertian direction
+        const bool pole = isZ ? zs && is_unit(mz) : ls && is_unit(mzb);
+        if (__any_sync(0xffffffffu, pole)) {
+            const double p = st * (isX ? cp : sp);
+            if (pole) {
+                nz = mz > 0 ? ct : -ct;
+                nxy = isX || mzb > 0 ? p : -p;
+            }
+        }
+        // M: the step before's end conditions (:1390-1466)
+        const bool end = isM && ls && (is_pos(r3) || below_minus(r3, tau) || (now.fl[e] & 1u));
+        const bool stop = (__ballot_sync(0xffffffffu, end) >> (lane | 3)) & 1u;
+        if (ls) {
+            va = nxy;
+            zp = z;
+            z = r3;
+            path = r4;
+            dt = dtau;
+            mzn = mz;
+            done = it;
+            event = end;
+        }
+        const double other = shfl_d(va, lane ^ 3);
+        if (!isZ && !isM) vb = other;
+        const double nmz = shfl_d(nz, lane & ~3), nsq = shfl_d(r8, lane & ~3), nh = shfl_d(r6, lane & ~3);
+        alive = alive && !stop && it < steps;
+        if (alive) {                                 // Z has walked step `it`
+            mzb = mz;
+            mz = nmz;
+            sq = nsq;
+            h2 = doubled(nh);
+        }
+    }
+    __syncwarp();
+    asm volatile("bar.sync 2, 64;\n" ::: "memory");
+    int cond = 0;
+    if (held) {
+        if (isZ) slot.muz = mz;
+        else if (!isM) *(isX ? &slot.mux : &slot.muy) = va;
+        else {
+            uint32_t flags = slot.flags & ~kRefl;
+            uint64_t k = now.k0[r] + 5 * (uint64_t)done + now.shift[r];
+            slot.i += done;
+            if (event) {
+                const uint32_t f = now.fl[base + done - 1];
+                cond = step_end(slot, a.seed, z, zp, dt, mzn, path, false, f & 1u, f & 2u, &k, &flags);
+            }
+            slot.z = z;
+            slot.path = path;
+            slot.k = k;
+            slot.flags = flags;
+        }
+    }
+    __syncwarp();
+    return cond;
+}
+
+__global__ void __launch_bounds__(64) walk_replay_kernel(const ReplayArgs a) {
+    __shared__ ReplayBlock B;
+    const int lane = threadIdx.x & 31;
+    const bool producer = threadIdx.x >= 32;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    if (threadIdx.x < kSlots) B.slots[threadIdx.x].flags = 0;
+    if (threadIdx.x == 0) {
+        B.ahead[0].n = 0;
+        B.ahead[0].S = 32;
+        B.stop = 0;
+    }
+    bool exhausted = false;
+    int n_born = 0, n_fin = 0;
+    const unsigned long long t0 = global_ns();
+    auto flush = [&]() {                             // the queued records, one per lane
+        if (lane < n_fin) {
+            const Finished &f = B.fin[lane];
+            finish_photon<false>(a, f.gid, f.ci, f.cond, f.i, f.wvl_um, f.mux, f.muy, f.muz, f.path, f.depth, nullptr);
+        }
+        n_fin = 0;
+        __syncwarp();
+    };
+    auto queue = [&](bool ended, const Slot &s, int cond) {
+        const unsigned m = __ballot_sync(0xffffffffu, ended);
+        if (ended) B.fin[n_fin + __popc(m & lt_mask)] =
+            Finished{s.mux, s.muy, s.muz, s.path, s.wvl_um, s.depth, s.gid, s.i, s.ci, cond};
+        n_fin += __popc(m);
+        __syncwarp();
+    };
+    for (uint32_t round = 0;; ++round) {
+        __syncthreads();
+        if (B.stop) break;
+        const Ahead &now = B.ahead[round & 1];
+        if (producer) {
+            draw_ahead(a, B, now, B.ahead[(round & 1) ^ 1], lane);
+            continue;
+        }
+        const int cond = walk_ahead(a, B, now, lane);
+        // ---- finished photons leave their slots
+        if (__any_sync(0xffffffffu, cond != 0)) {
+            Slot &s = B.slots[cond ? now.slot[lane >> 2] : 0];
+            queue(cond != 0, s, cond);
+            if (cond) s.flags = 0;
+            __syncwarp();
+            if (n_fin > 32 - kSlots) flush();
+        }
+        // ---- free slots take photons already born; 32 at most are born at once
+        unsigned idle = ~__ballot_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive)) &
+                        ((1u << a.slots) - 1u);
+        for (int tries = 0; tries < 4 && idle && n_born == 0 && !exhausted; ++tries) {
+            if (n_fin > 0) flush();
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(a.work, (unsigned long long)a.claim);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            const int64_t left = a.total - (int64_t)base;
+            const int valid = (int)max((int64_t)0, min((int64_t)a.claim, left));
+            exhausted = left <= a.claim;
+            int c1 = 0;
+            Slot s;
+            if (lane < valid) c1 = replay_birth(a, (int64_t)base + lane, s);
+            queue(lane < valid && c1 != 0, s, c1);
+            const unsigned m = __ballot_sync(0xffffffffu, lane < valid && c1 == 0);
+            if (lane < valid && c1 == 0) B.born[__popc(m & lt_mask)] = s;
+            n_born = __popc(m);
+            __syncwarp();
+            if (n_fin > 32 - kSlots) flush();
+        }
+        const int take = min(__popc(idle), n_born);
+        if (lane < take) B.slots[__fns(idle, 0, lane + 1)] = B.born[n_born - 1 - lane];
+        n_born -= take;
+        __syncwarp();
+        const bool any = __any_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive));
+        int stop = !any && exhausted && n_born == 0;
+        if ((round & 63u) == 63u && lane == 0) {     // time budget (watchdog)
+            if (global_ns() - t0 > a.budget_ns) atomicOr(a.status, kStatusBudget);
+            if (*(volatile unsigned int *)a.status) stop = 1;
+        }
+        if (lane == 0 && stop) B.stop = 1;
+    }
+    if (!producer && n_fin > 0) flush();
 }
 
 }  // namespace
 
-cudaError_t launch_walk_replay(const ReplayArgs &a, cudaStream_t s) {
+cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s) {
     if (a.total <= 0) return cudaSuccess;
-    const int block = 128;
-    const int64_t grid = (a.total + block - 1) / block;
-    if (a.pol) walk_replay_kernel<true><<<(unsigned)grid, block, 0, s>>>(a);
-    else walk_replay_kernel<false><<<(unsigned)grid, block, 0, s>>>(a);
+    if (a.pol) {
+        const int block = 128;
+        const int64_t grid = (a.total + block - 1) / block;
+        walk_replay_pol_kernel<<<(unsigned)grid, block, 0, s>>>(a);
+        return cudaGetLastError();
+    }
+    // four blocks (eight warps) an SM keep its four FP64 pipes busy; few photons are spread over
+    // all of them
+    ReplayArgs b = a;
+    const int64_t blocks = std::min<int64_t>(4 * (int64_t)std::max(1, sm_count), a.total);
+    const int64_t each = (a.total + blocks - 1) / blocks;
+    b.slots = (int32_t)std::min<int64_t>(kSlots, each);
+    b.claim = (int32_t)std::min<int64_t>(32, each);
+    walk_replay_kernel<<<(unsigned)blocks, 64, 0, s>>>(b);
     return cudaGetLastError();
 }
 
