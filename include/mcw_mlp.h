@@ -169,7 +169,8 @@ int mcw_mlp_gemm_grouped(const McwGemmGrouped *p, void *stream);
  *    every 128 rows, colsum[g * stride_colsum + (row / 128) * ld_colsum + j];
  *  - of MCW_EPI_F32 with colsum_in: colsum[g * stride_bias + i] = sum over q < colsum_chunks of
  *    colsum_in[g * stride_colsum + q * ld_colsum + i], i < m (a bias gradient beside its weight
- *    gradient). */
+ *    gradient); with colsum_rows > 0, colsum_in is the f32 matrix [k, m] itself (rows ld_colsum
+ *    apart), summed as mcw_mlp_colsum_grouped sums it in chunks of colsum_rows rows. */
 #define MCW_GEMM_BATCH_MAX 4
 typedef struct {
     int32_t m, n, k;
@@ -197,7 +198,7 @@ typedef struct {
     float *loss;
     int32_t colsum_chunks;
     int32_t trans_a, trans_b;
-    int32_t pad;
+    int32_t colsum_rows;
 } McwGemmProblem;
 
 int mcw_mlp_gemm_batch(const McwGemmProblem *p, int32_t n, void *stream);
@@ -255,6 +256,11 @@ int mcw_mlp_gather(const void *x_all, const float *t_all, int64_t ldt_all, int32
                    int64_t n_rows, const int32_t *counter_dev, int32_t batch, int32_t groups, void *x,
                    int64_t stride_x, void *xt, int64_t stride_xt, float *t, int64_t ldt, int64_t stride_t,
                    void *stream);
+
+/* The same batch at the beginning of a step (x and t only), with loss[g] = 0 (loss may be NULL). */
+int mcw_mlp_step_begin(const void *x_all, const float *t_all, int64_t ldt_all, int32_t n_out, const int32_t *perm,
+                       int64_t n_rows, const int32_t *counter_dev, int32_t batch, int32_t groups, void *x,
+                       int64_t stride_x, float *t, int64_t ldt, int64_t stride_t, float *loss, void *stream);
 
 /* *counter_dev += 1 and *step_dev += 1 (the end of a captured step). */
 int mcw_mlp_advance(int32_t *counter_dev, int32_t *step_dev, void *stream);

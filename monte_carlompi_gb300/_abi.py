@@ -122,7 +122,7 @@ class GemmProblemC(ctypes.Structure):
         ('colsum', ctypes.c_void_p), ('colsum_in', ctypes.c_void_p), ('stride_colsum', ctypes.c_int64),
         ('ld_colsum', ctypes.c_int64), ('weights', ctypes.c_void_p), ('loss', ctypes.c_void_p),
         ('colsum_chunks', ctypes.c_int32), ('trans_a', ctypes.c_int32), ('trans_b', ctypes.c_int32),
-        ('pad', ctypes.c_int32)]
+        ('colsum_rows', ctypes.c_int32)]
 
 
 class ColsumLayerC(ctypes.Structure):
@@ -147,7 +147,8 @@ MLP_EXPORTS = ['mcw_mlp_gemm', 'mcw_mlp_colsum', 'mcw_mlp_loss', 'mcw_mlp_adam',
                'mcw_mlp_forward_ensemble_f16',
                'mcw_mlp_gemm_grouped', 'mcw_mlp_gemm_batch', 'mcw_mlp_cast_rows', 'mcw_mlp_reduce_splits',
                'mcw_mlp_loss_grouped',
-               'mcw_mlp_colsum_grouped', 'mcw_mlp_adam_grouped', 'mcw_mlp_gather', 'mcw_mlp_advance']
+               'mcw_mlp_colsum_grouped', 'mcw_mlp_adam_grouped', 'mcw_mlp_gather', 'mcw_mlp_step_begin',
+               'mcw_mlp_advance']
 MLP_PACK_BYTES = 5 * 256 * 256 * 2 + 256 * 16 * 2
 MLP_BIAS_FLOATS = 3 * 256 + 649
 
@@ -243,6 +244,8 @@ def load(path=None):
                                  ctypes.c_int),
         'mcw_mlp_gather': ([vp, vp, i64, i32, vp, i64, vp, i32, i32, vp, i64, vp, i64, vp, i64, i64, vp],
                            ctypes.c_int),
+        'mcw_mlp_step_begin': ([vp, vp, i64, i32, vp, i64, vp, i32, i32, vp, i64, vp, i64, i64, vp, vp],
+                               ctypes.c_int),
         'mcw_mlp_advance': ([vp, vp, vp], ctypes.c_int),
     }
     for name, (args, res) in sig.items():

@@ -53,11 +53,11 @@ constexpr unsigned long long kWaitNs = 2000000000ull;
 
 __host__ __device__ constexpr int stage_bytes(int tn) { return kABytes + tn * TK * 2; }
 
-// One problem of a launch; CTAs [cta0, cta0 + tiles) are its.
+// One problem of a launch; CTAs [cta0, cta0 + tiles) are its, and from sum0 those of its column sums.
 struct GemmProb {
     CUtensorMap ta, tb;
     int32_t m, n, k, nt, mt;
-    int32_t splits, kps, cta0;      // K per split (a multiple of TK)
+    int32_t splits, kps, cta0, sum0; // K per split (a multiple of TK)
     const float *bias;
     long long s_bias;
     const float *aux;               // DSILU: pre-activations; LOSS: targets
@@ -69,9 +69,9 @@ struct GemmProb {
     __nv_bfloat16 *ct;
     long long ldct, s_ct;
     float *colsum;                  // SILU'/LOSS: column sums of every 128 rows; F32: their total, out
-    const float *colsum_in;         // F32: the column sums of the A operand's rows
-    long long s_colsum, ld_colsum;  // per group; per 128 rows
-    int32_t colsum_chunks, pad;
+    const float *colsum_in;         // F32: the column sums of the A operand's rows, or the f32 rows themselves
+    long long s_colsum, ld_colsum;  // per group; per 128 rows (per row)
+    int32_t colsum_chunks, colsum_rows;
     const float *weights;           // LOSS: per column
     float *loss;                    // LOSS: per group
 };
@@ -79,7 +79,7 @@ struct GemmProb {
 struct GemmBatch {
     GemmProb p[MCW_GEMM_BATCH_MAX];
     unsigned int *err;
-    int32_t np, stages;
+    int32_t np, stages, sums0;      // sums0: the first CTA of column sums
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -222,11 +222,41 @@ __device__ __forceinline__ void load_aux(const GemmProb &p, int g, int rbase, in
     for (int r = 0; r < 32; ++r) av[r] = (col_ok && rbase + r < p.m) ? __ldg(src + (size_t)(rbase + r) * p.ld_aux) : 0.f;
 }
 
+// Bias gradients beside weight gradients, 16 columns a CTA behind the tiles' CTAs: the sums of the
+// f32 rows colsum_in [k, m] over chunks of colsum_rows rows, rows q, q + 8, ... of a chunk added in
+// order for each q < 8 (a thread each), the eight sums in order, the chunks' sums in order
+// (mcw_mlp_colsum_grouped's order).  (In the tiles' own epilogue warps, a whole 128 columns fell to
+// one CTA of the first layer: 32 us for a launch of 8.)
+constexpr int kSumCols = 16;
+__device__ __forceinline__ void column_sums(const GemmProb &p, int cta, int tid, float *part) {
+    const int tiles = (p.m + kSumCols - 1) / kSumCols;
+    const int g = cta / tiles, c = tid % kSumCols, q0 = tid / kSumCols;
+    const int col = cta % tiles * kSumCols + c;
+    const float *src = p.colsum_in + (size_t)g * p.s_colsum + col;
+    float total = 0.f;
+    for (int r0 = 0; r0 < p.k; r0 += p.colsum_rows) {
+        const int r1 = min(p.k, r0 + p.colsum_rows);
+        float s = 0.f;
+        if (col < p.m) {
+#pragma unroll 16
+            for (int r = r0 + q0; r < r1; r += 8) s += __ldg(src + (size_t)r * p.ld_colsum);
+        }
+        part[tid] = s;
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += part[q * kSumCols + c];
+        total = r0 == 0 ? t : total + t;
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+    }
+    if (q0 == 0 && col < p.m) p.colsum[(size_t)g * p.s_bias + col] = total;
+}
+
 template <int kEpi, bool kAMn, bool kBMn, int TN>
 __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant__ GemmBatch batch) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_bar;
-    __shared__ float part[4][32];
+    __shared__ float part[4 * 32];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     constexpr uint32_t kTmemCols = TN < 32 ? 32 : TN;
@@ -237,6 +267,11 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int stages = batch.stages;
     int pi = 0;
+    if (kEpi == MCW_EPI_F32 && (int)blockIdx.x >= batch.sums0) {
+        while (pi + 1 < batch.np && (int)blockIdx.x >= batch.p[pi + 1].sum0) ++pi;
+        if (threadIdx.x < 128) column_sums(batch.p[pi], (int)blockIdx.x - batch.p[pi].sum0, (int)threadIdx.x, part);
+        return;
+    }
     while (pi + 1 < batch.np && (int)blockIdx.x >= batch.p[pi + 1].cta0) ++pi;
     const GemmProb &p = batch.p[pi];
     int t = (int)blockIdx.x - p.cta0;
@@ -330,15 +365,12 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
         uint32_t verdict;
         float av[32];
         if (kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) load_aux(p, g, rbase, n0 + lane, n0 + lane < p.n, av);
-        // F32 with column sums: the total of the chunks' sums of A's rows (bias gradient), in order
-        if (kEpi == MCW_EPI_F32 && p.colsum_in && n0 == 0 && sp == 0) {
-            const int o = rbase + lane;
-            if (o < p.m) {
-                const float *src = p.colsum_in + (size_t)g * p.s_colsum + o;
-                float s = 0.f;
-                for (int q = 0; q < p.colsum_chunks; ++q) s += src[(size_t)q * p.ld_colsum];
-                p.colsum[(size_t)g * p.s_bias + o] = s;
-            }
+        // the total of the 128-row sums of A's rows, in order
+        if (kEpi == MCW_EPI_F32 && p.colsum_in && p.colsum_rows == 0 && sp == 0 && n0 == 0 && rbase + lane < p.m) {
+            const float *src = p.colsum_in + (size_t)g * p.s_colsum + rbase + lane;
+            float s = 0.f;
+            for (int q = 0; q < p.colsum_chunks; ++q) s += src[(size_t)q * p.ld_colsum];
+            p.colsum[(size_t)g * p.s_bias + rbase + lane] = s;
         }
         // one verdict for the four warps: they meet at barriers below
         bool ok = wait_bar(&acc_bar, 0u, abort) && !*abort;
@@ -407,11 +439,11 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
                 // the next block's other input while this one's sums are put together
                 if (c0 + 32 < TN) load_aux(p, g, rbase, col + 32, col + 32 < p.n, av);
                 if (p.colsum) {
-                    part[warp][lane] = csum;
+                    part[warp * 32 + lane] = csum;
                     asm volatile("bar.sync 1, 128;\n" ::: "memory");
                     if (warp == 0 && col_ok)
                         p.colsum[(size_t)g * p.s_colsum + (size_t)mtile * p.ld_colsum + col] =
-                            ((part[0][lane] + part[1][lane]) + part[2][lane]) + part[3][lane];
+                            ((part[lane] + part[32 + lane]) + part[64 + lane]) + part[96 + lane];
                     asm volatile("bar.sync 1, 128;\n" ::: "memory");
                 }
             }
@@ -494,7 +526,7 @@ cudaError_t launch(const GemmBatch &b, unsigned grid, size_t smem, cudaStream_t 
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
         attr = cudaFuncSetAttribute(gemm_kernel<kEpi, kAMn, kBMn, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    227 * 1024 - 2048);
+                                    200 * 1024);
     });
     if (attr != cudaSuccess) return attr;
     gemm_kernel<kEpi, kAMn, kBMn, TN><<<grid, kThreads, smem, s>>>(b);
@@ -581,8 +613,14 @@ int launch_batch(const McwGemmProblem *q, int np, cudaStream_t stream) {
         d.c2 = static_cast<float *>(s.c2), d.ldc2 = s.ldc2, d.s_c2 = s.stride_c2;
         d.ct = static_cast<__nv_bfloat16 *>(s.ct), d.ldct = s.ldct, d.s_ct = s.stride_ct;
         d.colsum = s.colsum, d.colsum_in = s.colsum_in, d.s_colsum = s.stride_colsum, d.ld_colsum = s.ld_colsum;
-        d.colsum_chunks = s.colsum_chunks;
+        d.colsum_chunks = s.colsum_chunks, d.colsum_rows = s.colsum_rows;
         d.weights = s.weights, d.loss = s.loss;
+    }
+    b.sums0 = cta > 0x7fffffffLL ? 0 : (int32_t)cta;
+    for (int i = 0; i < np; ++i) {
+        b.p[i].sum0 = (int32_t)cta;
+        if (q[i].epilogue == MCW_EPI_F32 && q[i].colsum_in && q[i].colsum_rows > 0)
+            cta += (long long)((q[i].m + kSumCols - 1) / kSumCols) * q[i].groups;
     }
     if (cta > 0x7fffffffLL) return MCW_MLP_ERR_ARG;
     const size_t ring = (size_t)stages * stage_bytes(tn), tiles = 4 * kTileBytes;
@@ -640,7 +678,8 @@ int mcw_mlp_gemm_batch(const McwGemmProblem *q, int32_t n, void *stream) {
         if (s.epilogue == MCW_EPI_BIAS_SILU && !s.bias) return MCW_MLP_ERR_ARG;
         if ((s.epilogue == MCW_EPI_DSILU || s.epilogue == MCW_EPI_LOSS) && !s.aux) return MCW_MLP_ERR_ARG;
         if (s.epilogue == MCW_EPI_LOSS && (!s.loss || !s.bias)) return MCW_MLP_ERR_ARG;
-        if (s.epilogue == MCW_EPI_F32 && s.colsum_in && (!s.colsum || s.colsum_chunks < 0)) return MCW_MLP_ERR_ARG;
+        if (s.epilogue == MCW_EPI_F32 && s.colsum_in && (!s.colsum || s.colsum_chunks < 0 || s.colsum_rows < 0))
+            return MCW_MLP_ERR_ARG;
         if ((long long)s.groups * s.splits > 65535) return MCW_MLP_ERR_ARG;
         const int chunks = (s.k + TK - 1) / TK;
         const int per = (chunks + s.splits - 1) / s.splits;

@@ -182,15 +182,100 @@ __global__ void adam_grouped_kernel(float *w, const float *gr, float *mo, float 
     }
 }
 
+// The same by tiles, for layouts on 16-byte boundaries (adam_tiled): a block takes 32 rows x 64
+// columns of a transposed block, or 2,048 consecutive parameters outside them, eight a thread in
+// 16-byte loads and stores; the transposed copy goes through shared memory and leaves in runs of
+// 64 bytes (2-byte stores a column apart before).  Bound: 30 bytes a parameter, from L2; five
+// members 23 us one parameter a thread, @@ADAM@@ us now.
+struct AdamTiles {
+    TransposeTable tt;
+    int first[5];              // first tile of block q; first[n_blocks]: the rest
+    long long seg[6][2];       // the rest: [begin, end) between the blocks
+    int seg0[6], n_seg;        // first tile of segment s (after the blocks')
+    int tiles;
+};
+
+__device__ __forceinline__ void adam8(float *w, const float *gr, float *mo, float *ve, __nv_bfloat16 *w16, size_t e,
+                                      float lr, float c1, float c2, float b1, float b2, float eps, uint32_t (&h)[4]) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        float4 wv = reinterpret_cast<float4 *>(w + e)[q], mv = reinterpret_cast<float4 *>(mo + e)[q],
+               vv = reinterpret_cast<float4 *>(ve + e)[q];
+        const float4 gv = reinterpret_cast<const float4 *>(gr + e)[q];
+        float *wp = &wv.x, *mp = &mv.x, *vp = &vv.x;
+        const float *gp = &gv.x;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float gi = gp[k];
+            const float m = b1 * mp[k] + (1.f - b1) * gi;
+            const float v = b2 * vp[k] + (1.f - b2) * gi * gi;
+            mp[k] = m;
+            vp[k] = v;
+            wp[k] = wp[k] - lr * (m / c1) / (sqrtf(v / c2) + eps);
+        }
+        reinterpret_cast<float4 *>(w + e)[q] = wv;
+        reinterpret_cast<float4 *>(mo + e)[q] = mv;
+        reinterpret_cast<float4 *>(ve + e)[q] = vv;
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(wv.x, wv.y), hi = __floats2bfloat162_rn(wv.z, wv.w);
+        h[2 * q] = *reinterpret_cast<const uint32_t *>(&lo);
+        h[2 * q + 1] = *reinterpret_cast<const uint32_t *>(&hi);
+    }
+    *reinterpret_cast<uint4 *>(w16 + e) = make_uint4(h[0], h[1], h[2], h[3]);
+}
+
+__global__ void __launch_bounds__(256) adam_tiled_kernel(float *w, const float *gr, float *mo, float *ve,
+                                                         __nv_bfloat16 *w16, long long n, const float *lr_dev,
+                                                         const int *step_dev, float b1, float b2, float eps,
+                                                         __nv_bfloat16 *wt, long long s_t, const AdamTiles at) {
+    __shared__ __align__(16) __nv_bfloat16 tile[64][40];     // [column][row], rows of 80 bytes
+    __shared__ float corr[2];
+    const int g = blockIdx.y, t = blockIdx.x;
+    if (threadIdx.x == 0) {
+        const int step = *step_dev;
+        corr[0] = 1.f - powf(b1, (float)step);
+        corr[1] = 1.f - powf(b2, (float)step);
+    }
+    __syncthreads();
+    const float lr = *lr_dev, c1 = corr[0], c2 = corr[1];
+    const int nb = at.tt.n_blocks;
+    uint32_t h[4];
+    if (t >= at.first[nb]) {
+        int s = 0;
+        while (s + 1 < at.n_seg && t >= at.seg0[s + 1]) ++s;
+        const long long i = at.seg[s][0] + (long long)(t - at.seg0[s]) * 2048 + threadIdx.x * 8;
+        if (i < at.seg[s][1]) adam8(w, gr, mo, ve, w16, (size_t)g * n + i, lr, c1, c2, b1, b2, eps, h);
+        return;
+    }
+    int q = 0;
+    while (q + 1 < nb && t >= at.first[q + 1]) ++q;
+    const TransposeBlock &B = at.tt.b[q];
+    const int across = (B.cols + 63) / 64;
+    const int o0 = (t - at.first[q]) / across * 32, c0 = (t - at.first[q]) % across * 64;
+    const int row = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8;
+    h[0] = h[1] = h[2] = h[3] = 0u;
+    if (o0 + row < B.rows && c0 + c8 < B.cols)
+        adam8(w, gr, mo, ve, w16, (size_t)g * n + B.off + (size_t)(o0 + row) * B.cols + c0 + c8, lr, c1, c2, b1, b2, eps, h);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        tile[c8 + k][row] = __ushort_as_bfloat16((unsigned short)(h[k >> 1] >> ((k & 1) * 16)));
+    __syncthreads();
+    const int col = threadIdx.x >> 2, o8 = (threadIdx.x & 3) * 8;
+    // rows past the block's are the copy's zero padding
+    if (c0 + col < B.cols && o0 + o8 < B.ld_t)
+        *reinterpret_cast<uint4 *>(wt + (size_t)g * s_t + B.off_t + (size_t)(c0 + col) * B.ld_t + o0 + o8) =
+            *reinterpret_cast<const uint4 *>(&tile[col][o8]);
+}
+
 // Batch of the step: rows perm[g][b * batch + i] of the encoded inputs (bf16, row
 // pitch 16, as x [batch, 16] and transposed [16, batch]) and of the targets, b the
 // step's batch counter (device memory).
 __global__ void gather_kernel(const __nv_bfloat16 *x_all, const float *t_all, long long ldt_all, int n_out,
                               const int *perm, long long n_rows, const int *counter, int batch,
                               __nv_bfloat16 *x, long long s_x, __nv_bfloat16 *xt, long long s_xt, float *t,
-                              long long ldt, long long s_t) {
+                              long long ldt, long long s_t, float *loss) {
     const int g = blockIdx.y;
     const int i = blockIdx.x;             // row of the batch
+    if (loss && i == 0 && threadIdx.x == 0) loss[g] = 0.f;
     const long long idx = (long long)(*counter) * batch + i;
     if (idx >= n_rows) return;            // more steps than the epoch's batches: nothing to gather
     const long long src = perm[(size_t)g * n_rows + (size_t)idx];
@@ -199,7 +284,7 @@ __global__ void gather_kernel(const __nv_bfloat16 *x_all, const float *t_all, lo
     if (threadIdx.x < 16) {
         const __nv_bfloat16 v = x_all[(size_t)src * 16 + threadIdx.x];
         x[(size_t)g * s_x + (size_t)i * 16 + threadIdx.x] = v;
-        xt[(size_t)g * s_xt + (size_t)threadIdx.x * batch + i] = v;
+        if (xt) xt[(size_t)g * s_xt + (size_t)threadIdx.x * batch + i] = v;
     }
 }
 
@@ -208,6 +293,45 @@ __global__ void advance_kernel(int *counter, int *step) {
         *counter += 1;
         *step += 1;
     }
+}
+
+// The tiles of a layout whose blocks lie in ascending order on 16-byte boundaries; false otherwise.
+// wt is written up to ld_t only where the block's padding ends within its last eight rows.
+bool make_adam_tiles(const TransposeTable &tt, long long n, long long s_t, AdamTiles *out) {
+    AdamTiles a;
+    memset(&a, 0, sizeof(a));
+    a.tt = tt;
+    long long at = 0;
+    int tiles = 0;
+    for (int q = 0; q < tt.n_blocks; ++q) {
+        const TransposeBlock &b = tt.b[q];
+        if ((b.off & 7) || (b.off_t & 7) || (b.ld_t & 7) || (b.cols & 7) || b.off < at || b.ld_t != (b.rows + 7) / 8 * 8)
+            return false;
+        a.first[q] = tiles;
+        tiles += (b.rows + 31) / 32 * ((b.cols + 63) / 64);
+        at = b.off + (long long)b.rows * b.cols;
+        at = (at + 7) / 8 * 8;
+    }
+    if ((n & 7) || (s_t & 7)) return false;
+    a.first[tt.n_blocks] = tiles;
+    at = 0;
+    for (int q = 0; q <= tt.n_blocks; ++q) {
+        const long long end = q < tt.n_blocks ? tt.b[q].off : n;
+        if (end > at) {
+            a.seg[a.n_seg][0] = at;
+            a.seg[a.n_seg][1] = end;
+            a.seg0[a.n_seg++] = tiles;
+            tiles += (int)((end - at + 2047) / 2048);
+        }
+        if (q < tt.n_blocks) {
+            // a block that does not end on a boundary would share eight parameters with what follows
+            if (((long long)tt.b[q].rows * tt.b[q].cols) & 7) return false;
+            at = tt.b[q].off + (long long)tt.b[q].rows * tt.b[q].cols;
+        }
+    }
+    a.tiles = tiles;
+    *out = a;
+    return true;
 }
 
 }  // namespace
@@ -294,6 +418,14 @@ int mcw_mlp_adam_grouped(float *w, const float *g, float *m, float *v, void *w16
         tt.b[q].cols = blocks[q].cols;
     }
     tt.n_blocks = n_blocks;
+    AdamTiles at;
+    const uintptr_t align = (uintptr_t)w | (uintptr_t)g | (uintptr_t)m | (uintptr_t)v | (uintptr_t)w16 | (uintptr_t)wt;
+    if (!(align & 15) && make_adam_tiles(tt, n, stride_t, &at)) {
+        adam_tiled_kernel<<<dim3((unsigned)at.tiles, groups), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            w, g, m, v, static_cast<__nv_bfloat16 *>(w16), n, lr_dev, step_dev, beta1, beta2, eps,
+            static_cast<__nv_bfloat16 *>(wt), stride_t, at);
+        return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
+    }
     const dim3 grid((unsigned)((n + 255) / 256), groups);
     adam_grouped_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         w, g, m, v, static_cast<__nv_bfloat16 *>(w16), n, lr_dev, step_dev, beta1, beta2, eps,
@@ -310,7 +442,19 @@ int mcw_mlp_gather(const void *x_all, const float *t_all, int64_t ldt_all, int32
         return MCW_MLP_ERR_ARG;
     gather_kernel<<<dim3(batch, groups), 128, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16 *>(x_all), t_all, ldt_all, n_out, perm, n_rows, counter_dev, batch,
-        static_cast<__nv_bfloat16 *>(x), stride_x, static_cast<__nv_bfloat16 *>(xt), stride_xt, t, ldt, stride_t);
+        static_cast<__nv_bfloat16 *>(x), stride_x, static_cast<__nv_bfloat16 *>(xt), stride_xt, t, ldt, stride_t, nullptr);
+    return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
+}
+
+int mcw_mlp_step_begin(const void *x_all, const float *t_all, int64_t ldt_all, int32_t n_out, const int32_t *perm,
+                       int64_t n_rows, const int32_t *counter_dev, int32_t batch, int32_t groups, void *x,
+                       int64_t stride_x, float *t, int64_t ldt, int64_t stride_t, float *loss, void *stream) {
+    if (!x_all || !t_all || !perm || !counter_dev || !x || !t || batch < 1 || groups < 1 || n_out < 0 ||
+        n_rows < batch)
+        return MCW_MLP_ERR_ARG;
+    gather_kernel<<<dim3(batch, groups), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16 *>(x_all), t_all, ldt_all, n_out, perm, n_rows, counter_dev, batch,
+        static_cast<__nv_bfloat16 *>(x), stride_x, nullptr, 0, t, ldt, stride_t, loss);
     return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
 }
 

@@ -392,8 +392,8 @@ def flat_layout():
     Returns (lay, P, tlay, T): lay['W%d'] = (offset, rows, cols) of W_l [out, in]
     (layer 1's inputs padded to IN_PAD columns, held at zero), lay['b%d'] = (offset, n);
     P elements per member; tlay['W%d'] = (offset, ld) of the transposed bf16 copy
-    W_l^T [in, ld] (ld = out rounded up to 8) of W2, W3, W4, the B operands of the
-    backward products; T elements per member.  Every block starts on 8 elements."""
+    W_l^T [in, ld] (ld = out rounded up to 8) of W2, W3, W4 that Adam keeps beside the
+    weights; T elements per member.  Every block starts on 8 elements."""
     lay, off = {}, 0
     for layer, (fan_in, fan_out) in enumerate(zip(DIMS[:-1], DIMS[1:])):
         k = IN_PAD if layer == 0 else fan_in
@@ -421,13 +421,14 @@ def _dw_splits(rows):
 
 class EnsembleTrainer:
     """Adam steps of every member of an ensemble at once on the training engine
-    (include/mcw_mlp.h): per step one gather of the members' batches, the four forward
-    products (bias + SiLU epilogues keeping pre-activations and transposed
-    activations), the loss, the weight- and input-gradient products, the bias
-    gradients, Adam over the flat parameters and the step counter, each one launch for
-    all members.  Parameters live in flat [members, P] vectors (flat_layout).  The step
-    is captured in a CUDA graph on first use and replayed; learning rate, step count and
-    batch counter are device scalars, so the graph never changes."""
+    (include/mcw_mlp.h): per step one gather of the members' batches, the three hidden
+    products (bias + SiLU epilogues keeping pre-activations), the output product whose
+    epilogue is the loss and its gradient, three products back down the layers, all
+    weight and bias gradients, Adam over the flat parameters and the step counter, each
+    one launch for all members.  Parameters live in flat [members, P] vectors
+    (flat_layout).  The step is captured in a CUDA graph on first use and replayed;
+    learning rate, step count and batch counter are device scalars, so the graph never
+    changes."""
 
     def __init__(self, members, batch, x_all, t_all, w_out, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8,
                  use_graph=True):
@@ -484,100 +485,87 @@ class EnsembleTrainer:
         self.loss = torch.zeros(G, dtype=f32, device=dev)
         H, N = DIMS[1], DIMS[-1]
         self.x16 = torch.zeros((G, B, IN_PAD), dtype=bf16, device=dev)
-        self.xt = torch.zeros((G, IN_PAD, B), dtype=bf16, device=dev)
         self.t = torch.zeros((G, B, N), dtype=f32, device=dev)
         self.h = [torch.zeros((G, B, H), dtype=bf16, device=dev) for _ in range(3)]
-        self.ht = [torch.zeros((G, H, B), dtype=bf16, device=dev) for _ in range(3)]
         self.z = [torch.zeros((G, B, H), dtype=f32, device=dev) for _ in range(3)]
-        self.y = torch.zeros((G, B, OUT_PITCH), dtype=f32, device=dev)
-        # output gradient (pitch 656, the pad columns stay zero) and hidden-layer gradients
-        self.g32 = [torch.zeros((G, B, H), dtype=f32, device=dev) for _ in range(3)] + \
-                   [torch.zeros((G, B, OUT_PITCH), dtype=f32, device=dev)]
-        self.g16 = [torch.zeros((G, B, H), dtype=bf16, device=dev) for _ in range(3)] + \
-                   [torch.zeros((G, B, OUT_PITCH), dtype=bf16, device=dev)]
-        self.gt = [torch.zeros((G, H, B), dtype=bf16, device=dev) for _ in range(3)] + \
-                  [torch.zeros((G, OUT_PITCH, B), dtype=bf16, device=dev)]
+        # gradients of the layers' outputs (the last with pitch 656)
+        widths = [_align8(n) for n in (H, H, H, N)]
+        self.g16 = [torch.zeros((G, B, n), dtype=bf16, device=dev) for n in widths]
+        self.g32 = [torch.zeros((G, B, n), dtype=f32, device=dev) for n in widths]
+        # bias gradients: rows summed in chunks of 1,024 when the batch is large, then in order
+        self.colsum_rows = 1024 if B > 2048 else B
         self.splits = _dw_splits(B)
-        # bias gradients of large batches: rows summed in chunks of 1,024, then in order
-        self.colsum_rows = 1024 if B > 2048 else 0
-        n_chunks = (B + 1023) // 1024
-        self.colsum_part = torch.zeros(4 * G * n_chunks * OUT_PITCH, dtype=f32, device=dev) \
-            if self.colsum_rows else None
         if self.splits > 1:
-            largest = max(rows * cols for (_, rows, cols) in (self.lay['W%d' % q] for q in range(4)))
-            self.part = torch.zeros((self.splits, G, largest), dtype=f32, device=dev)
+            self.part = [torch.zeros((self.splits, G, rows * cols), dtype=f32, device=dev)
+                         for (_, rows, cols) in (self.lay['W%d' % q] for q in range(4))]
         self._build_calls()
 
     # ---- the calls of one step, built once (pointers never change)
-    def _gemm(self, epi, m, n, k, a, lda, sa, b, ldb, sb, c, ldc, sc, bias=None, aux=None, ldaux=0, saux=0,
-              c2=None, ldc2=0, sc2=0, ct=None, ldct=0, sct=0, splits=1, s_split=0):
-        ptr = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
-        bias_p = bias if isinstance(bias, int) else ptr(bias)
-        return _abi.GemmGroupedC(m, n, k, self.G, splits, epi, a if isinstance(a, int) else ptr(a), lda, sa,
-                                 b if isinstance(b, int) else ptr(b), ldb, sb, bias_p, self.P,
-                                 ptr(aux), ldaux, saux, c if isinstance(c, int) else ptr(c), ldc, sc, s_split,
-                                 ptr(c2), ldc2, sc2, ptr(ct), ldct, sct)
+    def _gemm(self, epi, m, n, k, a, lda, sa, b, ldb, sb, c, ldc, sc, **more):
+        return _abi.GemmProblemC(m=m, n=n, k=k, groups=self.G, splits=more.pop('splits', 1), epilogue=epi, a=a,
+                                 lda=lda, stride_a=sa, b=b, ldb=ldb, stride_b=sb, c=c, ldc=ldc, stride_c=sc, **more)
 
     def _build_calls(self):
-        G, B, P, T = self.G, self.B, self.P, self.T
+        G, B, P = self.G, self.B, self.P
         H, N = DIMS[1], DIMS[-1]
-        lay, tlay = self.lay, self.tlay
+        lay = self.lay
         w16 = self.w16.data_ptr()
-        wt = self.wt.data_ptr()
         par = self.params.data_ptr()
         grd = self.grad.data_ptr()
         bf, f4 = 2, 4
         fwd = []
-        a, lda, sa = self.x16, IN_PAD, B * IN_PAD
-        for layer in range(3):
+        acts = [(self.x16, IN_PAD)] + [(h, H) for h in self.h]      # inputs of layers 1..4
+        for layer in range(4):
+            a, lda = acts[layer]
             o, rows, cols = lay['W%d' % layer]
             ob, _ = lay['b%d' % layer]
-            fwd.append(self._gemm(_abi.EPI_BIAS_SILU, B, rows, cols, a, lda, sa, w16 + o * bf, cols, P,
-                                  self.h[layer], H, B * H, bias=par + ob * f4, c2=self.z[layer], ldc2=H,
-                                  sc2=B * H, ct=self.ht[layer], ldct=B, sct=H * B))
-            a, lda, sa = self.h[layer], H, B * H
-        o, rows, cols = lay['W3']
-        ob, _ = lay['b3']
-        fwd.append(self._gemm(_abi.EPI_BIAS_F32, B, N, H, self.h[2], H, B * H, w16 + o * bf, H, P,
-                              self.y, OUT_PITCH, B * OUT_PITCH, bias=par + ob * f4))
-        self.fwd_calls = fwd
-        bwd, reduce = [], []
-        # gradient of layer l's output: g[l] (layer 4: g[3], pitch 656)
-        acts_t = [self.xt] + self.ht          # transposed inputs of layers 1..4
-        for layer in (3, 2, 1, 0):
-            o, rows, cols = lay['W%d' % layer]
-            gt = self.gt[layer]
-            gpitch = OUT_PITCH if layer == 3 else H
-            # dW_l[o, i] = sum_b G[b, o] X[b, i]: A = G^T [rows, B], B = X^T [cols, B]
-            if self.splits == 1:
-                bwd.append(self._gemm(_abi.EPI_F32, rows, cols, B, gt, B, gpitch * B, acts_t[layer], B,
-                                      cols * B, grd + o * f4, cols, P))
+            common = (B, rows, cols, a.data_ptr(), lda, B * lda, w16 + o * bf, cols, P)
+            if layer < 3:
+                fwd.append(self._gemm(_abi.EPI_BIAS_SILU, *common, self.h[layer].data_ptr(), H, B * H,
+                                      bias=par + ob * f4, stride_bias=P, c2=self.z[layer].data_ptr(), ldc2=H,
+                                      stride_c2=B * H))
             else:
-                bwd.append(self._gemm(_abi.EPI_F32, rows, cols, B, gt, B, gpitch * B, acts_t[layer], B,
-                                      cols * B, self.part, cols, self.part.shape[2], splits=self.splits,
-                                      s_split=G * self.part.shape[2]))
-                reduce.append((len(bwd) - 1, (self.part.data_ptr(), G * self.part.shape[2], self.part.shape[2],
-                                              cols, grd + o * f4, P, cols, self.splits, G, rows, cols)))
-            if layer == 0:
-                break
-            # G_{l-1} = (G_l W_l) * silu'(Z_{l-1}): A = G_l [B, gpitch], B = W_l^T [cols, ld]
-            to, ld = tlay['W%d' % layer]
-            bwd.append(self._gemm(_abi.EPI_DSILU, B, cols, rows, self.g16[layer], gpitch, B * gpitch,
-                                  wt + to * bf, ld, T, self.g16[layer - 1], H, B * H, aux=self.z[layer - 1],
-                                  ldaux=H, saux=B * H, c2=self.g32[layer - 1], ldc2=H, sc2=B * H,
-                                  ct=self.gt[layer - 1], ldct=B, sct=H * B))
+                # the output layer leaves the loss and its gradient; the outputs are not stored
+                g = self.g16[3]
+                fwd.append(self._gemm(_abi.EPI_LOSS, *common, g.data_ptr(), g.shape[2], B * g.shape[2],
+                                      bias=par + ob * f4, stride_bias=P, aux=self.t.data_ptr(), ldaux=N,
+                                      stride_aux=B * N, weights=self.w_out.data_ptr(), loss=self.loss.data_ptr(),
+                                      c2=self.g32[3].data_ptr(), ldc2=g.shape[2], stride_c2=B * g.shape[2]))
+        self.fwd_calls = fwd
+        # G_{l-1} = (G_l W_l) * silu'(Z_{l-1}): A = G_l, B = W_l as it lies ([out, in])
+        bwd = []
+        for layer in (3, 2, 1):
+            o, rows, cols = lay['W%d' % layer]
+            g, prev = self.g16[layer], self.g16[layer - 1]
+            bwd.append(self._gemm(_abi.EPI_DSILU, B, cols, rows, g.data_ptr(), g.shape[2], B * g.shape[2],
+                                  w16 + o * bf, cols, P, prev.data_ptr(), H, B * H, trans_b=1,
+                                  aux=self.z[layer - 1].data_ptr(), ldaux=H, stride_aux=B * H,
+                                  c2=self.g32[layer - 1].data_ptr(), ldc2=H, stride_c2=B * H))
         self.bwd_calls = bwd
-        self.reduce_after = dict(reduce)
-        cols = (_abi.ColsumLayerC * 4)()
+        # dW_l[o, i] = sum_b G[b, o] X[b, i] and db_l[o] = sum_b G[b, o], the four layers in one launch
+        dw = (_abi.GemmProblemC * 4)()
+        self.reduce_calls = []
         for layer in range(4):
+            o, rows, cols = lay['W%d' % layer]
             ob, nb = lay['b%d' % layer]
-            pitch = OUT_PITCH if layer == 3 else H
-            cols[layer] = _abi.ColsumLayerC(self.g32[layer].data_ptr(), pitch, B * pitch, ob, nb, 0)
-        self.colsum_layers = cols
+            g = self.g16[layer]
+            a, lda = acts[layer]
+            c, sc, s_split = grd + o * f4, P, 0
+            if self.splits > 1:
+                part = self.part[layer]
+                c, sc, s_split = part.data_ptr(), rows * cols, G * rows * cols
+                self.reduce_calls.append((part.data_ptr(), s_split, sc, cols, grd + o * f4, P, cols, self.splits, G,
+                                          rows, cols))
+            dw[layer] = self._gemm(_abi.EPI_F32, rows, cols, B, g.data_ptr(), g.shape[2], B * g.shape[2],
+                                   a.data_ptr(), lda, B * lda, c, cols, sc, splits=self.splits, stride_split=s_split,
+                                   trans_a=1, trans_b=1, colsum=grd + ob * f4, stride_bias=P,
+                                   colsum_in=self.g32[layer].data_ptr(), ld_colsum=g.shape[2],
+                                   stride_colsum=B * g.shape[2], colsum_rows=self.colsum_rows)
+        self.dw_calls = dw
         tb = (_abi.TransposeBlockC * 3)()
         for q, layer in enumerate((1, 2, 3)):
             o, rows, cols_ = lay['W%d' % layer]
-            to, ld = tlay['W%d' % layer]
+            to, ld = self.tlay['W%d' % layer]
             tb[q] = _abi.TransposeBlockC(o, to, ld, rows, cols_)
         self.transpose_blocks = tb
 
@@ -587,30 +575,21 @@ class EnsembleTrainer:
 
     def _launch(self, adam=True):
         """The kernels of one step on the current stream (no host synchronisation)."""
-        torch = self.torch
         L = _abi.load()
-        st = _stream(torch)
+        st = _stream(self.torch)
         G, B = self.G, self.B
         N = DIMS[-1]
-        self._check(L.mcw_mlp_gather(self.x_all.data_ptr(), self.t_all.data_ptr(), self.t_all.shape[1], N,
-                                     self.perm.data_ptr(), self.n_rows, self.counter.data_ptr(), B, G,
-                                     self.x16.data_ptr(), B * IN_PAD, self.xt.data_ptr(), IN_PAD * B,
-                                     self.t.data_ptr(), N, B * N, st), 'mcw_mlp_gather')
+        self._check(L.mcw_mlp_step_begin(self.x_all.data_ptr(), self.t_all.data_ptr(), self.t_all.shape[1], N,
+                                         self.perm.data_ptr(), self.n_rows, self.counter.data_ptr(), B, G,
+                                         self.x16.data_ptr(), B * IN_PAD, self.t.data_ptr(), N, B * N,
+                                         self.loss.data_ptr(), st), 'mcw_mlp_step_begin')
         for c in self.fwd_calls:
-            self._check(L.mcw_mlp_gemm_grouped(ctypes.byref(c), st), 'forward GEMM')
-        self.loss.zero_()
-        self._check(L.mcw_mlp_loss_grouped(self.y.data_ptr(), OUT_PITCH, B * OUT_PITCH, self.t.data_ptr(), N,
-                                           B * N, self.w_out.data_ptr(), G, B, N, self.g32[3].data_ptr(),
-                                           OUT_PITCH, B * OUT_PITCH, self.g16[3].data_ptr(), B * OUT_PITCH,
-                                           self.gt[3].data_ptr(), B, OUT_PITCH * B, self.loss.data_ptr(), st),
-                    'mcw_mlp_loss_grouped')
-        for i, c in enumerate(self.bwd_calls):
-            self._check(L.mcw_mlp_gemm_grouped(ctypes.byref(c), st), 'backward GEMM')
-            if i in self.reduce_after:
-                self._check(L.mcw_mlp_reduce_splits(*self.reduce_after[i], st), 'mcw_mlp_reduce_splits')
-        self._check(L.mcw_mlp_colsum_grouped(self.colsum_layers, 4, G, B, self.grad.data_ptr(), self.P,
-                                             self.colsum_part.data_ptr() if self.colsum_part is not None else None,
-                                             self.colsum_rows, st), 'mcw_mlp_colsum_grouped')
+            self._check(L.mcw_mlp_gemm_batch(ctypes.byref(c), 1, st), 'forward product')
+        for c in self.bwd_calls:
+            self._check(L.mcw_mlp_gemm_batch(ctypes.byref(c), 1, st), 'backward product')
+        self._check(L.mcw_mlp_gemm_batch(self.dw_calls, 4, st), 'weight gradients')
+        for c in self.reduce_calls:
+            self._check(L.mcw_mlp_reduce_splits(*c, st), 'mcw_mlp_reduce_splits')
         if not adam:
             return
         self._check(L.mcw_mlp_adam_grouped(self.params.data_ptr(), self.grad.data_ptr(), self.m.data_ptr(),

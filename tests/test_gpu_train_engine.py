@@ -329,6 +329,21 @@ def test_gemm_batch_loss_and_column_sums(m, n):
     assert (db.double() - out32.double().sum(1)).abs().max() < 1e-5 * out32.double().sum(1).abs().max() + 1e-12
     ref = out16.cpu().double().transpose(1, 2) @ a.cpu().double()
     assert (dw.cpu().double() - ref).abs().max() < 1e-4 * ref.abs().max()
+    # and from the rows themselves, in mcw_mlp_colsum_grouped's order, for any number of column tiles
+    for rows in (m, 64, 1024):
+        for kk in (k, 40, 100):
+            one, two = torch.zeros(G, n, device='cuda'), torch.zeros(G, n, device='cuda')
+            dw = torch.zeros(G, n, kk, device='cuda')
+            x = a[:, :, :(kk + 7) // 8 * 8].contiguous()
+            q = _problem(_abi.EPI_F32, n, kk, m, gt, x, dw, 1, 1, groups=G, colsum=one.data_ptr(), stride_bias=n,
+                         colsum_in=out32.data_ptr(), ld_colsum=n, stride_colsum=m * n, colsum_rows=rows)
+            assert _abi.load().mcw_mlp_gemm_batch(ctypes.byref(q), 1, _stream()) == 0
+            layer = _abi.ColsumLayerC(out32.data_ptr(), n, m * n, 0, n, 0)
+            part = torch.zeros(G * ((m + rows - 1) // rows) * n, device='cuda')
+            assert _abi.load().mcw_mlp_colsum_grouped(ctypes.byref(layer), 1, G, m, two.data_ptr(), n,
+                                                      part.data_ptr(), rows, _stream()) == 0
+            torch.cuda.synchronize()
+            assert torch.equal(one, two), (rows, kk)
     # padded rows
     src = out32[0].contiguous()
     dst = torch.full((m, (n + 7) // 8 * 8), 5.0, dtype=torch.bfloat16, device='cuda')
