@@ -37,6 +37,7 @@
 #include <mutex>
 
 #include "../../include/mcw_mlp.h"
+#include "pdl.cuh"
 
 namespace mcw {
 
@@ -269,6 +270,8 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
     int pi = 0;
     if (kEpi == MCW_EPI_F32 && (int)blockIdx.x >= batch.sums0) {
         while (pi + 1 < batch.np && (int)blockIdx.x >= batch.p[pi + 1].sum0) ++pi;
+        after_previous();
+        let_next_start();
         if (threadIdx.x < 128) column_sums(batch.p[pi], (int)blockIdx.x - batch.p[pi].sum0, (int)threadIdx.x, part);
         return;
     }
@@ -304,6 +307,8 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     const uint32_t ring = smem_u32(smem);
+    after_previous();
+    let_next_start();
 
     if (warp == 4) {
         int issued = 0;
@@ -529,8 +534,7 @@ cudaError_t launch(const GemmBatch &b, unsigned grid, size_t smem, cudaStream_t 
                                     200 * 1024);
     });
     if (attr != cudaSuccess) return attr;
-    gemm_kernel<kEpi, kAMn, kBMn, TN><<<grid, kThreads, smem, s>>>(b);
-    return cudaGetLastError();
+    return launch_after(gemm_kernel<kEpi, kAMn, kBMn, TN>, grid, kThreads, smem, s, b);
 }
 
 // The combinations of epilogue and layouts that exist: a plain product takes any, a backward

@@ -10,6 +10,7 @@
 #include <cstring>
 
 #include "../../include/mcw_mlp.h"
+#include "pdl.cuh"
 
 namespace mcw {
 
@@ -230,6 +231,8 @@ __global__ void __launch_bounds__(256) adam_tiled_kernel(float *w, const float *
     __shared__ __align__(16) __nv_bfloat16 tile[64][40];     // [column][row], rows of 80 bytes
     __shared__ float corr[2];
     const int g = blockIdx.y, t = blockIdx.x;
+    after_previous();
+    let_next_start();
     if (threadIdx.x == 0) {
         const int step = *step_dev;
         corr[0] = 1.f - powf(b1, (float)step);
@@ -275,6 +278,8 @@ __global__ void gather_kernel(const __nv_bfloat16 *x_all, const float *t_all, lo
                               long long ldt, long long s_t, float *loss) {
     const int g = blockIdx.y;
     const int i = blockIdx.x;             // row of the batch
+    after_previous();
+    let_next_start();
     if (loss && i == 0 && threadIdx.x == 0) loss[g] = 0.f;
     const long long idx = (long long)(*counter) * batch + i;
     if (idx >= n_rows) return;            // more steps than the epoch's batches: nothing to gather
@@ -289,6 +294,8 @@ __global__ void gather_kernel(const __nv_bfloat16 *x_all, const float *t_all, lo
 }
 
 __global__ void advance_kernel(int *counter, int *step) {
+    after_previous();
+    let_next_start();
     if (threadIdx.x == 0) {
         *counter += 1;
         *step += 1;
@@ -421,10 +428,11 @@ int mcw_mlp_adam_grouped(float *w, const float *g, float *m, float *v, void *w16
     AdamTiles at;
     const uintptr_t align = (uintptr_t)w | (uintptr_t)g | (uintptr_t)m | (uintptr_t)v | (uintptr_t)w16 | (uintptr_t)wt;
     if (!(align & 15) && make_adam_tiles(tt, n, stride_t, &at)) {
-        adam_tiled_kernel<<<dim3((unsigned)at.tiles, groups), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            w, g, m, v, static_cast<__nv_bfloat16 *>(w16), n, lr_dev, step_dev, beta1, beta2, eps,
+        const cudaError_t e = launch_after(
+            adam_tiled_kernel, dim3((unsigned)at.tiles, groups), 256, 0, static_cast<cudaStream_t>(stream), w, g, m, v,
+            static_cast<__nv_bfloat16 *>(w16), n, lr_dev, step_dev, beta1, beta2, eps,
             static_cast<__nv_bfloat16 *>(wt), stride_t, at);
-        return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
+        return e == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
     }
     const dim3 grid((unsigned)((n + 255) / 256), groups);
     adam_grouped_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -452,16 +460,17 @@ int mcw_mlp_step_begin(const void *x_all, const float *t_all, int64_t ldt_all, i
     if (!x_all || !t_all || !perm || !counter_dev || !x || !t || batch < 1 || groups < 1 || n_out < 0 ||
         n_rows < batch)
         return MCW_MLP_ERR_ARG;
-    gather_kernel<<<dim3(batch, groups), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+    const cudaError_t e = launch_after(
+        gather_kernel, dim3(batch, groups), 128, 0, static_cast<cudaStream_t>(stream),
         static_cast<const __nv_bfloat16 *>(x_all), t_all, ldt_all, n_out, perm, n_rows, counter_dev, batch,
-        static_cast<__nv_bfloat16 *>(x), stride_x, nullptr, 0, t, ldt, stride_t, loss);
-    return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
+        static_cast<__nv_bfloat16 *>(x), stride_x, static_cast<__nv_bfloat16 *>(nullptr), 0, t, ldt, stride_t, loss);
+    return e == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
 }
 
 int mcw_mlp_advance(int32_t *counter_dev, int32_t *step_dev, void *stream) {
     if (!counter_dev || !step_dev) return MCW_MLP_ERR_ARG;
-    advance_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(counter_dev, step_dev);
-    return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
+    const cudaError_t e = launch_after(advance_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream), counter_dev, step_dev);
+    return e == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
 }
 
 }  // extern "C"
