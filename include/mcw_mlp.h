@@ -265,6 +265,38 @@ int mcw_mlp_step_begin(const void *x_all, const float *t_all, int64_t ldt_all, i
 /* *counter_dev += 1 and *step_dev += 1 (the end of a captured step). */
 int mcw_mlp_advance(int32_t *counter_dev, int32_t *step_dev, void *stream);
 
+/* ---- from the network's outputs to BRFs, FP64 (target space: y * std + mean = log(BRF / albedo +
+ * floor) for the 648 bins, log(albedo) last; mean and std [members, 649]; share [648] the bins'
+ * photon shares).  A bin's residual weight is 1 / (max(f, 1e-3) / (photons share) + (rel_noise f)^2 +
+ * model variance), or its share when photons is 0. */
+
+/* Members' BRFs [members, n, 648] and albedos [members, n] from fp16 outputs ys [members, n, pitch]. */
+int mcw_brf_members(const void *ys, int64_t pitch, int32_t members, int32_t n, const double *mean, const double *std,
+                    double floor, double *brf, double *albedo, void *stream);
+
+/* Their means over the members and the relative spread of the BRF (weighted RMS standard deviation
+ * over weighted RMS mean) per row. */
+int mcw_brf_stats(const double *brf, const double *albedo, int32_t members, int32_t n, const double *share,
+                  double *mean_brf, double *mean_albedo, double *spread, void *stream);
+
+/* cost[p * n_obs + o] = sum over bins of w (mean BRF of row p * n_obs + o of ys - obs[o])^2, w from
+ * the observation's own noise. */
+int mcw_brf_cost(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t n_obs, const double *mean,
+                 const double *std, double floor, const double *obs, const double *share, double photons,
+                 double rel_noise, double *cost, void *stream);
+
+/* Mean BRF f, its slope j and the members' variance v, each [n, 648] or NULL, from fp32 outputs y and
+ * tangents ydot [members, n, pitch]; with obs [n, 648]: jtr = sum w j (f - obs), jtj = sum w j^2. */
+int mcw_brf_jacobian(const float *y, const float *ydot, int64_t pitch, int32_t members, int32_t n, const double *mean,
+                     const double *std, double floor, double *f, double *j, double *v, const double *obs,
+                     const double *share, double photons, double rel_noise, double *jtr, double *jtj, void *stream);
+
+/* Standard deviation over the members of sum w j (BRF - mean BRF) / sum w j^2, and 1 / sqrt(sum j^2 /
+ * variance without the model's). */
+int mcw_brf_logr(const double *brf, const double *mean_brf, int32_t members, int32_t n, const double *f, const double *j,
+                 const double *v, const double *share, double photons, double rel_noise, double *spread, double *sigma,
+                 void *stream);
+
 #ifdef __cplusplus
 }
 #endif

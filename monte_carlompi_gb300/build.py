@@ -25,7 +25,7 @@ LIB = os.path.join(LIBDIR, 'libmcwalk.so')
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 
 # units whose FP64 arithmetic must keep the reference's rounding: no contraction
-NO_FMAD = {'walk_replay.cu', 'ssp_lut.cu'}
+NO_FMAD = {'walk_replay.cu', 'ssp_lut.cu', 'brf.cu'}
 # the FP32 production walk: flush denormals, approximate division and square root
 FAST_F32 = {'walk_f32.cu': ['-ftz=true', '-prec-div=false', '-prec-sqrt=false']}
 # tuning builds: extra -D flags for the FP32 walk and the fused inference kernel

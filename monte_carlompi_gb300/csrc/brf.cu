@@ -1,0 +1,308 @@
+// From the surrogate's standardised outputs to BRFs, in FP64: members' BRFs, their mean and
+// spread, a retrieval's costs and Gauss-Newton sums.  Compiled with --fmad=false: every product
+// and sum is rounded on its own, in the order of the array code these kernels took the place of
+// (surrogate.from_target, Ensemble.predict, inverse.surrogate_gn).
+//
+// Target space: y * std + mean = log(BRF / albedo + floor) for the 648 bins and log(albedo).
+//
+// What bounds them: FP64 (an exponential is about 25 operations, 64 cycles a warp each on a
+// sub-core), so every kernel takes each exponential once and keeps what it can in registers; a
+// block per row, a thread per bin, sums by block reduction.  128 observations, five members, one
+// retrieval (16-point grid, six iterations, spreads): 92 ms on the host's cores and elementwise
+// tensor kernels, 3.5 ms now.
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "../../include/mcw_mlp.h"
+
+namespace mcw {
+
+namespace {
+
+constexpr int kBins = MCW_MLP_OUT - 1;     // 648
+constexpr int kThreads = 224;              // 7 warps, three bins a thread (672)
+constexpr int kPer = 3;
+
+// Block sum (every thread gets it); `red` holds one value per warp.
+__device__ __forceinline__ double block_sum(double v, double *red) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = red[0];
+#pragma unroll
+    for (int q = 1; q < kThreads / 32; ++q) s += red[q];
+    return s;
+}
+
+__device__ __forceinline__ double unscaled(double y, double std, double mean) { return y * std + mean; }
+
+// BRF of one bin: (exp(y) - floor) * albedo.
+__device__ __forceinline__ double bin_brf(const __half *row, int b, const double *std, const double *mean, double floor,
+                                          double albedo) {
+    return (exp(unscaled((double)__half2float(row[b]), std[b], mean[b])) - floor) * albedo;
+}
+
+__device__ __forceinline__ double row_albedo(const __half *row, const double *std, const double *mean) {
+    return exp(unscaled((double)__half2float(row[kBins]), std[kBins], mean[kBins]));
+}
+
+// The larger of x and lo; NaN stays NaN.
+__device__ __forceinline__ double at_least(double x, double lo) { return x < lo ? lo : x; }
+
+// Weight of a bin's residual: 1 / variance (counting noise of `photons`, relative noise, the
+// model's variance), or the bin's share without photons.
+struct Noise {
+    double photons, rel;
+    const double *share;       // [648]
+    __device__ __forceinline__ double variance(double f, double model, int b) const {
+        const double v = at_least(f, 1e-3) / (photons * share[b]) + (rel * f) * (rel * f);
+        return v + model;
+    }
+};
+
+// Each member's BRF and albedo of row blockIdx.x.
+__global__ void __launch_bounds__(kThreads) members_kernel(const __half *ys, long long pitch, int n, const double *mean,
+                                                           const double *std, double floor, double *brf, double *alb) {
+    const int r = blockIdx.x, m = blockIdx.y;
+    const __half *row = ys + ((size_t)m * n + r) * pitch;
+    const double *mu = mean + (size_t)m * (kBins + 1), *sd = std + (size_t)m * (kBins + 1);
+    __shared__ double a;
+    if (threadIdx.x == 0) {
+        a = row_albedo(row, sd, mu);
+        alb[(size_t)m * n + r] = a;
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < kBins; b += kThreads)
+        brf[((size_t)m * n + r) * kBins + b] = bin_brf(row, b, sd, mu, floor, a);
+}
+
+// Mean BRF and albedo over the members, and the spread: the weighted RMS of the members' standard
+// deviation over the weighted RMS of the mean.
+__global__ void __launch_bounds__(kThreads) stats_kernel(const double *brf, const double *alb, int members, int n,
+                                                         const double *share, double *mean, double *alb_mean,
+                                                         double *spread) {
+    __shared__ double red[kThreads / 32];
+    const int r = blockIdx.x;
+    double num = 0.0, den = 0.0;
+    for (int b = threadIdx.x; b < kBins; b += kThreads) {
+        const double *p = brf + (size_t)r * kBins + b;
+        const size_t s = (size_t)n * kBins;
+        double t = 0.0;
+        for (int m = 0; m < members; ++m) t += p[m * s];
+        const double mu = t / members;
+        double v = 0.0;
+        for (int m = 0; m < members; ++m) {
+            const double d = p[m * s] - mu;
+            v += d * d;
+        }
+        mean[(size_t)r * kBins + b] = mu;
+        num += v / members * share[b];
+        den += mu * mu * share[b];
+    }
+    num = block_sum(num, red);
+    den = block_sum(den, red);
+    if (threadIdx.x == 0) {
+        spread[r] = sqrt(num / at_least(den, 1e-30));
+        double t = 0.0;
+        for (int m = 0; m < members; ++m) t += alb[(size_t)m * n + r];
+        alb_mean[r] = t / members;
+    }
+}
+
+// Cost of a grid point for an observation: sum over bins of w (mean BRF - obs)^2, w from the
+// observation's own noise.  Row blockIdx.x = point * n_obs + observation.
+__global__ void __launch_bounds__(kThreads) cost_kernel(const __half *ys, long long pitch, int members, int rows, int n_obs,
+                                                        const double *mean, const double *std, double floor,
+                                                        const double *obs, const Noise noise, double *cost) {
+    extern __shared__ double albs[];         // members
+    __shared__ double red[kThreads / 32];
+    const int r = blockIdx.x, o = r % n_obs;
+    for (int m = threadIdx.x; m < members; m += kThreads)
+        albs[m] = row_albedo(ys + ((size_t)m * rows + r) * pitch, std + (size_t)m * (kBins + 1), mean + (size_t)m * (kBins + 1));
+    __syncthreads();
+    double c = 0.0;
+    for (int b = threadIdx.x; b < kBins; b += kThreads) {
+        double t = 0.0;
+        for (int m = 0; m < members; ++m)
+            t += bin_brf(ys + ((size_t)m * rows + r) * pitch, b, std + (size_t)m * (kBins + 1),
+                         mean + (size_t)m * (kBins + 1), floor, albs[m]);
+        const double x = obs[(size_t)o * kBins + b];
+        const double d = t / members - x;
+        const double w = noise.photons != 0 ? 1.0 / noise.variance(x, 0.0, b) : noise.share[b];
+        c += w * (d * d);
+    }
+    c = block_sum(c, red);
+    if (threadIdx.x == 0) cost[r] = c;
+}
+
+// Mean BRF f, d f / d log r (j) and the members' variance (v) of row blockIdx.x from the outputs y
+// and their tangents, FP32 [members, n, pitch]; any of f_out, j_out, v_out may be null.  With obs:
+// the Gauss-Newton sums over the bins of w j (f - obs) and w j^2.
+__global__ void __launch_bounds__(kThreads) jacobian_kernel(const float *y, const float *ydot, long long pitch, int members,
+                                                            int n, const double *mean, const double *std, double floor,
+                                                            double *f_out, double *j_out, double *v_out,
+                                                            const double *obs, const Noise noise, double *jtr, double *jtj) {
+    extern __shared__ double sh[];           // albedo and its slope per member
+    __shared__ double red[kThreads / 32];
+    const int r = blockIdx.x;
+    for (int m = threadIdx.x; m < members; m += kThreads) {
+        const size_t at = ((size_t)m * n + r) * pitch + kBins;
+        const double sd = std[(size_t)m * (kBins + 1) + kBins];
+        const double a = exp(unscaled((double)y[at], sd, mean[(size_t)m * (kBins + 1) + kBins]));
+        sh[2 * m] = a;
+        sh[2 * m + 1] = a * ((double)ydot[at] * sd);
+    }
+    __syncthreads();
+    double sr = 0.0, sj = 0.0;
+    for (int b = threadIdx.x; b < kBins; b += kThreads) {
+        double f = 0.0, j = 0.0, f2 = 0.0;
+        for (int m = 0; m < members; ++m) {
+            const size_t at = ((size_t)m * n + r) * pitch + b;
+            const double sd = std[(size_t)m * (kBins + 1) + b], a = sh[2 * m];
+            const double shape = exp(unscaled((double)y[at], sd, mean[(size_t)m * (kBins + 1) + b]));
+            const double dp = (double)ydot[at] * sd;
+            const double fm = (shape - floor) * a;
+            f += fm;
+            f2 += fm * fm;
+            j += shape * dp * a + (shape - floor) * sh[2 * m + 1];
+        }
+        f = f / members;
+        j = j / members;
+        const double v = at_least(f2 / members - f * f, 0.0);
+        if (f_out) f_out[(size_t)r * kBins + b] = f;
+        if (j_out) j_out[(size_t)r * kBins + b] = j;
+        if (v_out) v_out[(size_t)r * kBins + b] = v;
+        if (obs) {
+            const double d = f - obs[(size_t)r * kBins + b];
+            const double w = noise.photons != 0 ? 1.0 / noise.variance(f, v, b) : noise.share[b];
+            sr += w * j * d;
+            sj += w * j * j;
+        }
+    }
+    if (!obs) return;
+    sr = block_sum(sr, red);
+    sj = block_sum(sj, red);
+    if (threadIdx.x == 0) {
+        jtr[r] = sr;
+        jtj[r] = sj;
+    }
+}
+
+// The members' standard deviation of log r at the solution (inverse.logr_spread) and the posterior
+// width the observation noise alone allows, 1 / sqrt(sum j^2 / var).
+__global__ void __launch_bounds__(kThreads) logr_kernel(const double *brf, const double *mean, int members, int n,
+                                                        const double *f, const double *j, const double *v,
+                                                        const Noise noise, double *spread, double *sigma) {
+    __shared__ double red[kThreads / 32];
+    const int r = blockIdx.x;
+    double wj[kPer], mu[kPer];
+    double sj = 0.0, sn = 0.0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int b = threadIdx.x + k * kThreads;
+        wj[k] = mu[k] = 0.0;
+        if (b < kBins) {
+            const size_t at = (size_t)r * kBins + b;
+            const double w = noise.photons != 0 ? 1.0 / noise.variance(f[at], v[at], b) : noise.share[b];
+            const double wn = noise.photons != 0 ? 1.0 / noise.variance(f[at], 0.0, b) : noise.share[b];
+            mu[k] = mean[at];
+            wj[k] = w * j[at];
+            sj += wj[k] * j[at];
+            sn += wn * j[at] * j[at];
+        }
+    }
+    sj = at_least(block_sum(sj, red), 1e-300);
+    sn = at_least(block_sum(sn, red), 1e-300);
+    // two passes over the members' shifts: their mean, then their deviation
+    double total = 0.0, var = 0.0;
+    for (int pass = 0; pass < 2; ++pass)
+        for (int m = 0; m < members; ++m) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                const int b = threadIdx.x + k * kThreads;
+                if (b < kBins) s += wj[k] * (brf[((size_t)m * n + r) * kBins + b] - mu[k]);
+            }
+            const double ds = block_sum(s, red) / sj;
+            if (pass == 0) {
+                total += ds;
+            } else {
+                const double d = ds - total / members;
+                var += d * d;
+            }
+        }
+    if (threadIdx.x == 0) {
+        spread[r] = sqrt(var / members);
+        sigma[r] = 1.0 / sqrt(sn);
+    }
+}
+
+bool rows_ok(int32_t members, int32_t n) { return members >= 1 && members <= 4096 && n >= 0; }
+int done() { return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA; }
+
+}  // namespace
+
+}  // namespace mcw
+
+using namespace mcw;
+
+extern "C" {
+
+int mcw_brf_members(const void *ys, int64_t pitch, int32_t members, int32_t n, const double *mean, const double *std,
+                    double floor, double *brf, double *albedo, void *stream) {
+    if (!ys || !mean || !std || !brf || !albedo || !rows_ok(members, n) || pitch < MCW_MLP_OUT) return MCW_MLP_ERR_ARG;
+    if (n == 0) return 0;
+    members_kernel<<<dim3(n, members), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __half *>(ys), pitch, n, mean, std, floor, brf, albedo);
+    return done();
+}
+
+int mcw_brf_stats(const double *brf, const double *albedo, int32_t members, int32_t n, const double *share,
+                  double *mean_brf, double *mean_albedo, double *spread, void *stream) {
+    if (!brf || !albedo || !share || !mean_brf || !mean_albedo || !spread || !rows_ok(members, n)) return MCW_MLP_ERR_ARG;
+    if (n == 0) return 0;
+    stats_kernel<<<n, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(brf, albedo, members, n, share, mean_brf,
+                                                                        mean_albedo, spread);
+    return done();
+}
+
+int mcw_brf_cost(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t n_obs, const double *mean,
+                 const double *std, double floor, const double *obs, const double *share, double photons,
+                 double rel_noise, double *cost, void *stream) {
+    if (!ys || !mean || !std || !obs || !share || !cost || points < 0 || n_obs < 0 ||
+        (long long)points * n_obs > 0x7fffffffLL || !rows_ok(members, points * n_obs) || pitch < MCW_MLP_OUT)
+        return MCW_MLP_ERR_ARG;
+    if (points * n_obs == 0) return 0;
+    cost_kernel<<<points * n_obs, kThreads, members * sizeof(double), static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __half *>(ys), pitch, members, points * n_obs, n_obs, mean, std, floor, obs,
+        Noise{photons, rel_noise, share}, cost);
+    return done();
+}
+
+int mcw_brf_jacobian(const float *y, const float *ydot, int64_t pitch, int32_t members, int32_t n, const double *mean,
+                     const double *std, double floor, double *f, double *j, double *v, const double *obs,
+                     const double *share, double photons, double rel_noise, double *jtr, double *jtj, void *stream) {
+    if (!y || !ydot || !mean || !std || !rows_ok(members, n) || pitch < MCW_MLP_OUT ||
+        (obs && (!share || !jtr || !jtj)))
+        return MCW_MLP_ERR_ARG;
+    if (n == 0) return 0;
+    jacobian_kernel<<<n, kThreads, 2 * members * sizeof(double), static_cast<cudaStream_t>(stream)>>>(
+        y, ydot, pitch, members, n, mean, std, floor, f, j, v, obs, Noise{photons, rel_noise, share}, jtr, jtj);
+    return done();
+}
+
+int mcw_brf_logr(const double *brf, const double *mean_brf, int32_t members, int32_t n, const double *f, const double *j,
+                 const double *v, const double *share, double photons, double rel_noise, double *spread, double *sigma,
+                 void *stream) {
+    if (!brf || !mean_brf || !f || !j || !v || !share || !spread || !sigma || !rows_ok(members, n)) return MCW_MLP_ERR_ARG;
+    if (n == 0) return 0;
+    logr_kernel<<<n, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(brf, mean_brf, members, n, f, j, v,
+                                                                       Noise{photons, rel_noise, share}, spread, sigma);
+    return done();
+}
+
+}  // extern "C"

@@ -19,6 +19,7 @@ import time
 
 import numpy as np
 
+from . import _abi
 from . import surrogate as S
 
 LOG_R = (math.log(S.R_RANGE[0]), math.log(S.R_RANGE[1]))
@@ -34,49 +35,64 @@ def noise_variance(f, photons, rel_noise=0.0, model_var=None):
     return v + model_var if model_var is not None else v
 
 
-def _brf_and_jacobian(ens, s, known, chunk=65536, with_var=False):
-    """Ensemble-mean BRF [n, 648] and d BRF / d log r [n, 648] at log r = s: one
-    forward-mode pass per member through the tensor-core kernels (the tangent of the
-    first input, d x0 / d log r = 2 / (log r_max - log r_min)), then the chain rule
-    through the target standardisation, exp and the albedo factor.  with_var: also the
-    variance of the members' BRFs per bin."""
-    import torch
+def _ptr(t):
+    return None if t is None else t.data_ptr()
+
+
+class _Slopes:
+    """BRF, d BRF / d log r_eff and the members' variance of an ensemble at n points: one
+    forward-mode pass of all members through the tensor-core kernels (the tangent of the first
+    input, d x0 / d log r = 2 / (log r_max - log r_min)), then the chain rule through the target
+    standardisation, exp and the albedo factor in one kernel."""
+
+    def __init__(self, ens, n):
+        import torch
+        self.torch = torch
+        self.n = n
+        self.net = S.EnsembleTangent(torch, ens.members, n, 2.0 / (LOG_R[1] - LOG_R[0]))
+        self.mean, self.std = ens.scaling()
+        self.share = torch.from_numpy(S.bin_weights()).cuda()
+
+    def at(self, s, known, obs=None, noise=(0.0, 0.0), arrays=True):
+        """At log r = s: (f, j, v) torch CUDA float64 [n, 648] (None without arrays) and, with obs
+        (torch CUDA float64 [n, 648]), the sums over the bins of w j (f - obs) and w j^2 [n]."""
+        torch = self.torch
+        x = torch.from_numpy(S.encode(np.exp(s), known[:, 0], known[:, 1], known[:, 2])).cuda()
+        y, ydot = self.net.run(x)
+        new = lambda *shape: torch.empty(shape, dtype=torch.float64, device=y.device)  # noqa: E731
+        f, j, v = (new(self.n, S.N_BRF) for _ in range(3)) if arrays else (None, None, None)
+        sums = new(2, self.n) if obs is not None else (None, None)
+        rc = _abi.load().mcw_brf_jacobian(_ptr(y), _ptr(ydot), y.shape[2], y.shape[0], self.n, _ptr(self.mean),
+                                          _ptr(self.std), S.BRF_FLOOR, _ptr(f), _ptr(j), _ptr(v), _ptr(obs),
+                                          _ptr(self.share), noise[0], noise[1], _ptr(sums[0]), _ptr(sums[1]),
+                                          S._stream(torch))
+        if rc:
+            raise _abi.McwError(rc, 'mcw_brf_jacobian failed')
+        return (f, j, v), sums
+
+
+def _brf_and_jacobian(ens, s, known, chunk=16384, with_var=False):
+    """Ensemble-mean BRF [n, 648] and d BRF / d log r [n, 648] at log r = s (_Slopes).  with_var:
+    also the variance of the members' BRFs per bin."""
     n = s.shape[0]
-    f_out = np.zeros((n, S.N_BRF))
-    j_out = np.zeros((n, S.N_BRF))
-    v_out = np.zeros((n, S.N_BRF))
-    dxds = 2.0 / (LOG_R[1] - LOG_R[0])
+    out = [np.zeros((n, S.N_BRF)) for _ in range(3)]
+    slopes = None
     for lo in range(0, n, chunk):
         hi = min(n, lo + chunk)
-        x = torch.from_numpy(S.encode(np.exp(s[lo:hi]), known[lo:hi, 0], known[lo:hi, 1],
-                                      known[lo:hi, 2])).cuda()
-        xdot = torch.zeros_like(x)
-        xdot[:, 0] = dxds
-        x16, xdot16 = S._cast(torch, x), S._cast(torch, xdot)
-        f_acc = torch.zeros((hi - lo, S.N_BRF), dtype=torch.float64, device='cuda')
-        j_acc = torch.zeros_like(f_acc)
-        f2_acc = torch.zeros_like(f_acc)
-        for m in ens.members:
-            y, ydot = S.forward_tangent(torch, x16, xdot16, m.w16, m.params[1::2])
-            yp = y.double() * m.y_std + m.y_mean                  # log(BRF / albedo + floor), log(albedo)
-            dp = ydot.double() * m.y_std
-            alb = torch.exp(yp[:, S.N_BRF])
-            shape = torch.exp(yp[:, :S.N_BRF])
-            fm = (shape - S.BRF_FLOOR) * alb[:, None]
-            f_acc += fm
-            f2_acc += fm * fm
-            j_acc += shape * dp[:, :S.N_BRF] * alb[:, None] + (shape - S.BRF_FLOOR) * (alb * dp[:, S.N_BRF])[:, None]
-        k = len(ens.members)
-        f_out[lo:hi] = (f_acc / k).cpu().numpy()
-        j_out[lo:hi] = (j_acc / k).cpu().numpy()
-        v_out[lo:hi] = torch.clamp(f2_acc / k - (f_acc / k) ** 2, min=0).cpu().numpy()
-    return (f_out, j_out, v_out) if with_var else (f_out, j_out)
+        if slopes is None or slopes.n != hi - lo:
+            slopes = _Slopes(ens, hi - lo)
+        arrays, _ = slopes.at(s[lo:hi], known[lo:hi])
+        for o, t in zip(out, arrays):
+            o[lo:hi] = t.cpu().numpy()
+    return tuple(out) if with_var else tuple(out[:2])
 
 
 def _gn_update(f, jac, obs, s, w, damping=1e-3, max_step=0.7):
     r = f - obs
-    jtr = (w * jac * r).sum(1)
-    jtj = (w * jac * jac).sum(1)
+    return _gn_step((w * jac * r).sum(1), (w * jac * jac).sum(1), s, damping, max_step)
+
+
+def _gn_step(jtr, jtj, s, damping=1e-3, max_step=0.7):
     step = -jtr / (jtj * (1 + damping) + 1e-30)
     step = np.clip(step, -max_step, max_step)
     return np.clip(s + step, LOG_R[0], LOG_R[1])
@@ -100,32 +116,57 @@ def surrogate_gn(ens, obs, known, iters=6, obs_photons=None, obs_noise=0.0, with
     without, by the bin's photon share.  Returns (s, brf at s, BRF spread at s, log r_eff
     spread at s) and, with with_noise, the posterior width of s from the observation
     noise alone, 1 / sqrt(sum_b J_b^2 / var_b)."""
+    if obs.ndim != 2 or obs.shape[1] != S.N_BRF or np.shape(known) != (obs.shape[0], 3):
+        raise ValueError('obs must be [n, %d] and known [n, 3]' % S.N_BRF)
+    parts = [_surrogate_gn(ens, obs[lo:lo + 4096], known[lo:lo + 4096], iters,
+                           (float(obs_photons or 0), float(obs_noise)))
+             for lo in range(0, obs.shape[0], 4096)]
+    if not parts:
+        parts = [(np.zeros(0), np.zeros((0, S.N_BRF)), np.zeros(0), np.zeros(0), np.zeros(0))]
+    out = tuple(np.concatenate([p[k] for p in parts]) for k in range(5))
+    return out if with_noise else out[:4]
+
+
+def _surrogate_gn(ens, obs, known, iters, noise):
+    """surrogate_gn of a few thousand observations: BRFs, residuals and their sums stay on the
+    device (FP64, csrc/brf.cu); the host holds log r_eff, encodes it and takes the steps."""
+    import torch
     n = obs.shape[0]
-    share = S.bin_weights()[None, :]
-    w0 = 1.0 / noise_variance(obs, obs_photons, obs_noise) if obs_photons else share
+    known = np.asarray(known, np.float64)
+    obs_d = torch.from_numpy(np.ascontiguousarray(obs, np.float64)).cuda()
+    slopes = _Slopes(ens, n)
+    L, st, k = _abi.load(), S._stream(torch), len(ens.members)
+
+    def check(rc, what):
+        if rc:
+            raise _abi.McwError(rc, '%s failed' % what)
+    # the grid: every observation at every point in one forward pass
     grid = np.linspace(LOG_R[0], LOG_R[1], 16)
+    r = np.repeat(np.array([math.exp(g) for g in grid]), n)
+    x = torch.from_numpy(S.encode(r, *np.tile(known, (16, 1)).T)).cuda()
+    ys = ens.predict_std(x)
+    cost_d = torch.empty((16, n), dtype=torch.float64, device='cuda')
+    check(L.mcw_brf_cost(_ptr(ys), ys.stride(1), k, 16, n, _ptr(slopes.mean), _ptr(slopes.std), S.BRF_FLOOR,
+                         _ptr(obs_d), _ptr(slopes.share), noise[0], noise[1], _ptr(cost_d), st), 'mcw_brf_cost')
+    cost = cost_d.cpu().numpy()
     best = np.full(n, np.inf)
     s = np.zeros(n)
-    for g in grid:
-        pred, _, _ = ens.predict(np.column_stack([np.full(n, math.exp(g)), known]))
-        cost = (w0 * (pred - obs) ** 2).sum(1)
-        better = cost < best
-        best[better] = cost[better]
+    for g, c in zip(grid, cost):
+        better = c < best
+        best[better] = c[better]
         s[better] = g
     for _ in range(iters):
-        f, jac, var = _brf_and_jacobian(ens, s, known, with_var=True)
-        w = 1.0 / noise_variance(f, obs_photons, obs_noise, var) if obs_photons else share
-        s = _gn_update(f, jac, obs, s, w)
-    pred, _, spread = ens.predict(np.column_stack([np.exp(s), known]))
-    f, jac, var = _brf_and_jacobian(ens, s, known, with_var=True)
-    members, _ = ens.predict_members(np.column_stack([np.exp(s), known]))
-    w = 1.0 / noise_variance(f, obs_photons, obs_noise, var) if obs_photons else share
-    spread_r = logr_spread(members, jac, w)
-    if not with_noise:
-        return s, pred, spread, spread_r
-    wn = 1.0 / noise_variance(f, obs_photons, obs_noise) if obs_photons else share
-    sigma = 1.0 / np.sqrt(np.maximum((wn * jac * jac).sum(1), 1e-300))
-    return s, pred, spread, spread_r, sigma
+        _, sums = slopes.at(s, known, obs_d, noise, arrays=False)
+        jtr, jtj = sums.cpu().numpy()
+        s = _gn_step(jtr, jtj, s)
+    x = torch.from_numpy(S.encode(np.exp(s), *known.T)).cuda()
+    brf, alb = ens.member_brfs(x)
+    pred, _, spread = ens.brf_stats(brf, alb)
+    (f, j, v), _ = slopes.at(s, known)
+    spread_r, sigma = torch.empty_like(spread), torch.empty_like(spread)
+    check(L.mcw_brf_logr(_ptr(brf), _ptr(pred), k, n, _ptr(f), _ptr(j), _ptr(v), _ptr(slopes.share), noise[0],
+                         noise[1], _ptr(spread_r), _ptr(sigma), st), 'mcw_brf_logr')
+    return (s,) + tuple(t.cpu().numpy() for t in (pred, spread, spread_r, sigma))
 
 
 def mc_gn(walker, obs, known, s0, n_photon=1000000, iters=3, h=0.05, seed=0x5EED0055, obs_photons=None,

@@ -271,6 +271,56 @@ def forward_tangent(torch, x16, xdot16, w16, biases):
     return y, ydot
 
 
+class EnsembleTangent:
+    """forward_tangent of every member of an ensemble on the same n inputs, each product one launch
+    for all members: the members' bf16 weights laid side by side and the buffers of one batch size,
+    made once for the evaluations of a retrieval.  The tangent is that of the first input, dx0."""
+
+    def __init__(self, torch, members, n, dx0):
+        self.torch = torch
+        self.n, self.G = n, len(members)
+        G, H, N, dev = self.G, DIMS[1], DIMS[-1], members[0].w16[0].device
+        bf16, f32 = torch.bfloat16, torch.float32
+        ws = [torch.stack([_rows16(torch, m.w16[layer]) for m in members]) for layer in range(4)]
+        bs = [torch.stack([m.params[2 * layer + 1].float() for m in members]) for layer in range(4)]
+        self.x = torch.zeros((G, n, 8), dtype=bf16, device=dev)
+        xdot = torch.zeros((G, n, 8), dtype=bf16, device=dev)
+        xdot[:, :, 0] = dx0
+        h = [torch.empty((G, n, H), dtype=bf16, device=dev) for _ in range(3)]
+        t = [torch.empty((G, n, H), dtype=bf16, device=dev) for _ in range(3)]
+        z = [torch.empty((G, n, H), dtype=f32, device=dev) for _ in range(3)]
+        self.y = torch.empty((G, n, Y_PITCH), dtype=f32, device=dev)
+        self.ydot = torch.empty((G, n, Y_PITCH), dtype=f32, device=dev)
+        self.keep = (ws, bs, xdot, h, t, z)
+
+        def call(epi, layer, a, c, **more):
+            w = ws[layer]
+            return _abi.GemmProblemC(m=n, n=w.shape[1], k=DIMS[layer], groups=G, splits=1, epilogue=epi, a=a.data_ptr(),
+                                     lda=a.shape[2], stride_a=n * a.shape[2], b=w.data_ptr(), ldb=w.shape[2],
+                                     stride_b=w.shape[1] * w.shape[2], c=c.data_ptr(), ldc=c.shape[2],
+                                     stride_c=n * c.shape[2], **more)
+        self.calls = []
+        a, d = self.x, xdot
+        for layer in range(3):
+            zl = dict(c2=z[layer].data_ptr(), ldc2=H, stride_c2=n * H)
+            self.calls.append(call(_abi.EPI_BIAS_SILU, layer, a, h[layer], bias=bs[layer].data_ptr(), stride_bias=H, **zl))
+            self.calls.append(call(_abi.EPI_DSILU, layer, d, t[layer], aux=z[layer].data_ptr(), ldaux=H, stride_aux=n * H))
+            a, d = h[layer], t[layer]
+        self.calls.append(call(_abi.EPI_BIAS_F32, 3, a, self.y, bias=bs[3].data_ptr(), stride_bias=N))
+        self.calls.append(call(_abi.EPI_F32, 3, d, self.ydot))
+
+    def run(self, x):
+        """x float32 [n, 4]; returns (y, ydot) fp32 [members, n, Y_PITCH], 649 columns used; valid
+        until the next call."""
+        self.x[:, :, :DIMS[0]] = x
+        L, st = _abi.load(), _stream(self.torch)
+        for c in self.calls:
+            rc = L.mcw_mlp_gemm_batch(ctypes.byref(c), 1, st)
+            if rc:
+                raise _abi.McwError(rc, 'ensemble tangent failed (n=%d)' % self.n)
+        return self.y, self.ydot
+
+
 def _mlp_function():
     import torch
 
@@ -732,24 +782,62 @@ class Ensemble:
         blob, bias = self.packed()
         return forward_ensemble(torch, x, blob, bias, len(self.members))
 
+    def scaling(self):
+        """The members' target scaling as rows: (mean, std), float64 [members, 649]."""
+        import torch
+        return (torch.stack([m.y_mean.double() for m in self.members]).contiguous(),
+                torch.stack([m.y_std.double() for m in self.members]).contiguous())
+
+    def member_brfs(self, x):
+        """Each member's BRF [members, n, 648] and albedo [members, n] (torch CUDA float64) for
+        encoded inputs x (torch CUDA float32 [n, 4])."""
+        import torch
+        ys = self.predict_std(x)
+        k, n = ys.shape[:2]
+        mean, std = self.scaling()
+        brf = torch.empty((k, n, N_BRF), dtype=torch.float64, device=x.device)
+        alb = torch.empty((k, n), dtype=torch.float64, device=x.device)
+        rc = _abi.load().mcw_brf_members(_ptr(ys), ys.stride(1), k, n, _ptr(mean), _ptr(std), BRF_FLOOR, _ptr(brf),
+                                         _ptr(alb), _stream(torch))
+        if rc:
+            raise _abi.McwError(rc, 'mcw_brf_members failed')
+        return brf, alb
+
+    def brf_stats(self, brf, alb):
+        """Mean BRF [n, 648], mean albedo [n] and relative spread [n] of member_brfs' result
+        (torch CUDA float64): the spread in the units of rel_rms, weighted RMS standard
+        deviation over weighted RMS BRF."""
+        import torch
+        k, n = alb.shape
+        mean = torch.empty((n, N_BRF), dtype=torch.float64, device=brf.device)
+        alb_mean, spread = torch.empty_like(alb[0]), torch.empty_like(alb[0])
+        share = torch.from_numpy(bin_weights()).to(brf.device)
+        rc = _abi.load().mcw_brf_stats(_ptr(brf), _ptr(alb), k, n, _ptr(share), _ptr(mean), _ptr(alb_mean),
+                                       _ptr(spread), _stream(torch))
+        if rc:
+            raise _abi.McwError(rc, 'mcw_brf_stats failed')
+        return mean, alb_mean, spread
+
+    def _chunks(self, raw, rows=16384):
+        import torch
+        x = encode(*np.asarray(raw, np.float64).T)
+        for lo in range(0, x.shape[0], rows):
+            yield torch.from_numpy(x[lo:lo + rows]).cuda()
+
     def predict_members(self, raw):
         """Each member's BRF [members, n, 648] and albedo [members, n]."""
-        import torch
-        x = torch.from_numpy(encode(*np.asarray(raw, np.float64).T)).cuda()
-        ys = self.predict_std(x)
-        outs = np.stack([(ys[k].double() * m.y_std + m.y_mean).cpu().numpy()
-                         for k, m in enumerate(self.members)])
-        brfs, albs = zip(*[from_target(o) for o in outs])
-        return np.stack(brfs), np.stack(albs)
+        parts = [[t.cpu().numpy() for t in self.member_brfs(x)] for x in self._chunks(raw)]
+        if not parts:
+            k = len(self.members)
+            return np.zeros((k, 0, N_BRF)), np.zeros((k, 0))
+        return np.concatenate([p[0] for p in parts], 1), np.concatenate([p[1] for p in parts], 1)
 
     def predict(self, raw):
         """Mean BRF [n, 648], mean albedo [n], relative ensemble spread of the BRF [n]."""
-        brfs, albs = self.predict_members(raw)
-        mean_brf = brfs.mean(0)
-        w = bin_weights()
-        # member spread in the units of rel_rms: weighted RMS std over weighted RMS BRF
-        spread = np.sqrt((brfs.std(0) ** 2 * w).sum(1) / np.maximum((mean_brf ** 2 * w).sum(1), 1e-30))
-        return mean_brf, albs.mean(0), spread
+        parts = [[t.cpu().numpy() for t in self.brf_stats(*self.member_brfs(x))] for x in self._chunks(raw)]
+        if not parts:
+            return np.zeros((0, N_BRF)), np.zeros(0), np.zeros(0)
+        return tuple(np.concatenate([p[k] for p in parts]) for k in range(3))
 
 
 def bin_weights():

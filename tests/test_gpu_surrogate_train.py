@@ -81,3 +81,71 @@ def test_gauss_newton_recovers_r_eff_on_network_brfs(trained):
     assert np.median(err) < 0.01, np.median(err)
     assert np.all(np.isfinite(s)) and np.all(s >= math.log(50) - 1e-9)
     assert np.all(np.isfinite(spread)) and np.all(np.isfinite(spread_r)) and np.all(spread_r >= 0)
+
+
+@pytest.mark.parametrize('n,members,weighted', [(1, 1, True), (33, 3, False), (130, 5, True)])
+def test_brf_kernels_match_numpy(n, members, weighted):
+    """Members' BRFs, their mean and spread, grid costs, Gauss-Newton sums and spreads of log r_eff
+    from random outputs against the array arithmetic, NaN kept where it arises."""
+    import torch
+    from monte_carlompi_gb300 import _abi
+    g = torch.Generator().manual_seed(n + members)
+    L, st = _abi.load(), surrogate._stream(torch)
+    pitch, bins = 656, surrogate.N_BRF
+    ys = (torch.randn(members, n, pitch, generator=g)).half().cuda()
+    y, yd = torch.randn(members, n, 652, generator=g).cuda(), torch.randn(members, n, 652, generator=g).cuda()
+    ys[0, n - 1, 5] = float('nan')
+    mean, std = (torch.randn(members, 649, generator=g) * 0.1).double(), (torch.rand(members, 649, generator=g) * 0.3).double()
+    obs = torch.rand(n, bins, generator=g).double()
+    share = surrogate.bin_weights()
+    photons, rel = (1e6, 0.01) if weighted else (0.0, 0.0)
+    new = lambda *shape: torch.empty(shape, dtype=torch.float64, device='cuda')  # noqa: E731
+    p = lambda t: t.data_ptr()  # noqa: E731
+    md, sd, od, wd = mean.cuda(), std.cuda(), obs.cuda(), torch.from_numpy(share).cuda()
+    brf, alb, mu, am, sp = new(members, n, bins), new(members, n), new(n, bins), new(n), new(n)
+    cost, f, j, v, sums = new(n), new(n, bins), new(n, bins), new(n, bins), new(2, n)
+    spread, sigma = new(n), new(n)
+    fl = surrogate.BRF_FLOOR
+    assert L.mcw_brf_members(p(ys), pitch, members, n, p(md), p(sd), fl, p(brf), p(alb), st) == 0
+    assert L.mcw_brf_stats(p(brf), p(alb), members, n, p(wd), p(mu), p(am), p(sp), st) == 0
+    assert L.mcw_brf_cost(p(ys), pitch, members, 1, n, p(md), p(sd), fl, p(od), p(wd), photons, rel, p(cost), st) == 0
+    assert L.mcw_brf_jacobian(p(y), p(yd), 652, members, n, p(md), p(sd), fl, p(f), p(j), p(v), p(od), p(wd), photons,
+                              rel, p(sums[0]), p(sums[1]), st) == 0
+    assert L.mcw_brf_logr(p(brf), p(mu), members, n, p(f), p(j), p(v), p(wd), photons, rel, p(spread), p(sigma), st) == 0
+    torch.cuda.synchronize()
+    o = ys[:, :, :649].cpu().double().numpy() * std.numpy()[:, None] + mean.numpy()[:, None]
+    rb, ra = zip(*[surrogate.from_target(q) for q in o])
+    rb, ra = np.stack(rb), np.stack(ra)
+    ok = dict(rtol=1e-11, atol=1e-13, equal_nan=True)
+    assert np.allclose(brf.cpu(), rb, **ok) and np.allclose(alb.cpu(), ra, **ok)
+    m = rb.mean(0)
+    assert np.allclose(mu.cpu(), m, **ok) and np.allclose(am.cpu(), ra.mean(0), **ok)
+    assert np.allclose(sp.cpu(), np.sqrt((rb.std(0) ** 2 * share).sum(1) / (m ** 2 * share).sum(1)), **ok)
+    on = obs.numpy()
+    w0 = 1 / inverse.noise_variance(on, photons, rel) if weighted else share[None]
+    assert np.allclose(cost.cpu(), (w0 * (m - on) ** 2).sum(1), **ok)
+    yp = y[:, :, :649].cpu().double().numpy() * std.numpy()[:, None] + mean.numpy()[:, None]
+    dp = yd[:, :, :649].cpu().double().numpy() * std.numpy()[:, None]
+    a, shape = np.exp(yp[..., bins:]), np.exp(yp[..., :bins])
+    fm = (shape - fl) * a
+    jm = shape * dp[..., :bins] * a + (shape - fl) * (a * dp[..., bins:])
+    rf, rj = fm.mean(0), jm.mean(0)
+    rv = np.maximum((fm ** 2).mean(0) - rf ** 2, 0)
+    assert np.allclose(f.cpu(), rf, **ok) and np.allclose(j.cpu(), rj, **ok)
+    assert np.allclose(v.cpu(), rv, rtol=1e-6, atol=1e-13)
+    vk = v.cpu().numpy()
+    w = 1 / inverse.noise_variance(rf, photons, rel, vk) if weighted else np.broadcast_to(share[None], rf.shape)
+    wn = 1 / inverse.noise_variance(rf, photons, rel) if weighted else share[None]
+    assert np.allclose(sums[0].cpu(), (w * rj * (rf - on)).sum(1), rtol=1e-9, atol=1e-9 * np.abs(w * rj * rf).sum(1).max())
+    assert np.allclose(sums[1].cpu(), (w * rj * rj).sum(1), rtol=1e-9)
+    got = spread.cpu().numpy()
+    assert np.allclose(got, inverse.logr_spread(rb, rj, w), rtol=1e-8, atol=1e-13, equal_nan=True)
+    assert np.allclose(sigma.cpu(), 1 / np.sqrt((wn * rj * rj).sum(1)), rtol=1e-9)
+
+
+def test_retrieval_refuses_arrays_of_other_shapes(trained):
+    ens = trained[0]
+    for obs, known in ((np.ones((4, 640)), np.ones((4, 3))), (np.ones((4, 648)), np.ones((3, 3))),
+                       (np.ones((4, 648)), np.ones((4, 2)))):
+        with pytest.raises(ValueError):
+            inverse.surrogate_gn(ens, obs, known)
