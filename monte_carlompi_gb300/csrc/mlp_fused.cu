@@ -10,27 +10,25 @@
 //    chunk signalled through its slot's mbarrier transaction count;
 //  * warp 9 (MMA) owns the tensor memory and issues tcgen05.mma (M = 128, K-major
 //    core-matrix operands, no swizzle) from shared memory into it: layer 1 (K = 4
-//    zero-padded to 16) and layers 2 and 3 with N = 256, the output layer as six
-//    N = 128 blocks ping-ponging between the two halves of the accumulator;
+//    zero-padded to 16) and layers 2 and 3 with N = 256, the output layer as five
+//    N = 128 blocks and one of N = 16 (columns 640 .. 655; its weights are copied for those
+//    alone), ping-ponging between the two halves of the accumulator;
 //  * warps 0-7 write the input tile and run the epilogues: hidden layers (bias,
 //    SiLU, bf16) write the next layer's A operand back into the 64 KB activation
-//    tile, so activations never leave shared memory; output blocks are transposed
-//    8 rows at a time through a small per-warp stage so that every output row is
-//    written as whole 128-byte runs (a warp's 16-byte stores cover 4 rows x 128 B).
+//    tile, so activations never leave shared memory; fp16 output rows leave as 32-byte stores
+//    from registers (f32 ones, and rows off 32-byte boundaries, 8 rows at a time through a
+//    small stage per warp as whole 128-byte runs).
 //    Epilogue warp w reads accumulator lanes 32 (w % 4) .. +31 (its rows).
 // Hand-offs are mbarriers: ring full/empty, accumulator full (tcgen05.commit) and
 // empty, activation tile ready.  Every wait is bounded by %globaltimer (2 s) and
 // checks a CTA-wide abort flag; a timeout sets bit 1 of the error flag read by
 // mcw_mlp_status, lets copies and MMAs in flight finish (bounded), frees the tensor
 // memory and leaves.
-#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <cstring>
-#include <mutex>
 
 #include "../../include/mcw_mlp.h"
 
@@ -48,28 +46,17 @@ constexpr int FK1 = 16;                 // layer-1 K, zero-padded
 #ifndef MCW_FUSED_SLOTS
 #define MCW_FUSED_SLOTS 2
 #endif
-#ifndef MCW_FUSED_EPI_WARPS
-#define MCW_FUSED_EPI_WARPS 8
-#endif
-#ifndef MCW_FUSED_TILES
-#define MCW_FUSED_TILES 1
-#endif
-#ifndef MCW_FUSED_CTAS_PER_SM
-#define MCW_FUSED_CTAS_PER_SM (MCW_FUSED_TILES == 1 ? 2 : 1)
-#endif
 constexpr int kSlots = MCW_FUSED_SLOTS;              // weight ring depth
-constexpr int kEpiWarps = MCW_FUSED_EPI_WARPS;       // 8 or 16
-constexpr int kCtasPerSm = MCW_FUSED_CTAS_PER_SM;
-// 128-row tiles a CTA carries at once, each with its own accumulator and activation
-// tile: the MMAs of one tile's next layer run while the other tile's epilogue does
-constexpr int kTiles = MCW_FUSED_TILES;
-static_assert(kTiles == 1 || kTiles == 2, "one or two tiles per CTA");
+constexpr int kEpiWarps = 8;
+constexpr int kCtasPerSm = 2;
 constexpr int kGroups = kEpiWarps / 4;               // column groups per accumulator lane quarter
 constexpr int kProducerWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1;
 constexpr int kThreads = 32 * (kEpiWarps + 2);
 constexpr int kEpiThreads = 32 * kEpiWarps;
 constexpr int kOutN = 128;                            // output block width
 constexpr int kOutBlocks = (FO + kOutN - 1) / kOutN;  // 6
+constexpr int kLastN = 16;                            // the last block's columns that exist, rounded up
+static_assert(FO - (kOutBlocks - 1) * kOutN <= kLastN, "last output block");
 // weight chunks, in the order the MMA warp consumes them
 constexpr int kHidK = 32;                             // k per hidden-layer chunk (256 rows)
 constexpr int kOutK = 64;                             // k per output chunk (128 rows)
@@ -84,14 +71,6 @@ constexpr int kRingBytes = kSlots * kChunkBytes;
 constexpr int kStagePitch = 36 * 4;                   // stage row: 32 floats + 16 B pad (no bank conflicts)
 constexpr int kStageWarp = 8 * kStagePitch;           // 8 rows per warp
 constexpr int kStageBytes = kEpiWarps * kStageWarp < 4096 ? 4096 : kEpiWarps * kStageWarp;
-#ifndef MCW_FUSED_TMA_OUT
-#define MCW_FUSED_TMA_OUT 1
-#endif
-// fp16 output through tensor stores: a warp's stage is 1 KB (8 rows x 128 bytes in the
-// tensor map's 128-byte swizzle), 1024-byte aligned; columns [0, kTmaCols) go through the
-// tensor map, the ragged rest (640 .. 648) through plain stores
-constexpr int kStageTma = 1024;
-constexpr int kTmaCols = (FO / 64) * 64;
 // biases in shared memory: b1, b2, b3 (256 each), b4 zero-padded to the six 128-column blocks
 constexpr int kB4Pad = 6 * 128;
 constexpr int kBiasFloats = 3 * 256 + kB4Pad;
@@ -99,10 +78,9 @@ constexpr int kBiasBytes = kBiasFloats * 4;
 constexpr int kHidCols = FH / kGroups;                // hidden columns per epilogue warp
 constexpr int kOutCols = kOutN / kGroups;             // output-block columns per epilogue warp
 static_assert(kEpiWarps % 4 == 0 && kHidCols % 32 == 0 && kOutCols % 32 == 0, "epilogue split");
-static_assert(kTiles * kActBytes + kRingBytes + kStageBytes + kBiasBytes <= 227 * 1024, "shared memory");
-constexpr size_t kSmemBytes = (size_t)kTiles * kActBytes + kRingBytes + kStageBytes + kBiasBytes;
-constexpr uint32_t kTmemCols = 256 * kTiles;
-constexpr int kSeqChunks = kTiles * kNumChunks;       // weight chunks a CTA consumes
+static_assert(kActBytes + kRingBytes + kStageBytes + kBiasBytes <= 227 * 1024, "shared memory");
+constexpr size_t kSmemBytes = (size_t)kActBytes + kRingBytes + kStageBytes + kBiasBytes;
+constexpr uint32_t kTmemCols = 256;
 constexpr unsigned long long kWaitNs = 2000000000ull;
 constexpr uint32_t kSuspendNs = 1000000;              // a waiting thread sleeps until the phase completes or 1 ms
 // F32 += BF16 x BF16, both K-major; N >> 3 in bits 17-22, M >> 4 in bits 24-28
@@ -112,21 +90,12 @@ __host__ __device__ constexpr uint32_t idesc(int n) {
 
 static_assert(kHidK * FH * 2 == kChunkBytes && kOutK * kOutN * 2 == kChunkBytes, "chunk sizes");
 static_assert(kW1Bytes + (kNumChunks - 1) * kChunkBytes == MCW_MLP_PACK_BYTES, "packed blob layout");
-static_assert(kTiles * kXBytes <= kStageBytes, "the input tiles live in the stage region");
-static_assert(kEpiWarps * kStageTma <= kStageBytes && (kTiles * kActBytes + kRingBytes) % 1024 == 0,
-              "tensor-store stages: 1 KB per epilogue warp, 1024-byte aligned");
-
-// The i-th weight chunk a CTA consumes: per layer the chunks of tile 0, then those of
-// tile 1 (the order in which the MMA warp issues the layers of its tiles).
-__host__ __device__ constexpr int chunk_at(int i) {
-    return i < kTiles ? 0
-         : i < kTiles * (1 + kHidChunks) ? 1 + (i - kTiles) % kHidChunks
-         : i < kTiles * (1 + 2 * kHidChunks) ? 1 + kHidChunks + (i - kTiles * (1 + kHidChunks)) % kHidChunks
-         : 1 + 2 * kHidChunks + (i - kTiles * (1 + 2 * kHidChunks)) % (kOutBlocks * kOutChunks);
-}
-
+static_assert(kXBytes <= kStageBytes, "the input tile lives in the stage region");
 __host__ __device__ constexpr size_t chunk_offset(int i) { return i == 0 ? 0 : kW1Bytes + (size_t)(i - 1) * kChunkBytes; }
-__host__ __device__ constexpr uint32_t chunk_bytes(int i) { return i == 0 ? kW1Bytes : kChunkBytes; }
+// (of the last output block only the rows of its first kLastN columns are copied)
+__host__ __device__ constexpr uint32_t chunk_bytes(int i) {
+    return i == 0 ? kW1Bytes : (i >= kNumChunks - kOutChunks ? kLastN * kOutK * 2 : kChunkBytes);
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -144,28 +113,18 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-#ifndef MCW_FUSED_SILU_TANH
-#define MCW_FUSED_SILU_TANH 1
-#endif
-__device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.f + __expf(-z)); }
-
 __device__ __forceinline__ float tanh_approx(float x) {
     float y;
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
-// SiLU of a pair of pre-activations.  With MCW_FUSED_SILU_TANH (the default):
-// z sigmoid(z) = h + h tanh(h), h = z / 2, one hardware tanh per value (relative
-// error about 2^-11, below the bf16 rounding of the stored activation) and packed
-// FP32 pair operations; otherwise z / (1 + exp(-z)) per value.
+// SiLU of a pair of pre-activations: z sigmoid(z) = h + h tanh(h), h = z / 2, one hardware
+// tanh per value (relative error about 2^-11, below the bf16 rounding of the stored
+// activation) and packed FP32 pair operations.
 __device__ __forceinline__ float2 silu2(const float2 z) {
-#if MCW_FUSED_SILU_TANH
     const float2 h = __fmul2_rn(z, make_float2(0.5f, 0.5f));
     return __ffma2_rn(h, make_float2(tanh_approx(h.x), tanh_approx(h.y)), h);
-#else
-    return make_float2(silu(z.x), silu(z.y));
-#endif
 }
 
 // Byte offset of element (row, k) in a K-major core-matrix tile whose rows are kdim long.
@@ -451,44 +410,31 @@ __device__ __forceinline__ void epilogue_out_half(uint32_t tlane, int blk, const
     __syncwarp();
 }
 
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n"
-                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y) : "memory");
-}
-// A tensor store of the ensemble's output map {columns, rows, member}: box {64, 8, 1}.
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, uint32_t src, int x, int y, int z) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];\n"
-                 :: "l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y), "r"(z) : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
-// the thread's tensor stores have read their shared-memory sources
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
-// the thread's tensor stores are complete
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
-
-// fp16 output through tensor stores: this warp's 64 columns, 8 rows at a time through its
-// 1 KB stage (16-byte chunk c of row r at r * 128 + (c ^ r) * 16, the map's 128-byte
-// swizzle, so the stage writes are free of bank conflicts), one tensor store per 8 rows
-// issued by lane 0; the warp goes on while the store drains.  The ragged block
-// (columns 640 .. 648) is written with plain stores from the same stage.
-template <bool kEnsemble>
-__device__ __forceinline__ void epilogue_out_half_tma(uint32_t tlane, int blk, const float *b4, unsigned char *stage,
-                                                      const CUtensorMap *ymap, __half *y, int ldy, int m, int row0,
-                                                      int member, int group, int lane) {
-    static_assert(kOutCols == 64, "tensor stores: 64 columns (128 bytes) per warp");
+// fp16 output by direct stores: a lane's row of 64 columns is 128 contiguous bytes, written as four
+// 32-byte stores, whole sectors, straight from registers.  Rows 32-byte aligned (y and its pitch).
+// The ragged block (columns 640 .. 648) goes out one value at a time.  (Through a 1 KB stage per warp
+// and tensor stores of 8 rows, every 8 rows waited for the copy before: 65,536 rows of one network 65
+// us, now 60, 300 rows 28, now 22.)
+__device__ __forceinline__ void epilogue_out_half_direct(uint32_t tlane, int blk, const float *b4, __half *y, int ldy,
+                                                         int m, int row0, int group, int lane) {
+    static_assert(kOutCols == 64, "64 columns (128 bytes) per lane");
     const int c0 = group * kOutCols;
     const int nb = blk * kOutN + c0;
     if (nb >= FO) return;
-    uint32_t hp[32];
+    const bool ok = row0 + lane < m;
+    __half *dst = y + (size_t)(row0 + lane) * ldy + nb;
     // both 32-column loads in flight before the one wait
     uint32_t ra[2][32];
     tmem_ld32_issue(tlane + (uint32_t)c0, ra[0]);
-    tmem_ld32_issue(tlane + (uint32_t)(c0 + 32), ra[1]);
+    const bool full = nb + kOutCols <= FO;
+    if (full) tmem_ld32_issue(tlane + (uint32_t)(c0 + 32), ra[1]);
     tmem_ld_wait(ra[0]);
-    tmem_ld_wait(ra[1]);
+    if (full) tmem_ld_wait(ra[1]);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
+        if (h == 1 && !full) break;
         const uint32_t (&v)[32] = ra[h];
+        uint32_t hp[16];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             const float4 b = *reinterpret_cast<const float4 *>(b4 + nb + 32 * h + 4 * q);
@@ -498,51 +444,31 @@ __device__ __forceinline__ void epilogue_out_half_tma(uint32_t tlane, int blk, c
                                          make_float2(b.z, b.w));
             const __half2 lo = __floats2half2_rn(zl.x, zl.y);
             const __half2 hi = __floats2half2_rn(zh.x, zh.y);
-            hp[16 * h + 2 * q] = *reinterpret_cast<const uint32_t *>(&lo);
-            hp[16 * h + 2 * q + 1] = *reinterpret_cast<const uint32_t *>(&hi);
+            hp[2 * q] = *reinterpret_cast<const uint32_t *>(&lo);
+            hp[2 * q + 1] = *reinterpret_cast<const uint32_t *>(&hi);
         }
-    }
-    const bool full = nb + kOutCols <= kTmaCols;
-    const int r = lane & 7;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        if (lane == 0) bulk_wait_read();          // the stage's last tensor store has read it
-        __syncwarp();
-        if ((lane >> 3) == p) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                *reinterpret_cast<uint4 *>(stage + r * 128 + ((q ^ r) << 4)) =
-                    make_uint4(hp[4 * q], hp[4 * q + 1], hp[4 * q + 2], hp[4 * q + 3]);
-        }
-        const int rbase = row0 + 8 * p;
         if (full) {
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-                if (kEnsemble)
-                    tma_store_3d(ymap, smem_u32(stage), nb, rbase, member);
-                else
-                    tma_store_2d(ymap, smem_u32(stage), nb, rbase);
-                bulk_commit();
-            }
-        } else {
-            __syncwarp();
-            if (nb + lane < FO) {
+            if (ok) {
 #pragma unroll
-                for (int rr = 0; rr < 8; ++rr)
-                    if (rbase + rr < m)
-                        y[(size_t)(rbase + rr) * ldy + nb + lane] = *reinterpret_cast<const __half *>(
-                            stage + rr * 128 + (((lane >> 3) ^ rr) << 4) + (lane & 7) * 2);
+                for (int q = 0; q < 2; ++q)
+                    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+                                 :: "l"(dst + 32 * h + 16 * q), "r"(hp[8 * q]), "r"(hp[8 * q + 1]), "r"(hp[8 * q + 2]),
+                                    "r"(hp[8 * q + 3]), "r"(hp[8 * q + 4]), "r"(hp[8 * q + 5]), "r"(hp[8 * q + 6]),
+                                    "r"(hp[8 * q + 7])
+                                 : "memory");
             }
+        } else if (ok) {
+#pragma unroll
+            for (int c = 0; c < FO - (kOutBlocks - 1) * kOutN; ++c)
+                dst[c] = __ushort_as_half((unsigned short)(hp[c >> 1] >> ((c & 1) * 16)));
         }
     }
-    __syncwarp();
 }
 
 struct Bars {
     uint64_t full[kSlots], empty[kSlots];   // weight ring
-    uint64_t accf[kTiles][2], acce[kTiles][2];  // accumulator halves per tile: full (MMA -> epilogue), empty
-    uint64_t act[kTiles];         // input / activation tile written (epilogue -> MMA)
+    uint64_t accf[2], acce[2];              // accumulator halves: full (MMA -> epilogue), empty
+    uint64_t act;                 // input / activation tile written (epilogue -> MMA)
     uint64_t fin;                 // every MMA of the CTA complete
 };
 
@@ -551,13 +477,13 @@ struct Bars {
 template <bool kHalf, bool kEnsemble>
 __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const float *b1, const float *b2,
                                                const float *b3, const float *b4, const unsigned char *blob, void *y,
-                                               int ldy, unsigned int *err, const CUtensorMap *ymap, int use_tma,
+                                               int ldy, unsigned int *err, int wide,
                                                int tiles, int bias_stride, long long blob_stride) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *act0 = smem;                                  // 64 KB activation tile per tile
-    unsigned char *ring = smem + kTiles * kActBytes;             // 2 x 16 KB weight chunks
-    unsigned char *stage_all = ring + kRingBytes;                // 16 KB output stage ...
-    unsigned char *xt0 = stage_all;                              // ... and, for layer 1, the input tiles
+    unsigned char *act = smem;                                   // 64 KB activation tile
+    unsigned char *ring = smem + kActBytes;                      // 16 KB weight chunks
+    unsigned char *stage_all = ring + kRingBytes;                // output stage ...
+    unsigned char *xt = stage_all;                               // ... and, for layer 1, the input tile
     float *sbias = reinterpret_cast<float *>(stage_all + kStageBytes);   // b1 | b2 | b3 | b4 (padded)
     __shared__ __align__(8) Bars bars;
     __shared__ uint32_t tmem_slot;
@@ -568,7 +494,7 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
     // (blockIdx.x / tiles), whose biases lie bias_stride floats and whose packed weights
     // blob_stride bytes after the previous member's, its output rows m * ldy after them
     // (member is recomputed where it is used, so it holds no register through the kernel)
-    const int m0 = (kEnsemble ? (int)blockIdx.x % tiles : (int)blockIdx.x) * FM * kTiles;
+    const int m0 = (kEnsemble ? (int)blockIdx.x % tiles : (int)blockIdx.x) * FM;
 
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n"
@@ -581,13 +507,11 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
             bar_init(&bars.full[i], 1);
             bar_init(&bars.empty[i], 1);
         }
-        for (int t = 0; t < kTiles; ++t) {
-            for (int i = 0; i < 2; ++i) {
-                bar_init(&bars.accf[t][i], 1);
-                bar_init(&bars.acce[t][i], kEpiThreads);
-            }
-            bar_init(&bars.act[t], kEpiThreads);
+        for (int i = 0; i < 2; ++i) {
+            bar_init(&bars.accf[i], 1);
+            bar_init(&bars.acce[i], kEpiThreads);
         }
+        bar_init(&bars.act, kEpiThreads);
         bar_init(&bars.fin, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n");
     }
@@ -597,109 +521,91 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
     if (warp == kProducerWarp) {
-        {
-            int issued = 0;
-            for (int i = 0; i < kSeqChunks; ++i) {
-                const int slot = i % kSlots;
-                if (i >= kSlots && !warp_wait(&bars.empty[slot], (uint32_t)(i / kSlots - 1) & 1u, abort)) break;
-                const int c = chunk_at(i);
-                if (elect_one())
-                    load_chunk(ring + slot * kChunkBytes,
-                               blob + (kEnsemble ? (size_t)((int)blockIdx.x / tiles) * (size_t)blob_stride : 0) +
-                                   chunk_offset(c),
-                               chunk_bytes(c), &bars.full[slot]);
-                __syncwarp();
-                issued = i + 1;
-            }
-            // the last copy into each slot has landed before the CTA can leave
-            for (int i = issued - kSlots < 0 ? 0 : issued - kSlots; i < issued; ++i)
-                wait_bar(&bars.full[i % kSlots], (uint32_t)(i / kSlots) & 1u, nullptr);
+        int issued = 0;
+        for (int i = 0; i < kNumChunks; ++i) {
+            const int slot = i % kSlots;
+            if (i >= kSlots && !warp_wait(&bars.empty[slot], (uint32_t)(i / kSlots - 1) & 1u, abort)) break;
+            if (elect_one())
+                load_chunk(ring + slot * kChunkBytes,
+                           blob + (kEnsemble ? (size_t)((int)blockIdx.x / tiles) * (size_t)blob_stride : 0) +
+                               chunk_offset(i),
+                           chunk_bytes(i), &bars.full[slot]);
+            __syncwarp();
+            issued = i + 1;
         }
+        // the last copy into each slot has landed before the CTA can leave
+        for (int i = issued - kSlots < 0 ? 0 : issued - kSlots; i < issued; ++i)
+            wait_bar(&bars.full[i % kSlots], (uint32_t)(i / kSlots) & 1u, nullptr);
     } else if (warp == kMmaWarp) {
-        {
-            const uint32_t ring_a = smem_u32(ring);
-            int chunk = 0;
-            uint32_t act_phase[kTiles];
-            for (int t = 0; t < kTiles; ++t) act_phase[t] = 0u;
-            bool ok = true;
-            auto take = [&](void) -> uint32_t {      // wait for the next chunk; its shared address
-                const int slot = chunk % kSlots;
-                ok = ok && warp_wait(&bars.full[slot], (uint32_t)(chunk / kSlots) & 1u, abort);
-                asm volatile("tcgen05.fence::after_thread_sync;\n");
-                return ring_a + (uint32_t)slot * kChunkBytes;
-            };
-            auto release = [&](void) {               // chunk's MMAs issued: free its slot when they finish
-                if (elect_one()) commit(&bars.empty[chunk % kSlots]);
-                __syncwarp();
-                ++chunk;
-            };
-            auto done = [&](uint64_t *bar) {         // arrive when the MMAs issued so far are complete
-                if (elect_one()) commit(bar);
-                __syncwarp();
-            };
-            auto wait_act = [&](int t) {             // tile t's input / activations written
-                ok = ok && warp_wait(&bars.act[t], act_phase[t], abort);
-                act_phase[t] ^= 1u;
-                asm volatile("tcgen05.fence::after_thread_sync;\n");
-            };
-            // layer 1 of each tile: input tile x W1
-            for (int t = 0; t < kTiles && ok; ++t) {
-                wait_act(t);
-                if (!ok) break;
+        const uint32_t ring_a = smem_u32(ring), act_a = smem_u32(act);
+        int chunk = 0;
+        uint32_t act_phase = 0u;
+        bool ok = true;
+        auto take = [&](void) -> uint32_t {      // wait for the next chunk; its shared address
+            const int slot = chunk % kSlots;
+            ok = ok && warp_wait(&bars.full[slot], (uint32_t)(chunk / kSlots) & 1u, abort);
+            asm volatile("tcgen05.fence::after_thread_sync;\n");
+            return ring_a + (uint32_t)slot * kChunkBytes;
+        };
+        auto release = [&](void) {               // chunk's MMAs issued: free its slot when they finish
+            if (elect_one()) commit(&bars.empty[chunk % kSlots]);
+            __syncwarp();
+            ++chunk;
+        };
+        auto done = [&](uint64_t *bar) {         // arrive when the MMAs issued so far are complete
+            if (elect_one()) commit(bar);
+            __syncwarp();
+        };
+        auto wait_act = [&](void) {              // the input / activations written
+            ok = ok && warp_wait(&bars.act, act_phase, abort);
+            act_phase ^= 1u;
+            asm volatile("tcgen05.fence::after_thread_sync;\n");
+        };
+        // layer 1: input tile x W1
+        wait_act();
+        if (ok) {
+            const uint32_t w = take();
+            if (ok) {
+                mma_steps<FK1, FK1, 1>(tmem, smem_u32(xt), 0, w, idesc(FH), false);
+                release();
+                done(&bars.accf[0]);
+            }
+        }
+        // layers 2 and 3: eight chunks of 32 k each
+        for (int layer = 0; layer < 2 && ok; ++layer) {
+            wait_act();
+            for (int c = 0; c < kHidChunks && ok; ++c) {
                 const uint32_t w = take();
                 if (!ok) break;
-                mma_steps<FK1, FK1, 1>(tmem + (uint32_t)(t * 256), smem_u32(xt0 + t * kXBytes), 0, w, idesc(FH), false);
+                mma_steps<FH, kHidK, kHidK / 16>(tmem, act_a, c * (kHidK / 16), w, idesc(FH), c > 0);
                 release();
-                done(&bars.accf[t][0]);
             }
-            // layers 2 and 3: eight chunks of 32 k each, tile by tile (one tile's MMAs run
-            // while the other's epilogue writes its activations)
-            for (int layer = 0; layer < 2 && ok; ++layer) {
-                for (int t = 0; t < kTiles && ok; ++t) {
-                    wait_act(t);
-                    const uint32_t act_a = smem_u32(act0 + t * kActBytes);
-                    for (int c = 0; c < kHidChunks && ok; ++c) {
-                        const uint32_t w = take();
-                        if (!ok) break;
-                        mma_steps<FH, kHidK, kHidK / 16>(tmem + (uint32_t)(t * 256), act_a, c * (kHidK / 16), w,
-                                                         idesc(FH), c > 0);
-                        release();
-                    }
-                    if (ok) done(&bars.accf[t][0]);
-                }
-            }
-            // output layer: six 128-column blocks per tile alternating between the halves
-            // of the tile's accumulator
-            for (int t = 0; t < kTiles && ok; ++t) {
-                wait_act(t);
-                const uint32_t act_a = smem_u32(act0 + t * kActBytes);
-                for (int j = 0; j < kOutBlocks && ok; ++j) {
-                    const int h = j & 1;
-                    if (j >= 2) {
-                        ok = warp_wait(&bars.acce[t][h], (uint32_t)((j >> 1) - 1) & 1u, abort);
-                        asm volatile("tcgen05.fence::after_thread_sync;\n");
-                        if (!ok) break;
-                    }
-                    for (int c = 0; c < kOutChunks && ok; ++c) {
-                        const uint32_t w = take();
-                        if (!ok) break;
-                        mma_steps<FH, kOutK, kOutK / 16>(tmem + (uint32_t)(t * 256 + h * kOutN), act_a,
-                                                         c * (kOutK / 16), w, idesc(kOutN), c > 0);
-                        release();
-                    }
-                    if (ok) done(&bars.accf[t][h]);
-                }
-            }
-            // every MMA issued by this thread has completed before the memory is freed
-            done(&bars.fin);
-            wait_bar(&bars.fin, 0, nullptr);
+            if (ok) done(&bars.accf[0]);
         }
+        // output layer: six blocks alternating between the halves of a tile's accumulator
+        if (ok) wait_act();
+        for (int j = 0; j < kOutBlocks && ok; ++j) {
+            const int h = j & 1;
+            if (j >= 2) {
+                ok = warp_wait(&bars.acce[h], (uint32_t)((j >> 1) - 1) & 1u, abort);
+                asm volatile("tcgen05.fence::after_thread_sync;\n");
+            }
+            const uint32_t id = j == kOutBlocks - 1 ? idesc(kLastN) : idesc(kOutN);
+            for (int c = 0; c < kOutChunks && ok; ++c) {
+                const uint32_t w = take();
+                if (!ok) break;
+                mma_steps<FH, kOutK, kOutK / 16>(tmem + (uint32_t)(h * kOutN), act_a, c * (kOutK / 16), w, id, c > 0);
+                release();
+            }
+            if (ok) done(&bars.accf[h]);
+        }
+        // every MMA issued by this warp has completed before the memory is freed
+        done(&bars.fin);
+        wait_bar(&bars.fin, 0, nullptr);
     } else {
         // epilogue warps
         const int quarter = warp & 3, group = warp >> 2;   // lane quarter, column group
         unsigned char *stage = stage_all + warp * kStageWarp;
-        uint32_t accf_phase[kTiles][2];
-        for (int t = 0; t < kTiles; ++t) accf_phase[t][0] = accf_phase[t][1] = 0u;
         // biases into shared memory (b4 zero past column 648), then the epilogue warps meet
         {
             const size_t bo = kEnsemble ? (size_t)((int)blockIdx.x / tiles) * (size_t)bias_stride : 0;
@@ -713,53 +619,48 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
             }
         }
         asm volatile("bar.sync 1, %0;\n" :: "n"(kEpiThreads) : "memory");
-        for (int t = 0; t < kTiles; ++t) {
-            if (threadIdx.x < FM) {
-                const int r = threadIdx.x, gm = m0 + t * FM + r;
+        {
+            const int r = threadIdx.x, gm = m0 + r;
+            if (r < FM) {
                 float xin[FIN];
 #pragma unroll
                 for (int k = 0; k < FIN; ++k) xin[k] = gm < m ? x[(size_t)gm * FIN + k] : 0.f;
                 const __nv_bfloat162 p0 = __floats2bfloat162_rn(xin[0], xin[1]);
                 const __nv_bfloat162 p1 = __floats2bfloat162_rn(xin[2], xin[3]);
-                unsigned char *xt = xt0 + t * kXBytes;
                 *reinterpret_cast<uint4 *>(xt + core_off(r, 0, FK1)) = make_uint4(
                     *reinterpret_cast<const uint32_t *>(&p0), *reinterpret_cast<const uint32_t *>(&p1), 0u, 0u);
                 *reinterpret_cast<uint4 *>(xt + core_off(r, 8, FK1)) = make_uint4(0u, 0u, 0u, 0u);
             }
             asm volatile("fence.proxy.async.shared::cta;\n");
-            arrive(&bars.act[t]);
-        }
-        const float *hb[3] = {sbias, sbias + 256, sbias + 512};
-        bool ok = true;
-        for (int layer = 0; layer < 3 && ok; ++layer) {
-            for (int t = 0; t < kTiles && ok; ++t) {
-                ok = wait_bar(&bars.accf[t][0], accf_phase[t][0], abort);
-                accf_phase[t][0] ^= 1u;
+            arrive(&bars.act);
+            const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16);
+            uint32_t accf_phase[2] = {0u, 0u};
+            bool ok = true;
+            for (int layer = 0; layer < 3 && ok; ++layer) {
+                ok = wait_bar(&bars.accf[0], accf_phase[0], abort);
+                accf_phase[0] ^= 1u;
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
-                const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * 256);
-                epilogue_hidden(tlane, hb[layer], act0 + t * kActBytes, quarter, group, lane);
+                epilogue_hidden(tlane, sbias + 256 * layer, act, quarter, group, lane);
                 asm volatile("fence.proxy.async.shared::cta;\n");
                 asm volatile("tcgen05.fence::before_thread_sync;\n");
-                arrive(&bars.act[t]);
+                arrive(&bars.act);
             }
-        }
-        for (int t = 0; t < kTiles && ok; ++t) {
-            const uint32_t tlane = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * 256);
-            const int row0 = m0 + t * FM + quarter * 32;
+            const int row0 = m0 + quarter * 32;
             for (int j = 0; j < kOutBlocks && ok; ++j) {
                 const int h = j & 1;
-                ok = wait_bar(&bars.accf[t][h], accf_phase[t][h], abort);
-                accf_phase[t][h] ^= 1u;
+                ok = wait_bar(&bars.accf[h], accf_phase[h], abort);
+                accf_phase[h] ^= 1u;
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
                 // this member's output rows (plain stores; the tensor map takes the member as a coordinate)
                 const int member = kEnsemble ? (int)blockIdx.x / tiles : 0;
                 const size_t yoff = kEnsemble ? (size_t)member * (size_t)m * (size_t)ldy : 0;
-                if (kHalf && use_tma)
-                    epilogue_out_half_tma<kEnsemble>(tlane + (uint32_t)(h * kOutN), j, sbias + 768,
-                                                     stage_all + warp * kStageTma,
-                                          ymap, static_cast<__half *>(y) + yoff, ldy, m, row0, member, group, lane);
+                if (kHalf && wide)
+                    epilogue_out_half_direct(tlane + (uint32_t)(h * kOutN), j, sbias + 768,
+                                             static_cast<__half *>(y) + yoff, ldy, m, row0, group, lane);
                 else if (kHalf)
                     epilogue_out_half(tlane + (uint32_t)(h * kOutN), j, sbias + 768, stage,
                                       static_cast<__half *>(y) + yoff, ldy, m, row0, group, lane);
@@ -767,10 +668,9 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
                     epilogue_out(tlane + (uint32_t)(h * kOutN), j, sbias + 768, stage, static_cast<float *>(y) + yoff,
                                  ldy, m, row0, group, lane);
                 asm volatile("tcgen05.fence::before_thread_sync;\n");
-                arrive(&bars.acce[t][h]);
+                arrive(&bars.acce[h]);
             }
         }
-        if (kHalf && use_tma && lane == 0) bulk_wait_all();   // this warp's tensor stores are done
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;\n");
@@ -788,19 +688,16 @@ template <bool kHalf>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) mlp_fused_kernel(const float *x, int m, const float *b1,
                                                                 const float *b2, const float *b3, const float *b4,
                                                                 const unsigned char *blob, void *y, int ldy,
-                                                                unsigned int *err,
-                                                                const __grid_constant__ CUtensorMap ymap,
-                                                                int use_tma) {
-    mlp_fused_body<kHalf, false>(x, m, b1, b2, b3, b4, blob, y, ldy, err, &ymap, use_tma, (int)gridDim.x, 0, 0);
+                                                                unsigned int *err, int wide) {
+    mlp_fused_body<kHalf, false>(x, m, b1, b2, b3, b4, blob, y, ldy, err, wide, (int)gridDim.x, 0, 0);
 }
 
 // An ensemble: fp16 outputs, tiles CTAs per member (mlp_fused_body).
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) mlp_fused_ensemble_kernel(
         const float *x, int m, const float *b1, const float *b2, const float *b3, const float *b4,
-        const unsigned char *blob, void *y, int ldy, unsigned int *err, const __grid_constant__ CUtensorMap ymap,
-        int use_tma, int tiles, int bias_stride, long long blob_stride) {
-    mlp_fused_body<true, true>(x, m, b1, b2, b3, b4, blob, y, ldy, err, &ymap, use_tma, tiles, bias_stride,
-                               blob_stride);
+        const unsigned char *blob, void *y, int ldy, unsigned int *err, int wide, int tiles, int bias_stride,
+        long long blob_stride) {
+    mlp_fused_body<true, true>(x, m, b1, b2, b3, b4, blob, y, ldy, err, wide, tiles, bias_stride, blob_stride);
 }
 
 // Rows [row0, row0 + rows_out) and k [k0, k0 + kdim) of W [n, k_in] (row-major bf16) as a
@@ -828,40 +725,6 @@ using namespace mcw;
 
 namespace {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    });
-    return fn;
-}
-
-// fp16 output [m, kTmaCols] at row pitch ldy halves, box 64 x 8, and for an ensemble
-// [members, m, kTmaCols] (members m * ldy halves apart), box 64 x 8 x 1, so that a box
-// passing row m - 1 of a member is clipped there; 128-byte swizzle.  False when the
-// driver entry point is missing or the layout breaks a tensor-map rule.
-bool make_out_map(CUtensorMap *map, void *y, int m, int ldy, int members) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn || (reinterpret_cast<uintptr_t>(y) & 15) || (ldy & 7) || ldy < kTmaCols || members < 1) return false;
-    const cuuint32_t rank = members > 1 ? 3 : 2;
-    const cuuint64_t dims[3] = {(cuuint64_t)kTmaCols, (cuuint64_t)m, (cuuint64_t)members};
-    const cuuint64_t strides[2] = {(cuuint64_t)ldy * 2, (cuuint64_t)m * (cuuint64_t)ldy * 2};
-    const cuuint32_t box[3] = {64, 8, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // members networks (1 for one network) on the same inputs: member e's biases bias_stride
 // floats and its packed weights blob_stride bytes after member e - 1's, its outputs at
 // y + e * m * ldy.
@@ -882,21 +745,20 @@ int forward(const float *x, int32_t m, const float *b1, const float *b2, const f
                           : reinterpret_cast<const void *>(mlp_fused_kernel<false>);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return MCW_MLP_ERR_CUDA;
-    const int tiles = (m + FM * kTiles - 1) / (FM * kTiles);
+    const int tiles = (m + FM - 1) / (FM);
     if ((long long)tiles * members > 0x7fffffffLL) return MCW_MLP_ERR_ARG;
     const unsigned grid = (unsigned)(tiles * members);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned char *wb = static_cast<const unsigned char *>(blob);
-    CUtensorMap ymap;
-    memset(&ymap, 0, sizeof(ymap));
-    const int use_tma = (half && MCW_FUSED_TMA_OUT && make_out_map(&ymap, y, m, ldy, members)) ? 1 : 0;
+    // rows on 32-byte boundaries take the 32-byte stores, others (16-byte) go through the stage
+    const int wide = half && (((uintptr_t)y | (uintptr_t)ldy * 2) & 31) == 0;
     if (half && members > 1)
-        mlp_fused_ensemble_kernel<<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, ymap,
-                                                                     use_tma, tiles, bias_stride, blob_stride);
+        mlp_fused_ensemble_kernel<<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, wide, tiles,
+                                                                     bias_stride, blob_stride);
     else if (half)
-        mlp_fused_kernel<true><<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, ymap, use_tma);
+        mlp_fused_kernel<true><<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, wide);
     else
-        mlp_fused_kernel<false><<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, ymap, 0);
+        mlp_fused_kernel<false><<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, 0);
     return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
 }
 
