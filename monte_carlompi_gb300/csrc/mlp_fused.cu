@@ -29,6 +29,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <mutex>
+#include <set>
+#include <utility>
 
 #include "../../include/mcw_mlp.h"
 
@@ -43,12 +46,9 @@ constexpr int FH = MCW_MLP_HIDDEN;      // 256
 constexpr int FO = MCW_MLP_OUT;         // 649
 constexpr int FIN = MCW_MLP_IN;         // 4
 constexpr int FK1 = 16;                 // layer-1 K, zero-padded
-#ifndef MCW_FUSED_SLOTS
-#define MCW_FUSED_SLOTS 2
-#endif
-constexpr int kSlots = MCW_FUSED_SLOTS;              // weight ring depth
+// weight ring depth: what two CTAs per SM leave beside their activations, or one CTA
+constexpr int kSlotsTwo = 2, kSlotsOne = 8;
 constexpr int kEpiWarps = 8;
-constexpr int kCtasPerSm = 2;
 constexpr int kGroups = kEpiWarps / 4;               // column groups per accumulator lane quarter
 constexpr int kProducerWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1;
 constexpr int kThreads = 32 * (kEpiWarps + 2);
@@ -67,7 +67,6 @@ constexpr int kW1Bytes = FH * FK1 * 2;                // 8 KB, chunk 0
 constexpr int kNumChunks = 1 + 2 * kHidChunks + kOutBlocks * kOutChunks;   // 41
 constexpr int kXBytes = FM * FK1 * 2;                 // 4 KB
 constexpr int kActBytes = FM * FH * 2;                // 64 KB
-constexpr int kRingBytes = kSlots * kChunkBytes;
 constexpr int kStagePitch = 36 * 4;                   // stage row: 32 floats + 16 B pad (no bank conflicts)
 constexpr int kStageWarp = 8 * kStagePitch;           // 8 rows per warp
 constexpr int kStageBytes = kEpiWarps * kStageWarp < 4096 ? 4096 : kEpiWarps * kStageWarp;
@@ -78,8 +77,8 @@ constexpr int kBiasBytes = kBiasFloats * 4;
 constexpr int kHidCols = FH / kGroups;                // hidden columns per epilogue warp
 constexpr int kOutCols = kOutN / kGroups;             // output-block columns per epilogue warp
 static_assert(kEpiWarps % 4 == 0 && kHidCols % 32 == 0 && kOutCols % 32 == 0, "epilogue split");
-static_assert(kActBytes + kRingBytes + kStageBytes + kBiasBytes <= 227 * 1024, "shared memory");
-constexpr size_t kSmemBytes = (size_t)kActBytes + kRingBytes + kStageBytes + kBiasBytes;
+constexpr size_t smem_bytes(int slots) { return (size_t)kActBytes + slots * kChunkBytes + kStageBytes + kBiasBytes; }
+static_assert(2 * (smem_bytes(kSlotsTwo) + 1024) <= 228 * 1024 && smem_bytes(kSlotsOne) <= 226 * 1024, "shared memory");
 constexpr uint32_t kTmemCols = 256;
 constexpr unsigned long long kWaitNs = 2000000000ull;
 constexpr uint32_t kSuspendNs = 1000000;              // a waiting thread sleeps until the phase completes or 1 ms
@@ -465,6 +464,7 @@ __device__ __forceinline__ void epilogue_out_half_direct(uint32_t tlane, int blk
     }
 }
 
+template <int kSlots>
 struct Bars {
     uint64_t full[kSlots], empty[kSlots];   // weight ring
     uint64_t accf[2], acce[2];              // accumulator halves: full (MMA -> epilogue), empty
@@ -474,7 +474,7 @@ struct Bars {
 
 // kEnsemble: the instance that carries several networks (tiles per member, member
 // strides); the one-network instance has none of that arithmetic.
-template <bool kHalf, bool kEnsemble>
+template <bool kHalf, bool kEnsemble, int kSlots>
 __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const float *b1, const float *b2,
                                                const float *b3, const float *b4, const unsigned char *blob, void *y,
                                                int ldy, unsigned int *err, int wide,
@@ -482,10 +482,10 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *act = smem;                                   // 64 KB activation tile
     unsigned char *ring = smem + kActBytes;                      // 16 KB weight chunks
-    unsigned char *stage_all = ring + kRingBytes;                // output stage ...
+    unsigned char *stage_all = ring + kSlots * kChunkBytes;                // output stage ...
     unsigned char *xt = stage_all;                               // ... and, for layer 1, the input tile
     float *sbias = reinterpret_cast<float *>(stage_all + kStageBytes);   // b1 | b2 | b3 | b4 (padded)
-    __shared__ __align__(8) Bars bars;
+    __shared__ __align__(8) Bars<kSlots> bars;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     volatile int *abort = &abort_flag;
@@ -520,16 +520,20 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
+    // the output blocks of this CTA: all six, or its share of them (the launch rule in forward())
+    const int j0 = kOutBlocks * (int)blockIdx.y / (int)gridDim.y, j1 = kOutBlocks * ((int)blockIdx.y + 1) / (int)gridDim.y;
     if (warp == kProducerWarp) {
         int issued = 0;
-        for (int i = 0; i < kNumChunks; ++i) {
+        const int hidden = 1 + 2 * kHidChunks, count = hidden + (j1 - j0) * kOutChunks;
+        for (int i = 0; i < count; ++i) {
+            const int c = i < hidden ? i : i + j0 * kOutChunks;
             const int slot = i % kSlots;
             if (i >= kSlots && !warp_wait(&bars.empty[slot], (uint32_t)(i / kSlots - 1) & 1u, abort)) break;
             if (elect_one())
                 load_chunk(ring + slot * kChunkBytes,
                            blob + (kEnsemble ? (size_t)((int)blockIdx.x / tiles) * (size_t)blob_stride : 0) +
-                               chunk_offset(i),
-                           chunk_bytes(i), &bars.full[slot]);
+                               chunk_offset(c),
+                           chunk_bytes(c), &bars.full[slot]);
             __syncwarp();
             issued = i + 1;
         }
@@ -584,10 +588,10 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
         }
         // output layer: six blocks alternating between the halves of a tile's accumulator
         if (ok) wait_act();
-        for (int j = 0; j < kOutBlocks && ok; ++j) {
-            const int h = j & 1;
-            if (j >= 2) {
-                ok = warp_wait(&bars.acce[h], (uint32_t)((j >> 1) - 1) & 1u, abort);
+        for (int j = j0; j < j1 && ok; ++j) {
+            const int h = (j - j0) & 1;
+            if (j - j0 >= 2) {
+                ok = warp_wait(&bars.acce[h], (uint32_t)(((j - j0) >> 1) - 1) & 1u, abort);
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
             }
             const uint32_t id = j == kOutBlocks - 1 ? idesc(kLastN) : idesc(kOutN);
@@ -648,8 +652,8 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
                 arrive(&bars.act);
             }
             const int row0 = m0 + quarter * 32;
-            for (int j = 0; j < kOutBlocks && ok; ++j) {
-                const int h = j & 1;
+            for (int j = j0; j < j1 && ok; ++j) {
+                const int h = (j - j0) & 1;
                 ok = wait_bar(&bars.accf[h], accf_phase[h], abort);
                 accf_phase[h] ^= 1u;
                 ok = __all_sync(0xffffffffu, ok);
@@ -683,21 +687,25 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
     }
 }
 
-// One network: CTA blockIdx.x carries rows 128 blockIdx.x ...
-template <bool kHalf>
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) mlp_fused_kernel(const float *x, int m, const float *b1,
+// One network: CTA blockIdx.x carries rows 128 blockIdx.x ...  kOne: the instance with one CTA per
+// SM and the deeper ring.
+template <bool kHalf, bool kOne>
+__global__ void __launch_bounds__(kThreads, kOne ? 1 : 2) mlp_fused_kernel(const float *x, int m, const float *b1,
                                                                 const float *b2, const float *b3, const float *b4,
                                                                 const unsigned char *blob, void *y, int ldy,
                                                                 unsigned int *err, int wide) {
-    mlp_fused_body<kHalf, false>(x, m, b1, b2, b3, b4, blob, y, ldy, err, wide, (int)gridDim.x, 0, 0);
+    mlp_fused_body<kHalf, false, kOne ? kSlotsOne : kSlotsTwo>(x, m, b1, b2, b3, b4, blob, y, ldy, err, wide,
+                                                               (int)gridDim.x, 0, 0);
 }
 
 // An ensemble: fp16 outputs, tiles CTAs per member (mlp_fused_body).
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) mlp_fused_ensemble_kernel(
+template <bool kOne>
+__global__ void __launch_bounds__(kThreads, kOne ? 1 : 2) mlp_fused_ensemble_kernel(
         const float *x, int m, const float *b1, const float *b2, const float *b3, const float *b4,
         const unsigned char *blob, void *y, int ldy, unsigned int *err, int wide, int tiles, int bias_stride,
         long long blob_stride) {
-    mlp_fused_body<true, true>(x, m, b1, b2, b3, b4, blob, y, ldy, err, wide, tiles, bias_stride, blob_stride);
+    mlp_fused_body<true, true, kOne ? kSlotsOne : kSlotsTwo>(x, m, b1, b2, b3, b4, blob, y, ldy, err, wide, tiles,
+                                                             bias_stride, blob_stride);
 }
 
 // Rows [row0, row0 + rows_out) and k [k0, k0 + kdim) of W [n, k_in] (row-major bf16) as a
@@ -725,6 +733,20 @@ using namespace mcw;
 
 namespace {
 
+// Lets a kernel take `bytes` of dynamic shared memory, asked once per device and kernel.
+cudaError_t allow_smem(const void *fn, size_t bytes) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void *>> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count({dev, fn})) return cudaSuccess;
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done.insert({dev, fn});
+    return e;
+}
+
 // members networks (1 for one network) on the same inputs: member e's biases bias_stride
 // floats and its packed weights blob_stride bytes after member e - 1's, its outputs at
 // y + e * m * ldy.
@@ -740,26 +762,37 @@ int forward(const float *x, int32_t m, const float *b1, const float *b2, const f
     if (m == 0) return 0;
     unsigned int *err = tc_err_flag();
     if (!err) return MCW_MLP_ERR_CUDA;
-    const void *fn = half ? (members > 1 ? reinterpret_cast<const void *>(mlp_fused_ensemble_kernel)
-                                         : reinterpret_cast<const void *>(mlp_fused_kernel<true>))
-                          : reinterpret_cast<const void *>(mlp_fused_kernel<false>);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (e != cudaSuccess) return MCW_MLP_ERR_CUDA;
-    const int tiles = (m + FM - 1) / (FM);
+    const int tiles = (m + FM - 1) / FM;
     if ((long long)tiles * members > 0x7fffffffLL) return MCW_MLP_ERR_ARG;
-    const unsigned grid = (unsigned)(tiles * members);
+    // Few tiles: each is shared out to as many CTAs as still have an SM of their own (six, three or
+    // two, each with its share of the output blocks; the hidden layers are computed by all of them),
+    // in the instance with the deeper weight ring.  300 rows of one network, f32: 29.2 us with
+    // three CTAs, 15.7 with eighteen; 2,048 rows of five members 23.9, now 20.7; 16,384 of one 29.7,
+    // now 27.4 (one CTA an SM); from 152 tiles on two CTAs share an SM.
+    const int work = tiles * members;
+    const int share = work * 6 <= 152 ? 6 : (work * 3 <= 152 ? 3 : (work * 2 <= 152 ? 2 : 1));
+    const bool one = work * share <= 152;
+    const dim3 grid((unsigned)work, (unsigned)share);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned char *wb = static_cast<const unsigned char *>(blob);
     // rows on 32-byte boundaries take the 32-byte stores, others (16-byte) go through the stage
     const int wide = half && (((uintptr_t)y | (uintptr_t)ldy * 2) & 31) == 0;
+    const size_t smem = smem_bytes(one ? kSlotsOne : kSlotsTwo);
+    auto run = [&](auto *fn, auto... more) -> cudaError_t {
+        const cudaError_t e = allow_smem(reinterpret_cast<const void *>(fn), smem);
+        if (e != cudaSuccess) return e;
+        fn<<<grid, kThreads, smem, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, wide, more...);
+        return cudaGetLastError();
+    };
+    cudaError_t e;
     if (half && members > 1)
-        mlp_fused_ensemble_kernel<<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, wide, tiles,
-                                                                     bias_stride, blob_stride);
+        e = one ? run(mlp_fused_ensemble_kernel<true>, tiles, bias_stride, blob_stride)
+                : run(mlp_fused_ensemble_kernel<false>, tiles, bias_stride, blob_stride);
     else if (half)
-        mlp_fused_kernel<true><<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, wide);
+        e = one ? run(mlp_fused_kernel<true, true>) : run(mlp_fused_kernel<true, false>);
     else
-        mlp_fused_kernel<false><<<grid, kThreads, kSmemBytes, s>>>(x, m, b1, b2, b3, b4, wb, y, ldy, err, 0);
-    return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
+        e = one ? run(mlp_fused_kernel<false, true>) : run(mlp_fused_kernel<false, false>);
+    return e == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA;
 }
 
 }  // namespace

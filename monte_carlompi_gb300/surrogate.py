@@ -68,11 +68,12 @@ def from_target(y):
 # ------------------------------------------------------------------ kernels
 
 def _stream(torch):
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle (a plain integer; making the Stream object takes several us)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _gemm(torch, epi, m, n, k, a, lda, b, ldb, c, ldc, trans_a=0, trans_b=0, bias=None, aux=None,
@@ -129,13 +130,16 @@ def forward_fused(torch, x, w16, biases, blob, half=False):
     """Inference of the whole network in one kernel (mcw_mlp_forward, or
     mcw_mlp_forward_f16 with half=True: outputs rounded to fp16, half the bytes);
     x float32 [m, 4]; returns a [m, 649] view of the output rows."""
-    x = x.contiguous().float()
+    if x.dtype != torch.float32 or not x.is_contiguous():
+        x = x.contiguous().float()
     m = x.shape[0]
     pitch = Y_PITCH_F16 if half else Y_PITCH
     y = torch.empty((m, pitch), dtype=torch.float16 if half else torch.float32, device=x.device)
-    b = [t.contiguous() for t in biases]
-    fn = _abi.load().mcw_mlp_forward_f16 if half else _abi.load().mcw_mlp_forward
-    rc = fn(_ptr(x), m, _ptr(b[0]), _ptr(b[1]), _ptr(b[2]), _ptr(b[3]), _ptr(blob), _ptr(y), pitch, _stream(torch))
+    b1, b2, b3, b4 = [t if t.is_contiguous() else t.contiguous() for t in biases]
+    L = _abi.load()
+    fn = L.mcw_mlp_forward_f16 if half else L.mcw_mlp_forward
+    rc = fn(x.data_ptr(), m, b1.data_ptr(), b2.data_ptr(), b3.data_ptr(), b4.data_ptr(), blob.data_ptr(), y.data_ptr(),
+            pitch, _stream(torch))
     if rc:
         raise _abi.McwError(rc, 'mcw_mlp_forward failed (m=%d)' % m)
     return y[:, :DIMS[-1]]

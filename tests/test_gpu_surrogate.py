@@ -320,3 +320,24 @@ def test_autograd_gradients_at_odd_row_counts(rows):
     for got, ref in [(xg.grad, xc.grad)] + [(p.grad, c.grad) for p, c in zip(params, cparams)]:
         got, ref = got.cpu().double().flatten(), ref.flatten()
         assert (got - ref).norm() < 3e-2 * ref.norm()
+
+
+@pytest.mark.parametrize('n', [1, 127, 129, 3200, 3201, 6401, 9729, 19457])
+def test_fused_forward_rows_do_not_depend_on_the_batch(n):
+    """The launch of few tiles shares a tile's output blocks out to six, three or two CTAs (up to 25,
+    50 and 76 tiles), and takes one CTA per SM up to 152: a row's outputs are the same bits in every
+    one of them, alone and in an ensemble, fp16 and fp32, and through the staged stores that a row
+    pitch off 32 bytes takes."""
+    nets = [surrogate.SurrogateMLP(seed=30 + k) for k in range(2)]
+    x = torch.rand(20000, 4, generator=torch.Generator().manual_seed(1)).cuda() * 2 - 1
+    for half in (False, True):
+        whole, part = nets[0].predict_std(x, half=half), nets[0].predict_std(x[:n], half=half)
+        assert torch.equal(whole[:n], part)
+    ens = surrogate.Ensemble(nets)
+    assert torch.equal(ens.predict_std(x)[:, :n], ens.predict_std(x[:n].contiguous()))
+    y = torch.full((n, 664), 3.0, dtype=torch.float16, device='cuda')      # 1,328-byte rows: 16-byte boundaries
+    b = nets[0].params[1::2]
+    rc = _abi.load().mcw_mlp_forward_f16(x.data_ptr(), n, *[t.data_ptr() for t in b], nets[0].packed().data_ptr(),
+                                         y.data_ptr(), 664, surrogate._stream(torch))
+    torch.cuda.synchronize()
+    assert rc == 0 and torch.equal(y[:, :649], part) and (y[:, 649:] == 3).all()
