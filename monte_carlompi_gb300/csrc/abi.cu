@@ -116,8 +116,9 @@ struct mcw_ctx {
     // 0, so no photon scatters isotropically (the deep-slab instance's HG step)
     std::vector<char> h_ice_aniso;
     // phase matrices of the polarised walk, one per ice table (n_rows 0 = none)
-    DevBuf phasedata, phase_tables, phasedata32, phase_tables32, phase_seeds;
+    DevBuf phasedata, phase_tables, phasedata32, phase_tables32, phase_seeds, phase_seg;
     std::vector<int32_t> phase_rows;
+    std::vector<DevPhase32> h_phase32;             // host copy of phase_tables32
     // workspace
     DevBuf cfgs, lut, tallies, counters, records, post, drain;
     HostBuf h_stage, h_tallies, h_counters;
@@ -524,7 +525,8 @@ int mcw_destroy(mcw_ctx *ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (DevBuf *b : {&ctx->tabdata, &ctx->ice_tables, &ctx->cfgs, &ctx->lut, &ctx->tallies, &ctx->counters,
-                      &ctx->records, &ctx->post, &ctx->drain})
+                      &ctx->records, &ctx->post, &ctx->drain, &ctx->phasedata, &ctx->phase_tables, &ctx->phasedata32,
+                      &ctx->phase_tables32, &ctx->phase_seeds, &ctx->phase_seg})
         b->release();
     ctx->h_stage.release();
     ctx->h_tallies.release();
@@ -724,6 +726,10 @@ int mcw_set_phase_matrices(mcw_ctx *ctx, const mcw_phase_table *tabs, int32_t n)
     auto f32 = [&](const double *p) { return p ? fbase + (p - dbase) : nullptr; };
     std::vector<uint16_t> seeds((size_t)n * kPhaseBuckets, 0);
     CUDA_TRY(ctx, ctx->phase_seeds.ensure(seeds.size() * sizeof(uint16_t)));
+    size_t seg_total = 1;
+    for (int32_t t = 0; t < n; ++t) seg_total += (size_t)(4 * tabs[t].n_angle[0] + 1) * dev[t].n_rows;
+    CUDA_TRY(ctx, ctx->phase_seg.ensure(seg_total * sizeof(float4)));
+    float4 *seg_at = (float4 *)ctx->phase_seg.p;
     for (int32_t t = 0; t < n; ++t) {
         const DevPhase &d = dev[t];
         DevPhase32 f{};
@@ -743,20 +749,22 @@ int mcw_set_phase_matrices(mcw_ctx *ctx, const mcw_phase_table *tabs, int32_t n)
                        memcmp(p.cos_asc[e], p.cos_asc[0], p.n_angle[0] * sizeof(double)) == 0;
             f.shared_grid = same ? 1 : 0;
             if (same && p.n_angle[0] <= 65535) {
-                // bucket seeds on the float copy of the grid (what the kernel compares)
+                // the first grid index at or above the middle of each bucket, on the float copy of
+                // the grid (what the kernel compares)
                 const int32_t m = p.n_angle[0];
-                const float lo = (float)p.cos_asc[0][0], hi = (float)p.cos_asc[0][m - 1];
-                const float scale = (float)kPhaseBuckets / (hi - lo);
                 uint16_t *sd = &seeds[(size_t)t * kPhaseBuckets];
-                int32_t j = 0;
-                for (int b = 0; b < kPhaseBuckets; ++b) {
-                    const float edge = lo + (float)b / scale;
-                    while (j < m && (float)p.cos_asc[0][j] < edge) ++j;
+                int32_t j = m;
+                for (int b = 0; b < kPhaseBuckets; ++b) {      // 1 - cos rises: cos falls
+                    const uint32_t bits = ((kBucketLow + (uint32_t)b) << 15) | 0x4000u;
+                    float d;
+                    memcpy(&d, &bits, sizeof(d));
+                    while (j > 0 && (float)p.cos_asc[0][j - 1] >= 1.0f - d) --j;
                     sd[b] = (uint16_t)j;
                 }
                 f.seed = (const uint16_t *)ctx->phase_seeds.p + (size_t)t * kPhaseBuckets;
-                f.seed_lo = lo;
-                f.seed_scale = scale;
+                f.seg = seg_at;
+                f.env = seg_at + (size_t)4 * m * d.n_rows;
+                seg_at += (size_t)(4 * m + 1) * d.n_rows;
             }
         }
         f.cos_max = (float)d.cos_max;
@@ -767,6 +775,11 @@ int mcw_set_phase_matrices(mcw_ctx *ctx, const mcw_phase_table *tabs, int32_t n)
     CUDA_TRY(ctx, cudaMemcpy(ctx->phasedata32.p, host32.data(), host32.size() * sizeof(float), cudaMemcpyHostToDevice));
     CUDA_TRY(ctx, cudaMemcpy(ctx->phase_seeds.p, seeds.data(), seeds.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
     CUDA_TRY(ctx, cudaMemcpy(ctx->phase_tables32.p, dev32.data(), n * sizeof(DevPhase32), cudaMemcpyHostToDevice));
+    // the copies above run in the default stream, from pageable memory: done before the kernel reads
+    CUDA_TRY(ctx, cudaStreamSynchronize(nullptr));
+    for (const DevPhase32 &f : dev32)
+        if (f.seg) CUDA_TRY(ctx, launch_phase_pack(f, const_cast<float4 *>(f.seg), const_cast<float4 *>(f.env), ctx->stream));
+    ctx->h_phase32 = dev32;
     for (int32_t t = 0; t < n; ++t) ctx->phase_rows[t] = tabs[t].n_rows;
     return MCW_OK;
 }
@@ -887,7 +900,10 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
                                 (mcw_record32 *)dev_records, 1, 32, seed);
         wa.phase = (const DevPhase32 *)ctx->phase_tables32.p;
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, st));
-        CUDA_TRY(ctx, launch_walk_pol32(wa, ctx->sm_count, st));
+        int32_t table = cfgs[0].ice_table;
+        for (int32_t i = 1; i < n_cfg; ++i)
+            if (cfgs[i].ice_table != table) table = -1;
+        CUDA_TRY(ctx, launch_walk_pol32(wa, table >= 0 ? &ctx->h_phase32[table] : nullptr, ctx->sm_count, st));
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev1, st));
         shape.block = 128;
     } else {

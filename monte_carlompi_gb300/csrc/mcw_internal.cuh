@@ -70,12 +70,18 @@ struct DevPhase32 {
     int32_t n_rows;
     int32_t shared_grid;         // 1: the six elements share one cos grid (one search serves all)
     float cos_max, cos_min, cos_cutoff, pad2;
-    // seeds of the search on the shared grid: seed[b] = first grid index with
-    // cos >= the lower edge of bucket b, kPhaseBuckets buckets uniform on [cos_min, cos_max]
+    // of a shared grid of at most 65,535 points (else null): seed[phase_bucket(cos)] = a grid index
+    // near cos, where the search of its segment begins
     const uint16_t *seed;
-    float seed_lo, seed_scale;
+    // seg[4 (row n_angle + k)]: the segment [k - 1, k] as {cos, cos, P11, P11}, {P12, P12, P22, P22},
+    // {P33, P33, P43, P43}, {P44, P44, 0, 0}, lower end first; env[row] = {a1, a2, b1, b2}
+    const float4 *seg, *env;
 };
-constexpr int kPhaseBuckets = 2048;
+
+// Buckets of cos that follow an angle grid: 256 to an octave of 1 - cos (grids are uniform in the
+// angle, so their cosines crowd at cos = 1, where 2,048 buckets uniform in cos held ten points each).
+constexpr uint32_t kBucketLow = 0x36800000u >> 15;              // 1 - cos = 2^-18
+constexpr int kPhaseBuckets = (int)((0x40000000u >> 15) - kBucketLow) + 1;   // ... 2
 
 // Phase matrices of one ice table on the device (mcw_phase_table, rows in the
 // device table's order).
@@ -220,8 +226,11 @@ constexpr int kDrainSlot = 6;
 // (sm_count SMs; a.drain must then hold grid * block slots).
 cudaError_t launch_walk_f32(const WalkArgs &a, bool impurity, int grid, int block, int sm_count, cudaStream_t s);
 cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s);
-// The FP32 polarised walk (a.phase set, a.records holding mcw_record32p).
-cudaError_t launch_walk_pol32(const WalkArgs &a, int sm_count, cudaStream_t s);
+// The FP32 polarised walk (a.phase set, a.records holding mcw_record32p).  only: the one phase table
+// that every config uses, or null.
+cudaError_t launch_walk_pol32(const WalkArgs &a, const DevPhase32 *only, int sm_count, cudaStream_t s);
+// Fill the seg and env tables of a phase table from its columns (DevPhase32).
+cudaError_t launch_phase_pack(const DevPhase32 &p, float4 *seg, float4 *env, cudaStream_t s);
 int walk_f32_max_blocks_per_sm(int block, int n_cfg, bool impurity);
 // The walk and drain kernels (their one parameter is a WalkArgs).
 bool walk_f32_is_kernel(const void *fn);

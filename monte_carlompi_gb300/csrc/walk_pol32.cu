@@ -23,6 +23,14 @@
 // l % n), so a step costs a few rounds instead of the slowest lane's candidate
 // count, and the last walks of a launch get the whole warp.
 //
+// What bounds it: the latency of a step, for the longest walks (800 steps of 200,000 photons'
+// mean 52), and instructions in between.  So a round finds its photons through a table in shared
+// memory and a constant one instead of bit searches, divisions and loops; the six elements of a
+// segment lie side by side with its two cosines (seg), so a lookup is a bucket and one or four
+// 16-byte loads instead of a search and 24 4-byte ones, and the accepted candidate's segment
+// serves the Stokes update; a launch on one phase table has it in its arguments.  200,000 photons
+// 3.12 ms, now 1.9, a million 7.3, now 4.9.
+//
 // Statistically equivalent restatements (identical distributions):
 //  * the envelope factor |Q cos 2b + U sin 2b| with 2b = arctan(U / Q) (:908-935)
 //    is sqrt(Q^2 + U^2), its closed form;
@@ -80,14 +88,19 @@ __device__ __forceinline__ int segment32(const float *x, int n, float xn) {
     return min(max(lo, 1), n - 1);
 }
 
+// The bucket of a cosine (kPhaseBuckets).
+__device__ __forceinline__ int phase_bucket(float xn) {
+    const uint32_t b = __float_as_uint(fmaxf(1.0f - xn, 3.814697265625e-06f)) >> 15;   // at least 2^-18
+    return (int)min(b - kBucketLow, (uint32_t)kPhaseBuckets - 1u);
+}
+
 // The same segment on the shared grid, the search seeded by its bucket: probe down
 // while the point before is still >= xn, then up while the point is < xn.
 __device__ __forceinline__ int segment_seeded(const DevPhase32 &ph, float xn) {
     const float *x = ph.cos_asc[0];
     const int n = ph.n_angle[0];
     if (!ph.seed) return segment32(x, n, xn);
-    const int b = min(max(__float2int_rd((xn - ph.seed_lo) * ph.seed_scale), 0), kPhaseBuckets - 1);
-    int k = __ldg(ph.seed + b);
+    int k = __ldg(ph.seed + phase_bucket(xn));
     while (k > 0 && __ldg(x + k - 1) >= xn) --k;
     while (k < n && __ldg(x + k) < xn) ++k;
     return min(max(k, 1), n - 1);
@@ -100,6 +113,32 @@ __device__ __forceinline__ float phase_at(const DevPhase32 &ph, int e, int row, 
     const float xl = __ldg(x + k - 1), xh = __ldg(x + k), yl = __ldg(y + k - 1), yh = __ldg(y + k);
     return fmaf(__fdividef(xn - xl, xh - xl), yh - yl, yl);
 }
+
+// The same segment from the seg table of a row (first quarters at base + 4 k): the bucket's segment
+// first, which carries its two cosines, then its neighbours.  s0: its first quarter.
+__device__ __forceinline__ int segment_packed(const DevPhase32 &ph, const float4 *base, float xn, float4 &s0) {
+    const int last = ph.n_angle[0] - 1;
+    int k = min(max((int)__ldg(ph.seed + phase_bucket(xn)), 1), last);
+    s0 = __ldg(base + 4 * k);
+    while (k > 1 && s0.x >= xn) s0 = __ldg(base + 4 * --k);
+    while (k < last && s0.y < xn) s0 = __ldg(base + 4 * ++k);
+    return k;
+}
+
+// sqrt of 0 or a normal x, correctly rounded: the hardware's reciprocal square root and one residual
+// (every mantissa of two binades was compared with sqrtf), without sqrtf's range branch.
+__device__ __forceinline__ float sqrt_pos(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float s = __fmul_rn(x, y);
+    const float r = fmaf(fmaf(-s, s, x), __fmul_rn(0.5f, y), s);
+    return x > 0.f ? r : x;
+}
+
+// Where xn lies in the segment whose first quarter is s (the same quotient for every element), and an
+// element's value there from its two ends.
+__device__ __forceinline__ float seg_pos(const float4 s, float xn) { return __fdividef(xn - s.x, s.y - s.x); }
+__device__ __forceinline__ float seg_val(float t, float lo, float hi) { return fmaf(t, hi - lo, lo); }
 
 // cos / sin of an azimuth 2 pi u, u in (0, 1): sincos of the angle shifted into
 // [-pi, pi) (where the fast intrinsic is accurate), negated back.
@@ -189,12 +228,14 @@ struct Envelope {
     float max1, max2, pa1;
 };
 
-__device__ __forceinline__ Envelope envelope(const PolPhoton &P) {
-    const DevPhase32 &ph = *P.ph;
+__device__ __forceinline__ Envelope envelope(const PolPhoton &P, const DevPhase32 &ph) {
     const float C = sqrtf(fmaf(P.Q, P.Q, P.U * P.U));
     Envelope v;
-    v.max1 = fmaf(fabsf(P.I), __ldg(ph.a1 + P.row), __ldg(ph.b1 + P.row) * C);
-    v.max2 = fmaf(fabsf(P.I), __ldg(ph.a2 + P.row), __ldg(ph.b2 + P.row) * C);
+    const float4 e = ph.env ? __ldg(ph.env + P.row)
+                            : make_float4(__ldg(ph.a1 + P.row), __ldg(ph.a2 + P.row), __ldg(ph.b1 + P.row),
+                                          __ldg(ph.b2 + P.row));
+    v.max1 = fmaf(fabsf(P.I), e.x, e.z * C);
+    v.max2 = fmaf(fabsf(P.I), e.y, e.w * C);
     const float area1 = (ph.cos_max - ph.cos_cutoff) * v.max1;
     const float area2 = (ph.cos_cutoff - ph.cos_min) * v.max2;
     v.pa1 = __fdividef(area1, area1 + area2);
@@ -204,7 +245,7 @@ __device__ __forceinline__ Envelope envelope(const PolPhoton &P) {
 // Candidate j of step n (:953-1001): its cosine and azimuth, and whether it passes.
 __device__ __forceinline__ bool candidate(const DevPhase32 &ph, int row, float I, float Q, float U,
                                           const Envelope &v, uint32_t n, uint32_t j, uint32_t lo, uint32_t hi,
-                                          const PhiloxKeys &ks, float &cos_theta, float &cphi, float &sphi) {
+                                          const PhiloxKeys &ks, float &cos_theta, float &cphi, float &sphi, int &seg) {
     const uint4 r = philox10(make_uint4(n, kTagPolCand | (j << 8), lo, hi), ks);
     const bool one = u01_f32(r.x) < v.pa1;
     const float uc = u01_f32(r.y);
@@ -213,7 +254,15 @@ __device__ __forceinline__ bool candidate(const DevPhase32 &ph, int row, float I
                     : fmaf(-uc, ph.cos_cutoff - ph.cos_min, ph.cos_cutoff);
     const float r3 = 1.000001f * u01_f32(r.w) * (one ? v.max1 : v.max2);
     float S11, S12;
-    if (ph.shared_grid) {
+    if (ph.seg) {
+        const float4 *base = ph.seg + 4 * (size_t)(row * ph.n_angle[0]);
+        float4 s0;
+        seg = segment_packed(ph, base, cos_theta, s0);
+        const float4 s1 = __ldg(base + 4 * seg + 1);
+        const float t = seg_pos(s0, cos_theta);
+        S11 = seg_val(t, s0.z, s0.w);
+        S12 = seg_val(t, s1.x, s1.y);
+    } else if (ph.shared_grid) {
         const int k = segment_seeded(ph, cos_theta);
         S11 = phase_at(ph, 0, row, k, cos_theta);
         S12 = phase_at(ph, 1, row, k, cos_theta);
@@ -228,8 +277,8 @@ __device__ __forceinline__ bool candidate(const DevPhase32 &ph, int row, float I
 
 // The rest of the step (monte_carlo3D.py:1227-1466) with its scattering angles.
 // Returns the end condition (0: still walking).
-__device__ __forceinline__ int pol_step_post(PolPhoton &P, const WalkArgs &a, float p_cos, float cphi, float sphi) {
-    const DevPhase32 &ph = *P.ph;
+__device__ __forceinline__ int pol_step_post(PolPhoton &P, const DevPhase32 &ph, const WalkArgs &a, float p_cos,
+                                             float cphi, float sphi, int p_seg) {
     const float dtau = (P.lam_surface && P.i == 1) ? 0.f : -__logf(u01_f32(P.sb.x));   // :1227-1229
     float nx = P.mux, ny = P.muy, nz = P.muz;
     if (P.i > 1) {
@@ -239,7 +288,7 @@ __device__ __forceinline__ int pol_step_post(PolPhoton &P, const WalkArgs &a, fl
             m0x = 0.f; m0y = 0.f; m0z = 1.f;
             ct = sqrtf(u01_f32(P.sb.w));
         }
-        const float st = sqrtf(fmaxf(0.f, fmaf(-ct, ct, 1.f)));
+        const float st = sqrt_pos(fmaxf(0.f, fmaf(-ct, ct, 1.f)));
         // sqrt(mu_x^2 + mu_y^2) stands for sqrt(1 - mu_z^2) (equal for a unit
         // direction; the frame stays orthogonal next to the pole in FP32); the
         // pole formula when it is 0 (or below FLT_MIN, where the reciprocal square
@@ -265,11 +314,26 @@ __device__ __forceinline__ int pol_step_post(PolPhoton &P, const WalkArgs &a, fl
             P.bref = false;
         } else {
             // into the scattering plane: phi_sca = arccos(cphi) in [0, pi]
-            const float sps = sqrtf(fmaxf(0.f, fmaf(-cphi, cphi, 1.f)));
+            const float sps = sqrt_pos(fmaxf(0.f, fmaf(-cphi, cphi, 1.f)));
             float Q = P.Q, U = P.U;
             rotate(Q, U, fmaf(2.f * cphi, cphi, -1.f), 2.f * sps * cphi);
             float Pe[6];
-            if (ph.shared_grid) {
+            if (ph.seg) {
+                // the accepted candidate's segment; a surface's Lambertian cosine looks up its own
+                const float4 *sg = ph.seg + 4 * (size_t)(P.row * ph.n_angle[0]);
+                float4 s0;
+                if (P.lam_surface) p_seg = segment_packed(ph, sg, ct, s0);
+                sg += 4 * p_seg;
+                s0 = __ldg(sg);
+                const float4 s1 = __ldg(sg + 1), s2 = __ldg(sg + 2), s3 = __ldg(sg + 3);
+                const float t = seg_pos(s0, ct);
+                Pe[0] = seg_val(t, s0.z, s0.w);
+                Pe[1] = seg_val(t, s1.x, s1.y);
+                Pe[2] = seg_val(t, s1.z, s1.w);
+                Pe[3] = seg_val(t, s2.x, s2.y);
+                Pe[4] = seg_val(t, s2.z, s2.w);
+                Pe[5] = seg_val(t, s3.x, s3.y);
+            } else if (ph.shared_grid) {
                 const int k = segment_seeded(ph, ct);
 #pragma unroll
                 for (int e = 0; e < 6; ++e) Pe[e] = phase_at(ph, e, P.row, k, ct);
@@ -287,7 +351,7 @@ __device__ __forceinline__ int pol_step_post(PolPhoton &P, const WalkArgs &a, fl
                 const float sign = (cphi == -1.f) ? 1.f : -1.f;   // phi_sca >= pi only at cos phi = -1
                 cos_i = fminf(fmaxf(__fdividef(fmaf(nz, ct, -m0z), sign * den), -1.f), 1.f);
             }
-            const float si = sqrtf(fmaxf(0.f, fmaf(-cos_i, cos_i, 1.f)));
+            const float si = sqrt_pos(fmaxf(0.f, fmaf(-cos_i, cos_i, 1.f)));
             float Qm = Qs, Um = Us;
             rotate(Qm, Um, fmaf(2.f * cos_i, cos_i, -1.f), -2.f * si * cos_i);
             const float inv_i = 1.f / Is;
@@ -353,9 +417,20 @@ __device__ __forceinline__ void pol_finish(const PolPhoton &P, const WalkArgs &a
     tally_global(a.tallies + P.ci, cond, P.i - 1, P.wvn_fx, theta, phi);
 }
 
+// Bits 0, n, 2n, ... below 32: the lanes of the photon of rank 0 when n photons share the warp.
+__constant__ uint32_t kEvery[33] = {
+    0u, 0xffffffffu, 0x55555555u, 0x49249249u, 0x11111111u, 0x42108421u, 0x41041041u, 0x10204081u, 0x01010101u,
+    0x08040201u, 0x40100401u, 0x00400801u, 0x01001001u, 0x04002001u, 0x10004001u, 0x40008001u, 0x00010001u,
+    0x00020001u, 0x00040001u, 0x00080001u, 0x00100001u, 0x00200001u, 0x00400001u, 0x00800001u, 0x01000001u,
+    0x02000001u, 0x04000001u, 0x08000001u, 0x10000001u, 0x20000001u, 0x40000001u, 0x80000001u, 0x00000001u};
+
 // Warp-synchronous: every lane of the warp stays in the loop until none has a
 // photon left, so the rejection rounds and claims can use the whole warp.
-__global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a) {
+// kOnly: every config uses the phase table `only`, whose pointers and bounds then are launch constants.
+template <bool kOnly>
+__global__ void __launch_bounds__(kPolBlock, 6) walk_pol32_kernel(const WalkArgs a, const DevPhase32 only) {
+    __shared__ uint8_t owners[kPolBlock / 32][32];   // per warp: the lane of the pending photon of each rank
+    uint8_t *owner_of = owners[threadIdx.x >> 5];
     const unsigned long long t0 = global_ns();
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -366,6 +441,8 @@ __global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a)
     bool have = false, exhausted = false;
     for (uint32_t it = 0;; ++it) {
         // ---- claims: lanes without a photon take the next ones, one atomic per warp
+        // (of a launch spread thin, a.lanes < 32, only its first a.lanes lanes, once)
+        if (a.lanes < 32 && (it > 0 || lane >= a.lanes)) exhausted = true;
         const unsigned need = __ballot_sync(0xffffffffu, !have && !exhausted);
         if (need) {
             unsigned long long base = 0;
@@ -388,11 +465,12 @@ __global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a)
         Envelope env{0.f, 0.f, 0.f};
         uint32_t jbase = 0;
         float p_cos = 1.f, cphi = 0.f, sphi = 0.f;
+        int p_seg = 1;
         if (have) {
             P.i += 1;
             P.sb = step_block(P, (uint32_t)P.i, kTagPolStep, a);
             if (P.i > 1) {
-                env = envelope(P);
+                env = envelope(P, kOnly ? only : *P.ph);
                 pending = true;
             }
         }
@@ -401,9 +479,13 @@ __global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a)
         // photon takes its lowest-indexed passing candidate
         unsigned pend = __ballot_sync(0xffffffffu, pending);
         for (uint32_t round = 0; pend; ++round) {
-            const int np = __popc(pend);
-            const int r = lane % np, q = lane / np;
-            const int owner = __fns(pend, 0, r + 1);
+            const int np = __popc(pend), me = __popc(pend & lt_mask);
+            // lane / np: (lane + 1/2) / np lies at least 1/64 from a whole number
+            const int q = (int)__fdividef((float)lane + 0.5f, (float)np), r = lane - q * np;
+            __syncwarp();
+            if (pending) owner_of[me] = (uint8_t)lane;
+            __syncwarp();
+            const int owner = owner_of[r];
             const int o_row = __shfl_sync(0xffffffffu, P.row, owner);
             const float o_I = __shfl_sync(0xffffffffu, P.I, owner);
             const float o_Q = __shfl_sync(0xffffffffu, P.Q, owner);
@@ -416,18 +498,17 @@ __global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a)
             const uint32_t o_lo = __shfl_sync(0xffffffffu, P.lo, owner);
             const uint32_t o_hi = __shfl_sync(0xffffffffu, P.hi, owner);
             const uint32_t o_j = __shfl_sync(0xffffffffu, jbase, owner) + (uint32_t)q;
-            const DevPhase32 *o_ph = reinterpret_cast<const DevPhase32 *>(
+            const DevPhase32 *o_ph = kOnly ? nullptr : reinterpret_cast<const DevPhase32 *>(
                 __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(P.ph), owner));
             float c_cos, c_cphi, c_sphi;
-            const bool pass = candidate(*o_ph, o_row, o_I, o_Q, o_U, o_env, o_n, o_j, o_lo, o_hi, a.keys,
-                                        c_cos, c_cphi, c_sphi);
+            int c_seg = 1;
+            const bool pass = candidate(kOnly ? only : *o_ph, o_row, o_I, o_Q, o_U, o_env, o_n, o_j, o_lo, o_hi, a.keys,
+                                        c_cos, c_cphi, c_sphi, c_seg);
             const unsigned acc = __ballot_sync(0xffffffffu, pass);
             int src = lane;
             bool got = false;
             if (pending) {
-                const int me = __popc(pend & lt_mask);
-                unsigned group = 0;
-                for (int l = me; l < 32; l += np) group |= 1u << l;
+                const unsigned group = kEvery[np] << me;
                 const unsigned hit = acc & group;
                 if (hit) {
                     src = __ffs(hit) - 1;
@@ -439,10 +520,12 @@ __global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a)
             const float w_cos = __shfl_sync(0xffffffffu, c_cos, src);
             const float w_cphi = __shfl_sync(0xffffffffu, c_cphi, src);
             const float w_sphi = __shfl_sync(0xffffffffu, c_sphi, src);
+            const int w_seg = __shfl_sync(0xffffffffu, c_seg, src);
             if (got) {
                 p_cos = w_cos;
                 cphi = w_cphi;
                 sphi = w_sphi;
+                p_seg = w_seg;
                 pending = false;
             } else if (pending && jbase >= kMaxCandidates) {
                 atomicOr(a.status, kStatusStream);   // a candidate range no envelope should need
@@ -461,7 +544,7 @@ __global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a)
 
         // ---- the rest of the step; finished photons leave their records
         if (have) {
-            const int cond = pol_step_post(P, a, p_cos, cphi, sphi);
+            const int cond = pol_step_post(P, kOnly ? only : *P.ph, a, p_cos, cphi, sphi, p_seg);
             if (cond > 0) {
                 pol_finish(P, a, cond);
                 have = false;
@@ -479,16 +562,51 @@ __global__ void __launch_bounds__(kPolBlock) walk_pol32_kernel(const WalkArgs a)
     }
 }
 
+// The seg and env tables of a phase table (DevPhase32), one segment a thread.
+__global__ void phase_pack_kernel(const DevPhase32 p, float4 *seg, float4 *env) {
+    const int m = p.n_angle[0];
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)p.n_rows * m) return;
+    const int row = (int)(i / m), hi = (int)(i % m), lo = max(hi - 1, 0);
+    const float *x = p.cos_asc[0];
+    float y[6][2];
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+        y[e][0] = p.p_asc[e][(size_t)row * m + lo];
+        y[e][1] = p.p_asc[e][(size_t)row * m + hi];
+    }
+    seg[4 * i] = make_float4(x[lo], x[hi], y[0][0], y[0][1]);
+    seg[4 * i + 1] = make_float4(y[1][0], y[1][1], y[2][0], y[2][1]);
+    seg[4 * i + 2] = make_float4(y[3][0], y[3][1], y[4][0], y[4][1]);
+    seg[4 * i + 3] = make_float4(y[5][0], y[5][1], 0.f, 0.f);
+    if (hi == 0) env[row] = make_float4(p.a1[row], p.a2[row], p.b1[row], p.b2[row]);
+}
+
 }  // namespace
 
-cudaError_t launch_walk_pol32(const WalkArgs &a, int sm_count, cudaStream_t s) {
+cudaError_t launch_phase_pack(const DevPhase32 &p, float4 *seg, float4 *env, cudaStream_t s) {
+    const long long total = (long long)p.n_rows * p.n_angle[0];
+    if (total <= 0) return cudaSuccess;
+    phase_pack_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(p, seg, env);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_walk_pol32(const WalkArgs &a, const DevPhase32 *only, int sm_count, cudaStream_t s) {
     if (a.total <= 0) return cudaSuccess;
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_pol32_kernel, kPolBlock, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_pol32_kernel<true>, kPolBlock, 0);
     if (e != cudaSuccess) return e;
-    const int64_t want = (a.total + kPolBlock - 1) / kPolBlock;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sm_count * std::max(per_sm, 1), want));
-    walk_pol32_kernel<<<grid, kPolBlock, 0, s>>>(a);
+    // six blocks: 200,000 photons 1.85 ms, with seven 2.02 (a long walk's steps wait for more
+    // warps), with four 1.99; a million 4.94 / 4.85 / 5.58
+    per_sm = std::min(per_sm, 6);
+    // few photons are spread over all warps: alone in a warp a photon has every lane for its
+    // rejection candidates; a step takes 1.5 us then, in a warp of 32 photons 2.5 (100 photons
+    // 1.26 ms, now 0.54)
+    const WalkSpread spread = spread_walk(a.total, (int64_t)sm_count * std::max(per_sm, 1), kPolBlock);
+    WalkArgs b = a;
+    b.lanes = spread.lanes;
+    if (only) walk_pol32_kernel<true><<<spread.grid, kPolBlock, 0, s>>>(b, *only);
+    else walk_pol32_kernel<false><<<spread.grid, kPolBlock, 0, s>>>(b, DevPhase32{});
     return cudaGetLastError();
 }
 

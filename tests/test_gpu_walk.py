@@ -785,3 +785,20 @@ def test_empty_run(walker):
     walker.set_tables([ice], imp)
     res = walker.walk([cfg], 1)
     assert res.records.size == 0 and int(res.tallies[0]['n_cond'].sum()) == 0
+
+
+@pytest.mark.parametrize('n', [1, 33, 3647, 3649, 30000])
+def test_pol32_records_independent_of_spread_and_table_path(walker, n):
+    """The first n records of a larger run, from one photon a warp to full warps; and the same
+    records when a second config on another ice table makes the launch take its phase tables from
+    memory instead of its arguments."""
+    g = load_golden('pol')
+    ice, imp = golden_tables(g)
+    walker.set_tables([ice, ice], imp)
+    walker.set_phase_matrices([golden_phase(g), golden_phase(g)])
+    cfg = dataclasses.replace(golden_config(g), n_photon=60000)
+    big = walker.walk([cfg], 8, mode='pol32').records
+    small = dataclasses.replace(cfg, n_photon=n)
+    assert np.array_equal(walker.walk([small], 8, mode='pol32').records, big[:n])
+    two = walker.walk([small, dataclasses.replace(small, ice_table=1)], 8, mode='pol32').records
+    assert np.array_equal(two[:n], big[:n])
