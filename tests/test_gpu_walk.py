@@ -491,6 +491,35 @@ def test_records_into_pinned_host_memory(walker):
             lib.mcw_host_free(ptr)
 
 
+@pytest.mark.parametrize('mode', ['f32', 'pol32', 'replay64'])
+@pytest.mark.parametrize('n', [1, 1000, 4099])
+@pytest.mark.parametrize('offset', [0, 8, 16])
+def test_records_into_pageable_host_memory(walker, mode, n, offset):
+    """Records of a walk into pageable host memory at any alignment (16-byte aligned: written
+    by the kernels; else copied) are those it leaves in device memory, and nothing beside
+    them is touched."""
+    import torch
+    if mode == 'pol32':
+        g = load_golden('pol')
+        (ice, imp), cfg = golden_tables(g), dataclasses.replace(golden_config(g), n_photon=n)
+    else:
+        cfg, ice, imp = cfg2_geometry(n)
+    walker.set_tables([ice], imp)
+    if mode == 'pol32':
+        walker.set_phase_matrices([golden_phase(g)])
+    dtype = {'f32': _abi.RECORD32, 'pol32': _abi.RECORD32P, 'replay64': _abi.RECORD64}[mode]
+    nbytes = n * dtype.itemsize
+    raw = np.full(nbytes + 64, 0xA5, np.uint8)
+    start = -raw.ctypes.data % 16 + offset
+    out = raw[start:start + nbytes].view(dtype)
+    a = walker.walk([cfg], 11, mode=mode, out=out)
+    device = torch.empty(nbytes, dtype=torch.uint8, device='cuda')
+    b = walker.walk([cfg], 11, mode=mode, records='device', device_ptr=device.data_ptr())
+    assert out.tobytes() == device.cpu().numpy().tobytes()
+    assert np.array_equal(a.tallies, b.tallies)
+    assert (raw[:start] == 0xA5).all() and (raw[start + nbytes:] == 0xA5).all()
+
+
 def test_pinned_host_records_with_drain_and_two_configs(walker):
     """Pinned host records of the FP32 walk, written by the kernels themselves, cover
     every photon: those finished by the drain kernel (weakly absorbing deep snow,
