@@ -191,11 +191,32 @@ struct __align__(16) FinishSlot {
     float muz, path, pad0, pad1;
 };
 
+// The lanes' values of a warp's scans, in shared memory: a lane's slot is 16 + lane, and the 16
+// slots below hold the identity, so that a lane without a left neighbour at some distance reads
+// the identity there: a store and a load of 16 bytes a round in place of four shuffles and as
+// many selects.  Two buffers in turn: a lane writes one only after the barrier of a round that
+// reads the other.
+struct PassScan {
+    float4 q[2][48];
+    float2 zp[2][48];
+};
+
+__device__ __forceinline__ void pass_scan_init(PassScan &S, int lane) {
+    if (lane < 16) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            S.q[b][lane] = make_float4(1.f, 0.f, 0.f, 0.f);
+            S.zp[b][lane] = make_float2(0.f, 0.f);
+        }
+    }
+}
+
 struct WarpQueues {
     BirthSlot birth[32];
     FinishSlot fin[kFinishCap];
     uint4 rmeta[3 * kSparseWarp];             // sparse round: each photon's stream, step and constants
     float4 pbuf[2 * kSparseSlots];            // sparse round: StepPre of up to 64 steps
+    PassScan scan;
     WarpTally tally;
 };
 
@@ -662,7 +683,7 @@ __device__ __forceinline__ int sparse_round(Photon &P, WarpQueues &q, const unsi
 // its steps' angles, optical path and absorption words (the same Philox blocks,
 // counter = step, as the step-by-step walk) and turns each step's rotation
 // R = Rz(phi) Ry(theta) into a unit quaternion; the lane's product, an inclusive
-// shuffle scan of Hamilton products across the chunk (rotations compose
+// scan of Hamilton products across the chunk (rotations compose
 // associatively) and the product W_c of the earlier chunks' totals give every
 // step's composed rotation P_k = R_1 ... R_k, so step k's direction is
 // O_0 P_k e_z.  Vertical positions and path lengths are scan sums the same way,
@@ -794,8 +815,8 @@ __device__ __forceinline__ void lane_draw(LaneSteps<LS> &L, const Photon &Q, uin
         L.reflm |= (uu.w < Q.R ? 1u : 0u) << t;
         if (kImp) L.impm |= (imp ? 1u : 0u) << t;
         const float ct = (lamb && t == 0) ? sqrtf(uu.x) : hg_cos<kDeep>(uu.x, Q.hg_a, Q.hg_b, Q.hg_c, Q.hg_d, Q.hg_e);
-        const float ch = sqrtf(fmaxf(0.f, __fmul_rn(0.5f, __fadd_rn(1.f, ct))));  // cos(theta / 2)
-        const float sh = sqrtf(fmaxf(0.f, __fmul_rn(0.5f, __fsub_rn(1.f, ct))));  // sin(theta / 2)
+        const float ch = sqrtf(fmaxf(0.f, fmaf(0.5f, ct, 0.5f)));       // cos(theta / 2)
+        const float sh = sqrtf(fmaxf(0.f, fmaf(-0.5f, ct, 0.5f)));      // sin(theta / 2)
         float sph, cph;                                                 // half the azimuth, uniform
         __sincosf(__fmul_rn(3.14159265358979324f, __fsub_rn(uu.y, 0.5f)), &sph, &cph);
         L.qs[t] = make_float4(__fmul_rn(cph, ch), -__fmul_rn(sph, sh), __fmul_rn(cph, sh), __fmul_rn(sph, ch));
@@ -934,41 +955,108 @@ __device__ __forceinline__ int pass_end(Photon &Q, int adv, bool ev, const float
 // One block pass over photon Q, held alike by every lane of the warp, the chunks
 // walked one after the other until the first with an event.  Q is updated alike
 // on every lane; returns the end condition.  Warp-collective.
+//
+// A chunk takes about 430 instructions a lane, bound by the FP32 pipe (a step's 20 wide
+// integer products hold it 80 cycles, the Hamilton products of the scan 160 a chunk) and
+// the issue slots, at 16 warps an SM.  The scans go through shared memory, and what only
+// the pass's last step needs is left to the pass's end (with shuffles and selects, and the
+// event's values kept for every chunk, 480 instructions: a sweep of 64 configs, 3.1e9
+// events of which 70% in passes, 24.9 -> 23.5 ms).  Two chunks a round with packed operations
+// are 300 instructions a chunk but hold the FP32 pipe as long (23.7 ms), and 128 registers:
+// the walk of 1e6 photons, which hardly reaches this, 332 -> 343 us; a third block an SM
+// (80 registers) spills, 24.3 ms.
 template <int LS, bool kImp, bool kDeep>
-__device__ __forceinline__ int block_pass(Photon &Q, const WalkArgs &a, int lane) {
+__device__ __forceinline__ int block_pass(Photon &Q, const WalkArgs &a, PassScan &S, int lane) {
     const bool reflected = (Q.flags & kFlagReflect) != 0;
-    const PassFrame F = pass_frame(Q, reflected);
+    float e1z2, e2z2, d0z;                 // the frame's z row, its first two doubled (exact)
+    {
+        const PassFrame F = pass_frame(Q, reflected);
+        e1z2 = 2.f * F.e1z, e2z2 = 2.f * F.e2z, d0z = F.d0z;
+    }
     float4 W = q_identity();               // rotation of the earlier chunks
     float Wz = 0.f, Wp = 0.f;              // their vertical moves and path increments
     for (int c = 0;; ++c) {
         LaneSteps<LS> L;
         lane_draw<LS, kImp, kDeep>(L, Q, (uint32_t)Q.i + 1u + (uint32_t)((32 * LS) * c + LS * lane),
                   reflected && c == 0 && lane == 0, a);
-        const float4 qi = warp_scan_q(lane_product<LS>(L), lane);
-        float4 xl = shfl_q(qi, (lane + 31) & 31);
-        if (lane == 0) xl = q_identity();
-        lane_prefixes<LS>(L, qmul(W, xl));
-        float dz[LS], zs, ps;
-        lane_moves<LS>(L, F, Q.inv_ext, dz, zs, ps);
-        warp_scan_2(zs, ps, lane);
-        float zx = __shfl_up_sync(0xffffffffu, zs, 1), px = __shfl_up_sync(0xffffffffu, ps, 1);
-        if (lane == 0) { zx = 0.f; px = 0.f; }
-        const LaneEvent E = lane_event<LS>(L, dz, Q, __fadd_rn(Wz, zx), __fadd_rn(Wp, px));
-        const unsigned ev = __ballot_sync(0xffffffffu, E.first < LS);
+        float4 q = lane_product<LS>(L);
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+            S.q[r & 1][16 + lane] = q;
+            __syncwarp();
+            q = qmul(S.q[r & 1][16 + lane - (1 << r)], q);
+        }
+        S.q[1][16 + lane] = q;
+        __syncwarp();
+        lane_prefixes<LS>(L, qmul(W, S.q[1][15 + lane]));
+        W = qmul(W, S.q[1][47]);
+        float zl[LS], pl[LS];
+#pragma unroll
+        for (int t = 0; t < LS; ++t) {
+            const float4 p = L.qs[t];
+            const float c0 = fmaf(p.y, p.w, __fmul_rn(p.x, p.z));
+            const float c1 = fmaf(p.z, p.w, -__fmul_rn(p.x, p.y));
+            const float c2 = fmaf(-2.f, fmaf(p.y, p.y, __fmul_rn(p.z, p.z)), 1.f);
+            const float dz = __fmul_rn(L.dtau[t], fmaf(e1z2, c0, fmaf(e2z2, c1, __fmul_rn(d0z, c2))));
+            const float inc = __fmul_rn(L.dtau[t], Q.inv_ext);
+            zl[t] = t == 0 ? dz : __fadd_rn(zl[t - 1], dz);
+            pl[t] = t == 0 ? inc : __fadd_rn(pl[t - 1], inc);
+        }
+        float2 zp = make_float2(zl[LS - 1], pl[LS - 1]);
+#pragma unroll
+        for (int r = 0; r < 5; ++r) {
+            S.zp[r & 1][16 + lane] = zp;
+            __syncwarp();
+            const float2 l = S.zp[r & 1][16 + lane - (1 << r)];
+            zp = make_float2(__fadd_rn(zp.x, l.x), __fadd_rn(zp.y, l.y));
+        }
+        S.zp[1][16 + lane] = zp;
+        __syncwarp();
+        const float2 before = S.zp[1][15 + lane], sum = S.zp[1][47];
+        const float zx = __fadd_rn(Wz, before.x);
+        bool event = false;
+        float zk[LS];
+#pragma unroll
+        for (int t = 0; t < LS; ++t) {
+            zk[t] = __fadd_rn(Q.z, __fadd_rn(zx, zl[t]));
+            event = event || zk[t] > 0.f || zk[t] < -Q.tau || ((L.absm >> t) & 1u);
+        }
+        const unsigned ev = __ballot_sync(0xffffffffu, event);
         if (ev || c == kPassChunks - 1) {
             const int e = ev ? __ffs(ev) - 1 : 31;
-            const float4 d = lane_step_dir<LS>(L, F, E.ts, Q.inv_ext);
+            int ts = LS - 1;
+            unsigned what = 0;
+            float zb = __fadd_rn(Q.z, zx);                             // before the step
+            float ze = 0.f, z0 = 0.f, pe = 0.f, dt = 0.f;
+            float4 rot = L.qs[0];
+            bool found = false;
+#pragma unroll
+            for (int t = 0; t < LS; ++t) {
+                const bool top = zk[t] > 0.f, bot = zk[t] < -Q.tau;
+                if (!found && (top || bot || ((L.absm >> t) & 1u) || t == LS - 1)) {
+                    found = true;
+                    ts = t;
+                    what = (top ? 1u : 0u) | (bot ? 2u : 0u) | (((L.impm >> t) & 1u) << 2) | (((L.reflm >> t) & 1u) << 3);
+                    ze = zk[t];
+                    z0 = zb;
+                    pe = __fadd_rn(__fadd_rn(Wp, before.y), pl[t]);
+                    rot = L.qs[t];
+                    dt = L.dtau[t];
+                }
+                zb = zk[t];
+            }
+            const float3 d = pass_dir(pass_frame(Q, reflected), rot);
             const float4 dir = make_float4(__shfl_sync(0xffffffffu, d.x, e), __shfl_sync(0xffffffffu, d.y, e),
-                                           __shfl_sync(0xffffffffu, d.z, e), __shfl_sync(0xffffffffu, d.w, e));
-            const int ts = __shfl_sync(0xffffffffu, E.ts, e);
-            const float ze = __shfl_sync(0xffffffffu, E.zk, e), zp = __shfl_sync(0xffffffffu, E.zp, e);
-            const float pe = __shfl_sync(0xffffffffu, E.pk, e);
-            const unsigned what = __shfl_sync(0xffffffffu, E.what, e);
-            return pass_end(Q, (32 * LS) * c + LS * e + ts + 1, ev != 0, dir, ze, zp, pe, what);
+                                           __shfl_sync(0xffffffffu, d.z, e),
+                                           __shfl_sync(0xffffffffu, __fmul_rn(dt, Q.inv_ext), e));
+            ts = __shfl_sync(0xffffffffu, ts, e);
+            ze = __shfl_sync(0xffffffffu, ze, e), z0 = __shfl_sync(0xffffffffu, z0, e);
+            pe = __shfl_sync(0xffffffffu, pe, e);
+            what = __shfl_sync(0xffffffffu, what, e);
+            return pass_end(Q, (32 * LS) * c + LS * e + ts + 1, ev != 0, dir, ze, z0, pe, what);
         }
-        W = qmul(W, shfl_q(qi, 31));
-        Wz = __fadd_rn(Wz, __shfl_sync(0xffffffffu, zs, 31));
-        Wp = __fadd_rn(Wp, __shfl_sync(0xffffffffu, ps, 31));
+        Wz = __fadd_rn(Wz, sum.x);
+        Wp = __fadd_rn(Wp, sum.y);
     }
 }
 
@@ -1168,6 +1256,7 @@ __global__ void __launch_bounds__(256, 2) walk_f32_kernel(const WalkArgs a) {
     const int32_t *claim_cfg = staged ? sclaim_cfg : a.claim_cfg;
     WarpQueues &q = queues[warp];
     warp_tally_reset(q.tally, lane);
+    pass_scan_init(q.scan, lane);
     __syncthreads();
 
     Photon P;
@@ -1303,10 +1392,10 @@ __global__ void __launch_bounds__(256, 2) walk_f32_kernel(const WalkArgs a) {
             Photon Q = shfl_photon(P, src);
             int c;
             if constexpr (kLongLaneSteps != kLaneSteps)
-                c = Q.i >= kLongWalk ? block_pass<kLongLaneSteps, kImpurity, kDeep>(Q, a, lane)
-                                     : block_pass<kLaneSteps, kImpurity, kDeep>(Q, a, lane);
+                c = Q.i >= kLongWalk ? block_pass<kLongLaneSteps, kImpurity, kDeep>(Q, a, q.scan, lane)
+                                     : block_pass<kLaneSteps, kImpurity, kDeep>(Q, a, q.scan, lane);
             else
-                c = block_pass<kLaneSteps, kImpurity, kDeep>(Q, a, lane);
+                c = block_pass<kLaneSteps, kImpurity, kDeep>(Q, a, q.scan, lane);
             if (lane == src) {
                 P.i = Q.i;
                 P.flags = Q.flags;

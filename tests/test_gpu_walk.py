@@ -332,6 +332,30 @@ def test_f32_records_independent_of_photon_count(walker, case):
     assert np.array_equal(small.records, big.records[:300])
 
 
+@pytest.mark.parametrize('n', [1, 33, 3000])
+@pytest.mark.parametrize('case', ['cfg2', 'imp'])
+@pytest.mark.parametrize('tau', [25.0, 4000.0])
+def test_f32_long_walks_same_records_in_warps_and_blocks(walker, case, n, tau):
+    """Walks past 256 steps (nearly conservative snow over a half-reflecting ground, thin
+    enough for bottom reflections or deep): passes walked by a warp, chunk after chunk
+    with its scans in shared memory, and by a block of the drain kernel, a warp per chunk
+    with its scans in registers, give the same records."""
+    cfg, ice, imp = cfg2_geometry(n) if case == 'cfg2' else _golden_case('imp', n)
+    cfg = dataclasses.replace(cfg, n_photon=n, ssa_ice_override=0.9998, tau_tot=tau, lambertian_bottom=True,
+                              lambertian_reflectance=0.9)
+    walker.set_tables([ice], imp)
+    saved = walker.get_launch()
+    try:
+        walker.set_launch(256, 0, 8, 0)
+        a = walker.walk([cfg], 7, mode='f32')
+        walker.set_launch(256, 0, 8, 256)
+        b = walker.walk([cfg], 7, mode='f32')
+    finally:
+        walker.set_launch(**saved)
+    assert n < 3000 or int(a.tallies['max_n_scat'][0]) > 256
+    assert np.array_equal(a.records, b.records) and np.array_equal(a.tallies, b.tallies)
+
+
 @pytest.mark.parametrize('n', [1, 2, 3, 5, 8, 12])
 def test_f32_sparse_rounds_same_records(walker, n):
     """A launch of n photons walks them in sparse rounds (32 / n steps of each photon
