@@ -342,7 +342,7 @@ def test_f32_long_walks_same_records_in_warps_and_blocks(walker, case, n, tau):
     with its scans in registers, give the same records."""
     cfg, ice, imp = cfg2_geometry(n) if case == 'cfg2' else _golden_case('imp', n)
     cfg = dataclasses.replace(cfg, n_photon=n, ssa_ice_override=0.9998, tau_tot=tau, lambertian_bottom=True,
-                              lambertian_reflectance=0.9)
+                              lambertian_reflectance=0.9, imp_cnc=1e-9 if case == 'imp' else 0.0)
     walker.set_tables([ice], imp)
     saved = walker.get_launch()
     try:
