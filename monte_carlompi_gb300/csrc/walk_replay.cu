@@ -12,23 +12,28 @@
 // pipe, however many of its lanes are active and whether or not it waits for the one before.  A
 // walk of one thread's own took about 170 of them per event, 5.6 us, and the longest walk of
 // 10,000 photons has 25,000 events.  So the work is laid out across lanes and warps:
-//  * a block of two warps holds up to eight photons.  The producer warp draws the steps ahead,
-//    32 at a time (all of one photon's, or four each of eight): angles, optical path, path
-//    increment, absorption; none of them depends on where the photon is;
-//  * the consumer warp walks the chain that remains with four lanes a photon: Z carries mu_z
-//    (which depends on mu_z alone) one step ahead of X, Y (mu_x, mu_y) and M (depth, path, end
-//    conditions), and each of the eleven FP64 instructions of a step serves all four;
+//  * a block of four warps holds up to sixteen photons and walks them in rounds of 32 steps (all of
+//    one photon's, or two each of sixteen), its warps a round apart: the first draws the steps
+//    (angles, optical path, path increment, absorption; none of them depends on where the photon
+//    is), the second walks mu_z, which depends on mu_z alone, the third mu_x and mu_y, the fourth
+//    depth and path, where a walk ends.  So a lone photon's step costs what the longest of the
+//    three chains costs, mu_z's twelve FP64 instructions one after the other;
+//  * in those chains every FP64 instruction takes its operands from another FP64 instruction or
+//    from memory: a result that a select, a shuffle or a test takes first costs 110 to 290 cycles
+//    on its way to the next instead of 66.  Directions about the vertical, which need one, are
+//    walked again with it when the chain turns out to have met one;
 //  * sqrt(1 - mu_z^2) and its reciprocal come from one Newton step and a residual correction
 //    (Markstein, IBM J. Res. Dev. 34, 1990), six operations, and the two divisions by it take
 //    three each.
-// The producer assumes that a step does nothing but scatter; a photon that ends, is reflected or
-// is replaced sits out the round that was drawn for it.  Every value is the one-thread walk's, in
+// The draws assume that a step does nothing but scatter: a photon that ends, is reflected or is
+// replaced sits out the two rounds under way.  Every value is the one-thread walk's, in
 // its order of operations: sqrt and quotients are correctly rounded but where the exact value
 // lies within 2^-28 ulp of a rounding boundary (of 1.2e9 random arguments one sqrt and two quotients differ from
 // CUDA's, by an ulp).
-// 10,000 photons of the driver's default run: 193.7 ms on one thread each, 30.5 ms now (0.94 us an
-// event of the longest: a result that another pipe selects or shuffles before the next FP64
-// instruction costs 110 to 117 cycles instead of 66).
+// 10,000 photons of the reference's default run: 193.7 ms on one thread each; 30.5 ms (0.94 us an
+// event of the longest walk) with one warp drawing and one walking, four lanes a photon, each
+// FP64 instruction serving all four through selects and shuffles; 16.0 ms now (0.47 us, 970
+// cycles an event, of which mu_z's chain is 880).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -365,7 +370,7 @@ __global__ void __launch_bounds__(128) walk_replay_pol_kernel(const ReplayArgs a
 
 // ---------------------------------------------------------------- the HG walk
 
-constexpr int kSlots = 8;                    // photons a block walks at once
+constexpr int kSlots = 16;                   // photons a block walks at once
 constexpr uint32_t kRefl = 1u, kSurface = 2u, kBottom = 4u, kIso = 8u, kActive = 16u;
 
 // A photon in flight (shared memory).
@@ -391,25 +396,26 @@ struct Finished {
 };
 
 // 32 steps drawn ahead, S of each of n photons: entry rank * S + t is step t of photon `rank`.
+// Each warp of the block adds its part, a round after the warp before it.
 struct Ahead {
     double ct[32], st[32], cp[32], sp[32], dtau[32], inc[32];
     uint32_t fl[32];                         // 1 absorbed here, 2 by ice
-    int32_t n, S;
-    int32_t slot[kSlots], steps[kSlots], lamb[kSlots], shift[kSlots];
-    uint64_t rid[kSlots], k0[kSlots], k1[kSlots];   // photon, its stream before and after the steps
-    // whether rank r's entries are those of its slot's photon as it stands
-    __device__ __forceinline__ bool holds(int r, const Slot *slots) const {
-        if (r >= n) return false;
-        const Slot &s = slots[slot[r]];
-        return (s.flags & kActive) && s.rid == rid[r] && s.k == k0[r] && (int)s.lambertian() == lamb[r];
-    }
+    int32_t n, S, pole;                      // pole: a step about the vertical among them
+    int32_t slot[kSlots], steps[kSlots], lamb[kSlots], first[kSlots], shift[kSlots];
+    uint32_t gen[kSlots];                    // the slot's count of events that the draws assume
+    uint64_t k0[kSlots];                     // the photon's stream before the steps
+    double mzb[32], sq[32], h2[32], mz[32];  // Z: mu_z before, sqrt(1 - mu_z^2), 1 / that, mu_z after
+    double x[32], y[32], z[32], path[32];    // XY and M: the state after the step
 };
 
 struct ReplayBlock {
-    Ahead ahead[2];
+    Ahead ahead[3];
     Slot slots[kSlots], born[32];
     Finished fin[32];
-    double lamb_ct[kSlots];
+    uint32_t gen[kSlots];                    // events of the slot's photons so far
+    uint32_t drawn_gen[kSlots];              // producer: the count at its last draw,
+    uint64_t next_k[kSlots];                 // and the stream after it
+    double mz[kSlots];                       // Z: mu_z after its last steps
     int32_t stop;
 };
 
@@ -443,6 +449,7 @@ __device__ __forceinline__ bool below_minus(double x, double t) {
     const uint64_t b = to_bits(x), m = b & 0x7fffffffffffffffull;
     return (b >> 63) && m > to_bits(t) && m <= 0x7ff0000000000000ull;
 }
+__device__ __forceinline__ bool is_nan(double x) { return (to_bits(x) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull; }
 __device__ __forceinline__ bool is_unit(double x) { return (to_bits(x) & 0x7fffffffffffffffull) == 0x3ff0000000000000ull; }
 
 // A power-of-two factor by the exponent (normal, finite x).
@@ -553,24 +560,21 @@ __device__ int replay_birth(const ReplayArgs &a, int64_t gid, Slot &out) {
     return cond;
 }
 
-// The producer's round: the next steps of the block's photons into `next`, assuming that those of
-// `now` (being walked) end in nothing.  Arrives at barrier 2 once it has read the slots.
-__device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, const Ahead &now, Ahead &next, int lane) {
+// The producer's round: the next steps of the block's photons into `next`, assuming that those
+// drawn before and not yet walked end in nothing.
+__device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, Ahead &next, int lane) {
     const unsigned act = __ballot_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive));
     const int n = __popc(act);
     const int S = n <= 1 ? 32 : 1 << (5 - (32 - __clz(n - 1)));       // 32 / n, a power of two
     const int rank = lane / S, t = lane % S;
     const bool mine = rank < n;
     const int si = mine ? __fns(act, 0, rank + 1) : 0;
+    const uint32_t gen = B.gen[si];
+    const bool first = B.drawn_gen[si] != gen;
     Slot s = B.slots[si];
-    bool lamb = s.lambertian();
-    for (int r = 0; r < now.n; ++r)
-        if (now.slot[r] == si && now.holds(r, B.slots)) {
-            s.k = now.k1[r];
-            lamb = (s.flags & kSurface) != 0;
-        }
+    if (!first) s.k = B.next_k[si];
+    const bool lamb = first ? s.lambertian() : (s.flags & kSurface) != 0;
     __syncwarp();
-    asm volatile("bar.arrive 2, 64;\n" ::: "memory");
     // a Lambertian direction first (:1238-1250): its photon's lanes test pairs of uniforms past the
     // step's five, and the first that passes is taken
     int shift = 0;
@@ -632,11 +636,14 @@ __device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, const Ahead &now
             next.slot[rank] = si;
             next.steps[rank] = steps;
             next.lamb[rank] = lamb ? 1 : 0;
+            next.first[rank] = first ? 1 : 0;
             next.shift[rank] = shift;
-            next.rid[rank] = s.rid;
+            next.gen[rank] = gen;
             next.k0[rank] = s.k;
-            next.k1[rank] = s.k + 5 * (uint64_t)steps + shift;
-            if (next.k1[rank] > (1ull << 33)) atomicOr(a.status, kStatusStream);
+            const uint64_t k1 = s.k + 5 * (uint64_t)steps + shift;
+            B.drawn_gen[si] = gen;
+            B.next_k[si] = k1;
+            if (k1 > (1ull << 33)) atomicOr(a.status, kStatusStream);
         }
     }
     if (lane == 0) {
@@ -645,124 +652,183 @@ __device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, const Ahead &now
     }
 }
 
-// The consumer's chain over the steps in `now` (see the top of the file).  Four lanes a photon: 0 Z,
-// 1 X, 2 Y, 3 M.  Returns, on an M lane, the photon's end condition.  The slots are written only
-// after barrier 2 (the producer has read them).
-__device__ int walk_ahead(const ReplayArgs &a, ReplayBlock &B, const Ahead &now, int lane) {
-    const int role = lane & 3, r = lane >> 2;
-    const bool isZ = role == 0, isM = role == 3, isX = role == 1;
-    const bool held = now.holds(r, B.slots);
-    const int si = held ? now.slot[r] : 0, S = now.S;
-    const int base = held ? r * S : 0, steps = held ? now.steps[r] : 0;
-    Slot &slot = B.slots[si];
+// Whether rank r's steps are those that its slot's photon takes: nothing has happened to it since.
+__device__ __forceinline__ bool holds(const ReplayBlock &B, const Ahead &A, int r) {
+    return r < A.n && A.gen[r] == B.gen[A.slot[r]];
+}
+
+// Z: the chain of mu_z over the steps drawn in the round before, a lane per photon:
+// mu_z' = mu_z ct - sqrt(1 - mu_z^2) st cp (:1277), which depends on mu_z alone.  kPole: with the
+// directions about the vertical (:1262-1269): mu_z = +-1, or a Lambertian direction.
+template <bool kPole>
+__device__ __forceinline__ double z_chain(Ahead &A, double mz, const int base, const int steps, const int S) {
+    double ct = A.ct[base], st = A.st[base], cp = A.cp[base];
+    for (int it = 0; it < S; ++it) {
+        const int e = base + it, e1 = base + min(it + 1, S - 1);
+        const double ct1 = A.ct[e1], st1 = A.st[e1], cp1 = A.cp[e1];
+        const double x = 1.0 - mz * mz;
+        const double y0 = rsqrt_seed(x), u = mz * ct;
+        const double h = halved(y0), g = x * y0;
+        const double r = fma(-g, h, 0.5);
+        const double g1 = fma(g, r, g), h1 = fma(h, r, h);
+        const double sq = fma(fma(-g1, g1, x), h1, g1);
+        double nz = (sq * -st) * cp + u;
+        if (kPole && is_unit(mz)) nz = to_bits(mz) >> 63 ? -ct : ct;
+        if (it < steps) {
+            A.mzb[e] = mz;
+            A.sq[e] = sq;
+            A.h2[e] = doubled(h1);
+            A.mz[e] = nz;
+        }
+        mz = nz;
+        ct = ct1, st = st1, cp = cp1;
+    }
+    return mz;
+}
+
+// A test of mu_z inside the chain costs 210 cycles a step beside its 880.  So it is walked without
+// one: past the vertical it is all NaN (0 times infinity), and then walked again with it.
+__device__ void walk_z(ReplayBlock &B, Ahead &A, int lane) {
+    const bool held = lane < kSlots && holds(B, A, lane & (kSlots - 1));
+    if (!__any_sync(0xffffffffu, held)) return;
+    const int S = A.S, base = held ? lane * S : 0, steps = held ? A.steps[lane] : 0, si = held ? A.slot[lane] : 0;
+    const double mz0 = !held ? 0.5 : (A.lamb[lane] ? 1.0 : (A.first[lane] ? B.slots[si].muz : B.mz[si]));
+    double mz = mz0;
+    bool pole = __any_sync(0xffffffffu, is_unit(mz0));
+    if (!pole) {
+        mz = z_chain<false>(A, mz0, base, steps, S);
+        // (a photon on a surface, of fewer steps, starts every one from the vertical)
+        pole = __any_sync(0xffffffffu, held && steps == S && is_nan(mz));
+    }
+    if (pole) mz = z_chain<true>(A, mz0, base, steps, S);
+    if (held) B.mz[si] = mz;
+    if (lane == 0) A.pole = pole ? 1 : 0;
+}
+
+// XY: mu_x and mu_y over the steps that Z walked in the round before, two lanes a photon:
+// mu_x' = st (mu_x mu_z cp - mu_y sp) / sqrt(1 - mu_z^2) + mu_x ct, mu_y' alike (:1270-1276).
+template <bool kPole>
+__device__ __forceinline__ void xy_chain(Ahead &A, double va, double vb, const int base, const int steps, const int S,
+                                         const bool isX, const int lane) {
+    double *out = isX ? A.x : A.y;
+    double mzb = A.mzb[base], ct = A.ct[base], st = A.st[base], cp = A.cp[base], sp = A.sp[base], sq = A.sq[base],
+           h2 = A.h2[base];
+    for (int it = 0; it < S; ++it) {
+        const int e = base + it, e1 = base + min(it + 1, S - 1);
+        const double mzb1 = A.mzb[e1], ct1 = A.ct[e1], st1 = A.st[e1], cp1 = A.cp[e1], sp1 = A.sp[e1], sq1 = A.sq[e1],
+                     h21 = A.h2[e1];
+        const double p = va * mzb, w = va * ct;
+        const double num = st * (p * cp + vb * (isX ? -sp : sp));
+        const double q = num * h2;
+        double nv = fma(fma(-q, sq, num), h2, q) + w;
+        if (kPole) {
+            const double v = st * (isX ? cp : sp);
+            if (is_unit(mzb)) nv = isX || !(to_bits(mzb) >> 63) ? v : -v;
+        }
+        if (it < steps) out[e] = nv;
+        va = nv;
+        vb = shfl_d(nv, lane ^ 1);
+        mzb = mzb1, ct = ct1, st = st1, cp = cp1, sp = sp1, sq = sq1, h2 = h21;
+    }
+}
+
+__device__ void walk_xy(ReplayBlock &B, Ahead &A, int lane) {
+    const int rk = lane >> 1;
+    const bool isX = !(lane & 1), held = holds(B, A, rk);
+    if (!__any_sync(0xffffffffu, held)) return;
+    const int S = A.S, base = held ? rk * S : 0, steps = held ? A.steps[rk] : 0;
+    const Slot &slot = B.slots[held ? A.slot[rk] : 0];
+    const bool lamb = !held || A.lamb[rk];
+    const double va = lamb ? 0.0 : (isX ? slot.mux : slot.muy), vb = lamb ? 0.0 : (isX ? slot.muy : slot.mux);
+    if (A.pole) xy_chain<true>(A, va, vb, base, steps, S, isX, lane);
+    else xy_chain<false>(A, va, vb, base, steps, S, isX, lane);
+}
+
+// M: depth and path over the same steps, two lanes a photon, and the first step with an end
+// condition (:1390-1466).  Returns, on the depth's lane, the steps walked, negative if the last is
+// such a step.
+__device__ int walk_m(ReplayBlock &B, Ahead &A, int lane) {
+    const int rk = lane >> 1;
+    const bool isz = !(lane & 1), held = holds(B, A, rk);
+    if (!__any_sync(0xffffffffu, held)) return 0;
+    A.z[lane] = A.dtau[lane] * A.mz[lane];
+    __syncwarp();
+    const int S = A.S, base = held ? rk * S : 0, steps = held ? A.steps[rk] : 0;
+    const Slot &slot = B.slots[held ? A.slot[rk] : 0];
     const double tau = slot.tau;
-    double mz = slot.muz, va = isX ? slot.mux : slot.muy, vb = isX ? slot.muy : slot.mux;
-    double z = slot.z, path = slot.path, zp = z, dt = 0, mzn = mz;
-    if (held && now.lamb[r]) { mz = 1.0; va = 0.0; vb = 0.0; }
-    double mzb = mz, sq = 1.0, h2 = 1.0;             // before the lagging step; sqrt(1 - mzb^2), 1 / that
-    bool alive = held;
-    int done = 0;                                    // M: steps walked
+    double acc = isz ? slot.z : slot.path;
+    const double *in = isz ? A.z : A.inc;
+    double *out = isz ? A.z : A.path;
+    int done = steps;
     bool event = false;
-    for (int it = 0; __any_sync(0xffffffffu, alive); ++it) {
-        const bool zs = alive && it < steps, ls = alive && it > 0;
-        const int lag = base + (it > 0 ? it - 1 : 0), cur = base + (it < S ? it : S - 1);
-        const int e = isZ ? cur : lag;
-        const double st = now.st[e], ct = isM ? now.ct[cur] : now.ct[e], cp = now.cp[e];
-        const double sp = isX ? -now.sp[e] : now.sp[e], dtau = now.dtau[e], inc = now.inc[e];
-        // 1: mz mz | a mzb | mz ct (Z's)
-        const double r1 = (isZ || isM ? mz : va) * (isZ ? mz : (isM ? ct : mzb));
-        const double u_z = shfl_d(r1, lane | 3);
-        // 2: 1 - . | . cp | dtau mz
-        const double r2 = fma(isM ? dtau : r1, isZ ? -1.0 : (isM ? mz : cp), isZ ? 1.0 : -0.0);
-        const double y0 = rsqrt_seed(isZ ? r2 : 1.0), h = halved(y0);
-        // 3: x y0 | b sp | z + .
-        const double r3 = fma(isZ ? r2 : (isM ? z : vb), isZ ? y0 : (isM ? 1.0 : sp), isM ? r2 : -0.0);
-        // 4: 1/2 - g h | sum | path + inc
-        const double r4 = fma(isZ ? r3 : (isM ? path : r2), isZ ? -h : 1.0, isZ ? 0.5 : (isM ? inc : r3));
-        // 5: g1 | st .
-        const double r5 = fma(isZ ? r3 : st, r4, isZ ? r3 : -0.0);
-        // 6: h1 | . / sq, approximate
-        const double r6 = fma(isZ ? h : r5, isZ ? r4 : h2, isZ ? h : -0.0);
-        // 7: residuals
-        const double r7 = fma(-(isZ ? r5 : r6), isZ ? r5 : sq, isZ ? r2 : r5);
-        // 8: sqrt | quotient
-        const double r8 = fma(r7, isZ ? r6 : h2, isZ ? r5 : r6);
-        // 9: -sq st | a ct
-        const double r9 = (isZ ? r8 : va) * (isZ ? -st : ct);
-        // 10: . cp | the new mu_x, mu_y
-        const double r10 = fma(isZ ? r9 : r8, isZ ? cp : 1.0, isZ ? -0.0 : r9);
-        // 11: the new mu_z
-        double nz = r10 + u_z, nxy = r10;
-        // about the vertical (:1262-1269): mu_z = +-1, or a Lambertian direction
-        const bool pole = isZ ? zs && is_unit(mz) : ls && is_unit(mzb);
-        if (__any_sync(0xffffffffu, pole)) {
-            const double p = st * (isX ? cp : sp);
-            if (pole) {
-                nz = mz > 0 ? ct : -ct;
-                nxy = isX || mzb > 0 ? p : -p;
+    double d = in[base];
+    uint32_t fl = A.fl[base];
+    for (int it = 0; it < S; ++it) {
+        const int e = base + it, e1 = base + min(it + 1, S - 1);
+        const double d1 = in[e1];
+        const uint32_t fl1 = A.fl[e1];
+        acc = acc + d;
+        if (it < steps) {
+            out[e] = acc;
+            if (!event && (is_pos(acc) || below_minus(acc, tau) || (fl & 1u))) {
+                event = true;
+                done = it + 1;
             }
         }
-        // M: the step before's end conditions (:1390-1466)
-        const bool end = isM && ls && (is_pos(r3) || below_minus(r3, tau) || (now.fl[e] & 1u));
-        const bool stop = (__ballot_sync(0xffffffffu, end) >> (lane | 3)) & 1u;
-        if (ls) {
-            va = nxy;
-            zp = z;
-            z = r3;
-            path = r4;
-            dt = dtau;
-            mzn = mz;
-            done = it;
-            event = end;
-        }
-        const double other = shfl_d(va, lane ^ 3);
-        if (!isZ && !isM) vb = other;
-        const double nmz = shfl_d(nz, lane & ~3), nsq = shfl_d(r8, lane & ~3), nh = shfl_d(r6, lane & ~3);
-        alive = alive && !stop && it < steps;
-        if (alive) {                                 // Z has walked step `it`
-            mzb = mz;
-            mz = nmz;
-            sq = nsq;
-            h2 = doubled(nh);
-        }
+        d = d1, fl = fl1;
     }
-    __syncwarp();
-    asm volatile("bar.sync 2, 64;\n" ::: "memory");
+    return event ? -done : done;
+}
+
+// The photons' states after the steps that XY and M walked: lane `rank` its photon's.  `walked`:
+// walk_m's result for it.  Returns its end condition.
+__device__ int commit(const ReplayArgs &a, ReplayBlock &B, const Ahead &A, int rank, int walked) {
+    const bool event = walked < 0;
+    const int done = event ? -walked : walked;
+    const int si = A.slot[rank], e = rank * A.S + done - 1;
+    Slot &slot = B.slots[si];
+    uint32_t flags = slot.flags & ~kRefl;
+    uint64_t k = A.k0[rank] + 5 * (uint64_t)done + A.shift[rank];
+    double z = A.z[e], path = A.path[e];
+    const double zp = done > 1 ? A.z[e - 1] : slot.z, mz = A.mz[e];
+    slot.mux = A.x[e];
+    slot.muy = A.y[e];
+    slot.muz = mz;
+    slot.i += done;
     int cond = 0;
-    if (held) {
-        if (isZ) slot.muz = mz;
-        else if (!isM) *(isX ? &slot.mux : &slot.muy) = va;
-        else {
-            uint32_t flags = slot.flags & ~kRefl;
-            uint64_t k = now.k0[r] + 5 * (uint64_t)done + now.shift[r];
-            slot.i += done;
-            if (event) {
-                const uint32_t f = now.fl[base + done - 1];
-                cond = step_end(slot, a.seed, z, zp, dt, mzn, path, false, f & 1u, f & 2u, &k, &flags);
-            }
-            slot.z = z;
-            slot.path = path;
-            slot.k = k;
-            slot.flags = flags;
-        }
+    if (event) {
+        const uint32_t f = A.fl[e];
+        cond = step_end(slot, a.seed, z, zp, A.dtau[e], mz, path, false, f & 1u, f & 2u, &k, &flags);
+        B.gen[si] += 1;
     }
-    __syncwarp();
+    slot.z = z;
+    slot.path = path;
+    slot.k = k;
+    slot.flags = flags;
     return cond;
 }
 
-__global__ void __launch_bounds__(64) walk_replay_kernel(const ReplayArgs a) {
+__global__ void __launch_bounds__(128, 4) walk_replay_kernel(const ReplayArgs a) {
     __shared__ ReplayBlock B;
     const int lane = threadIdx.x & 31;
-    const bool producer = threadIdx.x >= 32;
+    // the warps' parts, turned by a warp from one block of an SM to the next, so that each of its
+    // four FP64 pipes gets one of each part
+    enum { kDraw, kZ, kXY, kM };
+    const int part = ((int)(threadIdx.x >> 5) + (int)((4ull * blockIdx.x) / gridDim.x)) & 3;
     const unsigned lt_mask = (1u << lane) - 1u;
-    if (threadIdx.x < kSlots) B.slots[threadIdx.x].flags = 0;
-    if (threadIdx.x == 0) {
-        B.ahead[0].n = 0;
-        B.ahead[0].S = 32;
-        B.stop = 0;
+    if (threadIdx.x < kSlots) {
+        B.slots[threadIdx.x].flags = 0;
+        B.gen[threadIdx.x] = 1;
+        B.drawn_gen[threadIdx.x] = 0;
     }
+    if (threadIdx.x < 3) {
+        B.ahead[threadIdx.x].n = 0;
+        B.ahead[threadIdx.x].S = 32;
+    }
+    if (threadIdx.x == 0) B.stop = 0;
+    __syncthreads();
     bool exhausted = false;
-    int n_born = 0, n_fin = 0;
+    int n_born = 0, n_fin = 0, walked = 0;
     const unsigned long long t0 = global_ns();
     auto flush = [&]() {                             // the queued records, one per lane
         if (lane < n_fin) {
@@ -779,57 +845,72 @@ __global__ void __launch_bounds__(64) walk_replay_kernel(const ReplayArgs a) {
         n_fin += __popc(m);
         __syncwarp();
     };
+    int drawn = 0;                                   // the buffer drawn into this round
     for (uint32_t round = 0;; ++round) {
+        Ahead &now = B.ahead[drawn], &before = B.ahead[drawn == 0 ? 2 : drawn - 1],
+              &last = B.ahead[drawn == 2 ? 0 : drawn + 1];
+        if (part == kM) {
+            // ---- the steps of `now`, walked in the round before: states, ends
+            // (the buffer is the one that is drawn into next)
+            const bool mine = lane < kSlots && holds(B, now, lane & (kSlots - 1));
+            const int w = __shfl_sync(0xffffffffu, walked, (2 * lane) & 31);
+            const int si = mine ? now.slot[lane] : 0;
+            const int cond = mine ? commit(a, B, now, lane, w) : 0;
+            __syncwarp();
+            // ---- finished photons leave their slots
+            if (__any_sync(0xffffffffu, cond != 0)) {
+                Slot &s = B.slots[si];
+                if (n_fin > 32 - kSlots) flush();
+                queue(cond != 0, s, cond);
+                if (cond) s.flags = 0;
+                __syncwarp();
+            }
+            // ---- free slots take photons already born; 32 at most are born at once
+            unsigned idle = ~__ballot_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive)) &
+                            ((1u << a.slots) - 1u);
+            for (int tries = 0; tries < 4 && idle && n_born == 0 && !exhausted; ++tries) {
+                if (n_fin > 0) flush();
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(a.work, (unsigned long long)a.claim);
+                base = __shfl_sync(0xffffffffu, base, 0);
+                const int64_t left = a.total - (int64_t)base;
+                const int valid = (int)max((int64_t)0, min((int64_t)a.claim, left));
+                exhausted = left <= a.claim;
+                int c1 = 0;
+                Slot s;
+                if (lane < valid) c1 = replay_birth(a, (int64_t)base + lane, s);
+                queue(lane < valid && c1 != 0, s, c1);
+                const unsigned m = __ballot_sync(0xffffffffu, lane < valid && c1 == 0);
+                if (lane < valid && c1 == 0) B.born[__popc(m & lt_mask)] = s;
+                n_born = __popc(m);
+                __syncwarp();
+            }
+            const int take = min(__popc(idle), n_born);
+            if (lane < take) {
+                const int f = __fns(idle, 0, lane + 1);
+                B.slots[f] = B.born[n_born - 1 - lane];
+                B.gen[f] += 1;
+            }
+            n_born -= take;
+            __syncwarp();
+            const bool any = __any_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive));
+            int stop = !any && exhausted && n_born == 0;
+            if ((round & 63u) == 63u && lane == 0) { // time budget (watchdog)
+                if (global_ns() - t0 > a.budget_ns) atomicOr(a.status, kStatusBudget);
+                if (*(volatile unsigned int *)a.status) stop = 1;
+            }
+            if (lane == 0 && stop) B.stop = 1;
+        }
         __syncthreads();
         if (B.stop) break;
-        const Ahead &now = B.ahead[round & 1];
-        if (producer) {
-            draw_ahead(a, B, now, B.ahead[(round & 1) ^ 1], lane);
-            continue;
-        }
-        const int cond = walk_ahead(a, B, now, lane);
-        // ---- finished photons leave their slots
-        if (__any_sync(0xffffffffu, cond != 0)) {
-            Slot &s = B.slots[cond ? now.slot[lane >> 2] : 0];
-            queue(cond != 0, s, cond);
-            if (cond) s.flags = 0;
-            __syncwarp();
-            if (n_fin > 32 - kSlots) flush();
-        }
-        // ---- free slots take photons already born; 32 at most are born at once
-        unsigned idle = ~__ballot_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive)) &
-                        ((1u << a.slots) - 1u);
-        for (int tries = 0; tries < 4 && idle && n_born == 0 && !exhausted; ++tries) {
-            if (n_fin > 0) flush();
-            unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(a.work, (unsigned long long)a.claim);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            const int64_t left = a.total - (int64_t)base;
-            const int valid = (int)max((int64_t)0, min((int64_t)a.claim, left));
-            exhausted = left <= a.claim;
-            int c1 = 0;
-            Slot s;
-            if (lane < valid) c1 = replay_birth(a, (int64_t)base + lane, s);
-            queue(lane < valid && c1 != 0, s, c1);
-            const unsigned m = __ballot_sync(0xffffffffu, lane < valid && c1 == 0);
-            if (lane < valid && c1 == 0) B.born[__popc(m & lt_mask)] = s;
-            n_born = __popc(m);
-            __syncwarp();
-            if (n_fin > 32 - kSlots) flush();
-        }
-        const int take = min(__popc(idle), n_born);
-        if (lane < take) B.slots[__fns(idle, 0, lane + 1)] = B.born[n_born - 1 - lane];
-        n_born -= take;
-        __syncwarp();
-        const bool any = __any_sync(0xffffffffu, lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive));
-        int stop = !any && exhausted && n_born == 0;
-        if ((round & 63u) == 63u && lane == 0) {     // time budget (watchdog)
-            if (global_ns() - t0 > a.budget_ns) atomicOr(a.status, kStatusBudget);
-            if (*(volatile unsigned int *)a.status) stop = 1;
-        }
-        if (lane == 0 && stop) B.stop = 1;
+        if (part == kDraw) draw_ahead(a, B, now, lane);
+        else if (part == kZ) walk_z(B, before, lane);
+        else if (part == kXY) walk_xy(B, last, lane);
+        else walked = walk_m(B, last, lane);
+        __syncthreads();
+        drawn = drawn == 2 ? 0 : drawn + 1;
     }
-    if (!producer && n_fin > 0) flush();
+    if (part == kM && n_fin > 0) flush();
 }
 
 }  // namespace
@@ -842,14 +923,14 @@ cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s
         walk_replay_pol_kernel<<<(unsigned)grid, block, 0, s>>>(a);
         return cudaGetLastError();
     }
-    // four blocks (eight warps) an SM keep its four FP64 pipes busy; few photons are spread over
-    // all of them
+    // four blocks an SM (126 registers), a warp of each part on each of its four FP64 pipes; few
+    // photons are spread over all of them
     ReplayArgs b = a;
     const int64_t blocks = std::min<int64_t>(4 * (int64_t)std::max(1, sm_count), a.total);
     const int64_t each = (a.total + blocks - 1) / blocks;
     b.slots = (int32_t)std::min<int64_t>(kSlots, each);
     b.claim = (int32_t)std::min<int64_t>(32, each);
-    walk_replay_kernel<<<(unsigned)blocks, 64, 0, s>>>(b);
+    walk_replay_kernel<<<(unsigned)blocks, 128, 0, s>>>(b);
     return cudaGetLastError();
 }
 

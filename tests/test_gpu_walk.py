@@ -855,3 +855,21 @@ def test_pol32_records_independent_of_spread_and_table_path(walker, n):
     assert np.array_equal(walker.walk([small], 8, mode='pol32').records, big[:n])
     two = walker.walk([small, dataclasses.replace(small, ice_table=1)], 8, mode='pol32').records
     assert np.array_equal(two[:n], big[:n])
+
+
+@pytest.mark.parametrize('n', [1, 2, 3, 5, 16, 17, 700])
+@pytest.mark.parametrize('case', ['cfg2', 'vertical', 'imp', 'lamsurf'])
+def test_replay_records_independent_of_photon_count(walker, case, n):
+    """Replay records of n photons (one photon's 32 steps a round up to two steps of sixteen, slots
+    refilled as walks end) are the first n of a run that fills every block: a beam along the
+    vertical (the pole case), reflections at the bottom, impurities and a Lambertian surface."""
+    if case in ('cfg2', 'vertical'):
+        cfg, ice, imp = cfg2_geometry(n)
+        if case == 'vertical':
+            cfg = dataclasses.replace(cfg, theta0_deg=0.0, tau_tot=8.0, lambertian_reflectance=0.9)
+    else:
+        cfg, ice, imp = _golden_case(case, n)
+    walker.set_tables([ice], imp)
+    big = walker.walk([dataclasses.replace(cfg, n_photon=11000)], 3, mode='replay64').records
+    got = walker.walk([cfg], 3, mode='replay64').records
+    assert np.array_equal(got, big[:n])
