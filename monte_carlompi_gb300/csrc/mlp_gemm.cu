@@ -19,11 +19,17 @@
 //    for the weight gradient of 65,536 rows);
 //  * the copying and the issuing loops are run by whole warps, one elected lane issuing: under
 //    `lane == 0` every tcgen05.mma took about 200 cycles to issue (its descriptors had to be moved
-//    into uniform registers; a chain of 1,024 chunks 440 us, now 201);
+//    into uniform registers; a chain of 1,024 chunks 440 us, then 201), and the next stage's
+//    barrier is looked at before a stage's MMAs are issued;
 //  * tiles are 64 or 32 columns wide, so that four CTAs share an SM or a small product is spread
 //    over more SMs (the rules in launch_batch have the times).
 // The epilogue goes through a 32 x 33 tile per warp once: a lane then holds one output column of
 // 32 rows, so loads and stores are whole row runs, and bias gradients are the lane's running sum.
+// At large sizes it is what bounds the launch, by its instructions: a block with all its rows and
+// columns has an instance without predicates, its pointers moving a row at a time, and the SiLU'
+// quotient takes five instructions instead of a division (32 instead of 47 instructions an element
+// with a bias and SiLU, 70 instead of 96 with SiLU', 19 instead of 26 for the output: the autograd
+// pass of 65,536 rows 742 -> 625 us with the stages above, the ensemble's training step 92 -> 81).
 //
 // Every mbarrier wait is bounded (2 s of %globaltimer); a wait that runs out raises bit 2 of
 // mcw_mlp_status, the CTA waits (bounded) for its copies and MMAs in flight, frees its tensor
@@ -80,7 +86,7 @@ struct GemmProb {
 struct GemmBatch {
     GemmProb p[MCW_GEMM_BATCH_MAX];
     unsigned int *err;
-    int32_t np, stages, sums0;      // sums0: the first CTA of column sums
+    int32_t np, stages, sub, sums0; // K chunks a stage; the first CTA of column sums
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -92,8 +98,14 @@ __device__ __forceinline__ unsigned long long now_ns() {
 }
 
 __device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.f + __expf(-z)); }
+// The sigmoid's quotient by a Newton step on the hardware's reciprocal (Markstein, IBM J. Res. Dev.
+// 34, 1990), which flushes divisors past 2^126.
 __device__ __forceinline__ float dsilu(float z) {
-    const float s = 1.f / (1.f + __expf(-z));
+    const float d = 1.f + __expf(-z);
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    float s = fmaf(fmaf(-d, y, 1.f), y, y);
+    if (d > 8.5e37f) s = 1.f / d;
     return s * (1.f + z * (1.f - s));
 }
 
@@ -102,6 +114,17 @@ __device__ __forceinline__ bool try_wait(uint64_t *bar, uint32_t parity) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
+
+// Whether the phase has completed, without waiting.
+__device__ __forceinline__ bool test_wait(uint64_t *bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return done != 0;
@@ -217,10 +240,85 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 
 // The other input of a 32 x 32 block, one column per lane: rows rbase .. rbase + 31 of column
 // `col` (pre-activations or targets); all loads in flight at once.
-__device__ __forceinline__ void load_aux(const GemmProb &p, int g, int rbase, int col, bool col_ok, float (&av)[32]) {
-    const float *src = p.aux + (size_t)g * p.s_aux + col;
+__device__ __forceinline__ void load_aux(const GemmProb &p, int g, int rbase, int col, bool full, float (&av)[32]) {
+    const float *src = p.aux + (size_t)g * p.s_aux + (size_t)rbase * p.ld_aux + col;
+    if (full) {
 #pragma unroll
-    for (int r = 0; r < 32; ++r) av[r] = (col_ok && rbase + r < p.m) ? __ldg(src + (size_t)(rbase + r) * p.ld_aux) : 0.f;
+        for (int r = 0; r < 32; ++r, src += p.ld_aux) av[r] = __ldg(src);
+    } else {
+#pragma unroll
+        for (int r = 0; r < 32; ++r, src += p.ld_aux) av[r] = (col < p.n && rbase + r < p.m) ? __ldg(src) : 0.f;
+    }
+}
+
+// One 32 x 32 block of a tile, its product in `tile`: a lane's column, row by row.  kFull: the block
+// has all its rows and columns.
+template <int kEpi, bool kFull>
+__device__ __forceinline__ void block_rows(const GemmProb &p, int g, int sp, int rbase, int col, float *tile, int lane,
+                                           const float (&av)[32], float &csum, float &lsum) {
+    const bool col_ok = kFull || col < p.n;
+    const int rows = kFull ? 32 : (col_ok ? min(32, p.m - rbase) : 0);
+    float bias = 0.f, wc = 1.f;
+    if (kEpi != MCW_EPI_F32 && kEpi != MCW_EPI_DSILU && p.bias && col_ok) bias = __ldg(p.bias + (size_t)g * p.s_bias + col);
+    if (kEpi == MCW_EPI_LOSS && p.weights && col_ok) wc = __ldg(p.weights + col);
+    const float scale = kEpi == MCW_EPI_LOSS ? 1.f / ((float)p.m * (float)p.n) : 0.f;
+    constexpr bool k16 = kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS;
+    float *c32 = nullptr;
+    long long ld32 = 0;
+    __nv_bfloat16 *c16 = nullptr;
+    if (!k16) {
+        ld32 = p.ldc;
+        c32 = static_cast<float *>(p.c) + (size_t)sp * p.s_split + (size_t)g * p.s_c + (size_t)rbase * ld32 + col;
+    } else {
+        c16 = static_cast<__nv_bfloat16 *>(p.c) + (size_t)g * p.s_c + (size_t)rbase * p.ldc + col;
+        ld32 = p.ldc2;
+        if (p.c2) c32 = p.c2 + (size_t)g * p.s_c2 + (size_t)rbase * ld32 + col;
+    }
+    const bool has32 = !k16 || p.c2 != nullptr;
+    const bool turned = (kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_DSILU) && p.ct;
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+        float z = tile[r * 33 + lane];
+        const bool in = kFull || r < rows;
+        if (kEpi == MCW_EPI_BIAS_F32 || kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_LOSS) z += bias;
+        if (kEpi == MCW_EPI_DSILU) z *= dsilu(av[r]);
+        if (kEpi == MCW_EPI_LOSS) {
+            const float d = z - av[r];
+            if (in) lsum += wc * d * d * scale;
+            z = 2.f * wc * d * scale;
+        }
+        if ((kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) && in) csum += z;
+        if (has32) {
+            if (in) *c32 = z;
+            c32 += ld32;
+        }
+        if (k16) {
+            const __nv_bfloat16 h = __float2bfloat16(kEpi == MCW_EPI_BIAS_SILU ? silu(z) : z);
+            if (in) *c16 = h;
+            c16 += p.ldc;
+            if (turned) tile[r * 33 + lane] = __bfloat162float(h);
+        }
+    }
+    if (turned && col_ok && rows > 0) {
+        // transposed copy [n, m]: the lane's column is a run of 32 rows
+        __nv_bfloat16 *dst = p.ct + (size_t)g * p.s_ct + (size_t)col * p.ldct + rbase;
+        const bool wide = rows == 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+        for (int q = 0; q < 4; ++q) {
+            uint32_t h[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t lo = __float_as_uint(tile[(8 * q + 2 * k) * 33 + lane]) >> 16;
+                h[k] = lo | (__float_as_uint(tile[(8 * q + 2 * k + 1) * 33 + lane]) & 0xffff0000u);
+            }
+            if (wide) {
+                reinterpret_cast<uint4 *>(dst)[q] = make_uint4(h[0], h[1], h[2], h[3]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (8 * q + k < rows) dst[8 * q + k] = __ushort_as_bfloat16((unsigned short)(h[k / 2] >> (16 * (k % 2))));
+            }
+        }
+    }
 }
 
 // Bias gradients beside weight gradients, 16 columns a CTA behind the tiles' CTAs: the sums of the
@@ -253,7 +351,7 @@ __device__ __forceinline__ void column_sums(const GemmProb &p, int cta, int tid,
     if (q0 == 0 && col < p.m) p.colsum[(size_t)g * p.s_bias + col] = total;
 }
 
-template <int kEpi, bool kAMn, bool kBMn, int TN>
+template <int kEpi, bool kAMn, bool kBMn, int TN, int kSub>
 __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant__ GemmBatch batch) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_bar;
@@ -310,51 +408,70 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
     after_previous();
     let_next_start();
 
+    // K chunks a stage holds, and the stages of this CTA's share
+    const int nst = (nch + kSub - 1) / kSub;
+    constexpr uint32_t stage = (uint32_t)(kSub * stage_bytes(TN));
     if (warp == 4) {
         int issued = 0;
-        for (int kc = 0, s = 0, use = 0; kc < nch; ++kc) {
-            if (use > 0 && !warp_wait(&empty_bar[s], (uint32_t)((use - 1) & 1), abort)) break;
-            const uint32_t sa = ring + (uint32_t)s * stage_bytes(TN);
-            const int k0 = kbeg + kc * TK;
+        bool ready = true;                       // the stage's last use is over
+        for (int i = 0, s = 0, use = 0; i < nst; ++i) {
+            if (!ready && !warp_wait(&empty_bar[s], (uint32_t)((use - 1) & 1), abort)) break;
+            const int s1 = s + 1 == stages ? 0 : s + 1, use1 = s1 == 0 ? use + 1 : use;
+            const bool peek = use1 == 0 || test_wait(&empty_bar[s1], (uint32_t)((use1 - 1) & 1));
+            const int c0 = i * kSub, cn = kSub == 1 ? 1 : min(kSub, nch - c0);
             if (elect_one()) {
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n"
-                             :: "r"(smem_u32(&full_bar[s])), "r"((uint32_t)stage_bytes(TN)) : "memory");
-                load_operand<kAMn, TM>(sa, &p.ta, k0, m0, g, &full_bar[s]);
-                load_operand<kBMn, TN>(sa + kABytes, &p.tb, k0, n0, g, &full_bar[s]);
+                             :: "r"(smem_u32(&full_bar[s])), "r"((uint32_t)(cn * stage_bytes(TN))) : "memory");
+#pragma unroll
+                for (int c = 0; c < kSub; ++c) {
+                    if (c >= cn) break;
+                    const uint32_t sa = ring + (uint32_t)s * stage + (uint32_t)(c * stage_bytes(TN));
+                    const int k0 = kbeg + (c0 + c) * TK;
+                    load_operand<kAMn, TM>(sa, &p.ta, k0, m0, g, &full_bar[s]);
+                    load_operand<kBMn, TN>(sa + kABytes, &p.tb, k0, n0, g, &full_bar[s]);
+                }
             }
-            __syncwarp();
-            issued = kc + 1;
-            if (++s == stages) s = 0, ++use;
+            ready = __all_sync(0xffffffffu, peek);
+            issued = i + 1;
+            s = s1, use = use1;
         }
         // the last copy into each stage has landed before the CTA can leave
-        for (int kc = max(0, issued - stages); kc < issued; ++kc)
-            drain_bar(&full_bar[kc % stages], (uint32_t)((kc / stages) & 1));
+        for (int i = max(0, issued - stages); i < issued; ++i)
+            drain_bar(&full_bar[i % stages], (uint32_t)((i / stages) & 1));
     } else if (warp == 5) {
-        bool any = false;
-        for (int kc = 0, s = 0, use = 0; kc < nch; ++kc) {
-            if (!warp_wait(&full_bar[s], (uint32_t)(use & 1), abort)) break;
+        bool any = false, ready = false;
+        for (int i = 0, s = 0, use = 0; i < nst; ++i) {
+            if (!ready && !warp_wait(&full_bar[s], (uint32_t)(use & 1), abort)) break;
+            // (the next stage is looked at before this one's MMAs are issued, not after)
+            const int s1 = s + 1 == stages ? 0 : s + 1, use1 = s1 == 0 ? use + 1 : use;
+            const bool peek = i + 1 < nst && test_wait(&full_bar[s1], (uint32_t)(use1 & 1));
             asm volatile("tcgen05.fence::after_thread_sync;\n");
-            const uint32_t sa = ring + (uint32_t)s * stage_bytes(TN);
-            const int steps = (min(TK, kend - kbeg - kc * TK) + 15) / 16;
+            const int c0 = i * kSub, cn = kSub == 1 ? 1 : min(kSub, nch - c0);
             if (elect_one()) {
 #pragma unroll
-                for (int q = 0; q < TK / 16; ++q) {
-                    if (q < steps) {
-                        const uint64_t da = operand_desc<kAMn, TM>(sa, q);
-                        const uint64_t db = operand_desc<kBMn, TN>(sa + kABytes, q);
-                        const uint32_t accumulate = (kc > 0 || q > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\t"
-                            "setp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-                            :: "r"(tmem), "l"(da), "l"(db), "r"(kIdesc), "r"(accumulate));
+                for (int c = 0; c < kSub; ++c) {
+                    if (c >= cn) break;
+                    const uint32_t sa = ring + (uint32_t)s * stage + (uint32_t)(c * stage_bytes(TN));
+                    const int steps = (min(TK, kend - kbeg - (c0 + c) * TK) + 15) / 16;
+#pragma unroll
+                    for (int q = 0; q < TK / 16; ++q) {
+                        if (q < steps) {
+                            const uint64_t da = operand_desc<kAMn, TM>(sa, q);
+                            const uint64_t db = operand_desc<kBMn, TN>(sa + kABytes, q);
+                            const uint32_t accumulate = (c0 + c > 0 || q > 0) ? 1u : 0u;
+                            asm volatile(
+                                "{\n\t.reg .pred p;\n\t"
+                                "setp.ne.b32 p, %4, 0;\n\t"
+                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+                                :: "r"(tmem), "l"(da), "l"(db), "r"(kIdesc), "r"(accumulate));
+                        }
                     }
                 }
                 commit(&empty_bar[s]);
             }
-            __syncwarp();
+            ready = __all_sync(0xffffffffu, peek);
             any = true;
-            if (++s == stages) s = 0, ++use;
+            s = s1, use = use1;
         }
         // the accumulator is complete when every MMA issued above is (no MMA: arrives now)
         if (elect_one()) {
@@ -369,7 +486,8 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
         const int rbase = m0 + warp * 32;
         uint32_t verdict;
         float av[32];
-        if (kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) load_aux(p, g, rbase, n0 + lane, n0 + lane < p.n, av);
+        const bool all_rows = rbase + 32 <= p.m;
+        if (kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) load_aux(p, g, rbase, n0 + lane, all_rows && n0 + 32 <= p.n, av);
         // the total of the 128-row sums of A's rows, in order
         if (kEpi == MCW_EPI_F32 && p.colsum_in && p.colsum_rows == 0 && sp == 0 && n0 == 0 && rbase + lane < p.m) {
             const float *src = p.colsum_in + (size_t)g * p.s_colsum + rbase + lane;
@@ -388,7 +506,6 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
         ok = verdict != 0;
         asm volatile("tcgen05.fence::after_thread_sync;\n");
         float lsum = 0.f;
-        const float scale = 1.f / ((float)p.m * (float)p.n);
 #pragma unroll 1
         for (int c0 = 0; c0 < TN && ok; c0 += 32) {
             const int nb = n0 + c0;
@@ -403,46 +520,12 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
                 for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = nch > 0 ? __uint_as_float(v[j]) : 0.f;
                 __syncwarp();
             }
-            float bias = 0.f, wc = 1.f;
-            if (kEpi != MCW_EPI_F32 && kEpi != MCW_EPI_DSILU && p.bias && col_ok)
-                bias = __ldg(p.bias + (size_t)g * p.s_bias + col);
-            if (kEpi == MCW_EPI_LOSS && p.weights && col_ok) wc = __ldg(p.weights + col);
             float csum = 0.f;
-            uint32_t packed[16];
-            float *c32 = nullptr;
-            long long ld32 = 0;
-            if (kEpi == MCW_EPI_F32 || kEpi == MCW_EPI_BIAS_F32) {
-                c32 = static_cast<float *>(p.c) + (size_t)sp * p.s_split + (size_t)g * p.s_c + col;
-                ld32 = p.ldc;
-            } else if (p.c2) {
-                c32 = p.c2 + (size_t)g * p.s_c2 + col;
-                ld32 = p.ldc2;
-            }
-            __nv_bfloat16 *c16 = static_cast<__nv_bfloat16 *>(p.c) + (size_t)g * p.s_c + col;
-            const int rows = min(32, p.m - rbase);
-#pragma unroll
-            for (int r = 0; r < 32; ++r) {
-                float z = tile[r * 33 + lane];
-                const bool in = col_ok && r < rows;
-                if (kEpi == MCW_EPI_BIAS_F32 || kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_LOSS) z += bias;
-                if (kEpi == MCW_EPI_DSILU) z *= dsilu(av[r]);
-                if (kEpi == MCW_EPI_LOSS) {
-                    const float d = z - av[r];
-                    if (in) lsum += wc * d * d * scale;
-                    z = 2.f * wc * d * scale;
-                }
-                if ((kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) && in) csum += z;
-                if (c32 && in) c32[(size_t)(rbase + r) * ld32] = z;
-                if (kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) {
-                    const __nv_bfloat16 h = __float2bfloat16(kEpi == MCW_EPI_BIAS_SILU ? silu(z) : z);
-                    if (in) c16[(size_t)(rbase + r) * p.ldc] = h;
-                    const uint32_t bits = (uint32_t)__bfloat16_as_ushort(h);
-                    packed[r >> 1] = (r & 1) ? (packed[r >> 1] | bits << 16) : bits;
-                }
-            }
+            if (all_rows && nb + 32 <= p.n) block_rows<kEpi, true>(p, g, sp, rbase, col, tile, lane, av, csum, lsum);
+            else block_rows<kEpi, false>(p, g, sp, rbase, col, tile, lane, av, csum, lsum);
             if (kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) {
                 // the next block's other input while this one's sums are put together
-                if (c0 + 32 < TN) load_aux(p, g, rbase, col + 32, col + 32 < p.n, av);
+                if (c0 + 32 < TN && nb + 32 < p.n) load_aux(p, g, rbase, col + 32, all_rows && nb + 64 <= p.n, av);
                 if (p.colsum) {
                     part[warp * 32 + lane] = csum;
                     asm volatile("bar.sync 1, 128;\n" ::: "memory");
@@ -450,20 +533,6 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
                         p.colsum[(size_t)g * p.s_colsum + (size_t)mtile * p.ld_colsum + col] =
                             ((part[lane] + part[32 + lane]) + part[64 + lane]) + part[96 + lane];
                     asm volatile("bar.sync 1, 128;\n" ::: "memory");
-                }
-            }
-            if ((kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_DSILU) && p.ct && col_ok && rows > 0) {
-                // transposed copy [n, m]: the lane's column is a run of 32 rows
-                __nv_bfloat16 *dst = p.ct + (size_t)g * p.s_ct + (size_t)col * p.ldct + rbase;
-                if (rows == 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        reinterpret_cast<uint4 *>(dst)[q] =
-                            make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-                } else {
-#pragma unroll
-                    for (int r = 0; r < 32; ++r)
-                        if (r < rows) dst[r] = __ushort_as_bfloat16((unsigned short)(packed[r >> 1] >> ((r & 1) * 16)));
                 }
             }
             __syncwarp();
@@ -525,16 +594,16 @@ bool make_map(CUtensorMap *map, const void *base, long long inner, long long row
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int kEpi, bool kAMn, bool kBMn, int TN>
+template <int kEpi, bool kAMn, bool kBMn, int TN, int kSub = 1>
 cudaError_t launch(const GemmBatch &b, unsigned grid, size_t smem, cudaStream_t s) {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(gemm_kernel<kEpi, kAMn, kBMn, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    200 * 1024);
+        attr = cudaFuncSetAttribute(gemm_kernel<kEpi, kAMn, kBMn, TN, kSub>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    208 * 1024);
     });
     if (attr != cudaSuccess) return attr;
-    return launch_after(gemm_kernel<kEpi, kAMn, kBMn, TN>, grid, kThreads, smem, s, b);
+    return launch_after(gemm_kernel<kEpi, kAMn, kBMn, TN, kSub>, grid, kThreads, smem, s, b);
 }
 
 // The combinations of epilogue and layouts that exist: a plain product takes any, a backward
@@ -547,6 +616,7 @@ template <int TN>
 cudaError_t launch_n(int epi, const GemmBatch &b, bool ta, bool tb, unsigned grid, size_t smem, cudaStream_t s) {
     switch (epi) {
         case MCW_EPI_F32:
+            if (ta && tb && b.sub == 2) return launch<MCW_EPI_F32, true, true, TN, 2>(b, grid, smem, s);
             if (ta) return tb ? launch<MCW_EPI_F32, true, true, TN>(b, grid, smem, s)
                               : launch<MCW_EPI_F32, true, false, TN>(b, grid, smem, s);
             return tb ? launch<MCW_EPI_F32, false, true, TN>(b, grid, smem, s)
@@ -580,18 +650,20 @@ int launch_batch(const McwGemmProblem *q, int np, cudaStream_t stream) {
         const int c = ((q[i].k + TK - 1) / TK + q[i].splits - 1) / q[i].splits;
         chunks = c > chunks ? c : chunks;
     }
-    // 64 columns a tile when that leaves two tiles per SM, except for the SiLU' product, whose
-    // first block's pre-activations are loaded behind the product; 65,536 rows with tiles of
-    // 32 / 64 / 128 columns: 256 x 256 bias + SiLU 53 / 49 / 57 us, 256 x 649 output 84 / 72 / 73,
-    // SiLU' of 649 99 / 101 / 135, of 256 75 / 89 / 119
-    const int tn = t64 >= 304 && q[0].epilogue != MCW_EPI_DSILU ? 64 : 32;
+    // 64 columns a tile when that leaves two tiles per SM: at 65,536 rows with tiles of 32 / 64
+    // columns the SiLU' product of 649 takes 92 / 72 us, of 256 62 / 55 (bias + SiLU 256 x 256 53 / 42,
+    // the 256 x 649 output 84 / 70)
+    const int tn = t64 >= 304 ? 64 : 32;
     // two stages when the launch fills the SMs several times over (four CTAs of an SM overlap each
-    // other), else up to eight, or as many as the chunks: the weight gradients of 65,536 rows, one
-    // chain of 1,024 chunks per tile, take 464 / 317 / 246 / 201 us with 2 / 3 / 4 / 8 stages
+    // other), else up to eight, or as many as the chunks; five of two chunks each for a transposed
+    // product with an SM to a CTA and a long chain, where a stage's handover (120 ns beside 20 ns an
+    // MMA) is what is left: the weight gradients of 65,536 rows, 1,024 chunks a tile, take
+    // 464 / 317 / 246 / 201 us with 2 / 3 / 4 / 8 stages, 176 with 5 of two
     const long long ctas = tn == 64 ? t64 : t32;
-    int stages = ctas > 304 ? 2 : (ctas > 152 ? 4 : kMaxStages);
-    stages = stages > chunks ? chunks : stages;
-    b.stages = stages;
+    const int stages = ctas > 304 ? 2 : (ctas > 152 ? 4 : kMaxStages);
+    b.stages = stages > chunks ? chunks : stages;
+    b.sub = q[0].epilogue == MCW_EPI_F32 && ta && tb && ctas <= 152 && chunks >= 4 * kMaxStages ? 2 : 1;
+    if (b.sub == 2) b.stages = 5;
     long long cta = 0;
     for (int i = 0; i < np; ++i) {
         const McwGemmProblem &s = q[i];
@@ -627,7 +699,7 @@ int launch_batch(const McwGemmProblem *q, int np, cudaStream_t stream) {
             cta += (long long)((q[i].m + kSumCols - 1) / kSumCols) * q[i].groups;
     }
     if (cta > 0x7fffffffLL) return MCW_MLP_ERR_ARG;
-    const size_t ring = (size_t)stages * stage_bytes(tn), tiles = 4 * kTileBytes;
+    const size_t ring = (size_t)b.stages * b.sub * stage_bytes(tn), tiles = 4 * kTileBytes;
     const size_t smem = (ring > tiles ? ring : tiles) + 1024;
     cudaError_t e;
     if (tn == 64) e = launch_n<64>(q[0].epilogue, b, ta, tb, (unsigned)cta, smem, stream);

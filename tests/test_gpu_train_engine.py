@@ -281,6 +281,54 @@ def test_gemm_batch_layouts_match_float64(ta, tb, m, n, k):
         assert (c[:, mm] == 7).all() and (c[:, :, nn] == 7).all()
 
 
+@pytest.mark.parametrize('k', [2047, 2048, 2049, 2112, 2113, 4200])
+def test_gemm_batch_long_chain_matches_float64(k):
+    """A transposed product of few tiles and a long K, two chunks of 64 a stage: a last stage of
+    one chunk, chunks cut short, and more stages than the ring holds."""
+    m, n = 200, 72
+    g = torch.Generator().manual_seed(k)
+    a = torch.randn((2, k, m), generator=g).to(torch.bfloat16).cuda()
+    b = (torch.randn((2, k, n), generator=g) * 0.1).to(torch.bfloat16).cuda()
+    c = torch.full((2, m + 1, n + 1), 7.0, device='cuda')
+    q = _problem(_abi.EPI_F32, m, n, k, a, b, c, 1, 1, groups=2)
+    _status_clear()
+    assert _abi.load().mcw_mlp_gemm_batch(ctypes.byref(q), 1, _stream()) == 0
+    torch.cuda.synchronize()
+    _status_ok()
+    ref = a.cpu().double().transpose(1, 2) @ b.cpu().double()
+    err = (c[:, :m, :n].cpu().double() - ref).abs().max().item()
+    assert err <= 1e-4 * max(1.0, ref.abs().max().item()) + 1e-5 * math.sqrt(k), err
+    assert (c[:, m] == 7).all() and (c[:, :, n] == 7).all()
+
+
+@pytest.mark.parametrize('m,n', [(128, 64), (31, 33), (640, 649)])
+def test_silu_derivative_over_the_range(m, n):
+    """The SiLU' epilogue from pre-activations of -100 to 100, infinities and NaN against float64:
+    exp's argument is rounded at |z| 2^-23, the rest to a few units of 2^-24, and the sigmoid is 0
+    where exp(-z) leaves FP32's range."""
+    a = torch.ones(1, m, 8, dtype=torch.bfloat16, device='cuda') / 8
+    b = torch.ones(1, n, 8, dtype=torch.bfloat16, device='cuda')
+    z = torch.linspace(-100, 100, m * n).reshape(m, n)
+    z[0, 0], z[0, 1], z[1, 0] = float('nan'), float('inf'), float('-inf')
+    z[1, 1], z[2, 2] = 0.0, -88.0
+    zc = z.cuda()
+    out16 = torch.zeros(1, m, n, dtype=torch.bfloat16, device='cuda')
+    out32 = torch.zeros(1, m, n, device='cuda')
+    q = _problem(_abi.EPI_DSILU, m, n, 8, a, b, out16, 0, 0, aux=zc.data_ptr(), ldaux=n, stride_aux=m * n,
+                 c2=out32.data_ptr(), ldc2=n, stride_c2=m * n)
+    assert _abi.load().mcw_mlp_gemm_batch(ctypes.byref(q), 1, _stream()) == 0
+    torch.cuda.synchronize()
+    got = out32[0].cpu().double()
+    zd = z.double()
+    s = torch.where(torch.exp(-zd) > 3.4028235e38, 0.0, torch.sigmoid(zd))
+    ref = s * (1 + zd * (1 - s))
+    tol = 2e-5 * s * (1 + zd.abs()) + 1e-37
+    odd = ~torch.isfinite(zd)
+    assert (((got - ref).abs() <= tol) | odd).all()
+    assert torch.isnan(got[0, 0]) and torch.isnan(got[1, 0])
+    assert torch.equal(out16.float(), out32.to(torch.bfloat16).float()) or torch.isnan(out32).any()
+
+
 @pytest.mark.parametrize('m,n', [(1, 649), (130, 40), (700, 256)])
 def test_gemm_batch_loss_and_column_sums(m, n):
     """The loss epilogue, the column sums of SiLU' and loss results over every 128 rows, their
