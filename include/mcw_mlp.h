@@ -291,6 +291,19 @@ int mcw_brf_jacobian(const float *y, const float *ydot, int64_t pitch, int32_t m
                      const double *std, double floor, double *f, double *j, double *v, const double *obs,
                      const double *share, double photons, double rel_noise, double *jtr, double *jtj, void *stream);
 
+/* The network's inputs x [points * n, 4] of every observation (known [n, 3]: wavelength, mu0, depth) at
+ * every log r of s [points], scaled to [-1, 1]; hull (host, 8 values): origin and width of log r,
+ * wavelength, mu0 and log depth. */
+int mcw_brf_encode(const double *s, int32_t points, const double *known, int32_t n, const double *hull, float *x,
+                   void *stream);
+
+/* log r of n observations: with cost [points, n] the grid value of the lowest (0 where none is below
+ * infinity), else s + clip(-jtr / (jtj (1 + damping) + 1e-30), +-max_step) within [lo, hi]; then its
+ * inputs, x [n, 4] and x16 bf16 [members, n, 8] (columns 0 to 3), either may be NULL. */
+int mcw_brf_gn_step(const double *cost, const double *grid, int32_t points, const double *jtr, const double *jtj,
+                    double damping, double max_step, double lo, double hi, const double *known, int32_t n,
+                    const double *hull, double *s, float *x, void *x16, int32_t members, void *stream);
+
 /* Standard deviation over the members of sum w j (BRF - mean BRF) / sum w j^2, and 1 / sqrt(sum j^2 /
  * variance without the model's). */
 int mcw_brf_logr(const double *brf, const double *mean_brf, int32_t members, int32_t n, const double *f, const double *j,

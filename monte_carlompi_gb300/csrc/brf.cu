@@ -9,7 +9,9 @@
 // sub-core), so every kernel takes each exponential once and keeps what it can in registers; a
 // block per row, a thread per bin, sums by block reduction.  128 observations, five members, one
 // retrieval (16-point grid, six iterations, spreads): 92 ms on the host's cores and elementwise
-// tensor kernels, 3.3 ms now.
+// tensor kernels; 3.3 ms with these kernels and the steps and the encoding of log r on the host, a
+// wait for the device and two copies an iteration; 2.0 ms with the steps here too.
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -241,6 +243,61 @@ __global__ void __launch_bounds__(kThreads) logr_kernel(const double *brf, const
     }
 }
 
+// The network's inputs, scaled to [-1, 1] over the training hull (surrogate.encode): log r_eff,
+// wavelength, mu0, log depth, each (x - origin) over the width.
+struct Hull {
+    double origin[4], width[4];
+    __device__ __forceinline__ float scaled(int q, double x) const { return (float)(2 * (x - origin[q]) / width[q] - 1); }
+    __device__ __forceinline__ float4 encode(double s, const double *known) const {
+        return make_float4(scaled(0, log(exp(s))), scaled(1, known[0]), scaled(2, known[1]), scaled(3, log(known[2])));
+    }
+};
+
+// Row p * n + o: observation o at log r = s[p].
+__global__ void encode_kernel(const double *s, int points, int n, const double *known, const Hull hull, float4 *x) {
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row < points * n) x[row] = hull.encode(s[row / n], known + 3 * (row % n));
+}
+
+__device__ __forceinline__ double clipped(double x, double lo, double hi) { return x < lo ? lo : (x > hi ? hi : x); }
+
+// log r of every observation: the grid point of the lowest cost, or a damped Gauss-Newton step from
+// where it is; then the network's inputs there, FP32 (x) and bf16 for every member (x16, rows of 8),
+// either may be null.
+__global__ void gn_kernel(const double *cost, const double *grid, int points, const double *jtr, const double *jtj,
+                          double damping, double max_step, double lo, double hi, const double *known, int n,
+                          const Hull hull, double *s, float4 *x, __nv_bfloat16 *x16, int members) {
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= n) return;
+    double at;
+    if (cost) {
+        double best = __longlong_as_double(0x7ff0000000000000ll);
+        at = 0.0;
+        for (int p = 0; p < points; ++p) {
+            const double c = cost[(size_t)p * n + o];
+            if (c < best) best = c, at = grid[p];
+        }
+    } else {
+        const double step = clipped(-jtr[o] / (jtj[o] * (1 + damping) + 1e-30), -max_step, max_step);
+        at = clipped(s[o] + step, lo, hi);
+    }
+    s[o] = at;
+    const float4 e = hull.encode(at, known + 3 * (size_t)o);
+    if (x) x[o] = e;
+    if (x16)
+        for (int m = 0; m < members; ++m) {
+            __nv_bfloat162 *d = reinterpret_cast<__nv_bfloat162 *>(x16 + ((size_t)m * n + o) * 8);
+            d[0] = __floats2bfloat162_rn(e.x, e.y);
+            d[1] = __floats2bfloat162_rn(e.z, e.w);
+        }
+}
+
+Hull hull_of(const double *h) {
+    Hull r;
+    for (int q = 0; q < 4; ++q) r.origin[q] = h[2 * q], r.width[q] = h[2 * q + 1];
+    return r;
+}
+
 bool rows_ok(int32_t members, int32_t n) { return members >= 1 && members <= 4096 && n >= 0; }
 int done() { return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA; }
 
@@ -292,6 +349,30 @@ int mcw_brf_jacobian(const float *y, const float *ydot, int64_t pitch, int32_t m
     if (n == 0) return 0;
     jacobian_kernel<<<n, kThreads, 2 * members * sizeof(double), static_cast<cudaStream_t>(stream)>>>(
         y, ydot, pitch, members, n, mean, std, floor, f, j, v, obs, Noise{photons, rel_noise, share}, jtr, jtj);
+    return done();
+}
+
+int mcw_brf_encode(const double *s, int32_t points, const double *known, int32_t n, const double *hull, float *x,
+                   void *stream) {
+    if (!s || !known || !hull || !x || points < 0 || n < 0 || (long long)points * n > 0x7fffffffLL - 128 ||
+        (reinterpret_cast<uintptr_t>(x) & 15))
+        return MCW_MLP_ERR_ARG;
+    if (points * n == 0) return 0;
+    encode_kernel<<<(points * n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+        s, points, n, known, hull_of(hull), reinterpret_cast<float4 *>(x));
+    return done();
+}
+
+int mcw_brf_gn_step(const double *cost, const double *grid, int32_t points, const double *jtr, const double *jtj,
+                    double damping, double max_step, double lo, double hi, const double *known, int32_t n,
+                    const double *hull, double *s, float *x, void *x16, int32_t members, void *stream) {
+    if (!known || !hull || !s || n < 0 || n > 0x7fffffff - 128 || members < 0 || (cost ? !grid || points < 0 : !jtr || !jtj) ||
+        (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(x16) & 15))
+        return MCW_MLP_ERR_ARG;
+    if (n == 0) return 0;
+    gn_kernel<<<(n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(
+        cost, grid, points, jtr, jtj, damping, max_step, lo, hi, known, n, hull_of(hull), s,
+        reinterpret_cast<float4 *>(x), static_cast<__nv_bfloat16 *>(x16), members);
     return done();
 }
 

@@ -14,6 +14,7 @@ solution, gives the log r_eff that member would move the answer to; their standa
 deviation is the surrogate's own relative uncertainty in r_eff).  The reference has no inverse; this consumes the same BRF definition
 (post_processing.py:73-81, 2-D form).
 """
+import ctypes
 import math
 import time
 
@@ -23,6 +24,7 @@ from . import _abi
 from . import surrogate as S
 
 LOG_R = (math.log(S.R_RANGE[0]), math.log(S.R_RANGE[1]))
+DAMPING, MAX_STEP = 1e-3, 0.7
 
 
 def noise_variance(f, photons, rel_noise=0.0, model_var=None):
@@ -53,22 +55,30 @@ class _Slopes:
         self.mean, self.std = ens.scaling()
         self.share = torch.from_numpy(S.bin_weights()).cuda()
 
-    def at(self, s, known, obs=None, noise=(0.0, 0.0), arrays=True):
-        """At log r = s: (f, j, v) torch CUDA float64 [n, 648] (None without arrays) and, with obs
-        (torch CUDA float64 [n, 648]), the sums over the bins of w j (f - obs) and w j^2 [n]."""
-        torch = self.torch
-        x = torch.from_numpy(S.encode(np.exp(s), known[:, 0], known[:, 1], known[:, 2])).cuda()
+    def at(self, s, known):
+        """(f, j, v) torch CUDA float64 [n, 648] at log r = s (host arrays s [n], known [n, 3])."""
+        return self.arrays(self.torch.from_numpy(S.encode(np.exp(s), *known.T)).cuda())
+
+    def arrays(self, x=None):
+        """(f, j, v) of inputs x, or of those the network's buffer holds."""
+        f, j, v = (self.torch.empty((self.n, S.N_BRF), dtype=self.torch.float64, device=self.share.device) for _ in range(3))
+        self._evaluate(x, f, j, v, None, (0.0, 0.0), None)
+        return f, j, v
+
+    def sums(self, obs, noise, out):
+        """The sums over the bins of w j (f - obs) and w j^2 into out [2, n] (obs torch CUDA float64
+        [n, 648]), of the inputs the network's buffer holds."""
+        self._evaluate(None, None, None, None, obs, noise, out)
+
+    def _evaluate(self, x, f, j, v, obs, noise, out):
         y, ydot = self.net.run(x)
-        new = lambda *shape: torch.empty(shape, dtype=torch.float64, device=y.device)  # noqa: E731
-        f, j, v = (new(self.n, S.N_BRF) for _ in range(3)) if arrays else (None, None, None)
-        sums = new(2, self.n) if obs is not None else (None, None)
+        jtr, jtj = (None, None) if out is None else (out[0], out[1])
         rc = _abi.load().mcw_brf_jacobian(_ptr(y), _ptr(ydot), y.shape[2], y.shape[0], self.n, _ptr(self.mean),
                                           _ptr(self.std), S.BRF_FLOOR, _ptr(f), _ptr(j), _ptr(v), _ptr(obs),
-                                          _ptr(self.share), noise[0], noise[1], _ptr(sums[0]), _ptr(sums[1]),
-                                          S._stream(torch))
+                                          _ptr(self.share), noise[0], noise[1], _ptr(jtr), _ptr(jtj),
+                                          S._stream(self.torch))
         if rc:
             raise _abi.McwError(rc, 'mcw_brf_jacobian failed')
-        return (f, j, v), sums
 
 
 def _brf_and_jacobian(ens, s, known, chunk=16384, with_var=False):
@@ -81,18 +91,18 @@ def _brf_and_jacobian(ens, s, known, chunk=16384, with_var=False):
         hi = min(n, lo + chunk)
         if slopes is None or slopes.n != hi - lo:
             slopes = _Slopes(ens, hi - lo)
-        arrays, _ = slopes.at(s[lo:hi], known[lo:hi])
+        arrays = slopes.at(s[lo:hi], known[lo:hi])
         for o, t in zip(out, arrays):
             o[lo:hi] = t.cpu().numpy()
     return tuple(out) if with_var else tuple(out[:2])
 
 
-def _gn_update(f, jac, obs, s, w, damping=1e-3, max_step=0.7):
+def _gn_update(f, jac, obs, s, w, damping=DAMPING, max_step=MAX_STEP):
     r = f - obs
     return _gn_step((w * jac * r).sum(1), (w * jac * jac).sum(1), s, damping, max_step)
 
 
-def _gn_step(jtr, jtj, s, damping=1e-3, max_step=0.7):
+def _gn_step(jtr, jtj, s, damping=DAMPING, max_step=MAX_STEP):
     step = -jtr / (jtj * (1 + damping) + 1e-30)
     step = np.clip(step, -max_step, max_step)
     return np.clip(s + step, LOG_R[0], LOG_R[1])
@@ -128,45 +138,46 @@ def surrogate_gn(ens, obs, known, iters=6, obs_photons=None, obs_noise=0.0, with
 
 
 def _surrogate_gn(ens, obs, known, iters, noise):
-    """surrogate_gn of a few thousand observations: BRFs, residuals and their sums stay on the
-    device (FP64, csrc/brf.cu); the host holds log r_eff, encodes it and takes the steps."""
+    """surrogate_gn of a few thousand observations, queued on the device from the grid to the
+    spreads (FP64, csrc/brf.cu) without the host waiting in between."""
     import torch
     n = obs.shape[0]
-    known = np.asarray(known, np.float64)
+    f64 = dict(dtype=torch.float64, device='cuda')
+    known_d = torch.from_numpy(np.ascontiguousarray(known, np.float64)).cuda()
     obs_d = torch.from_numpy(np.ascontiguousarray(obs, np.float64)).cuda()
     slopes = _Slopes(ens, n)
     L, st, k = _abi.load(), S._stream(torch), len(ens.members)
+    hull = (ctypes.c_double * 8)(*S.hull())
 
     def check(rc, what):
         if rc:
             raise _abi.McwError(rc, '%s failed' % what)
     # the grid: every observation at every point in one forward pass
-    grid = np.linspace(LOG_R[0], LOG_R[1], 16)
-    r = np.repeat(np.array([math.exp(g) for g in grid]), n)
-    x = torch.from_numpy(S.encode(r, *np.tile(known, (16, 1)).T)).cuda()
+    grid = torch.from_numpy(np.linspace(LOG_R[0], LOG_R[1], 16)).cuda()
+    x = torch.empty((16 * n, S.DIMS[0]), dtype=torch.float32, device='cuda')
+    check(L.mcw_brf_encode(_ptr(grid), 16, _ptr(known_d), n, hull, _ptr(x), st), 'mcw_brf_encode')
     ys = ens.predict_std(x)
-    cost_d = torch.empty((16, n), dtype=torch.float64, device='cuda')
+    cost = torch.empty((16, n), **f64)
     check(L.mcw_brf_cost(_ptr(ys), ys.stride(1), k, 16, n, _ptr(slopes.mean), _ptr(slopes.std), S.BRF_FLOOR,
-                         _ptr(obs_d), _ptr(slopes.share), noise[0], noise[1], _ptr(cost_d), st), 'mcw_brf_cost')
-    cost = cost_d.cpu().numpy()
-    best = np.full(n, np.inf)
-    s = np.zeros(n)
-    for g, c in zip(grid, cost):
-        better = c < best
-        best[better] = c[better]
-        s[better] = g
+                         _ptr(obs_d), _ptr(slopes.share), noise[0], noise[1], _ptr(cost), st), 'mcw_brf_cost')
+    s, sums = torch.empty(n, **f64), torch.empty((2, n), **f64)
+    x = torch.empty((n, S.DIMS[0]), dtype=torch.float32, device='cuda')
+
+    def step(cost_p):
+        check(L.mcw_brf_gn_step(cost_p, _ptr(grid), 16, _ptr(sums[0]), _ptr(sums[1]), DAMPING, MAX_STEP, LOG_R[0],
+                                LOG_R[1], _ptr(known_d), n, hull, _ptr(s), _ptr(x), _ptr(slopes.net.x), k, st),
+              'mcw_brf_gn_step')
+    step(_ptr(cost))
     for _ in range(iters):
-        _, sums = slopes.at(s, known, obs_d, noise, arrays=False)
-        jtr, jtj = sums.cpu().numpy()
-        s = _gn_step(jtr, jtj, s)
-    x = torch.from_numpy(S.encode(np.exp(s), *known.T)).cuda()
-    brf, alb = ens.member_brfs(x)
+        slopes.sums(obs_d, noise, sums)
+        step(None)
+    brf, alb = ens._member_brfs(x, slopes.mean, slopes.std)
     pred, _, spread = ens.brf_stats(brf, alb)
-    (f, j, v), _ = slopes.at(s, known)
+    f, j, v = slopes.arrays()
     spread_r, sigma = torch.empty_like(spread), torch.empty_like(spread)
     check(L.mcw_brf_logr(_ptr(brf), _ptr(pred), k, n, _ptr(f), _ptr(j), _ptr(v), _ptr(slopes.share), noise[0],
                          noise[1], _ptr(spread_r), _ptr(sigma), st), 'mcw_brf_logr')
-    return (s,) + tuple(t.cpu().numpy() for t in (pred, spread, spread_r, sigma))
+    return tuple(t.cpu().numpy() for t in (s, pred, spread, spread_r, sigma))
 
 
 def mc_gn(walker, obs, known, s0, n_photon=1000000, iters=3, h=0.05, seed=0x5EED0055, obs_photons=None,

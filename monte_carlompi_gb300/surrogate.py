@@ -46,6 +46,15 @@ def encode(r_eff, wvl, mu0, depth):
     return x.astype(np.float32)
 
 
+def hull():
+    """Origin and width of log r_eff, wavelength, mu0 and log depth, as encode scales them."""
+    out = []
+    for lo, hi in ((math.log(R_RANGE[0]), math.log(R_RANGE[1])), WVL_RANGE, MU_RANGE,
+                   (math.log(DEPTH_RANGE[0]), math.log(DEPTH_RANGE[1]))):
+        out += [lo, hi - lo]
+    return out
+
+
 def in_hull(r_eff, wvl, mu0, depth):
     x = encode(r_eff, wvl, mu0, depth)
     return np.all(np.abs(x) <= 1.0 + 1e-6, axis=-1)
@@ -314,9 +323,10 @@ class EnsembleTangent:
         self.calls.append(call(_abi.EPI_F32, 3, d, self.ydot))
 
     def run(self, x):
-        """x float32 [n, 4]; returns (y, ydot) fp32 [members, n, Y_PITCH], 649 columns used; valid
-        until the next call."""
-        self.x[:, :, :DIMS[0]] = x
+        """x float32 [n, 4], or None for what self.x (bf16 [members, n, 8]) holds; returns (y, ydot)
+        fp32 [members, n, Y_PITCH], 649 columns used; valid until the next call."""
+        if x is not None:
+            self.x[:, :, :DIMS[0]] = x
         L, st = _abi.load(), _stream(self.torch)
         for c in self.calls:
             rc = L.mcw_mlp_gemm_batch(ctypes.byref(c), 1, st)
@@ -795,10 +805,12 @@ class Ensemble:
     def member_brfs(self, x):
         """Each member's BRF [members, n, 648] and albedo [members, n] (torch CUDA float64) for
         encoded inputs x (torch CUDA float32 [n, 4])."""
+        return self._member_brfs(x, *self.scaling())
+
+    def _member_brfs(self, x, mean, std):
         import torch
         ys = self.predict_std(x)
         k, n = ys.shape[:2]
-        mean, std = self.scaling()
         brf = torch.empty((k, n, N_BRF), dtype=torch.float64, device=x.device)
         alb = torch.empty((k, n), dtype=torch.float64, device=x.device)
         rc = _abi.load().mcw_brf_members(_ptr(ys), ys.stride(1), k, n, _ptr(mean), _ptr(std), BRF_FLOOR, _ptr(brf),

@@ -83,6 +83,50 @@ def test_gauss_newton_recovers_r_eff_on_network_brfs(trained):
     assert np.all(np.isfinite(spread)) and np.all(np.isfinite(spread_r)) and np.all(spread_r >= 0)
 
 
+@pytest.mark.parametrize('n,members', [(1, 1), (127, 3), (129, 5), (1000, 2)])
+def test_retrieval_steps_match_numpy(n, members):
+    """Inputs encoded on the device, the grid's best point and the damped step against
+    surrogate.encode and inverse._gn_step: steps cut at both ends, equal, infinite and NaN costs.
+    float32 inputs: one rounding of a float64 value that may differ by an ulp."""
+    import ctypes
+    import torch
+    from monte_carlompi_gb300 import _abi
+    rng = np.random.default_rng(n)
+    L, st, p = _abi.load(), surrogate._stream(torch), lambda t: t.data_ptr()
+    raw = surrogate.sample_inputs(n, n + 1)
+    known = torch.from_numpy(np.ascontiguousarray(raw[:, 1:])).cuda()
+    hull = (ctypes.c_double * 8)(*surrogate.hull())
+    grid = np.linspace(*inverse.LOG_R, 16)
+    grid_d = torch.from_numpy(grid).cuda()
+    x = torch.empty((16 * n, 4), device='cuda')
+    assert L.mcw_brf_encode(p(grid_d), 16, p(known), n, hull, p(x), st) == 0
+    ref = surrogate.encode(np.repeat(np.exp(grid), n), *np.tile(raw[:, 1:], (16, 1)).T)
+    assert np.allclose(x.cpu().numpy(), ref, rtol=1.2e-7, atol=1e-7)
+    cost = rng.random((16, n))
+    cost[3, 0], cost[7:, n // 2], cost[:, n - 1] = np.nan, cost[7, n // 2], (np.inf if n > 1 else cost[:, 0])
+    s = torch.empty(n, dtype=torch.float64, device='cuda')
+    x1, x16 = torch.empty((n, 4), device='cuda'), torch.zeros((members, n, 8), dtype=torch.bfloat16, device='cuda')
+    jtr, jtj = rng.normal(size=n) * 10, rng.random(n) * np.where(np.arange(n) % 3, 10.0, 0.1)
+    cost_d, jtr_d, jtj_d = (torch.from_numpy(v).cuda() for v in (cost, jtr, jtj))
+
+    def step(c):
+        assert L.mcw_brf_gn_step(c, p(grid_d), 16, p(jtr_d), p(jtj_d), 1e-3, 0.7, *inverse.LOG_R, p(known), n, hull, p(s),
+                                 p(x1), p(x16), members, st) == 0
+        assert torch.equal(x16[:, :, :4], x1.to(torch.bfloat16).expand(members, n, 4)) and not x16[:, :, 4:].any()
+        assert np.allclose(x1.cpu().numpy(), surrogate.encode(np.exp(s.cpu().numpy()), *raw[:, 1:].T), rtol=1.2e-7, atol=1e-7)
+        return s.cpu().numpy()
+    best, want = np.full(n, np.inf), np.zeros(n)
+    for g, c in zip(grid, cost):
+        better = c < best
+        best[better], want[better] = c[better], g
+    got = step(p(cost_d))
+    assert np.array_equal(got, want)
+    for _ in range(3):
+        want = inverse._gn_step(jtr, jtj, got)
+        got = step(None)
+        assert np.allclose(got, want, rtol=0, atol=1e-15)
+
+
 @pytest.mark.parametrize('n,members,weighted', [(1, 1, True), (33, 3, False), (130, 5, True)])
 def test_brf_kernels_match_numpy(n, members, weighted):
     """Members' BRFs, their mean and spread, grid costs, Gauss-Newton sums and spreads of log r_eff
