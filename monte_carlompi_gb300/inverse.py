@@ -172,7 +172,7 @@ def _surrogate_gn(ens, obs, known, iters, noise):
         slopes.sums(obs_d, noise, sums)
         step(None)
     brf, alb = ens._member_brfs(x, slopes.mean, slopes.std)
-    pred, _, spread = ens.brf_stats(brf, alb)
+    pred, _, spread = ens._brf_stats(brf, alb, slopes.share)
     f, j, v = slopes.arrays()
     spread_r, sigma = torch.empty_like(spread), torch.empty_like(spread)
     check(L.mcw_brf_logr(_ptr(brf), _ptr(pred), k, n, _ptr(f), _ptr(j), _ptr(v), _ptr(slopes.share), noise[0],

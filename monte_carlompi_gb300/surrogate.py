@@ -824,10 +824,13 @@ class Ensemble:
         (torch CUDA float64): the spread in the units of rel_rms, weighted RMS standard
         deviation over weighted RMS BRF."""
         import torch
+        return self._brf_stats(brf, alb, torch.from_numpy(bin_weights()).to(brf.device))
+
+    def _brf_stats(self, brf, alb, share):
+        import torch
         k, n = alb.shape
         mean = torch.empty((n, N_BRF), dtype=torch.float64, device=brf.device)
         alb_mean, spread = torch.empty_like(alb[0]), torch.empty_like(alb[0])
-        share = torch.from_numpy(bin_weights()).to(brf.device)
         rc = _abi.load().mcw_brf_stats(_ptr(brf), _ptr(alb), k, n, _ptr(share), _ptr(mean), _ptr(alb_mean),
                                        _ptr(spread), _stream(torch))
         if rc:

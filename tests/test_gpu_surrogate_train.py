@@ -83,6 +83,26 @@ def test_gauss_newton_recovers_r_eff_on_network_brfs(trained):
     assert np.all(np.isfinite(spread)) and np.all(np.isfinite(spread_r)) and np.all(spread_r >= 0)
 
 
+@pytest.mark.parametrize('lo,hi', [(-750.0, 750.0), (-1.0, 1.0), (-701.0, -699.0), (699.0, 701.0), (-6e-8, 6e-8)])
+def test_members_exponential_over_the_range(lo, hi):
+    """exp of a member's outputs (floor 0, albedo 1) against numpy's: an ulp of each."""
+    import torch
+    from monte_carlompi_gb300 import _abi
+    n, bins = 40, surrogate.N_BRF
+    ys = torch.linspace(lo, hi, n * bins).reshape(1, n, bins).half()
+    if hi == 750:
+        ys[0, 0, :3] = torch.tensor([float('nan'), float('inf'), float('-inf')])
+    ys = torch.cat([ys, torch.zeros(1, n, 1).half()], 2).cuda().contiguous()
+    mean, std = torch.zeros(1, 649, dtype=torch.float64, device='cuda'), torch.ones(1, 649, dtype=torch.float64, device='cuda')
+    brf, alb = torch.empty((1, n, bins), dtype=torch.float64, device='cuda'), torch.empty((1, n), dtype=torch.float64, device='cuda')
+    p = lambda t: t.data_ptr()  # noqa: E731
+    assert _abi.load().mcw_brf_members(p(ys), 649, 1, n, p(mean), p(std), 0.0, p(brf), p(alb), surrogate._stream(torch)) == 0
+    with np.errstate(over='ignore', under='ignore'):
+        ref = np.exp(ys[:, :, :bins].cpu().double().numpy())
+    assert np.allclose(brf.cpu().numpy(), ref, rtol=4.45e-16, atol=1e-323, equal_nan=True)
+    assert (alb.cpu().numpy() == 1).all()
+
+
 @pytest.mark.parametrize('n,members', [(1, 1), (127, 3), (129, 5), (1000, 2)])
 def test_retrieval_steps_match_numpy(n, members):
     """Inputs encoded on the device, the grid's best point and the damped step against
