@@ -23,13 +23,14 @@
 //    barrier is looked at before a stage's MMAs are issued;
 //  * tiles are 64 or 32 columns wide, so that four CTAs share an SM or a small product is spread
 //    over more SMs (the rules in launch_batch have the times).
-// The epilogue goes through a 32 x 33 tile per warp once: a lane then holds one output column of
+// The epilogue goes through a 32 x 32 tile per warp once: a lane then holds one output column of
 // 32 rows, so loads and stores are whole row runs, and bias gradients are the lane's running sum.
 // At large sizes it is what bounds the launch, by its instructions: a block with all its rows and
-// columns has an instance without predicates, its pointers moving a row at a time, and the SiLU'
-// quotient takes five instructions instead of a division (32 instead of 47 instructions an element
-// with a bias and SiLU, 70 instead of 96 with SiLU', 19 instead of 26 for the output: the autograd
-// pass of 65,536 rows 742 -> 625 us with the stages above, the ensemble's training step 92 -> 81).
+// columns has an instance without predicates, its pointers moving a row at a time; with 16-bit
+// outputs and even strides a lane takes two columns of every other row; and the SiLU' quotient
+// takes five instructions instead of a division.  Instructions an element 47 -> 28 with a bias and
+// SiLU, 96 -> 50 with SiLU', 26 -> 18 for the output; the autograd pass of 65,536 rows 742 -> 591 us
+// with the stages below, the ensemble's training step 92 -> 76 us.
 //
 // Every mbarrier wait is bounded (2 s of %globaltimer); a wait that runs out raises bit 2 of
 // mcw_mlp_status, the CTA waits (bounded) for its copies and MMAs in flight, frees its tensor
@@ -54,7 +55,8 @@ namespace {
 constexpr int TM = 128, TK = 64;
 constexpr int kMaxStages = 8;
 constexpr int kABytes = TM * TK * 2;              // 16 KB
-constexpr int kTileBytes = 32 * 33 * 4;           // an epilogue warp's tile
+constexpr int kPitch = 34;                        // floats a row of an epilogue warp's 32 x 32 tile
+constexpr int kTileBytes = 32 * kPitch * 4;
 constexpr int kThreads = 192;
 constexpr unsigned long long kWaitNs = 2000000000ull;
 
@@ -81,6 +83,7 @@ struct GemmProb {
     int32_t colsum_chunks, colsum_rows;
     const float *weights;           // LOSS: per column
     float *loss;                    // LOSS: per group
+    int32_t pairs;                  // 16-bit outputs, and what goes with them, on pairs of columns
 };
 
 struct GemmBatch {
@@ -251,6 +254,58 @@ __device__ __forceinline__ void load_aux(const GemmProb &p, int g, int rbase, in
     }
 }
 
+// The same for block_pairs: rows 2 i + lane / 16, two columns a lane.
+__device__ __forceinline__ void load_aux_pairs(const GemmProb &p, int g, int rbase, int nb, int lane, float (&av)[32]) {
+    const float *src = p.aux + (size_t)g * p.s_aux + (size_t)(rbase + (lane >> 4)) * p.ld_aux + nb + 2 * (lane & 15);
+#pragma unroll
+    for (int i = 0; i < 16; ++i, src += 2 * p.ld_aux) {
+        const float2 v = __ldg(reinterpret_cast<const float2 *>(src));
+        av[2 * i] = v.x, av[2 * i + 1] = v.y;
+    }
+}
+
+// One whole 32 x 32 block of a tile with 16-bit outputs: two rows at a time, two columns a lane, so
+// that an address, a load and a store serve two elements.  csum: the sums of the lane's columns.
+template <int kEpi>
+__device__ __forceinline__ void block_pairs(const GemmProb &p, int g, int rbase, int nb, const float *tile, int lane,
+                                            const float (&av)[32], float2 &csum, float &lsum) {
+    const int col = nb + 2 * (lane & 15), row = rbase + (lane >> 4);
+    float2 bias = make_float2(0.f, 0.f), wc = make_float2(1.f, 1.f);
+    if (kEpi != MCW_EPI_DSILU && p.bias) {
+        const float *b = p.bias + (size_t)g * p.s_bias + col;
+        bias = make_float2(__ldg(b), __ldg(b + 1));
+    }
+    if (kEpi == MCW_EPI_LOSS && p.weights) wc = make_float2(__ldg(p.weights + col), __ldg(p.weights + col + 1));
+    const float scale = kEpi == MCW_EPI_LOSS ? 1.f / ((float)p.m * (float)p.n) : 0.f;
+    __nv_bfloat16 *c16 = static_cast<__nv_bfloat16 *>(p.c) + (size_t)g * p.s_c + (size_t)row * p.ldc + col;
+    float *c32 = p.c2 ? p.c2 + (size_t)g * p.s_c2 + (size_t)row * p.ldc2 + col : nullptr;
+    const bool has32 = p.c2 != nullptr;
+    const float *src = tile + (lane >> 4) * kPitch + 2 * (lane & 15);
+    csum = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        float2 z = *reinterpret_cast<const float2 *>(src + 2 * i * kPitch);
+        if (kEpi != MCW_EPI_DSILU) z.x += bias.x, z.y += bias.y;
+        if (kEpi == MCW_EPI_DSILU) z.x *= dsilu(av[2 * i]), z.y *= dsilu(av[2 * i + 1]);
+        if (kEpi == MCW_EPI_LOSS) {
+            const float dx = z.x - av[2 * i], dy = z.y - av[2 * i + 1];
+            lsum += wc.x * dx * dx * scale;
+            lsum += wc.y * dy * dy * scale;
+            z.x = 2.f * wc.x * dx * scale, z.y = 2.f * wc.y * dy * scale;
+        }
+        if (kEpi != MCW_EPI_BIAS_SILU) csum.x += z.x, csum.y += z.y;
+        if (has32) {
+            *reinterpret_cast<float2 *>(c32) = z;
+            c32 += 2 * p.ldc2;
+        }
+        if (kEpi == MCW_EPI_BIAS_SILU) z.x = silu(z.x), z.y = silu(z.y);
+        *reinterpret_cast<__nv_bfloat162 *>(c16) = __floats2bfloat162_rn(z.x, z.y);
+        c16 += 2 * p.ldc;
+    }
+    csum.x += __shfl_xor_sync(0xffffffffu, csum.x, 16);
+    csum.y += __shfl_xor_sync(0xffffffffu, csum.y, 16);
+}
+
 // One 32 x 32 block of a tile, its product in `tile`: a lane's column, row by row.  kFull: the block
 // has all its rows and columns.
 template <int kEpi, bool kFull>
@@ -278,7 +333,7 @@ __device__ __forceinline__ void block_rows(const GemmProb &p, int g, int sp, int
     const bool turned = (kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_DSILU) && p.ct;
 #pragma unroll
     for (int r = 0; r < 32; ++r) {
-        float z = tile[r * 33 + lane];
+        float z = tile[r * kPitch + lane];
         const bool in = kFull || r < rows;
         if (kEpi == MCW_EPI_BIAS_F32 || kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_LOSS) z += bias;
         if (kEpi == MCW_EPI_DSILU) z *= dsilu(av[r]);
@@ -296,7 +351,7 @@ __device__ __forceinline__ void block_rows(const GemmProb &p, int g, int sp, int
             const __nv_bfloat16 h = __float2bfloat16(kEpi == MCW_EPI_BIAS_SILU ? silu(z) : z);
             if (in) *c16 = h;
             c16 += p.ldc;
-            if (turned) tile[r * 33 + lane] = __bfloat162float(h);
+            if (turned) tile[r * kPitch + lane] = __bfloat162float(h);
         }
     }
     if (turned && col_ok && rows > 0) {
@@ -307,8 +362,8 @@ __device__ __forceinline__ void block_rows(const GemmProb &p, int g, int sp, int
             uint32_t h[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const uint32_t lo = __float_as_uint(tile[(8 * q + 2 * k) * 33 + lane]) >> 16;
-                h[k] = lo | (__float_as_uint(tile[(8 * q + 2 * k + 1) * 33 + lane]) & 0xffff0000u);
+                const uint32_t lo = __float_as_uint(tile[(8 * q + 2 * k) * kPitch + lane]) >> 16;
+                h[k] = lo | (__float_as_uint(tile[(8 * q + 2 * k + 1) * kPitch + lane]) & 0xffff0000u);
             }
             if (wide) {
                 reinterpret_cast<uint4 *>(dst)[q] = make_uint4(h[0], h[1], h[2], h[3]);
@@ -487,7 +542,14 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
         uint32_t verdict;
         float av[32];
         const bool all_rows = rbase + 32 <= p.m;
-        if (kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) load_aux(p, g, rbase, n0 + lane, all_rows && n0 + 32 <= p.n, av);
+        constexpr bool k16 = kEpi == MCW_EPI_BIAS_SILU || kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS;
+        constexpr bool kAux = kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS;
+        auto aux_of = [&](int nb) {                   // block nb's other input
+            const bool whole = all_rows && nb + 32 <= p.n;
+            if (whole && p.pairs) load_aux_pairs(p, g, rbase, nb, lane, av);
+            else load_aux(p, g, rbase, nb + lane, whole, av);
+        };
+        if (kAux) aux_of(n0);
         // the total of the 128-row sums of A's rows, in order
         if (kEpi == MCW_EPI_F32 && p.colsum_in && p.colsum_rows == 0 && sp == 0 && n0 == 0 && rbase + lane < p.m) {
             const float *src = p.colsum_in + (size_t)g * p.s_colsum + rbase + lane;
@@ -511,23 +573,35 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
             const int nb = n0 + c0;
             if (nb >= p.n) break;                                   // block-uniform
             const int col = nb + lane;
-            const bool col_ok = col < p.n;
+            const bool col_ok = col < p.n, whole = all_rows && nb + 32 <= p.n;
             {
                 uint32_t v[32];
                 tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
                 __syncwarp();
+                float2 *dst = reinterpret_cast<float2 *>(tile + lane * kPitch);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = nch > 0 ? __uint_as_float(v[j]) : 0.f;
+                for (int j = 0; j < 16; ++j) {
+                    if (nch > 0) dst[j] = make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                    else dst[j] = make_float2(0.f, 0.f);
+                }
                 __syncwarp();
             }
             float csum = 0.f;
-            if (all_rows && nb + 32 <= p.n) block_rows<kEpi, true>(p, g, sp, rbase, col, tile, lane, av, csum, lsum);
-            else block_rows<kEpi, false>(p, g, sp, rbase, col, tile, lane, av, csum, lsum);
-            if (kEpi == MCW_EPI_DSILU || kEpi == MCW_EPI_LOSS) {
+            float2 csum2 = make_float2(0.f, 0.f);
+            const bool pairs = k16 && whole && p.pairs;
+            if constexpr (k16) {
+                if (pairs) block_pairs<kEpi>(p, g, rbase, nb, tile, lane, av, csum2, lsum);
+            }
+            if (!pairs) {
+                if (whole) block_rows<kEpi, true>(p, g, sp, rbase, col, tile, lane, av, csum, lsum);
+                else block_rows<kEpi, false>(p, g, sp, rbase, col, tile, lane, av, csum, lsum);
+            }
+            if (kAux) {
                 // the next block's other input while this one's sums are put together
-                if (c0 + 32 < TN && nb + 32 < p.n) load_aux(p, g, rbase, col + 32, all_rows && nb + 64 <= p.n, av);
+                if (c0 + 32 < TN && nb + 32 < p.n) aux_of(nb + 32);
                 if (p.colsum) {
-                    part[warp * 32 + lane] = csum;
+                    if (!pairs) part[warp * 32 + lane] = csum;
+                    else if (lane < 16) part[warp * 32 + 2 * lane] = csum2.x, part[warp * 32 + 2 * lane + 1] = csum2.y;
                     asm volatile("bar.sync 1, 128;\n" ::: "memory");
                     if (warp == 0 && col_ok)
                         p.colsum[(size_t)g * p.s_colsum + (size_t)mtile * p.ld_colsum + col] =
@@ -651,8 +725,8 @@ int launch_batch(const McwGemmProblem *q, int np, cudaStream_t stream) {
         chunks = c > chunks ? c : chunks;
     }
     // 64 columns a tile when that leaves two tiles per SM: at 65,536 rows with tiles of 32 / 64
-    // columns the SiLU' product of 649 takes 92 / 72 us, of 256 62 / 55 (bias + SiLU 256 x 256 53 / 42,
-    // the 256 x 649 output 84 / 70)
+    // columns the SiLU' product of 649 takes 92 / 69 us, of 256 62 / 51 (bias + SiLU 256 x 256 53 / 36,
+    // the 256 x 649 output 84 / 72)
     const int tn = t64 >= 304 ? 64 : 32;
     // two stages when the launch fills the SMs several times over (four CTAs of an SM overlap each
     // other), else up to eight, or as many as the chunks; five of two chunks each for a transposed
@@ -691,6 +765,11 @@ int launch_batch(const McwGemmProblem *q, int np, cudaStream_t stream) {
         d.colsum = s.colsum, d.colsum_in = s.colsum_in, d.s_colsum = s.stride_colsum, d.ld_colsum = s.ld_colsum;
         d.colsum_chunks = s.colsum_chunks, d.colsum_rows = s.colsum_rows;
         d.weights = s.weights, d.loss = s.loss;
+        auto even = [](const void *p, long long ld, long long stride, int bytes) {
+            return !p || (!(reinterpret_cast<uintptr_t>(p) % (2 * bytes)) && !(ld & 1) && !(stride & 1));
+        };
+        d.pairs = (s.epilogue == MCW_EPI_BIAS_SILU || s.epilogue == MCW_EPI_DSILU || s.epilogue == MCW_EPI_LOSS) && !s.ct &&
+                  even(s.c, s.ldc, s.stride_c, 2) && even(s.c2, s.ldc2, s.stride_c2, 4) && even(s.aux, s.ldaux, s.stride_aux, 4);
     }
     b.sums0 = cta > 0x7fffffffLL ? 0 : (int32_t)cta;
     for (int i = 0; i < np; ++i) {
