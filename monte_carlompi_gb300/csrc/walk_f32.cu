@@ -652,6 +652,37 @@ __device__ __forceinline__ int sparse_round(Photon &P, WarpQueues &q, const unsi
                 xs[u] = q.pbuf[2 * (t0 + u)];
                 ys[u] = q.pbuf[2 * (t0 + u) + 1];
             }
+            // a group that does nothing but scatter (most do) is a chain of rotations without a
+            // branch; its result is dropped, and the group walked step by step, when a step
+            // starts the photon, is reflected or along the vertical, or ends in something (a lone
+            // photon's 256 steps 24 -> 14 us with impurities 29 -> 16; the launch of 1,000 photons
+            // of deep snow 97 -> 85, of 100,000 154 -> 148, of 1e6 330 -> 322)
+            bool plain = P.i != 0 && !(P.flags & (kFlagReflect | kFlagLamSurface));
+            if (plain) {
+                float mx = P.mux, my = P.muy, mz = P.muz, z = P.z, path = P.path, pathc = P.pathc;
+#pragma unroll
+                for (int u = 0; u < kStepsPerRound; ++u) {
+                    const float s2 = horiz2(mx, my);
+                    const float3 g = rotate(mx, my, mz, s2, xs[u].x, xs[u].y, ys[u].y, ys[u].x, u == kStepsPerRound - 1);
+                    const float2 zi = __ffma2_rn(make_float2(ys[u].z, ys[u].z), make_float2(g.z, P.inv_ext),
+                                                 make_float2(z, 0.f));
+                    const float y = zi.y - pathc;
+                    const float tt = path + y;
+                    pathc = (tt - path) - y;
+                    path = tt;
+                    z = zi.x;
+                    const bool imp = kImpurity && ((impm >> (t0 + u)) & 1u);
+                    plain = plain && s2 > 0.f && !(z > 0.f) && !(z < -P.tau) &&
+                            !(ys[u].w < (imp ? P.coalb_imp : P.coalb_ice));
+                    mx = g.x, my = g.y, mz = g.z;
+                }
+                if (plain) {
+                    P.i += kStepsPerRound;
+                    P.mux = mx, P.muy = my, P.muz = mz;
+                    P.z = z, P.path = path, P.pathc = pathc;
+                    continue;
+                }
+            }
             // each photon's lane leaves at its end condition (at most kSparseWarp lanes walk
             // here, so the divergence costs little); the state is the one after that step,
             // as in the dense rounds

@@ -873,3 +873,18 @@ def test_replay_records_independent_of_photon_count(walker, case, n):
     big = walker.walk([dataclasses.replace(cfg, n_photon=11000)], 3, mode='replay64').records
     got = walker.walk([cfg], 3, mode='replay64').records
     assert np.array_equal(got, big[:n])
+
+
+@pytest.mark.parametrize('n', [1, 2, 4, 8])
+@pytest.mark.parametrize('theta0,tau', [(0.0, 3.0), (0.0, 40.0), (75.0, 3.0)])
+def test_f32_sparse_groups_same_records(walker, n, theta0, tau):
+    """Sparse rounds walk groups of four steps without a branch where nothing but scattering
+    happens in them: the first n records of a launch of full warps, beams along the vertical
+    and slabs thin enough for reflections and exits in most groups."""
+    cfg, ice, imp = cfg2_geometry(20000)
+    cfg = dataclasses.replace(cfg, theta0_deg=theta0, tau_tot=tau, lambertian_reflectance=0.9)
+    walker.set_tables([ice], imp)
+    for seed in range(8):
+        big = walker.walk([dataclasses.replace(cfg, n_photon=5000)], seed, mode='f32').records
+        small = walker.walk([dataclasses.replace(cfg, n_photon=n)], seed, mode='f32').records
+        assert np.array_equal(small, big[:n])
