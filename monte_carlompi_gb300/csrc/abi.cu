@@ -735,6 +735,10 @@ int mcw_set_phase_matrices(mcw_ctx *ctx, const mcw_phase_table *tabs, int32_t n)
             d.cos_max = p.cos_max;
             d.cos_min = p.cos_min;
             d.cos_cutoff = p.cos_cutoff;
+            d.shared_grid = 1;
+            for (int e = 1; e < 6; ++e)
+                if (p.n_angle[e] != p.n_angle[0] || memcmp(p.cos_asc[e], p.cos_asc[0], p.n_angle[0] * sizeof(double)))
+                    d.shared_grid = 0;
         }
         dev[t] = d;
     }

@@ -91,7 +91,7 @@ struct DevPhase {
     const double *a1, *a2, *b1, *b2;
     int32_t n_angle[6];
     int32_t n_rows;
-    int32_t pad;
+    int32_t shared_grid;         // 1: the six elements share one cos grid
     double cos_max, cos_min, cos_cutoff;
 };
 

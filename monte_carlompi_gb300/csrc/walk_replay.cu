@@ -46,26 +46,6 @@ namespace mcw {
 
 namespace {
 
-// Sequential reader of one photon's replay stream: uniform k uses Philox
-// block k >> 1 (counter (block, tag, photon lo, photon hi)), 64-bit word k & 1.
-struct ReplayStream {
-    uint64_t seed, photon, k;
-    uint4 x;
-    bool overrun;
-
-    __device__ double next() {
-        if ((k & 1) == 0) {
-            uint64_t b = k >> 1;
-            if (b > 0xffffffffull) overrun = true;
-            x = philox10_seed(make_uint4((uint32_t)b, kTagWalk, (uint32_t)photon,
-                                         (uint32_t)(photon >> 32)), seed);
-        }
-        uint64_t w = (k & 1) ? (((uint64_t)x.w << 32) | x.z) : (((uint64_t)x.y << 32) | x.x);
-        ++k;
-        return u01_f64(w);
-    }
-};
-
 __device__ double replay_uniform(uint64_t seed, uint32_t tag, uint64_t photon, uint64_t k) {
     uint4 x = philox10_seed(make_uint4((uint32_t)(k >> 1), tag, (uint32_t)photon,
                                        (uint32_t)(photon >> 32)), seed);
@@ -129,245 +109,6 @@ __device__ void finish_photon(const ReplayArgs &a, int64_t gid, int ci, int cond
     }
 }
 
-// scipy interp1d (linear) on an ascending grid: searchsorted (left) clipped to
-// [1, n-1], then the two-term form of interp1d._call_linear.
-__device__ double interp_n(const double *x, const double *y, int n, double xn) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (x[mid] < xn) lo = mid + 1; else hi = mid;
-    }
-    const int k = lo < 1 ? 1 : (lo > n - 1 ? n - 1 : lo);
-    const double xl = x[k - 1], xh = x[k], yl = y[k - 1], yh = y[k];
-    return ((xn - xl) / (xh - xl)) * yh + ((xh - xn) / (xh - xl)) * yl;
-}
-
-__device__ __forceinline__ double phase_el(const DevPhase &ph, int e, int row, double ct) {
-    return interp_n(ph.cos_asc[e], ph.p_asc[e] + (size_t)row * ph.n_angle[e], ph.n_angle[e], ct);
-}
-
-// rotate_stokes_vector (monte_carlo3D.py:1090-1109)
-__device__ __forceinline__ void rotate_stokes(double angle, const double in[4], double out[4]) {
-    const double d = 2 * angle;
-    const double cd = cos(d), sd = sin(d);
-    out[0] = in[0];
-    out[1] = in[1] * cd + in[2] * sd;
-    out[2] = -in[1] * sd + in[2] * cd;
-    out[3] = in[3];
-}
-
-// Scattering cosine and azimuth of the polarised walk for the photon's Stokes
-// vector st: the two-area rejection sampler of populate_pdfs (:905-1004).
-// Returns false if the stream ran out or the time budget passed.
-__device__ bool polarised_angles(const DevPhase &ph, int row, const double st[4], ReplayStream &s,
-                                 double &p_rand, double &phi_rand, unsigned long long t0,
-                                 unsigned long long budget_ns) {
-    const double I = st[0], Q = st[1], U = st[2];
-    const double two_beta = (Q == 0) ? atan(U / 1e-15) : atan(U / Q);          // :908-911
-    const double C = fabs(Q * cos(two_beta) + U * sin(two_beta));               // :935
-    const double max_val1 = fabs(I) * ph.a1[row] + ph.b1[row] * C;              // :931-937
-    const double max_val2 = fabs(I) * ph.a2[row] + ph.b2[row] * C;              // :940-947
-    const double area1 = (ph.cos_max - ph.cos_cutoff) * max_val1;               // :949-951
-    const double area2 = (ph.cos_cutoff - ph.cos_min) * max_val2;
-    const double percent_area1 = area1 / (area1 + area2);
-    double area_rand = s.next();                                                // :953-957
-    double cos_theta = s.next();
-    double two_phi = 2 * (s.next() * kTwoPi);
-    int area;
-    if (area_rand < percent_area1) {                                            // :963-973
-        area = 1;
-        cos_theta = cos_theta * (ph.cos_max - ph.cos_cutoff) + ph.cos_cutoff;
-    } else {
-        area = 2;
-        cos_theta = -cos_theta * (ph.cos_cutoff - ph.cos_min) + ph.cos_cutoff;
-    }
-    double r3 = 1, pf = 0;                                                      // :976-1001
-    for (int64_t k = 0; r3 > pf; ++k) {
-        if (k > 0) {
-            area_rand = s.next();
-            if (area_rand < percent_area1) {
-                area = 1;
-                cos_theta = s.next() * (ph.cos_max - ph.cos_cutoff) + ph.cos_cutoff;
-            } else {
-                area = 2;
-                cos_theta = -s.next() * (ph.cos_cutoff - ph.cos_min) + ph.cos_cutoff;
-            }
-            two_phi = s.next() * (4 * kPi);
-        }
-        r3 = 1.000001 * s.next();
-        if (area == 1) r3 = r3 * max_val1;
-        else r3 = r3 * max_val2;
-        const double S11 = phase_el(ph, 0, row, cos_theta);
-        const double S12 = phase_el(ph, 1, row, cos_theta);
-        pf = I * S11 + S12 * (Q * cos(two_phi) + U * sin(two_phi));
-        if (s.overrun) return false;
-        if ((k & 255) == 255 && global_ns() - t0 > budget_ns) return false;
-    }
-    p_rand = cos_theta;
-    phi_rand = two_phi / 2.;
-    return true;
-}
-
-__global__ void __launch_bounds__(128) walk_replay_pol_kernel(const ReplayArgs a) {
-    const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= a.total) return;
-    const int ci = find_config(a.prefix, a.n_cfg, gid);
-    const DevConfig c = a.cfgs[ci];
-
-    const uint64_t rid = c.rng_base + (uint64_t)(gid - c.offset);  // stream id
-    const double wvl = replay_wavelength(c, a.seed, rid);
-    const Optics o = photon_optics(c, a.ice[c.ice_table], a.imp, wvl);
-    const bool lam_surface = (c.flags & kFlagLamSurface) != 0;
-    const bool lam_bottom = (c.flags & kFlagLamBottom) != 0;
-    const double tau_tot = c.tau_tot_d, R = c.R_d;
-
-    ReplayStream s{a.seed, rid, 0, make_uint4(0, 0, 0, 0), false};
-    double tau_rand = -log(s.next());  // initial_pdfs, :1035-1038
-    double ssa_rand = s.next();
-    double ext_rand = s.next();
-    double p_rand = 0, phi_rand = 0;
-    double st[4] = {1, 0, 0, 0};                                      // :1132
-    const DevPhase ph = a.phase[c.ice_table];
-    for (int k = 0; k < 4; ++k) st[k] = c.stokes0[k];
-
-    double mux_0 = c.mux0_d, muy_0 = 0, muz_0 = c.muz0_d;             // :1121-1124
-    double muz2_0 = muz_0 * muz_0;
-    double mux_n = 0, muy_n = 0, muz_n = 0;
-    double z_prev = 0, path_length = 0;
-    const double ext_cff = o.ext_cff_mss * c.rho_snw;                 // :1355-1356
-    bool bottom_reflection = false;
-    int condition = 0;
-    int64_t i = 0;
-    const unsigned long long t0 = global_ns();
-
-    while (condition == 0) {                                          // :1212
-        i += 1;
-        if (i > 1) {                                                  // :1215-1224
-            if (!polarised_angles(ph, o.row, st, s, p_rand, phi_rand, t0, a.budget_ns)) {
-                atomicOr(a.status, s.overrun ? kStatusStream : kStatusBudget);
-                break;
-            }
-            tau_rand = -log(s.next());
-            ssa_rand = s.next();
-            ext_rand = s.next();
-        }
-        double dtau = tau_rand;                                       // :1227-1229
-        if (lam_surface && i == 1) dtau = 0;
-        double costheta, sintheta;
-        if (i == 1) {                                                 // :1232-1237
-            costheta = 1;
-            sintheta = 0;
-        } else if (lam_surface || bottom_reflection) {                // :1238-1250
-            mux_0 = 0.;
-            muy_0 = 0.;
-            muz_0 = 1.;
-            for (;;) {
-                double theta_rand = 0 + (kPi / 2 - 0) * s.next();
-                double r1 = s.next();
-                if (r1 < 2 * sin(theta_rand) * cos(theta_rand)) {
-                    costheta = cos(theta_rand);
-                    sintheta = sqrt(1 - costheta * costheta);
-                    break;
-                }
-                if (s.overrun) { costheta = 1; sintheta = 0; break; }
-            }
-        } else {                                                      // :1251-1253
-            costheta = p_rand;
-            sintheta = sqrt(1 - costheta * costheta);
-        }
-        if (i > 1) {                                                  // :1255-1281
-            double cosphi = cos(phi_rand), sinphi = sin(phi_rand);
-            if (muz_0 == 1) {
-                mux_n = sintheta * cosphi;
-                muy_n = sintheta * sinphi;
-                muz_n = costheta;
-            } else if (muz_0 == -1) {
-                mux_n = sintheta * cosphi;
-                muy_n = -sintheta * sinphi;
-                muz_n = -costheta;
-            } else {
-                double sq = sqrt(1 - muz2_0);
-                mux_n = (sintheta * (mux_0 * muz_0 * cosphi - muy_0 * sinphi)) / sq + mux_0 * costheta;
-                muy_n = (sintheta * (muy_0 * muz_0 * cosphi + mux_0 * sinphi)) / sq + muy_0 * costheta;
-                muz_n = -sq * sintheta * cosphi + muz_0 * costheta;
-            }
-            if (bottom_reflection) {                                  // :1283-1285
-                st[0] = 1; st[1] = 0; st[2] = 0; st[3] = 0;
-                bottom_reflection = false;
-            } else {                                                  // :1287-1342
-                const double cos2theta = costheta * costheta;
-                const double phi_sca = acos(cosphi);
-                double sp[4], sc[4], sm[4];
-                rotate_stokes(phi_sca, st, sp);
-                const double P11 = phase_el(ph, 0, o.row, costheta), P12 = phase_el(ph, 1, o.row, costheta);
-                const double P22 = phase_el(ph, 2, o.row, costheta), P33 = phase_el(ph, 3, o.row, costheta);
-                const double P43 = phase_el(ph, 4, o.row, costheta), P44 = phase_el(ph, 5, o.row, costheta);
-                sc[0] = sp[0] * P11 + sp[1] * P12;
-                sc[1] = sp[0] * P12 + sp[1] * P22;
-                sc[2] = sp[2] * P33 - sp[3] * P43;
-                sc[3] = sp[2] * P43 + sp[3] * P44;
-                const double den = sqrt((1 - cos2theta) * (1 - muz_n * muz_n));
-                double cos_i;
-                if (den == 0) {
-                    cos_i = 0;
-                } else {
-                    const double num = muz_n * costheta - muz_0;
-                    const double sign = (phi_sca >= kPi) ? 1 : -1;
-                    cos_i = num / (sign * den);
-                    if (cos_i < -1) cos_i = -1;
-                    else if (cos_i > 1) cos_i = 1;
-                }
-                rotate_stokes(-acos(cos_i), sc, sm);
-                const double I_merd = sm[0];
-                for (int k = 0; k < 4; ++k) st[k] = sm[k] / I_merd;
-            }
-        } else {                                                      // :1344-1347
-            mux_n = mux_0;
-            muy_n = muy_0;
-            muz_n = muz_0;
-        }
-        double z_i = z_prev + dtau * muz_n;                           // :1352
-        if (i > 1) {                                                  // :1364-1369
-            mux_0 = mux_n;
-            muy_0 = muy_n;
-            muz_0 = muz_n;
-            muz2_0 = muz_0 * muz_0;
-        }
-        path_length += dtau / ext_cff;                                // :1372
-        bool ice = ext_rand > o.p_imp;                                // :1375-1383
-        double ssa_event = ice ? o.ssa_ice : o.ssa_imp;
-        if (lam_surface) ssa_event = R;                               // :1385-1387
-        if (z_i > 0) {                                                // :1390-1397
-            condition = 1;
-            path_length += -((z_i * dtau) / ((z_i - z_prev) * ext_cff));
-        } else if (z_i < -tau_tot) {                                  // :1399-1459
-            path_length += -(((z_i + tau_tot) * dtau) / ((z_i - z_prev) * ext_cff));
-            double dtau_correction = -(((z_i + tau_tot) / (z_prev - z_i)) * dtau);
-            z_i = z_i - (muz_n * dtau_correction);
-            const int leave = (i == 1) ? 3 : 2;
-            if (lam_bottom) {
-                if (s.next() <= R) bottom_reflection = true;
-                else condition = leave;
-            } else {
-                condition = leave;
-            }
-        } else if (ssa_rand >= ssa_event) {                           // :1461-1466
-            condition = ice ? 4 : 5;
-        }
-        z_prev = z_i;
-        if (s.overrun) {
-            atomicOr(a.status, kStatusStream);
-            break;
-        }
-        if ((i & 1023) == 0 && global_ns() - t0 > a.budget_ns) {
-            atomicOr(a.status, kStatusBudget);
-            break;
-        }
-    }
-
-    finish_photon<true>(a, gid, ci, condition, i, o.wvl_um, mux_0, muy_0, muz_0, path_length, o.snow_depth, st);
-}
-
 // ---------------------------------------------------------------- the HG walk
 
 constexpr int kSlots = 16;                   // photons a block walks at once
@@ -383,7 +124,7 @@ struct Slot {
     uint64_t rid, k;                         // stream id, next uniform
     int64_t gid;
     int64_t i;                               // steps walked
-    int32_t ci;
+    int32_t ci, row;                         // config, ice-table row
     uint32_t flags;
     __device__ __forceinline__ bool lambertian() const { return (flags & (kRefl | kSurface)) != 0; }
 };
@@ -544,6 +285,7 @@ __device__ int replay_birth(const ReplayArgs &a, int64_t gid, Slot &out) {
     s.p_imp = o.p_imp;
     s.wvl_um = o.wvl_um;
     s.depth = o.snow_depth;
+    s.row = o.row;
     s.mux = c.mux0_d;                                                 // :1121-1124
     s.muy = 0;
     s.muz = c.muz0_d;
@@ -913,14 +655,315 @@ __global__ void __launch_bounds__(128, 4) walk_replay_kernel(const ReplayArgs a)
     if (part == kM && n_fin > 0) flush();
 }
 
+// ---------------------------------------------------------------- the polarised walk
+
+// Order of doubles as integers (no FP64 operation), -0 with 0.
+__device__ __forceinline__ int64_t order_of(double x) {
+    const int64_t b = (int64_t)to_bits(x);
+    return b >= 0 ? b : ((int64_t)0x8000000000000000ull - b);
+}
+
+// 1 / b and a / b by it, b normal (div_res in two parts).
+__device__ __forceinline__ double rcp_res(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    return fma(fma(-b, y, 1.0), y, y);
+}
+__device__ __forceinline__ double quotient(double a, double b, double rb) {
+    const double q = a * rb;
+    return fma(fma(-q, b, a), rb, q);
+}
+
+// Whether |x| lies between 2^-255 and 2^256: the ranges of the two functions above and of sqrt_res hold.
+__device__ __forceinline__ bool moderate(double x) {
+    const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+    return h >= 0x30000000u && h < 0x4ff00000u;
+}
+
+// The square root of 1 - c^2 and the like, in [0, 1] but for rounding (then NaN).
+__device__ __forceinline__ double sqrt_unit(double x) {
+    return !(to_bits(x) >> 63) && moderate(x) ? sqrt_res(x) : sqrt(x);
+}
+
+// scipy interp1d (linear) on an ascending grid: searchsorted (left) clipped to [1, n - 1], then the
+// two-term form of interp1d._call_linear: the upper end's index and both weights.
+struct Segment {
+    int k;
+    double lo, hi;
+};
+__device__ __forceinline__ Segment segment_of(const DevPhase &ph, int e, double xn) {
+    const double *x = ph.cos_asc[e];
+    const int n = ph.n_angle[e];
+    const int64_t key = order_of(xn);
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (order_of(__ldg(x + mid)) < key) lo = mid + 1; else hi = mid;
+    }
+    Segment s;
+    s.k = lo < 1 ? 1 : (lo > n - 1 ? n - 1 : lo);
+    const double xl = __ldg(x + s.k - 1), xh = __ldg(x + s.k), w = xh - xl;
+    if (moderate(w)) {
+        const double rw = rcp_res(w);
+        s.hi = quotient(xn - xl, w, rw);
+        s.lo = quotient(xh - xn, w, rw);
+    } else {
+        s.hi = (xn - xl) / w;
+        s.lo = (xh - xn) / w;
+    }
+    return s;
+}
+__device__ __forceinline__ double element(const DevPhase &ph, int e, int row, const Segment &s) {
+    const double *y = ph.p_asc[e] + (size_t)row * ph.n_angle[e] + s.k;
+    return s.hi * __ldg(y) + s.lo * __ldg(y - 1);
+}
+
+// rotate_stokes_vector (monte_carlo3D.py:1090-1109)
+__device__ __forceinline__ void rotate_stokes(double angle, const double in[4], double out[4]) {
+    const double d = 2 * angle;
+    double sd, cd;
+    sincos(d, &sd, &cd);
+    out[0] = in[0];
+    out[1] = in[1] * cd + in[2] * sd;
+    out[2] = -in[1] * sd + in[2] * cd;
+    out[3] = in[3];
+}
+
+// The envelope of the rejection sampler for a Stokes vector (populate_pdfs, :905-951).
+struct PolEnvelope {
+    double max1, max2, part1;
+};
+__device__ PolEnvelope pol_envelope(const DevPhase &ph, int row, const double st[4]) {
+    const double I = st[0], Q = st[1], U = st[2];
+    const double two_beta = (Q == 0) ? atan(U / 1e-15) : atan(U / Q);  // :908-911
+    double sb, cb;
+    sincos(two_beta, &sb, &cb);
+    const double C = fabs(Q * cb + U * sb);                           // :935
+    PolEnvelope v;
+    v.max1 = fabs(I) * ph.a1[row] + ph.b1[row] * C;                   // :931-937
+    v.max2 = fabs(I) * ph.a2[row] + ph.b2[row] * C;                   // :940-947
+    const double area1 = (ph.cos_max - ph.cos_cutoff) * v.max1;       // :949-951
+    const double area2 = (ph.cos_cutoff - ph.cos_min) * v.max2;
+    v.part1 = area1 / (area1 + area2);
+    return v;
+}
+
+// The sampler's candidate whose four uniforms begin at k (:953-1001): its cosine and doubled azimuth,
+// and whether it passes.
+__device__ __forceinline__ bool pol_candidate(const DevPhase &ph, const Slot &s, uint64_t seed, uint64_t k, const double st[4],
+                                              const PolEnvelope &v, double &cos_theta, double &two_phi) {
+    const uint4 x0 = stream_block(seed, s.rid, k >> 1), x1 = stream_block(seed, s.rid, (k >> 1) + 1),
+                x2 = stream_block(seed, s.rid, (k >> 1) + 2);
+    const bool odd = k & 1;
+    const double u0 = u01_bits(word(x0, odd)), u1 = u01_bits(odd ? word(x1, false) : word(x0, true)),
+                 u2 = u01_bits(word(x1, odd)), u3 = u01_bits(odd ? word(x2, false) : word(x1, true));
+    const bool one = u0 < v.part1;                                    // :963-973
+    cos_theta = one ? u1 * (ph.cos_max - ph.cos_cutoff) + ph.cos_cutoff
+                    : -u1 * (ph.cos_cutoff - ph.cos_min) + ph.cos_cutoff;
+    two_phi = 2 * (u2 * kTwoPi);
+    const double r3 = 1.000001 * u3 * (one ? v.max1 : v.max2);        // :976-1001
+    const Segment g0 = segment_of(ph, 0, cos_theta);
+    const Segment g1 = ph.shared_grid ? g0 : segment_of(ph, 1, cos_theta);
+    const double S11 = element(ph, 0, s.row, g0), S12 = element(ph, 1, s.row, g1);
+    double sp, cp;
+    sincos(two_phi, &sp, &cp);
+    const double pf = st[0] * S11 + S12 * (st[1] * cp + st[2] * sp);
+    return !(r3 > pf);
+}
+
+// A step of photon s past its first with its scattering angles (:1227-1466); returns its end
+// condition.  Its uniforms begin at s.k.
+__device__ int pol_step(const DevPhase &ph, Slot &s, uint64_t seed, double st[4], double p_rand, double two_phi) {
+    const double dtau = -log(uniform_at(seed, s.rid, s.k));
+    const double ssa_rand = uniform_at(seed, s.rid, s.k + 1);
+    const bool ice = uniform_at(seed, s.rid, s.k + 2) > s.p_imp;      // :1375-1383
+    s.k += 3;
+    const bool reflected = (s.flags & kRefl) != 0;
+    double mux = s.mux, muy = s.muy, muz = s.muz, ct = p_rand;
+    if (s.lambertian()) {                                             // :1238-1250
+        mux = muy = 0.;
+        muz = 1.;
+        for (int tries = 0;; ++tries) {
+            const double theta = 0 + (kPi / 2 - 0) * uniform_at(seed, s.rid, s.k);
+            const double r1 = uniform_at(seed, s.rid, s.k + 1);
+            double sn;
+            sincos(theta, &sn, &ct);
+            s.k += 2;
+            if (r1 < 2 * sn * ct || tries >= 131072) break;           // no stream needs as many
+        }
+    }
+    const double sint = sin_from(ct);                                 // :1251-1253
+    const double phi = two_phi / 2.;
+    double sinphi, cosphi;
+    sincos(phi, &sinphi, &cosphi);
+    double nx, ny, nz;
+    if (is_unit(muz)) {                                               // :1262-1269
+        const bool up = !(to_bits(muz) >> 63);
+        nx = sint * cosphi;
+        ny = up ? sint * sinphi : -sint * sinphi;
+        nz = up ? ct : -ct;
+    } else {                                                          // :1270-1281
+        const double sq = sqrt_unit(1 - muz * muz);
+        const double tx = sint * (mux * muz * cosphi - muy * sinphi), ty = sint * (muy * muz * cosphi + mux * sinphi);
+        if (moderate(sq)) {
+            const double rq = rcp_res(sq);
+            nx = quotient(tx, sq, rq) + mux * ct;
+            ny = quotient(ty, sq, rq) + muy * ct;
+        } else {
+            nx = tx / sq + mux * ct;
+            ny = ty / sq + muy * ct;
+        }
+        nz = -sq * sint * cosphi + muz * ct;
+    }
+    if (reflected) {                                                  // :1283-1285
+        st[0] = 1; st[1] = 0; st[2] = 0; st[3] = 0;
+    } else {                                                          // :1287-1342
+        const double phi_sca = acos(cosphi);
+        double sp[4], sc[4], sm[4], P[6];
+        rotate_stokes(phi_sca, st, sp);
+        const Segment g = segment_of(ph, 0, ct);
+#pragma unroll
+        for (int e = 0; e < 6; ++e) P[e] = element(ph, e, s.row, e == 0 || ph.shared_grid ? g : segment_of(ph, e, ct));
+        const double P11 = P[0], P12 = P[1], P22 = P[2], P33 = P[3], P43 = P[4], P44 = P[5];
+        sc[0] = sp[0] * P11 + sp[1] * P12;
+        sc[1] = sp[0] * P12 + sp[1] * P22;
+        sc[2] = sp[2] * P33 - sp[3] * P43;
+        sc[3] = sp[2] * P43 + sp[3] * P44;
+        const double den = sqrt_unit((1 - ct * ct) * (1 - nz * nz));
+        double cos_i = 0;
+        if (!(den == 0)) {
+            const double sign = (phi_sca >= kPi) ? 1 : -1;
+            const double num = nz * ct - muz, d = sign * den;
+            cos_i = moderate(d) ? div_res(num, d) : num / d;
+            if (cos_i < -1) cos_i = -1;
+            else if (cos_i > 1) cos_i = 1;
+        }
+        rotate_stokes(-acos(cos_i), sc, sm);
+        if (moderate(sm[0])) {
+            const double ri = rcp_res(sm[0]);
+            st[0] = 1;
+#pragma unroll
+            for (int k = 1; k < 4; ++k) st[k] = quotient(sm[k], sm[0], ri);
+        } else {
+            const double I_merd = sm[0];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) st[k] = sm[k] / I_merd;
+        }
+    }
+    s.flags &= ~kRefl;
+    const double zp = s.z;
+    s.z = zp + dtau * nz;                                             // :1352
+    s.mux = nx, s.muy = ny, s.muz = nz;                               // :1364-1369
+    const double q0 = dtau * s.rext;
+    s.path += fma(fma(-q0, s.ext, dtau), s.rext, q0);                 // dtau / ext (:1372)
+    s.i += 1;
+    return step_end(s, seed, s.z, zp, dtau, nz, s.path, false, ssa_rand >= (ice ? s.ssa_ice : s.ssa_imp), ice, &s.k, &s.flags);
+}
+
+// 2^glog lanes a photon, the same state in each: they test candidates of the sampler side by side
+// (a candidate takes four uniforms of the photon's stream, so candidate j's are known; the first that
+// passes is the sampler's), and walk the rest of the step alike.  A group whose photon ends takes the
+// next.  Bound by FP64 instructions, 64 cycles a warp each however many lanes take part.  So searches
+// compare bits, the six elements share one segment's weights where they share a grid, quotients by
+// one divisor its reciprocal, and sine and cosine come together: about 60 a candidate and 430 a
+// step's rest (145 and 650 with one thread a photon, whose warp also waited for the slowest of 32
+// samplers).  Hexagonal plates, 100 um, tau as below 40: 50 photons 40.4 -> 9.4 ms, 1,000
+// 80.8 -> 20.3, 10,000 95.6 -> 34.9, 40,000 153 -> 87; a lone photon's step 17 us.
+__global__ void __launch_bounds__(128, 3) walk_replay_pol_kernel(const ReplayArgs a, const int glog) {
+    const int lane = threadIdx.x & 31, G = 1 << glog, gl = lane & (G - 1), g0 = lane - gl;
+    const unsigned group = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << g0;
+    Slot s{};
+    double st[4] = {1, 0, 0, 0};
+    bool have = false, exhausted = false;
+    const unsigned long long t0 = global_ns();
+    for (uint32_t it = 0;; ++it) {
+        int cond = 0;
+        const unsigned need = __ballot_sync(0xffffffffu, !have && !exhausted && gl == 0);
+        bool born = false;
+        if (need) {
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(a.work, (unsigned long long)__popc(need));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (!have && !exhausted) {
+                const unsigned long long n = base + __popc(need & ((1u << g0) - 1u));
+                if (n < (unsigned long long)a.total) {
+                    cond = replay_birth(a, (int64_t)n, s);
+                    const DevConfig &c = a.cfgs[s.ci];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) st[k] = c.stokes0[k];
+                    have = born = true;
+                } else {
+                    exhausted = true;
+                }
+            }
+        }
+        if (!__any_sync(0xffffffffu, have)) break;
+        // ---- the scattering angles of the photons walking on
+        const DevPhase &ph = a.phase[have ? a.cfgs[s.ci].ice_table : 0];
+        bool pending = have && !born;
+        PolEnvelope env{0, 0, 0};
+        if (pending) env = pol_envelope(ph, s.row, st);
+        double p_rand = 1, two_phi = 0;
+        uint32_t j0 = 0;
+        for (uint32_t round = 0; __any_sync(0xffffffffu, pending); ++round) {
+            bool pass = false;
+            double c = 1, t = 0;
+            if (pending) pass = pol_candidate(ph, s, a.seed, s.k + 4 * (uint64_t)(j0 + gl), st, env, c, t);
+            const unsigned hit = __ballot_sync(0xffffffffu, pass) & group;
+            const int src = hit ? __ffs(hit) - 1 : lane;
+            c = shfl_d(c, src);
+            t = shfl_d(t, src);
+            if (pending && hit) {
+                p_rand = c;
+                two_phi = t;
+                s.k += 4 * (uint64_t)(j0 + (uint32_t)(src - g0) + 1);
+                pending = false;
+            }
+            j0 += (uint32_t)G;
+            if ((round & 255u) == 255u) {
+                int over = 0;
+                if (lane == 0) over = global_ns() - t0 > a.budget_ns;
+                if (__shfl_sync(0xffffffffu, over, 0)) {
+                    if (lane == 0) atomicOr(a.status, kStatusBudget);
+                    return;
+                }
+            }
+        }
+        if (have && !born) {
+            cond = pol_step(ph, s, a.seed, st, p_rand, two_phi);
+            if (s.k > (1ull << 33)) {
+                if (gl == 0) atomicOr(a.status, kStatusStream);
+                have = false;
+            }
+        }
+        if (cond > 0) {
+            if (gl == 0) finish_photon<true>(a, s.gid, s.ci, cond, s.i, s.wvl_um, s.mux, s.muy, s.muz, s.path, s.depth, st);
+            have = false;
+        }
+        if ((it & 63u) == 63u) {                                      // time budget (watchdog)
+            int stop = 0;
+            if (lane == 0) stop = (global_ns() - t0 > a.budget_ns) || *(volatile unsigned int *)a.status;
+            if (__shfl_sync(0xffffffffu, stop, 0)) {
+                if (lane == 0 && global_ns() - t0 > a.budget_ns) atomicOr(a.status, kStatusBudget);
+                return;
+            }
+        }
+    }
+}
+
 }  // namespace
 
 cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s) {
     if (a.total <= 0) return cudaSuccess;
     if (a.pol) {
-        const int block = 128;
-        const int64_t grid = (a.total + block - 1) / block;
-        walk_replay_pol_kernel<<<(unsigned)grid, block, 0, s>>>(a);
+        // three blocks an SM (140 registers), and as many lanes a photon as let all photons walk at
+        // once: a lane more tests a candidate for nothing, but a photon more in a warp shares its rest
+        const int64_t warps = 12 * (int64_t)std::max(1, sm_count);
+        int glog = 5;
+        while (glog > 0 && warps << (5 - glog) < a.total) --glog;
+        const int64_t each = 4 << (5 - glog);                         // photons a block at a time
+        const int64_t grid = std::min<int64_t>(3 * (int64_t)std::max(1, sm_count), (a.total + each - 1) / each);
+        walk_replay_pol_kernel<<<(unsigned)grid, 128, 0, s>>>(a, glog);
         return cudaGetLastError();
     }
     // four blocks an SM (126 registers), a warp of each part on each of its four FP64 pipes; few

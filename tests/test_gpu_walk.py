@@ -888,3 +888,23 @@ def test_f32_sparse_groups_same_records(walker, n, theta0, tau):
         big = walker.walk([dataclasses.replace(cfg, n_photon=5000)], seed, mode='f32').records
         small = walker.walk([dataclasses.replace(cfg, n_photon=n)], seed, mode='f32').records
         assert np.array_equal(small, big[:n])
+
+
+@pytest.mark.parametrize('n', [1, 5, 1900, 4000, 9000])
+@pytest.mark.parametrize('case', ['plates', 'thin', 'surface'])
+def test_polarised_replay_independent_of_photon_count(walker, case, n):
+    """Polarised replay records of n photons, 32 lanes a photon down to four, are the first n of a
+    run of one lane a photon; a thin slab over a reflecting ground and a Lambertian surface too."""
+    g = load_golden('pol')
+    ice, imp = golden_tables(g)
+    walker.set_tables([ice], imp)
+    walker.set_phase_matrices([golden_phase(g)])
+    cfg = dataclasses.replace(golden_config(g), tau_tot=2.0 if case != 'plates' else 8.0)
+    if case == 'thin':
+        cfg = dataclasses.replace(cfg, theta0_deg=0.0, lambertian_bottom=True, lambertian_reflectance=0.9)
+    elif case == 'surface':
+        cfg = dataclasses.replace(cfg, lambertian_surface=True, lambertian_reflectance=0.5)
+    total = 60000 if case == 'plates' else 30000
+    big = walker.walk([dataclasses.replace(cfg, n_photon=total)], 3, mode='pol64').records
+    got = walker.walk([dataclasses.replace(cfg, n_photon=n)], 3, mode='pol64').records
+    assert got.tobytes() == big[:n].tobytes()
