@@ -615,7 +615,7 @@ def run_train(args):
             'data': 'synthetic',
             'config': {'net': '4-256-256-256-649 SiLU', 'members': members, 'batch': batch,
                        'engine': 'grouped tcgen05 GEMMs fed by TMA, one CUDA graph per step '
-                                 '(16 launches for all members)'},
+                                 '(11 launches for all members)'},
             'layerwise_ms_per_step': ms_layer, 'speedup_vs_layerwise': ms_layer / ms_grouped,
             'fwd_bwd_65536': {'ms': ms_big, 'layerwise_ms': ms_big_layer, 'speedup': ms_big_layer / ms_big,
                               'tflops': tflops, 'splits': one.splits},

@@ -1,8 +1,8 @@
 // GEMM of the surrogate network on the 5th-generation tensor cores:
 // C[m, n] = sum_k A(m, k) B(n, k), bf16 operands stored K-major ([m, k], [n, k]) or
 // transposed ([k, m], [k, n]), FP32 accumulation in tensor memory, fused epilogues
-// (bias, bias + SiLU, SiLU' product of the backward pass).  Used for the forward and
-// the backward GEMMs of training.
+// (bias, bias + SiLU, SiLU' product of the backward pass).  Takes the products whose
+// operands the copies of mlp_gemm.cu cannot (off 16-byte boundaries).
 //
 // One CTA of four warps computes a 128 x 128 tile.  K is walked in chunks of 64
 // through two shared-memory buffers: all threads stage chunk k + 1 as 8 x 16-byte
