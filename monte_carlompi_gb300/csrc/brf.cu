@@ -9,10 +9,10 @@
 // exponential once, ten operations by table, divides once where it can, and keeps what it can in
 // registers; a block per row, a thread per bin, sums by block reduction.  16 grid points of 128
 // observations, five members: 362 us with CUDA's exp and a division a weight a point, 254 now; a
-// Jacobian 46 and 40.  128 observations, five members, one
-// retrieval (16-point grid, six iterations, spreads): 92 ms on the host's cores and elementwise
-// tensor kernels; 3.3 ms with these kernels and the steps and the encoding of log r on the host, a
-// wait for the device and two copies an iteration; 1.8 ms with the steps here too.
+// Jacobian 46 and 40.  One retrieval of 128 observations with five members (16-point grid, six
+// iterations, spreads): 92 ms on the host's cores and elementwise tensor kernels; 3.3 ms with these kernels and the steps and the encoding of log r on the host, a
+// wait for the device and two copies an iteration; 1.5 ms with the steps here too and the network
+// laid out while the grid's costs are worked out.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

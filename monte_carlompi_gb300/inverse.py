@@ -47,13 +47,13 @@ class _Slopes:
     input, d x0 / d log r = 2 / (log r_max - log r_min)), then the chain rule through the target
     standardisation, exp and the albedo factor in one kernel."""
 
-    def __init__(self, ens, n):
+    def __init__(self, ens, n, scaling=None, share=None):
         import torch
         self.torch = torch
         self.n = n
         self.net = S.EnsembleTangent(torch, ens.members, n, 2.0 / (LOG_R[1] - LOG_R[0]))
-        self.mean, self.std = ens.scaling()
-        self.share = torch.from_numpy(S.bin_weights()).cuda()
+        self.mean, self.std = ens.scaling() if scaling is None else scaling
+        self.share = torch.from_numpy(S.bin_weights()).cuda() if share is None else share
 
     def at(self, s, known):
         """(f, j, v) torch CUDA float64 [n, 648] at log r = s (host arrays s [n], known [n, 3])."""
@@ -145,7 +145,8 @@ def _surrogate_gn(ens, obs, known, iters, noise):
     f64 = dict(dtype=torch.float64, device='cuda')
     known_d = torch.from_numpy(np.ascontiguousarray(known, np.float64)).cuda()
     obs_d = torch.from_numpy(np.ascontiguousarray(obs, np.float64)).cuda()
-    slopes = _Slopes(ens, n)
+    share = torch.from_numpy(S.bin_weights()).cuda()
+    mean, std = ens.scaling()
     L, st, k = _abi.load(), S._stream(torch), len(ens.members)
     hull = (ctypes.c_double * 8)(*S.hull())
 
@@ -158,8 +159,10 @@ def _surrogate_gn(ens, obs, known, iters, noise):
     check(L.mcw_brf_encode(_ptr(grid), 16, _ptr(known_d), n, hull, _ptr(x), st), 'mcw_brf_encode')
     ys = ens.predict_std(x)
     cost = torch.empty((16, n), **f64)
-    check(L.mcw_brf_cost(_ptr(ys), ys.stride(1), k, 16, n, _ptr(slopes.mean), _ptr(slopes.std), S.BRF_FLOOR,
-                         _ptr(obs_d), _ptr(slopes.share), noise[0], noise[1], _ptr(cost), st), 'mcw_brf_cost')
+    check(L.mcw_brf_cost(_ptr(ys), ys.stride(1), k, 16, n, _ptr(mean), _ptr(std), S.BRF_FLOOR,
+                         _ptr(obs_d), _ptr(share), noise[0], noise[1], _ptr(cost), st), 'mcw_brf_cost')
+    # (laid out while the grid's costs are being worked out)
+    slopes = _Slopes(ens, n, (mean, std), share)
     s, sums = torch.empty(n, **f64), torch.empty((2, n), **f64)
     x = torch.empty((n, S.DIMS[0]), dtype=torch.float32, device='cuda')
 
@@ -171,11 +174,11 @@ def _surrogate_gn(ens, obs, known, iters, noise):
     for _ in range(iters):
         slopes.sums(obs_d, noise, sums)
         step(None)
-    brf, alb = ens._member_brfs(x, slopes.mean, slopes.std)
-    pred, _, spread = ens._brf_stats(brf, alb, slopes.share)
+    brf, alb = ens._member_brfs(x, mean, std)
+    pred, _, spread = ens._brf_stats(brf, alb, share)
     f, j, v = slopes.arrays()
     spread_r, sigma = torch.empty_like(spread), torch.empty_like(spread)
-    check(L.mcw_brf_logr(_ptr(brf), _ptr(pred), k, n, _ptr(f), _ptr(j), _ptr(v), _ptr(slopes.share), noise[0],
+    check(L.mcw_brf_logr(_ptr(brf), _ptr(pred), k, n, _ptr(f), _ptr(j), _ptr(v), _ptr(share), noise[0],
                          noise[1], _ptr(spread_r), _ptr(sigma), st), 'mcw_brf_logr')
     return tuple(t.cpu().numpy() for t in (s, pred, spread, spread_r, sigma))
 

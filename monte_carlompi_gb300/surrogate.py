@@ -104,15 +104,6 @@ def _cast(torch, x):
     return y
 
 
-def _colsum(torch, g):
-    m, n = g.shape
-    out = torch.empty(n, dtype=torch.float32, device=g.device)
-    rc = _abi.load().mcw_mlp_colsum(_ptr(g), m, n, n, _ptr(out), _stream(torch))
-    if rc:
-        raise _abi.McwError(rc, 'mcw_mlp_colsum failed')
-    return out
-
-
 # engine of training's GEMMs (forward with kept pre-activations, and the backward
 # layouts: transposed operands, silu' epilogue); inference runs the fused tcgen05
 # kernel (forward_fused)
