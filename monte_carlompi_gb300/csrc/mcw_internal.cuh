@@ -219,6 +219,8 @@ cudaError_t launch_post(const void *recs, bool f64, size_t stride, int64_t n, in
                         unsigned long long *bins_fx, unsigned int *bins_cnt, mcw_post_stats *stats, int sms,
                         cudaStream_t s);
 cudaError_t launch_lut(const LutArgs &a, cudaStream_t s);
+cudaError_t launch_results(const mcw_tally *tallies, int n_cfg, mcw_tally *to, const uint32_t *counters,
+                           uint32_t *counters_to, int words, cudaStream_t s);
 // Photons the walk hands over to its drain queue are packed as this many float4.
 constexpr int kDrainSlot = 6;
 // impurity: some config has imp_cnc > 0 (the kernel instance with the species draw).

@@ -908,3 +908,24 @@ def test_polarised_replay_independent_of_photon_count(walker, case, n):
     big = walker.walk([dataclasses.replace(cfg, n_photon=total)], 3, mode='pol64').records
     got = walker.walk([dataclasses.replace(cfg, n_photon=n)], 3, mode='pol64').records
     assert got.tobytes() == big[:n].tobytes()
+
+
+@pytest.mark.parametrize('mode', ['f32', 'replay64'])
+@pytest.mark.parametrize('n_cfg', [1, 2, 16, 17, 40])
+def test_tallies_of_few_and_many_configs(walker, mode, n_cfg):
+    """Tallies and counters come back by a kernel: each config's condition counts and events are
+    those of its records, call after call."""
+    cfg, ice, imp = cfg2_geometry(50)
+    walker.set_tables([ice], imp)
+    cfgs = [dataclasses.replace(cfg, n_photon=50 + 7 * k, theta0_deg=k) for k in range(n_cfg)]
+    for seed in (1, 2):
+        res = walker.walk(cfgs, seed, mode=mode)
+        lo = 0
+        for k, c in enumerate(cfgs):
+            rec = res.records[lo:lo + c.n_photon]
+            lo += c.n_photon
+            assert (rec['config'] == k).all()
+            counts = np.bincount(rec['condition'], minlength=6)
+            assert np.array_equal(res.tallies[k]['n_cond'][1:6], counts[1:6])
+            assert int(res.tallies[k]['n_events']) == int(rec['n_scat'].astype(np.int64).sum())
+        assert res.stats['n_photon'] == lo
