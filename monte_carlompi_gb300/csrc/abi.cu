@@ -369,7 +369,7 @@ Shape pick_shape(const mcw_ctx *ctx, const mcw_launch &l, const Plan &plan) {
     if (occ <= 0) occ = 1;
     s.bps = (l.blocks_per_sm > 0) ? std::min(l.blocks_per_sm, occ) : occ;
     s.chunk = l.regen_chunk;
-    const WalkSpread spread = spread_walk(total, (int64_t)ctx->sm_count * s.bps, s.block);
+    const WalkSpread spread = spread_walk_f32(total, ctx->sm_count, s.bps, s.block);
     s.grid = spread.grid;
     s.lanes = spread.lanes;
     return s;
@@ -461,6 +461,8 @@ WalkArgs walk_args(const mcw_ctx *ctx, const Plan &plan, DevBuf &cfgs, DevBuf &l
 }
 
 constexpr int32_t kDrainSpread = 512;
+// FP32 records in pageable memory up to this size are written by the walk, more are copied
+constexpr size_t kDirectBytes = 4u << 20;
 
 // Attach the drain queue (one slot per thread of the walk grid) when handover is on.
 int attach_drain(mcw_ctx *ctx, WalkArgs &wa, DevBuf &drain, const Shape &shape) {
@@ -878,9 +880,11 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
             at.devicePointer && ((uintptr_t)at.devicePointer % 16) == 0) {
             dev_records = at.devicePointer;
             direct = true;
-        } else if (reach_pageable(ctx, records, (size_t)plan.total * rec_size, 16, true)) {
-            // pageable memory, where the GPU walks the host's page tables: written the same way
-            // (a call of 100,003 FP32 records 222 -> 197 us, 10,000 126 -> 118)
+        } else if ((mode != MCW_MODE_F32 || (size_t)plan.total * rec_size <= kDirectBytes) &&
+                   reach_pageable(ctx, records, (size_t)plan.total * rec_size, 16, true)) {
+            // pageable memory, where the GPU walks the host's page tables: written the same way, but
+            // for many records of the fastest walk (a call of 100,003 FP32 records 222 -> 197 us,
+            // 10,000 126 -> 118; 737,905 of short walks 262 by the copy, 318 without)
             dev_records = records;
             direct = true;
         } else {

@@ -213,6 +213,15 @@ inline WalkSpread spread_walk(int64_t total, int64_t max_grid, int block) {
     return {(int)grid, (int)lanes};
 }
 
+// The FP32 walk's, per_sm blocks an SM: photons that fit eight warps an SM take no more, which walk
+// faster than sixteen with half as many photons each (30,000 photons with soot 92 against 101 us,
+// 3,000 to 30,000 of others the same to 3% less).
+inline WalkSpread spread_walk_f32(int64_t total, int sms, int per_sm, int block) {
+    const int eight = block < 256 ? 256 / block : 1;
+    if (total <= (int64_t)sms * 256 && eight < per_sm) per_sm = eight;
+    return spread_walk(total, (int64_t)sms * per_sm, block);
+}
+
 // Kernel launchers (defined in the .cu files).
 // recs: n records of `stride` bytes starting with an mcw_record64 (f64) or mcw_record32.
 cudaError_t launch_post(const void *recs, bool f64, size_t stride, int64_t n, int n_cfg, int n_bins,

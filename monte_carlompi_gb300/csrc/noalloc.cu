@@ -233,7 +233,7 @@ extern "C" int mcw_walk_noalloc(const mcw_config *cfg, const mcw_ssp_table *ice_
         const bool impurity = c.imp_cnc > 0;
         int bps = walk_f32_max_blocks_per_sm(256, 1, impurity);
         if (bps < 1) bps = 1;
-        const WalkSpread spread = spread_walk(c.n_photon, (int64_t)sms * bps, 256);
+        const WalkSpread spread = spread_walk_f32(c.n_photon, sms, bps, 256);
         wa.lanes = spread.lanes;
         if (launch_walk_f32(wa, impurity, spread.grid, 256, sms, st) != cudaSuccess) return MCW_ERR_CUDA;
     }

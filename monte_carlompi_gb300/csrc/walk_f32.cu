@@ -652,6 +652,9 @@ __device__ __forceinline__ int sparse_round(Photon &P, WarpQueues &q, const unsi
                 xs[u] = q.pbuf[2 * (t0 + u)];
                 ys[u] = q.pbuf[2 * (t0 + u) + 1];
             }
+            // (not in the deep instance with impurities, whose full rounds lose 5% beside it: 271,683
+            // photons 262 -> 271 us, 685,962 631 -> 664)
+            if constexpr (!(kDeep && kImpurity)) {
             // a group that does nothing but scatter (most do) is a chain of rotations without a
             // branch; its result is dropped, and the group walked step by step, when a step
             // starts the photon, is reflected or along the vertical, or ends in something (a lone
@@ -682,6 +685,7 @@ __device__ __forceinline__ int sparse_round(Photon &P, WarpQueues &q, const unsi
                     P.z = z, P.path = path, P.pathc = pathc;
                     continue;
                 }
+            }
             }
             // each photon's lane leaves at its end condition (at most kSparseWarp lanes walk
             // here, so the divergence costs little); the state is the one after that step,
