@@ -612,8 +612,13 @@ __global__ void __launch_bounds__(kThreads, 4) gemm_kernel(const __grid_constant
             __syncwarp();
         }
         if (kEpi == MCW_EPI_LOSS) {
+            // one addition to the loss a tile: the sum of many rounds at each
             for (int o = 16; o; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-            if (ok && lane == 0) atomicAdd(p.loss + g, lsum);
+            if (ok) {
+                if (lane == 0) part[warp * 32] = lsum;
+                asm volatile("bar.sync 1, 128;\n" ::: "memory");
+                if (warp == 0 && lane == 0) atomicAdd(p.loss + g, (part[0] + part[32]) + (part[64] + part[96]));
+            }
         }
         if (!ok && lane == 0) atomicOr(batch.err, 4u);
     }
