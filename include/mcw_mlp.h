@@ -310,6 +310,18 @@ int mcw_brf_logr(const double *brf, const double *mean_brf, int32_t members, int
                  const double *v, const double *share, double photons, double rel_noise, double *spread, double *sigma,
                  void *stream);
 
+/* The three with the relative noise of every observation and bin, rel_noise [n, 648] on the device. */
+int mcw_brf_cost_noise(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t n_obs,
+                       const double *mean, const double *std, double floor, const double *obs, const double *share,
+                       double photons, const double *rel_noise, double *cost, void *stream);
+int mcw_brf_jacobian_noise(const float *y, const float *ydot, int64_t pitch, int32_t members, int32_t n,
+                           const double *mean, const double *std, double floor, double *f, double *j, double *v,
+                           const double *obs, const double *share, double photons, const double *rel_noise, double *jtr,
+                           double *jtj, void *stream);
+int mcw_brf_logr_noise(const double *brf, const double *mean_brf, int32_t members, int32_t n, const double *f,
+                       const double *j, const double *v, const double *share, double photons, const double *rel_noise,
+                       double *spread, double *sigma, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

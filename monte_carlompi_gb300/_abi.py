@@ -149,7 +149,8 @@ MLP_EXPORTS = ['mcw_mlp_gemm', 'mcw_mlp_colsum', 'mcw_mlp_loss', 'mcw_mlp_adam',
                'mcw_mlp_loss_grouped',
                'mcw_mlp_colsum_grouped', 'mcw_mlp_adam_grouped', 'mcw_mlp_gather', 'mcw_mlp_step_begin',
                'mcw_mlp_advance', 'mcw_brf_members', 'mcw_brf_stats', 'mcw_brf_cost', 'mcw_brf_jacobian',
-               'mcw_brf_encode', 'mcw_brf_gn_step', 'mcw_brf_logr']
+               'mcw_brf_encode', 'mcw_brf_gn_step', 'mcw_brf_logr',
+               'mcw_brf_cost_noise', 'mcw_brf_jacobian_noise', 'mcw_brf_logr_noise']
 MLP_PACK_BYTES = 5 * 256 * 256 * 2 + 256 * 16 * 2
 MLP_BIAS_FLOATS = 3 * 256 + 649
 
@@ -255,6 +256,10 @@ def load(path=None):
         'mcw_brf_encode': ([vp, i32, vp, i32, vp, vp, vp], ctypes.c_int),
         'mcw_brf_gn_step': ([vp, vp, i32, vp, vp, dbl, dbl, dbl, dbl, vp, i32, vp, vp, vp, vp, i32, vp], ctypes.c_int),
         'mcw_brf_logr': ([vp, vp, i32, i32, vp, vp, vp, vp, dbl, dbl, vp, vp, vp], ctypes.c_int),
+        'mcw_brf_cost_noise': ([vp, i64, i32, i32, i32, vp, vp, dbl, vp, vp, dbl, vp, vp, vp], ctypes.c_int),
+        'mcw_brf_jacobian_noise': ([vp, vp, i64, i32, i32, vp, vp, dbl, vp, vp, vp, vp, vp, dbl, vp, vp, vp, vp],
+                                   ctypes.c_int),
+        'mcw_brf_logr_noise': ([vp, vp, i32, i32, vp, vp, vp, vp, dbl, vp, vp, vp, vp], ctypes.c_int),
         'mcw_mlp_advance': ([vp, vp, vp], ctypes.c_int),
     }
     for name, (args, res) in sig.items():

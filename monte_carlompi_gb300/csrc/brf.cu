@@ -101,8 +101,10 @@ __device__ __forceinline__ double at_least(double x, double lo) { return x < lo 
 struct Noise {
     double photons, rel;
     const double *share;       // [648]
-    __device__ __forceinline__ double variance(double f, double model, int b) const {
-        const double v = at_least(f, 1e-3) / (photons * share[b]) + (rel * f) * (rel * f);
+    const double *rel_bins;    // relative noise per row and bin [n, 648] in place of rel, or null
+    __device__ __forceinline__ double variance(double f, double model, int r, int b) const {
+        const double q = rel_bins ? rel_bins[(size_t)r * kBins + b] : rel;
+        const double v = at_least(f, 1e-3) / (photons * share[b]) + (q * f) * (q * f);
         return v + model;
     }
 };
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(kThreads) cost_kernel(const __half *ys, long l
         x[k] = w[k] = 0.0;
         if (b < kBins) {
             x[k] = obs[(size_t)o * kBins + b];
-            w[k] = noise.photons != 0 ? 1.0 / noise.variance(x[k], 0.0, b) : noise.share[b];
+            w[k] = noise.photons != 0 ? 1.0 / noise.variance(x[k], 0.0, o, b) : noise.share[b];
         }
     }
     for (int p = 0; p < np; ++p) {
@@ -245,7 +247,7 @@ __global__ void __launch_bounds__(kThreads) jacobian_kernel(const float *y, cons
         if (v_out) v_out[(size_t)r * kBins + b] = v;
         if (obs) {
             const double d = f - obs[(size_t)r * kBins + b];
-            const double w = noise.photons != 0 ? 1.0 / noise.variance(f, v, b) : noise.share[b];
+            const double w = noise.photons != 0 ? 1.0 / noise.variance(f, v, r, b) : noise.share[b];
             sr += w * j * d;
             sj += w * j * j;
         }
@@ -274,8 +276,8 @@ __global__ void __launch_bounds__(kThreads) logr_kernel(const double *brf, const
         wj[k] = mu[k] = 0.0;
         if (b < kBins) {
             const size_t at = (size_t)r * kBins + b;
-            const double w = noise.photons != 0 ? 1.0 / noise.variance(f[at], v[at], b) : noise.share[b];
-            const double wn = noise.photons != 0 ? 1.0 / noise.variance(f[at], 0.0, b) : noise.share[b];
+            const double w = noise.photons != 0 ? 1.0 / noise.variance(f[at], v[at], r, b) : noise.share[b];
+            const double wn = noise.photons != 0 ? 1.0 / noise.variance(f[at], 0.0, r, b) : noise.share[b];
             mu[k] = mean[at];
             wj[k] = w * j[at];
             sj += wj[k] * j[at];
@@ -366,6 +368,41 @@ Hull hull_of(const double *h) {
 bool rows_ok(int32_t members, int32_t n) { return members >= 1 && members <= 4096 && n >= 0; }
 int done() { return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA; }
 
+int cost(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t n_obs, const double *mean,
+         const double *std, double floor, const double *obs, const Noise &noise, double *cost, void *stream) {
+    if (!ys || !mean || !std || !obs || !noise.share || !cost || points < 0 || n_obs < 0 ||
+        (long long)points * n_obs > 0x7fffffffLL || !rows_ok(members, points * n_obs) || pitch < MCW_MLP_OUT)
+        return MCW_MLP_ERR_ARG;
+    if (points * n_obs == 0) return 0;
+    const int per = members <= 1024 ? 4 : 1;       // points a block, within 32 KB of albedos
+    cost_kernel<<<(points + per - 1) / per * n_obs, kThreads, per * members * sizeof(double),
+                  static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __half *>(ys), pitch, members, points, per, n_obs, mean, std, floor, obs, noise, cost);
+    return done();
+}
+
+int jacobian(const float *y, const float *ydot, int64_t pitch, int32_t members, int32_t n, const double *mean,
+             const double *std, double floor, double *f, double *j, double *v, const double *obs, const Noise &noise,
+             double *jtr, double *jtj, void *stream) {
+    if (!y || !ydot || !mean || !std || !rows_ok(members, n) || pitch < MCW_MLP_OUT ||
+        (obs && (!noise.share || !jtr || !jtj)))
+        return MCW_MLP_ERR_ARG;
+    if (n == 0) return 0;
+    jacobian_kernel<<<n, kThreads, 2 * members * sizeof(double), static_cast<cudaStream_t>(stream)>>>(
+        y, ydot, pitch, members, n, mean, std, floor, f, j, v, obs, noise, jtr, jtj);
+    return done();
+}
+
+int logr(const double *brf, const double *mean_brf, int32_t members, int32_t n, const double *f, const double *j,
+         const double *v, const Noise &noise, double *spread, double *sigma, void *stream) {
+    if (!brf || !mean_brf || !f || !j || !v || !noise.share || !spread || !sigma || !rows_ok(members, n))
+        return MCW_MLP_ERR_ARG;
+    if (n == 0) return 0;
+    logr_kernel<<<n, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(brf, mean_brf, members, n, f, j, v, noise,
+                                                                       spread, sigma);
+    return done();
+}
+
 }  // namespace
 
 }  // namespace mcw
@@ -394,29 +431,33 @@ int mcw_brf_stats(const double *brf, const double *albedo, int32_t members, int3
 
 int mcw_brf_cost(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t n_obs, const double *mean,
                  const double *std, double floor, const double *obs, const double *share, double photons,
-                 double rel_noise, double *cost, void *stream) {
-    if (!ys || !mean || !std || !obs || !share || !cost || points < 0 || n_obs < 0 ||
-        (long long)points * n_obs > 0x7fffffffLL || !rows_ok(members, points * n_obs) || pitch < MCW_MLP_OUT)
-        return MCW_MLP_ERR_ARG;
-    if (points * n_obs == 0) return 0;
-    const int per = members <= 1024 ? 4 : 1;       // points a block, within 32 KB of albedos
-    cost_kernel<<<(points + per - 1) / per * n_obs, kThreads, per * members * sizeof(double),
-                  static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half *>(ys), pitch, members, points, per, n_obs, mean, std, floor, obs,
-        Noise{photons, rel_noise, share}, cost);
-    return done();
+                 double rel_noise, double *out, void *stream) {
+    return cost(ys, pitch, members, points, n_obs, mean, std, floor, obs, Noise{photons, rel_noise, share, nullptr}, out,
+                stream);
+}
+
+int mcw_brf_cost_noise(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t n_obs,
+                       const double *mean, const double *std, double floor, const double *obs, const double *share,
+                       double photons, const double *rel_noise, double *out, void *stream) {
+    if (!rel_noise) return MCW_MLP_ERR_ARG;
+    return cost(ys, pitch, members, points, n_obs, mean, std, floor, obs, Noise{photons, 0.0, share, rel_noise}, out,
+                stream);
 }
 
 int mcw_brf_jacobian(const float *y, const float *ydot, int64_t pitch, int32_t members, int32_t n, const double *mean,
                      const double *std, double floor, double *f, double *j, double *v, const double *obs,
                      const double *share, double photons, double rel_noise, double *jtr, double *jtj, void *stream) {
-    if (!y || !ydot || !mean || !std || !rows_ok(members, n) || pitch < MCW_MLP_OUT ||
-        (obs && (!share || !jtr || !jtj)))
-        return MCW_MLP_ERR_ARG;
-    if (n == 0) return 0;
-    jacobian_kernel<<<n, kThreads, 2 * members * sizeof(double), static_cast<cudaStream_t>(stream)>>>(
-        y, ydot, pitch, members, n, mean, std, floor, f, j, v, obs, Noise{photons, rel_noise, share}, jtr, jtj);
-    return done();
+    return jacobian(y, ydot, pitch, members, n, mean, std, floor, f, j, v, obs,
+                    Noise{photons, rel_noise, share, nullptr}, jtr, jtj, stream);
+}
+
+int mcw_brf_jacobian_noise(const float *y, const float *ydot, int64_t pitch, int32_t members, int32_t n,
+                           const double *mean, const double *std, double floor, double *f, double *j, double *v,
+                           const double *obs, const double *share, double photons, const double *rel_noise, double *jtr,
+                           double *jtj, void *stream) {
+    if (!rel_noise) return MCW_MLP_ERR_ARG;
+    return jacobian(y, ydot, pitch, members, n, mean, std, floor, f, j, v, obs, Noise{photons, 0.0, share, rel_noise},
+                    jtr, jtj, stream);
 }
 
 int mcw_brf_encode(const double *s, int32_t points, const double *known, int32_t n, const double *hull, float *x,
@@ -446,11 +487,14 @@ int mcw_brf_gn_step(const double *cost, const double *grid, int32_t points, cons
 int mcw_brf_logr(const double *brf, const double *mean_brf, int32_t members, int32_t n, const double *f, const double *j,
                  const double *v, const double *share, double photons, double rel_noise, double *spread, double *sigma,
                  void *stream) {
-    if (!brf || !mean_brf || !f || !j || !v || !share || !spread || !sigma || !rows_ok(members, n)) return MCW_MLP_ERR_ARG;
-    if (n == 0) return 0;
-    logr_kernel<<<n, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(brf, mean_brf, members, n, f, j, v,
-                                                                       Noise{photons, rel_noise, share}, spread, sigma);
-    return done();
+    return logr(brf, mean_brf, members, n, f, j, v, Noise{photons, rel_noise, share, nullptr}, spread, sigma, stream);
+}
+
+int mcw_brf_logr_noise(const double *brf, const double *mean_brf, int32_t members, int32_t n, const double *f,
+                       const double *j, const double *v, const double *share, double photons, const double *rel_noise,
+                       double *spread, double *sigma, void *stream) {
+    if (!rel_noise) return MCW_MLP_ERR_ARG;
+    return logr(brf, mean_brf, members, n, f, j, v, Noise{photons, 0.0, share, rel_noise}, spread, sigma, stream);
 }
 
 }  // extern "C"

@@ -41,6 +41,20 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
+class _Noise:
+    """An observation's photons (0: none) and relative noise, one number or a torch CUDA float64
+    [n, 648], as the kernels of csrc/brf.cu take them."""
+
+    def __init__(self, photons, rel):
+        self.photons, self.rel = photons, rel
+
+    def entry(self, name):
+        return getattr(_abi.load(), name if isinstance(self.rel, float) else name + '_noise')
+
+    def args(self):
+        return self.photons, self.rel if isinstance(self.rel, float) else _ptr(self.rel)
+
+
 class _Slopes:
     """BRF, d BRF / d log r_eff and the members' variance of an ensemble at n points: one
     forward-mode pass of all members through the tensor-core kernels (the tangent of the first
@@ -62,7 +76,7 @@ class _Slopes:
     def arrays(self, x=None):
         """(f, j, v) of inputs x, or of those the network's buffer holds."""
         f, j, v = (self.torch.empty((self.n, S.N_BRF), dtype=self.torch.float64, device=self.share.device) for _ in range(3))
-        self._evaluate(x, f, j, v, None, (0.0, 0.0), None)
+        self._evaluate(x, f, j, v, None, _Noise(0.0, 0.0), None)
         return f, j, v
 
     def sums(self, obs, noise, out):
@@ -73,10 +87,10 @@ class _Slopes:
     def _evaluate(self, x, f, j, v, obs, noise, out):
         y, ydot = self.net.run(x)
         jtr, jtj = (None, None) if out is None else (out[0], out[1])
-        rc = _abi.load().mcw_brf_jacobian(_ptr(y), _ptr(ydot), y.shape[2], y.shape[0], self.n, _ptr(self.mean),
-                                          _ptr(self.std), S.BRF_FLOOR, _ptr(f), _ptr(j), _ptr(v), _ptr(obs),
-                                          _ptr(self.share), noise[0], noise[1], _ptr(jtr), _ptr(jtj),
-                                          S._stream(self.torch))
+        rc = noise.entry('mcw_brf_jacobian')(_ptr(y), _ptr(ydot), y.shape[2], y.shape[0], self.n, _ptr(self.mean),
+                                             _ptr(self.std), S.BRF_FLOOR, _ptr(f), _ptr(j), _ptr(v), _ptr(obs),
+                                             _ptr(self.share), *noise.args(), _ptr(jtr), _ptr(jtj),
+                                             S._stream(self.torch))
         if rc:
             raise _abi.McwError(rc, 'mcw_brf_jacobian failed')
 
@@ -122,14 +136,18 @@ def surrogate_gn(ens, obs, known, iters=6, obs_photons=None, obs_noise=0.0, with
     """Gauss-Newton on s = log r_eff through the surrogate; starts from the best of a
     16-point grid.  With obs_photons, every bin's residual is weighted by the inverse of
     its variance (noise_variance: the observation's counting noise for obs_photons
-    photons and its relative noise obs_noise, plus the ensemble's variance in that bin);
+    photons and its relative noise obs_noise, a number or an array that broadcasts to
+    obs's shape, plus the ensemble's variance in that bin);
     without, by the bin's photon share.  Returns (s, brf at s, BRF spread at s, log r_eff
     spread at s) and, with with_noise, the posterior width of s from the observation
     noise alone, 1 / sqrt(sum_b J_b^2 / var_b)."""
     if obs.ndim != 2 or obs.shape[1] != S.N_BRF or np.shape(known) != (obs.shape[0], 3):
         raise ValueError('obs must be [n, %d] and known [n, 3]' % S.N_BRF)
-    parts = [_surrogate_gn(ens, obs[lo:lo + 4096], known[lo:lo + 4096], iters,
-                           (float(obs_photons or 0), float(obs_noise)))
+    photons = np.asarray(obs_photons or 0, np.float64).item()
+    rel = np.asarray(obs_noise if photons else 0, np.float64)        # (weights without photons take no noise)
+    rel = rel.item() if rel.size == 1 else np.broadcast_to(rel, obs.shape)
+    parts = [_surrogate_gn(ens, obs[lo:lo + 4096], known[lo:lo + 4096], iters, photons,
+                           rel if isinstance(rel, float) else rel[lo:lo + 4096])
              for lo in range(0, obs.shape[0], 4096)]
     if not parts:
         parts = [(np.zeros(0), np.zeros((0, S.N_BRF)), np.zeros(0), np.zeros(0), np.zeros(0))]
@@ -137,7 +155,7 @@ def surrogate_gn(ens, obs, known, iters=6, obs_photons=None, obs_noise=0.0, with
     return out if with_noise else out[:4]
 
 
-def _surrogate_gn(ens, obs, known, iters, noise):
+def _surrogate_gn(ens, obs, known, iters, photons, rel):
     """surrogate_gn of a few thousand observations, queued on the device from the grid to the
     spreads (FP64, csrc/brf.cu) without the host waiting in between."""
     import torch
@@ -146,6 +164,7 @@ def _surrogate_gn(ens, obs, known, iters, noise):
     known_d = torch.from_numpy(np.ascontiguousarray(known, np.float64)).cuda()
     obs_d = torch.from_numpy(np.ascontiguousarray(obs, np.float64)).cuda()
     share = torch.from_numpy(S.bin_weights()).cuda()
+    noise = _Noise(photons, rel if isinstance(rel, float) else torch.from_numpy(np.array(rel)).cuda())
     mean, std = ens.scaling()
     L, st, k = _abi.load(), S._stream(torch), len(ens.members)
     hull = (ctypes.c_double * 8)(*S.hull())
@@ -159,8 +178,8 @@ def _surrogate_gn(ens, obs, known, iters, noise):
     check(L.mcw_brf_encode(_ptr(grid), 16, _ptr(known_d), n, hull, _ptr(x), st), 'mcw_brf_encode')
     ys = ens.predict_std(x)
     cost = torch.empty((16, n), **f64)
-    check(L.mcw_brf_cost(_ptr(ys), ys.stride(1), k, 16, n, _ptr(mean), _ptr(std), S.BRF_FLOOR,
-                         _ptr(obs_d), _ptr(share), noise[0], noise[1], _ptr(cost), st), 'mcw_brf_cost')
+    check(noise.entry('mcw_brf_cost')(_ptr(ys), ys.stride(1), k, 16, n, _ptr(mean), _ptr(std), S.BRF_FLOOR,
+                                      _ptr(obs_d), _ptr(share), *noise.args(), _ptr(cost), st), 'mcw_brf_cost')
     # (laid out while the grid's costs are being worked out)
     slopes = _Slopes(ens, n, (mean, std), share)
     s, sums = torch.empty(n, **f64), torch.empty((2, n), **f64)
@@ -178,8 +197,8 @@ def _surrogate_gn(ens, obs, known, iters, noise):
     pred, _, spread = ens._brf_stats(brf, alb, share)
     f, j, v = slopes.arrays()
     spread_r, sigma = torch.empty_like(spread), torch.empty_like(spread)
-    check(L.mcw_brf_logr(_ptr(brf), _ptr(pred), k, n, _ptr(f), _ptr(j), _ptr(v), _ptr(share), noise[0],
-                         noise[1], _ptr(spread_r), _ptr(sigma), st), 'mcw_brf_logr')
+    check(noise.entry('mcw_brf_logr')(_ptr(brf), _ptr(pred), k, n, _ptr(f), _ptr(j), _ptr(v), _ptr(share),
+                                      *noise.args(), _ptr(spread_r), _ptr(sigma), st), 'mcw_brf_logr')
     return tuple(t.cpu().numpy() for t in (s, pred, spread, spread_r, sigma))
 
 

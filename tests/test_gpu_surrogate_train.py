@@ -213,3 +213,61 @@ def test_retrieval_refuses_arrays_of_other_shapes(trained):
                        (np.ones((4, 648)), np.ones((4, 2)))):
         with pytest.raises(ValueError):
             inverse.surrogate_gn(ens, obs, known)
+
+
+def test_retrieval_takes_noise_per_bin_and_per_observation(trained):
+    """obs_noise as an array: the same number in every place is the number, in every form that
+    broadcasts; a noise of each observation's own is that of a retrieval of it alone (its rows of the
+    network and of the sums do not depend on the others); a noise per bin weights the costs, the
+    Gauss-Newton sums and the spreads as the array arithmetic does."""
+    from monte_carlompi_gb300 import _abi
+    ens, ds, hold = trained
+    n, rng = 7, np.random.default_rng(11)
+    known, photons = ds.raw[:n, 1:], 1e6
+    obs = ds.brf[:n] * (1 + 0.02 * rng.standard_normal((n, surrogate.N_BRF)))
+
+    def solve(noise, rows=slice(None), **kw):
+        return inverse.surrogate_gn(ens, obs[rows], known[rows], obs_photons=kw.get('photons', photons),
+                                    obs_noise=noise, with_noise=True)
+    want = solve(0.02)
+    for shape in ((1,), (1, 1), (surrogate.N_BRF,), (1, surrogate.N_BRF), (n, 1), (n, surrogate.N_BRF)):
+        for a, b in zip(solve(np.full(shape, 0.02)), want):
+            assert np.array_equal(a, b), shape
+    for a, b in zip(solve(0.02, photons=np.array([photons])), want):
+        assert np.array_equal(a, b)
+    for a, b in zip(solve(np.full((n, 1), 0.3), photons=None), solve(0.0, photons=None)):
+        assert np.array_equal(a, b)
+    each = np.linspace(0.005, 0.1, n)
+    got = solve(each[:, None])
+    for i in range(n):
+        for a, b in zip(got, solve(float(each[i]), slice(i, i + 1))):
+            assert np.allclose(a[i], b[0], rtol=1e-9, atol=1e-12), i
+    with pytest.raises(ValueError):
+        solve(np.ones((n + 1, 1)))
+    # the kernels against the array arithmetic (test_brf_kernels_match_numpy's tolerances)
+    rel = rng.uniform(0.0, 0.2, (n, surrogate.N_BRF))
+    m, bins = 3, surrogate.N_BRF
+    g = torch.Generator().manual_seed(5)
+    ys = torch.randn(m, n, 656, generator=g).half().cuda()
+    y, yd = torch.randn(m, n, 652, generator=g).cuda(), torch.randn(m, n, 652, generator=g).cuda()
+    mean, std = torch.zeros(m, 649, dtype=torch.float64, device='cuda'), torch.full((m, 649), 0.2, dtype=torch.float64, device='cuda')
+    od, wd, rd = (torch.from_numpy(np.ascontiguousarray(t)).cuda() for t in (obs, surrogate.bin_weights(), rel))
+    new = lambda *shape: torch.empty(shape, dtype=torch.float64, device='cuda')  # noqa: E731
+    p, fl, st = (lambda t: t.data_ptr()), surrogate.BRF_FLOOR, surrogate._stream(torch)  # noqa: E731
+    brf, alb, mu, am, sp = new(m, n, bins), new(m, n), new(n, bins), new(n), new(n)
+    cost, f, j, v, sums, spread, sigma = new(n), new(n, bins), new(n, bins), new(n, bins), new(2, n), new(n), new(n)
+    L = _abi.load()
+    assert L.mcw_brf_members(p(ys), 656, m, n, p(mean), p(std), fl, p(brf), p(alb), st) == 0
+    assert L.mcw_brf_stats(p(brf), p(alb), m, n, p(wd), p(mu), p(am), p(sp), st) == 0
+    assert L.mcw_brf_cost_noise(p(ys), 656, m, 1, n, p(mean), p(std), fl, p(od), p(wd), photons, p(rd), p(cost), st) == 0
+    assert L.mcw_brf_jacobian_noise(p(y), p(yd), 652, m, n, p(mean), p(std), fl, p(f), p(j), p(v), p(od), p(wd), photons,
+                                    p(rd), p(sums[0]), p(sums[1]), st) == 0
+    assert L.mcw_brf_logr_noise(p(brf), p(mu), m, n, p(f), p(j), p(v), p(wd), photons, p(rd), p(spread), p(sigma), st) == 0
+    rb, rmu, rf, rj, rv = (t.cpu().numpy() for t in (brf, mu, f, j, v))
+    w0, w = 1 / inverse.noise_variance(obs, photons, rel), 1 / inverse.noise_variance(rf, photons, rel, rv)
+    assert np.allclose(cost.cpu(), (w0 * (rmu - obs) ** 2).sum(1), rtol=1e-11, atol=1e-13)
+    assert np.allclose(sums[0].cpu(), (w * rj * (rf - obs)).sum(1), rtol=1e-9, atol=1e-9 * np.abs(w * rj * rf).sum(1).max())
+    assert np.allclose(sums[1].cpu(), (w * rj * rj).sum(1), rtol=1e-9)
+    assert np.allclose(spread.cpu(), inverse.logr_spread(rb, rj, w), rtol=1e-8, atol=1e-13)
+    wn = 1 / inverse.noise_variance(rf, photons, rel)
+    assert np.allclose(sigma.cpu(), 1 / np.sqrt((wn * rj * rj).sum(1)), rtol=1e-9)
