@@ -26,7 +26,8 @@ extern "C" {
 #define MCW_OK 0
 #define MCW_ERR_ARG (-1)     /* invalid argument (reference: ValueError / bad kwargs) */
 #define MCW_ERR_CUDA (-2)    /* a CUDA runtime call failed */
-#define MCW_ERR_BUDGET (-3)  /* the kernel's time budget ran out; results are partial */
+#define MCW_ERR_BUDGET (-3)  /* the kernel's time budget ran out; results are partial (a replay leaves
+                                condition 0 in the records of the photons that did not end) */
 #define MCW_ERR_STREAM (-4)  /* a replay photon needed more than 2^33 uniforms */
 #define MCW_ERR_OOM (-5)     /* device or pinned allocation failed */
 #define MCW_ERR_STATE (-6)   /* call made in the wrong state (e.g. no SSP tables) */

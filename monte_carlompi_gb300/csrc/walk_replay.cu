@@ -112,6 +112,7 @@ __device__ void finish_photon(const ReplayArgs &a, int64_t gid, int ci, int cond
 // ---------------------------------------------------------------- the HG walk
 
 constexpr int kSlots = 16;                   // photons a block walks at once
+constexpr uint64_t kMaxUniforms = 1ull << 33;    // of a photon's stream
 constexpr uint32_t kRefl = 1u, kSurface = 2u, kBottom = 4u, kIso = 8u, kActive = 16u;
 
 // A photon in flight (shared memory).
@@ -302,6 +303,23 @@ __device__ int replay_birth(const ReplayArgs &a, int64_t gid, Slot &out) {
     return cond;
 }
 
+// The photons that no block has claimed when the time is out, 32 a warp at a time.  Warp-collective.
+template <bool kPol>
+__device__ __noinline__ void leave_unwalked(const ReplayArgs &a, int lane) {
+    for (;;) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(a.work, 32ull);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= (unsigned long long)a.total) return;
+        if (base + lane < (unsigned long long)a.total) {
+            Slot s;
+            const int cond = replay_birth(a, (int64_t)(base + lane), s);
+            finish_photon<kPol>(a, s.gid, s.ci, cond, s.i, s.wvl_um, s.mux, s.muy, s.muz, s.path, s.depth,
+                                kPol ? a.cfgs[s.ci].stokes0 : nullptr);
+        }
+    }
+}
+
 // The producer's round: the next steps of the block's photons into `next`, assuming that those
 // drawn before and not yet walked end in nothing.
 __device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, Ahead &next, int lane) {
@@ -385,7 +403,6 @@ __device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, Ahead &next, int
             const uint64_t k1 = s.k + 5 * (uint64_t)steps + shift;
             B.drawn_gen[si] = gen;
             B.next_k[si] = k1;
-            if (k1 > (1ull << 33)) atomicOr(a.status, kStatusStream);
         }
     }
     if (lane == 0) {
@@ -523,7 +540,7 @@ __device__ int walk_m(ReplayBlock &B, Ahead &A, int lane) {
 }
 
 // The photons' states after the steps that XY and M walked: lane `rank` its photon's.  `walked`:
-// walk_m's result for it.  Returns its end condition.
+// walk_m's result for it.  Returns its end condition (-1: out of its stream).
 __device__ int commit(const ReplayArgs &a, ReplayBlock &B, const Ahead &A, int rank, int walked) {
     const bool event = walked < 0;
     const int done = event ? -walked : walked;
@@ -541,8 +558,12 @@ __device__ int commit(const ReplayArgs &a, ReplayBlock &B, const Ahead &A, int r
     if (event) {
         const uint32_t f = A.fl[e];
         cond = step_end(slot, a.seed, z, zp, A.dtau[e], mz, path, false, f & 1u, f & 2u, &k, &flags);
-        B.gen[si] += 1;
     }
+    if (k > kMaxUniforms) {
+        atomicOr(a.status, kStatusStream);
+        if (cond == 0) cond = -1;
+    }
+    if (event || cond) B.gen[si] += 1;
     slot.z = z;
     slot.path = path;
     slot.k = k;
@@ -603,7 +624,7 @@ __global__ void __launch_bounds__(128, 4) walk_replay_kernel(const ReplayArgs a)
             if (__any_sync(0xffffffffu, cond != 0)) {
                 Slot &s = B.slots[si];
                 if (n_fin > 32 - kSlots) flush();
-                queue(cond != 0, s, cond);
+                queue(cond != 0, s, max(cond, 0));
                 if (cond) s.flags = 0;
                 __syncwarp();
             }
@@ -639,7 +660,7 @@ __global__ void __launch_bounds__(128, 4) walk_replay_kernel(const ReplayArgs a)
             int stop = !any && exhausted && n_born == 0;
             if ((round & 63u) == 63u && lane == 0) { // time budget (watchdog)
                 if (global_ns() - t0 > a.budget_ns) atomicOr(a.status, kStatusBudget);
-                if (*(volatile unsigned int *)a.status) stop = 1;
+                if (*(volatile unsigned int *)a.status & kStatusBudget) stop = 1;
             }
             if (lane == 0 && stop) B.stop = 1;
         }
@@ -652,7 +673,15 @@ __global__ void __launch_bounds__(128, 4) walk_replay_kernel(const ReplayArgs a)
         __syncthreads();
         drawn = drawn == 2 ? 0 : drawn + 1;
     }
-    if (part == kM && n_fin > 0) flush();
+    if (part != kM) return;
+    if (n_fin > 0) flush();
+    // out of time: the photons in flight leave their records as they stand, those not begun yet after
+    // their first step, with condition 0 unless that step is their last
+    queue(lane < kSlots && (B.slots[lane & (kSlots - 1)].flags & kActive), B.slots[lane & (kSlots - 1)], 0);
+    if (n_fin > 0) flush();
+    queue(lane < n_born, B.born[lane], 0);
+    if (n_fin > 0) flush();
+    if (!exhausted) leave_unwalked<false>(a, lane);
 }
 
 // ---------------------------------------------------------------- the polarised walk
@@ -874,9 +903,9 @@ __global__ void __launch_bounds__(128, 3) walk_replay_pol_kernel(const ReplayArg
     const unsigned group = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << g0;
     Slot s{};
     double st[4] = {1, 0, 0, 0};
-    bool have = false, exhausted = false;
+    bool have = false, exhausted = false, stop = false;
     const unsigned long long t0 = global_ns();
-    for (uint32_t it = 0;; ++it) {
+    for (uint32_t it = 0; !stop; ++it) {
         int cond = 0;
         const unsigned need = __ballot_sync(0xffffffffu, !have && !exhausted && gl == 0);
         bool born = false;
@@ -923,32 +952,35 @@ __global__ void __launch_bounds__(128, 3) walk_replay_pol_kernel(const ReplayArg
             if ((round & 255u) == 255u) {
                 int over = 0;
                 if (lane == 0) over = global_ns() - t0 > a.budget_ns;
-                if (__shfl_sync(0xffffffffu, over, 0)) {
-                    if (lane == 0) atomicOr(a.status, kStatusBudget);
-                    return;
-                }
+                stop = __shfl_sync(0xffffffffu, over, 0) != 0;
+                if (stop) break;
             }
         }
-        if (have && !born) {
+        if (stop && lane == 0) atomicOr(a.status, kStatusBudget);
+        bool over = false;                                            // out of its stream
+        if (have && !born && !stop) {
             cond = pol_step(ph, s, a.seed, st, p_rand, two_phi);
-            if (s.k > (1ull << 33)) {
-                if (gl == 0) atomicOr(a.status, kStatusStream);
-                have = false;
-            }
+            over = s.k > kMaxUniforms;
+            if (over && gl == 0) atomicOr(a.status, kStatusStream);
         }
-        if (cond > 0) {
+        if (cond > 0 || over) {
             if (gl == 0) finish_photon<true>(a, s.gid, s.ci, cond, s.i, s.wvl_um, s.mux, s.muy, s.muz, s.path, s.depth, st);
             have = false;
         }
-        if ((it & 63u) == 63u) {                                      // time budget (watchdog)
-            int stop = 0;
-            if (lane == 0) stop = (global_ns() - t0 > a.budget_ns) || *(volatile unsigned int *)a.status;
-            if (__shfl_sync(0xffffffffu, stop, 0)) {
-                if (lane == 0 && global_ns() - t0 > a.budget_ns) atomicOr(a.status, kStatusBudget);
-                return;
+        if ((it & 63u) == 63u && !stop) {                             // time budget (watchdog)
+            int late = 0;
+            if (lane == 0) {
+                if (global_ns() - t0 > a.budget_ns) atomicOr(a.status, kStatusBudget);
+                late = *(volatile unsigned int *)a.status & kStatusBudget;
             }
+            stop = __shfl_sync(0xffffffffu, late, 0) != 0;
         }
     }
+    if (!stop) return;
+    // as the HG walk's photons do (walk_replay_kernel)
+    if (have && gl == 0) finish_photon<true>(a, s.gid, s.ci, 0, s.i, s.wvl_um, s.mux, s.muy, s.muz, s.path, s.depth, st);
+    __syncwarp();
+    leave_unwalked<true>(a, lane);
 }
 
 }  // namespace

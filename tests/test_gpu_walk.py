@@ -929,3 +929,36 @@ def test_tallies_of_few_and_many_configs(walker, mode, n_cfg):
             assert np.array_equal(res.tallies[k]['n_cond'][1:6], counts[1:6])
             assert int(res.tallies[k]['n_events']) == int(rec['n_scat'].astype(np.int64).sum())
         assert res.stats['n_photon'] == lo
+
+
+@pytest.mark.parametrize('mode,n', [('replay64', 300), ('replay64', 60000), ('pol64', 40), ('pol64', 60000)])
+def test_replay_stopped_by_its_budget_leaves_every_record(walker, mode, n):
+    """A replay out of time: photons that ended leave the records of a whole run, those in flight and
+    those not begun a record with condition 0, their wavelength and the steps they walked; no record
+    of the caller's array is left as it was."""
+    g = load_golden('pol' if mode == 'pol64' else 'cfg1')
+    ice, imp = golden_tables(g)
+    cfg = dataclasses.replace(golden_config(g), n_photon=n)
+    if mode == 'pol64':
+        cfg = dataclasses.replace(cfg, tau_tot=8.0)
+    walker.set_tables([ice], imp)
+    if mode == 'pol64':
+        walker.set_phase_matrices([golden_phase(g)])
+    whole = walker.walk([cfg], 4, mode=mode).records
+    got = np.empty(n, whole.dtype)
+    got.view(np.uint8)[:] = 0xee
+    walker.set_budget(1e-6)
+    try:
+        with pytest.raises(_abi.BudgetExceeded):
+            walker.walk([cfg], 4, mode=mode, out=got)
+    finally:
+        walker.set_budget(_abi.DEFAULT_BUDGET_S)
+    ended = got['condition'] > 0
+    assert (got['condition'] >= 0).all() and (got['condition'] <= 5).all() and (~ended).any()
+    assert got[ended].tobytes() == whole[ended].tobytes()
+    left = got[~ended]
+    assert np.array_equal(left['wvn'], whole[~ended]['wvn']) and (left['config'] == 0).all()
+    assert (left['n_scat'] >= 0).all() and (left['n_scat'] <= whole[~ended]['n_scat']).all()
+    assert np.isfinite(left['theta_n']).all() and (left['flags'] <= 1).all()
+    again = walker.walk([cfg], 4, mode=mode).records
+    assert again.tobytes() == whole.tobytes()
