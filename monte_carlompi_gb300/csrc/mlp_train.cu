@@ -136,8 +136,7 @@ __global__ void colsum_finish_kernel(const ColsumTable tab, int groups, int chun
     out[(size_t)g * s_out + L.off + col] = t;
 }
 
-// Transposed bf16 copies of weight blocks written by Adam (the B operands of the
-// backward products): wt[g * s_t + off_t + c * ld_t + o] = w[o, c] for the block's
+// Transposed bf16 copies of weight blocks written by Adam: wt[g * s_t + off_t + c * ld_t + o] = w[o, c] for the block's
 // rows o < rows and columns c < cols, which start at offset off in the flat layout.
 struct TransposeBlock {
     long long off, off_t, ld_t;
@@ -263,10 +262,15 @@ __global__ void __launch_bounds__(256) adam_tiled_kernel(float *w, const float *
         tile[c8 + k][row] = __ushort_as_bfloat16((unsigned short)(h[k >> 1] >> ((k & 1) * 16)));
     __syncthreads();
     const int col = threadIdx.x >> 2, o8 = (threadIdx.x & 3) * 8;
-    // rows past the block's are the copy's zero padding
-    if (c0 + col < B.cols && o0 + o8 < B.ld_t)
-        *reinterpret_cast<uint4 *>(wt + (size_t)g * s_t + B.off_t + (size_t)(c0 + col) * B.ld_t + o0 + o8) =
-            *reinterpret_cast<const uint4 *>(&tile[col][o8]);
+    // (what lies past the block's rows, up to ld_t, is the caller's)
+    if (c0 + col < B.cols && o0 + o8 < B.rows) {
+        __nv_bfloat16 *dst = wt + (size_t)g * s_t + B.off_t + (size_t)(c0 + col) * B.ld_t + o0 + o8;
+        if (o0 + o8 + 8 <= B.rows) {
+            *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(&tile[col][o8]);
+        } else {
+            for (int k = 0; o0 + o8 + k < B.rows; ++k) dst[k] = tile[col][o8 + k];
+        }
+    }
 }
 
 // Batch of the step: rows perm[g][b * batch + i] of the encoded inputs (bf16, row
@@ -303,7 +307,6 @@ __global__ void advance_kernel(int *counter, int *step) {
 }
 
 // The tiles of a layout whose blocks lie in ascending order on 16-byte boundaries; false otherwise.
-// wt is written up to ld_t only where the block's padding ends within its last eight rows.
 bool make_adam_tiles(const TransposeTable &tt, long long n, long long s_t, AdamTiles *out) {
     AdamTiles a;
     memset(&a, 0, sizeof(a));
@@ -312,7 +315,7 @@ bool make_adam_tiles(const TransposeTable &tt, long long n, long long s_t, AdamT
     int tiles = 0;
     for (int q = 0; q < tt.n_blocks; ++q) {
         const TransposeBlock &b = tt.b[q];
-        if ((b.off & 7) || (b.off_t & 7) || (b.ld_t & 7) || (b.cols & 7) || b.off < at || b.ld_t != (b.rows + 7) / 8 * 8)
+        if ((b.off & 7) || (b.off_t & 7) || (b.ld_t & 7) || (b.cols & 7) || b.off < at)
             return false;
         a.first[q] = tiles;
         tiles += (b.rows + 31) / 32 * ((b.cols + 63) / 64);

@@ -401,3 +401,30 @@ def test_gemm_batch_loss_and_column_sums(m, n):
     torch.cuda.synchronize()
     assert rc == 0 and torch.equal(dst[:, :n], src.to(torch.bfloat16)) and (dst[:, n:] == 0).all()
     assert (cs.double().sum(0) - src.double().sum(0)).abs().max() < 1e-5 * src.double().sum(0).abs().max() + 1e-12
+
+
+@pytest.mark.parametrize('rows,ld', [(1, 8), (12, 16), (31, 40), (32, 32), (33, 48), (649, 656)])
+def test_grouped_adam_writes_no_padding_of_the_transposed_copies(rows, ld):
+    """wt[offset_t + c ld_t + o] is written for o < rows alone: what lies between the columns' ends,
+    and behind the last column's, keeps what the caller had there."""
+    G, cols = 2, 72
+    n = rows * cols + 16
+    off_t, stride_t = 8, 8 + (cols - 1) * ld + rows + 24
+    stride_t += -stride_t % 8
+    g = torch.Generator().manual_seed(rows)
+    w, gr = torch.randn(G, n, generator=g).cuda(), torch.randn(G, n, generator=g).cuda()
+    m, v = torch.zeros_like(w), torch.zeros_like(w)
+    w16 = torch.zeros(G, n, dtype=torch.bfloat16, device='cuda')
+    wt = torch.full((G, stride_t), 7.0, dtype=torch.bfloat16, device='cuda')
+    lr, step = torch.full((1,), 1e-3, device='cuda'), torch.ones(1, dtype=torch.int32, device='cuda')
+    blk = (_abi.TransposeBlockC * 1)(_abi.TransposeBlockC(8, off_t, ld, rows, cols))
+    assert _abi.load().mcw_mlp_adam_grouped(w.data_ptr(), gr.data_ptr(), m.data_ptr(), v.data_ptr(), w16.data_ptr(), n, G,
+                                            lr.data_ptr(), step.data_ptr(), 0.9, 0.999, 1e-8, wt.data_ptr(), stride_t,
+                                            blk, 1, _stream()) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(w16, w.to(torch.bfloat16))
+    want = torch.full_like(wt, 7.0)
+    for c in range(cols):
+        at = off_t + c * ld
+        want[:, at:at + rows] = w16[:, 8 + c:8 + rows * cols:cols]
+    assert torch.equal(wt, want)
