@@ -29,11 +29,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
-#include <set>
-#include <utility>
 
 #include "../../include/mcw_mlp.h"
+#include "smem_limit.cuh"
 
 namespace mcw {
 
@@ -732,20 +730,6 @@ __global__ void pack_kernel(const __nv_bfloat16 *w, int n, int k_in, int row0, i
 using namespace mcw;
 
 namespace {
-
-// Lets a kernel take `bytes` of dynamic shared memory, asked once per device and kernel.
-cudaError_t allow_smem(const void *fn, size_t bytes) {
-    static std::mutex mu;
-    static std::set<std::pair<int, const void *>> done;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(mu);
-    if (done.count({dev, fn})) return cudaSuccess;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) done.insert({dev, fn});
-    return e;
-}
 
 // members networks (1 for one network) on the same inputs: member e's biases bias_stride
 // floats and its packed weights blob_stride bytes after member e - 1's, its outputs at

@@ -45,6 +45,7 @@
 
 #include "../../include/mcw_mlp.h"
 #include "pdl.cuh"
+#include "smem_limit.cuh"
 
 namespace mcw {
 
@@ -675,14 +676,10 @@ bool make_map(CUtensorMap *map, const void *base, long long inner, long long row
 
 template <int kEpi, bool kAMn, bool kBMn, int TN, int kSub = 1>
 cudaError_t launch(const GemmBatch &b, unsigned grid, size_t smem, cudaStream_t s) {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(gemm_kernel<kEpi, kAMn, kBMn, TN, kSub>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    208 * 1024);
-    });
-    if (attr != cudaSuccess) return attr;
-    return launch_after(gemm_kernel<kEpi, kAMn, kBMn, TN, kSub>, grid, kThreads, smem, s, b);
+    auto *kernel = gemm_kernel<kEpi, kAMn, kBMn, TN, kSub>;
+    const cudaError_t e = allow_smem(reinterpret_cast<const void *>(kernel), 208 * 1024);
+    if (e != cudaSuccess) return e;
+    return launch_after(kernel, grid, kThreads, smem, s, b);
 }
 
 // The combinations of epilogue and layouts that exist: a plain product takes any, a backward
