@@ -20,6 +20,7 @@
 #include <cstdint>
 
 #include "../../include/mcw_mlp.h"
+#include "smem_limit.cuh"
 
 namespace mcw {
 
@@ -365,7 +366,9 @@ Hull hull_of(const double *h) {
     return r;
 }
 
-bool rows_ok(int32_t members, int32_t n) { return members >= 1 && members <= 4096 && n >= 0; }
+// The Jacobian keeps 16 bytes a member in shared memory, the costs 8: 200 KB of the 227 at the most.
+constexpr int kMaxMembers = 12800;
+bool rows_ok(int32_t members, int32_t n) { return members >= 1 && members <= kMaxMembers && n >= 0; }
 int done() { return cudaGetLastError() == cudaSuccess ? 0 : MCW_MLP_ERR_CUDA; }
 
 int cost(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t n_obs, const double *mean,
@@ -374,9 +377,11 @@ int cost(const void *ys, int64_t pitch, int32_t members, int32_t points, int32_t
         (long long)points * n_obs > 0x7fffffffLL || !rows_ok(members, points * n_obs) || pitch < MCW_MLP_OUT)
         return MCW_MLP_ERR_ARG;
     if (points * n_obs == 0) return 0;
-    const int per = members <= 1024 ? 4 : 1;       // points a block, within 32 KB of albedos
-    cost_kernel<<<(points + per - 1) / per * n_obs, kThreads, per * members * sizeof(double),
-                  static_cast<cudaStream_t>(stream)>>>(
+    const int per = members <= 1024 ? 4 : 1;       // points a block, within 32 KB of albedos for the usual ensembles
+    const size_t smem = per * members * sizeof(double);
+    if (smem > 40 * 1024 && allow_smem(reinterpret_cast<const void *>(cost_kernel), kMaxMembers * sizeof(double)) != cudaSuccess)
+        return MCW_MLP_ERR_CUDA;
+    cost_kernel<<<(points + per - 1) / per * n_obs, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __half *>(ys), pitch, members, points, per, n_obs, mean, std, floor, obs, noise, cost);
     return done();
 }
@@ -388,7 +393,10 @@ int jacobian(const float *y, const float *ydot, int64_t pitch, int32_t members, 
         (obs && (!noise.share || !jtr || !jtj)))
         return MCW_MLP_ERR_ARG;
     if (n == 0) return 0;
-    jacobian_kernel<<<n, kThreads, 2 * members * sizeof(double), static_cast<cudaStream_t>(stream)>>>(
+    const size_t smem = 2 * members * sizeof(double);
+    if (smem > 40 * 1024 && allow_smem(reinterpret_cast<const void *>(jacobian_kernel), kMaxMembers * 2 * sizeof(double)) != cudaSuccess)
+        return MCW_MLP_ERR_CUDA;
+    jacobian_kernel<<<n, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
         y, ydot, pitch, members, n, mean, std, floor, f, j, v, obs, noise, jtr, jtj);
     return done();
 }

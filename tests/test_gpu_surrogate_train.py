@@ -271,3 +271,36 @@ def test_retrieval_takes_noise_per_bin_and_per_observation(trained):
     assert np.allclose(spread.cpu(), inverse.logr_spread(rb, rj, w), rtol=1e-8, atol=1e-13)
     wn = 1 / inverse.noise_variance(rf, photons, rel)
     assert np.allclose(sigma.cpu(), 1 / np.sqrt((wn * rj * rj).sum(1)), rtol=1e-9)
+
+
+@pytest.mark.parametrize('members', [1024, 1025, 3037, 4096, 12800])
+def test_costs_and_slopes_of_many_members(members):
+    """The kernels that keep a share of every member in shared memory, past 48 KB of it, against the
+    array arithmetic; a member more than they hold is refused."""
+    from monte_carlompi_gb300 import _abi
+    n, bins, fl, L, st = 2, surrogate.N_BRF, surrogate.BRF_FLOOR, _abi.load(), surrogate._stream(torch)
+    g = torch.Generator().manual_seed(members)
+    y, yd = torch.randn(members, n, 652, generator=g).half(), torch.randn(members, n, 652, generator=g)
+    ys, y32, ydd = y.cuda(), y.float().cuda(), yd.cuda()
+    mean, std = torch.zeros(members, 649, dtype=torch.float64, device='cuda'), torch.full((members, 649), 0.2, dtype=torch.float64, device='cuda')
+    obs = torch.rand(n, bins, generator=g).double()
+    od, wd = obs.cuda(), torch.from_numpy(surrogate.bin_weights()).cuda()
+    new = lambda *shape: torch.empty(shape, dtype=torch.float64, device='cuda')  # noqa: E731
+    p = lambda t: t.data_ptr()  # noqa: E731
+    cost, f, j, v, sums = new(n), new(n, bins), new(n, bins), new(n, bins), new(2, n)
+
+    def run(k):
+        return (L.mcw_brf_cost(p(ys), 652, k, 1, n, p(mean), p(std), fl, p(od), p(wd), 0.0, 0.0, p(cost), st),
+                L.mcw_brf_jacobian(p(y32), p(ydd), 652, k, n, p(mean), p(std), fl, p(f), p(j), p(v), p(od), p(wd), 0.0, 0.0,
+                                   p(sums[0]), p(sums[1]), st))
+    assert run(members) == (0, 0) and run(12801) == (-1, -1)
+    torch.cuda.synchronize()
+    yp, dp = y[:, :, :649].double().numpy() * 0.2, yd[:, :, :649].double().numpy() * 0.2
+    a, shape = np.exp(yp[..., bins:]), np.exp(yp[..., :bins])
+    rf = ((shape - fl) * a).mean(0)
+    rj = (shape * dp[..., :bins] * a + (shape - fl) * (a * dp[..., bins:])).mean(0)
+    # (sums of some thousand terms of the order of one, in another order than numpy's)
+    assert np.allclose(f.cpu(), rf, rtol=1e-11, atol=1e-13) and np.allclose(j.cpu(), rj, rtol=1e-10, atol=1e-12)
+    share = surrogate.bin_weights()
+    assert np.allclose(cost.cpu(), (share * (rf - obs.numpy()) ** 2).sum(1), rtol=1e-10)
+    assert np.allclose(sums[1].cpu(), (share * rj * rj).sum(1), rtol=1e-9)
