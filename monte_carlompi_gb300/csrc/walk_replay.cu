@@ -24,12 +24,13 @@
 //    walked again with it when the chain turns out to have met one;
 //  * sqrt(1 - mu_z^2) and its reciprocal come from one Newton step and a residual correction
 //    (Markstein, IBM J. Res. Dev. 34, 1990), six operations, and the two divisions by it take
-//    three each.
+//    three each (rounded.cuh).
 // The draws assume that a step does nothing but scatter: a photon that ends, is reflected or is
 // replaced sits out the two rounds under way.  Every value is the one-thread walk's, in
-// its order of operations: sqrt and quotients are correctly rounded but where the exact value
-// lies within 2^-28 ulp of a rounding boundary (of 1.2e9 random arguments one sqrt and two quotients differ from
-// CUDA's, by an ulp).
+// its order of operations, every square root and quotient correctly rounded: the fourth warp looks
+// at the residuals of all steps of a round side by side, and a step whose rounding they leave open (some
+// five in a million) is walked again with sqrt() and /, its photon's draws ahead dropped as at an
+// event.  10,000 photons of the reference's default run 18.7 ms without the look, 19.3 with it.
 // 10,000 photons of the reference's default run: 193.7 ms on one thread each; 30.5 ms (0.94 us an
 // event of the longest walk) with one warp drawing and one walking, four lanes a photon, each
 // FP64 instruction serving all four through selects and shuffles; 16.0 ms now (0.47 us, 970
@@ -39,6 +40,7 @@
 #include <algorithm>
 
 #include "mcw_internal.cuh"
+#include "rounded.cuh"
 #include "ssp_device.cuh"
 #include "tally.cuh"
 
@@ -148,6 +150,7 @@ struct Ahead {
     uint64_t k0[kSlots];                     // the photon's stream before the steps
     double mzb[32], sq[32], h2[32], mz[32];  // Z: mu_z before, sqrt(1 - mu_z^2), 1 / that, mu_z after
     double x[32], y[32], z[32], path[32];    // XY and M: the state after the step
+    double numx[32], quox[32], numy[32], quoy[32];   // XY: the quotients by sqrt(1 - mu_z^2) in them
 };
 
 struct ReplayBlock {
@@ -162,7 +165,6 @@ struct ReplayBlock {
 };
 
 __device__ __forceinline__ double from_bits(uint64_t b) { return __longlong_as_double((long long)b); }
-__device__ __forceinline__ uint64_t to_bits(double x) { return (uint64_t)__double_as_longlong(x); }
 
 // u01_f64 by its bits: 1.m - (1 - 2^-53), exact, one FP64 operation.
 __device__ __forceinline__ double u01_bits(uint64_t w) {
@@ -194,43 +196,10 @@ __device__ __forceinline__ bool below_minus(double x, double t) {
 __device__ __forceinline__ bool is_nan(double x) { return (to_bits(x) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull; }
 __device__ __forceinline__ bool is_unit(double x) { return (to_bits(x) & 0x7fffffffffffffffull) == 0x3ff0000000000000ull; }
 
-// A power-of-two factor by the exponent (normal, finite x).
-__device__ __forceinline__ double halved(double x) { return __hiloint2double(__double2hiint(x) - 0x00100000, __double2loint(x)); }
-__device__ __forceinline__ double doubled(double x) { return __hiloint2double(__double2hiint(x) + 0x00100000, __double2loint(x)); }
-
-__device__ __forceinline__ double rsqrt_seed(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    return y;
-}
-
-// sqrt(x), x normal and in (0, 1]: a Newton step from the hardware's approximation, then the
-// residual's correction.
-__device__ __forceinline__ double sqrt_res(double x) {
-    const double y = rsqrt_seed(x), h = halved(y);
-    const double g = x * y;
-    const double r = fma(-g, h, 0.5);
-    const double g1 = fma(g, r, g), h1 = fma(h, r, h);
-    return fma(fma(-g1, g1, x), h1, g1);
-}
-
-// a / b, b normal: a Newton step on the hardware's reciprocal, then the residual's correction.
-__device__ __forceinline__ double div_res(double a, double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = fma(fma(-b, y, 1.0), y, y);
-    const double q = a * y;
-    return fma(fma(-q, b, a), y, q);
-}
-
 __device__ __forceinline__ double shfl_d(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
 
 // sqrt(1 - ct^2) as the reference writes it (ct = +-1: 0; past it, by rounding: NaN).
-__device__ __forceinline__ double sin_from(double ct) {
-    const double x = 1 - ct * ct;
-    const uint64_t b = to_bits(x);
-    return b == 0 || (b >> 63) ? sqrt(x) : sqrt_res(x);
-}
+__device__ __forceinline__ double sin_from(double ct) { return sqrt_rn(1 - ct * ct); }
 
 // The end of a step (:1390-1466) at depth z (z_prev before it): the path's exit correction, the
 // bottom's reflectance draw (uniform *k, taken when drawn), the end condition (0: walking on, or
@@ -377,20 +346,20 @@ __device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, Ahead &next, int
         } else if (s.flags & kIso) {                                  // Henyey_Greenstein2 (:790-800)
             ct = 1 - 2 * u0;
         } else {
-            const double q = div_res(s.hg_b, s.hg_c + s.hg_d * u0);
+            const double den = s.hg_c + s.hg_d * u0;
+            const double q = quotient_rn(s.hg_b, den, rcp_res(den));
             ct = s.hg_e * (s.hg_a - q * q);
         }
         double sp, cp;
         sincos(u1 * kTwoPi, &sp, &cp);
         const double dtau = -log(u2);
-        const double q0 = dtau * s.rext;                              // dtau / ext (:1372)
         const bool ice = u4 > s.p_imp;                                // :1375-1383
         next.ct[lane] = ct;
         next.st[lane] = sin_from(ct);
         next.cp[lane] = cp;
         next.sp[lane] = sp;
         next.dtau[lane] = dtau;
-        next.inc[lane] = fma(fma(-q0, s.ext, dtau), s.rext, q0);
+        next.inc[lane] = quotient_rn(dtau, s.ext, s.rext);            // :1372
         next.fl[lane] = (u3 >= (ice ? s.ssa_ice : s.ssa_imp) ? 1u : 0u) | (ice ? 2u : 0u);
         if (t == 0) {
             next.slot[rank] = si;
@@ -425,12 +394,9 @@ __device__ __forceinline__ double z_chain(Ahead &A, double mz, const int base, c
     for (int it = 0; it < S; ++it) {
         const int e = base + it, e1 = base + min(it + 1, S - 1);
         const double ct1 = A.ct[e1], st1 = A.st[e1], cp1 = A.cp[e1];
-        const double x = 1.0 - mz * mz;
-        const double y0 = rsqrt_seed(x), u = mz * ct;
-        const double h = halved(y0), g = x * y0;
-        const double r = fma(-g, h, 0.5);
-        const double g1 = fma(g, r, g), h1 = fma(h, r, h);
-        const double sq = fma(fma(-g1, g1, x), h1, g1);
+        const double u = mz * ct;
+        double h1;
+        const double sq = sqrt_res(1.0 - mz * mz, h1);
         double nz = (sq * -st) * cp + u;
         if (kPole && is_unit(mz)) nz = to_bits(mz) >> 63 ? -ct : ct;
         if (it < steps) {
@@ -469,7 +435,7 @@ __device__ void walk_z(ReplayBlock &B, Ahead &A, int lane) {
 template <bool kPole>
 __device__ __forceinline__ void xy_chain(Ahead &A, double va, double vb, const int base, const int steps, const int S,
                                          const bool isX, const int lane) {
-    double *out = isX ? A.x : A.y;
+    double *out = isX ? A.x : A.y, *nums = isX ? A.numx : A.numy, *quos = isX ? A.quox : A.quoy;
     double mzb = A.mzb[base], ct = A.ct[base], st = A.st[base], cp = A.cp[base], sp = A.sp[base], sq = A.sq[base],
            h2 = A.h2[base];
     for (int it = 0; it < S; ++it) {
@@ -478,13 +444,17 @@ __device__ __forceinline__ void xy_chain(Ahead &A, double va, double vb, const i
                      h21 = A.h2[e1];
         const double p = va * mzb, w = va * ct;
         const double num = st * (p * cp + vb * (isX ? -sp : sp));
-        const double q = num * h2;
-        double nv = fma(fma(-q, sq, num), h2, q) + w;
+        const double q = quotient_res(num, sq, h2);
+        double nv = q + w;
         if (kPole) {
             const double v = st * (isX ? cp : sp);
             if (is_unit(mzb)) nv = isX || !(to_bits(mzb) >> 63) ? v : -v;
         }
-        if (it < steps) out[e] = nv;
+        if (it < steps) {
+            out[e] = nv;
+            nums[e] = num;
+            quos[e] = q;
+        }
         va = nv;
         vb = shfl_d(nv, lane ^ 1);
         mzb = mzb1, ct = ct1, st = st1, cp = cp1, sp = sp1, sq = sq1, h2 = h21;
@@ -539,13 +509,45 @@ __device__ int walk_m(ReplayBlock &B, Ahead &A, int lane) {
     return event ? -done : done;
 }
 
+// The steps of A, a bit each, whose square root or quotients the chains may have rounded otherwise than
+// sqrt() and / do (rounded.cuh).  A lane a step: six FP64 instructions for all of them, where a test in
+// the chains would take as many a step.
+__device__ unsigned uncertain_steps(const Ahead &A, int lane) {
+    const double mz = A.mzb[lane], sq = A.sq[lane];
+    // (about the vertical there is neither; past it, by rounding, all is NaN either way)
+    const bool sure = is_unit(mz) || is_nan(sq) ||
+                      (sqrt_certain(sq, 1.0 - mz * mz) && quotient_certain(A.quox[lane], A.numx[lane], sq) &&
+                       quotient_certain(A.quoy[lane], A.numy[lane], sq));
+    return __ballot_sync(0xffffffffu, !sure);
+}
+
+// Step e, the `t`-th of its photon's, again with sqrt() and /, from the state before it.
+__device__ __noinline__ void step_again(const Slot &slot, Ahead &A, int e, int t) {
+    const double mux = t > 0 ? A.x[e - 1] : slot.mux, muy = t > 0 ? A.y[e - 1] : slot.muy, muz = A.mzb[e];
+    const double ct = A.ct[e], st = A.st[e], cp = A.cp[e], sp = A.sp[e];
+    const double sq = sqrt(1 - muz * muz);
+    A.x[e] = (st * (mux * muz * cp - muy * sp)) / sq + mux * ct;
+    A.y[e] = (st * (muy * muz * cp + mux * sp)) / sq + muy * ct;
+    A.mz[e] = -sq * st * cp + muz * ct;
+    A.z[e] = (t > 0 ? A.z[e - 1] : slot.z) + A.dtau[e] * A.mz[e];
+    A.path[e] = (t > 0 ? A.path[e - 1] : slot.path) + A.inc[e];
+}
+
 // The photons' states after the steps that XY and M walked: lane `rank` its photon's.  `walked`:
-// walk_m's result for it.  Returns its end condition (-1: out of its stream).
-__device__ int commit(const ReplayArgs &a, ReplayBlock &B, const Ahead &A, int rank, int walked) {
-    const bool event = walked < 0;
-    const int done = event ? -walked : walked;
-    const int si = A.slot[rank], e = rank * A.S + done - 1;
+// walk_m's result for it; `uncertain`: the steps to be walked again, where the photon's draws ahead
+// end as at an event.  Returns its end condition (-1: out of its stream).
+__device__ int commit(const ReplayArgs &a, ReplayBlock &B, Ahead &A, int rank, int walked, unsigned uncertain) {
+    bool event = walked < 0;
+    int done = event ? -walked : walked;
+    const int si = A.slot[rank];
     Slot &slot = B.slots[si];
+    const unsigned mine = (uncertain >> (rank * A.S)) & (0xffffffffu >> (32 - done));
+    if (mine) {
+        event = true;
+        done = __ffs(mine);
+        step_again(slot, A, rank * A.S + done - 1, done - 1);
+    }
+    const int e = rank * A.S + done - 1;
     uint32_t flags = slot.flags & ~kRefl;
     uint64_t k = A.k0[rank] + 5 * (uint64_t)done + A.shift[rank];
     double z = A.z[e], path = A.path[e];
@@ -618,7 +620,8 @@ __global__ void __launch_bounds__(128, 4) walk_replay_kernel(const ReplayArgs a)
             const bool mine = lane < kSlots && holds(B, now, lane & (kSlots - 1));
             const int w = __shfl_sync(0xffffffffu, walked, (2 * lane) & 31);
             const int si = mine ? now.slot[lane] : 0;
-            const int cond = mine ? commit(a, B, now, lane, w) : 0;
+            const unsigned uncertain = uncertain_steps(now, lane);
+            const int cond = mine ? commit(a, B, now, lane, w, uncertain) : 0;
             __syncwarp();
             // ---- finished photons leave their slots
             if (__any_sync(0xffffffffu, cond != 0)) {
@@ -692,28 +695,6 @@ __device__ __forceinline__ int64_t order_of(double x) {
     return b >= 0 ? b : ((int64_t)0x8000000000000000ull - b);
 }
 
-// 1 / b and a / b by it, b normal (div_res in two parts).
-__device__ __forceinline__ double rcp_res(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    return fma(fma(-b, y, 1.0), y, y);
-}
-__device__ __forceinline__ double quotient(double a, double b, double rb) {
-    const double q = a * rb;
-    return fma(fma(-q, b, a), rb, q);
-}
-
-// Whether |x| lies between 2^-255 and 2^256: the ranges of the two functions above and of sqrt_res hold.
-__device__ __forceinline__ bool moderate(double x) {
-    const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
-    return h >= 0x30000000u && h < 0x4ff00000u;
-}
-
-// The square root of 1 - c^2 and the like, in [0, 1] but for rounding (then NaN).
-__device__ __forceinline__ double sqrt_unit(double x) {
-    return !(to_bits(x) >> 63) && moderate(x) ? sqrt_res(x) : sqrt(x);
-}
-
 // scipy interp1d (linear) on an ascending grid: searchsorted (left) clipped to [1, n - 1], then the
 // two-term form of interp1d._call_linear: the upper end's index and both weights.
 struct Segment {
@@ -732,14 +713,9 @@ __device__ __forceinline__ Segment segment_of(const DevPhase &ph, int e, double 
     Segment s;
     s.k = lo < 1 ? 1 : (lo > n - 1 ? n - 1 : lo);
     const double xl = __ldg(x + s.k - 1), xh = __ldg(x + s.k), w = xh - xl;
-    if (moderate(w)) {
-        const double rw = rcp_res(w);
-        s.hi = quotient(xn - xl, w, rw);
-        s.lo = quotient(xh - xn, w, rw);
-    } else {
-        s.hi = (xn - xl) / w;
-        s.lo = (xh - xn) / w;
-    }
+    const double rw = rcp_res(w);
+    s.hi = quotient_rn(xn - xl, w, rw);
+    s.lo = quotient_rn(xh - xn, w, rw);
     return s;
 }
 __device__ __forceinline__ double element(const DevPhase &ph, int e, int row, const Segment &s) {
@@ -832,16 +808,10 @@ __device__ int pol_step(const DevPhase &ph, Slot &s, uint64_t seed, double st[4]
         ny = up ? sint * sinphi : -sint * sinphi;
         nz = up ? ct : -ct;
     } else {                                                          // :1270-1281
-        const double sq = sqrt_unit(1 - muz * muz);
+        const double sq = sqrt_rn(1 - muz * muz), rq = rcp_res(sq);
         const double tx = sint * (mux * muz * cosphi - muy * sinphi), ty = sint * (muy * muz * cosphi + mux * sinphi);
-        if (moderate(sq)) {
-            const double rq = rcp_res(sq);
-            nx = quotient(tx, sq, rq) + mux * ct;
-            ny = quotient(ty, sq, rq) + muy * ct;
-        } else {
-            nx = tx / sq + mux * ct;
-            ny = ty / sq + muy * ct;
-        }
+        nx = quotient_rn(tx, sq, rq) + mux * ct;
+        ny = quotient_rn(ty, sq, rq) + muy * ct;
         nz = -sq * sint * cosphi + muz * ct;
     }
     if (reflected) {                                                  // :1283-1285
@@ -858,33 +828,26 @@ __device__ int pol_step(const DevPhase &ph, Slot &s, uint64_t seed, double st[4]
         sc[1] = sp[0] * P12 + sp[1] * P22;
         sc[2] = sp[2] * P33 - sp[3] * P43;
         sc[3] = sp[2] * P43 + sp[3] * P44;
-        const double den = sqrt_unit((1 - ct * ct) * (1 - nz * nz));
+        const double den = sqrt_rn((1 - ct * ct) * (1 - nz * nz));
         double cos_i = 0;
         if (!(den == 0)) {
             const double sign = (phi_sca >= kPi) ? 1 : -1;
             const double num = nz * ct - muz, d = sign * den;
-            cos_i = moderate(d) ? div_res(num, d) : num / d;
+            cos_i = quotient_rn(num, d, rcp_res(d));
             if (cos_i < -1) cos_i = -1;
             else if (cos_i > 1) cos_i = 1;
         }
         rotate_stokes(-acos(cos_i), sc, sm);
-        if (moderate(sm[0])) {
-            const double ri = rcp_res(sm[0]);
-            st[0] = 1;
+        const double ri = rcp_res(sm[0]);
+        st[0] = moderate(sm[0]) ? 1 : sm[0] / sm[0];
 #pragma unroll
-            for (int k = 1; k < 4; ++k) st[k] = quotient(sm[k], sm[0], ri);
-        } else {
-            const double I_merd = sm[0];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) st[k] = sm[k] / I_merd;
-        }
+        for (int k = 1; k < 4; ++k) st[k] = quotient_rn(sm[k], sm[0], ri);
     }
     s.flags &= ~kRefl;
     const double zp = s.z;
     s.z = zp + dtau * nz;                                             // :1352
     s.mux = nx, s.muy = ny, s.muz = nz;                               // :1364-1369
-    const double q0 = dtau * s.rext;
-    s.path += fma(fma(-q0, s.ext, dtau), s.rext, q0);                 // dtau / ext (:1372)
+    s.path += quotient_rn(dtau, s.ext, s.rext);                       // :1372
     s.i += 1;
     return step_end(s, seed, s.z, zp, dtau, nz, s.path, false, ssa_rand >= (ice ? s.ssa_ice : s.ssa_imp), ice, &s.k, &s.flags);
 }
