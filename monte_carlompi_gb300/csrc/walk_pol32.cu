@@ -29,7 +29,7 @@
 // segment lie side by side with its two cosines (seg), so a lookup is a bucket and one or four
 // 16-byte loads instead of a search and 24 4-byte ones, and the accepted candidate's segment
 // serves the Stokes update; a launch on one phase table has it in its arguments.  200,000 photons
-// 3.12 ms, now 1.9, a million 7.3, now 4.9.
+// 3.12 ms, now 2.0, a million 7.3, now 5.0.
 //
 // Statistically equivalent restatements (identical distributions):
 //  * the envelope factor |Q cos 2b + U sin 2b| with 2b = arctan(U / Q) (:908-935)
@@ -123,16 +123,6 @@ __device__ __forceinline__ int segment_packed(const DevPhase32 &ph, const float4
     while (k > 1 && s0.x >= xn) s0 = __ldg(base + 4 * --k);
     while (k < last && s0.y < xn) s0 = __ldg(base + 4 * ++k);
     return k;
-}
-
-// sqrt of 0 or a normal x, correctly rounded: the hardware's reciprocal square root and one residual
-// (every mantissa of two binades was compared with sqrtf), without sqrtf's range branch.
-__device__ __forceinline__ float sqrt_pos(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    const float s = __fmul_rn(x, y);
-    const float r = fmaf(fmaf(-s, s, x), __fmul_rn(0.5f, y), s);
-    return x > 0.f ? r : x;
 }
 
 // Where xn lies in the segment whose first quarter is s (the same quotient for every element), and an
@@ -288,7 +278,7 @@ __device__ __forceinline__ int pol_step_post(PolPhoton &P, const DevPhase32 &ph,
             m0x = 0.f; m0y = 0.f; m0z = 1.f;
             ct = sqrtf(u01_f32(P.sb.w));
         }
-        const float st = sqrt_pos(fmaxf(0.f, fmaf(-ct, ct, 1.f)));
+        const float st = sqrtf(fmaxf(0.f, fmaf(-ct, ct, 1.f)));
         // sqrt(mu_x^2 + mu_y^2) stands for sqrt(1 - mu_z^2) (equal for a unit
         // direction; the frame stays orthogonal next to the pole in FP32); the
         // pole formula when it is 0 (or below FLT_MIN, where the reciprocal square
@@ -314,7 +304,7 @@ __device__ __forceinline__ int pol_step_post(PolPhoton &P, const DevPhase32 &ph,
             P.bref = false;
         } else {
             // into the scattering plane: phi_sca = arccos(cphi) in [0, pi]
-            const float sps = sqrt_pos(fmaxf(0.f, fmaf(-cphi, cphi, 1.f)));
+            const float sps = sqrtf(fmaxf(0.f, fmaf(-cphi, cphi, 1.f)));
             float Q = P.Q, U = P.U;
             rotate(Q, U, fmaf(2.f * cphi, cphi, -1.f), 2.f * sps * cphi);
             float Pe[6];
@@ -351,7 +341,7 @@ __device__ __forceinline__ int pol_step_post(PolPhoton &P, const DevPhase32 &ph,
                 const float sign = (cphi == -1.f) ? 1.f : -1.f;   // phi_sca >= pi only at cos phi = -1
                 cos_i = fminf(fmaxf(__fdividef(fmaf(nz, ct, -m0z), sign * den), -1.f), 1.f);
             }
-            const float si = sqrt_pos(fmaxf(0.f, fmaf(-cos_i, cos_i, 1.f)));
+            const float si = sqrtf(fmaxf(0.f, fmaf(-cos_i, cos_i, 1.f)));
             float Qm = Qs, Um = Us;
             rotate(Qm, Um, fmaf(2.f * cos_i, cos_i, -1.f), -2.f * si * cos_i);
             const float inv_i = 1.f / Is;
