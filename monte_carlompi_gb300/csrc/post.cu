@@ -30,18 +30,6 @@ __device__ __forceinline__ int np_bin(double x, int n, double step) {
     return i;
 }
 
-// 1 / x of a record's wavenumber: two Newton steps on the hardware's approximation (4 FMAs;
-// FP64 is scarce on this GPU, and IEEE division takes about ten operations), within an ulp of
-// the quotient; the division itself outside the range where the steps are safe.
-__device__ __forceinline__ double recip(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double y1 = fma(fma(-x, y, 1.0), y, y);
-    const double y2 = fma(fma(-x, y1, 1.0), y1, y1);
-    const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-    return (e > 64u && e < 1983u) ? y2 : 1.0 / x;
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -93,7 +81,7 @@ __device__ __forceinline__ void post_direct(mcw_post_stats *st, const PostRec &r
     atomicAdd(reinterpret_cast<unsigned long long *>(&st->n_cond[r.cond]), 1ull);
     atomicAdd(reinterpret_cast<unsigned long long *>(&st->sum_n_scat), (unsigned long long)r.nscat);
     atomicAdd(&st->sum_path_length, r.path);
-    atomicAdd(&st->sum_wavelength, recip(r.wvn));
+    atomicAdd(&st->sum_wavelength, 1.0 / r.wvn);
 }
 
 // A warp's running totals of its current config, a share in every lane's registers.
@@ -115,7 +103,7 @@ struct PostSums {
         }
         nscat += (unsigned long long)r.nscat;
         path += r.path;
-        wvl += recip(r.wvn);
+        wvl += 1.0 / r.wvn;
     }
     __device__ __forceinline__ void flush(mcw_post_stats *st, int lane) {
         unsigned long long mine = 0;

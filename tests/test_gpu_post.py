@@ -128,3 +128,15 @@ def test_records_in_any_order_match_numpy(walker, n, n_bins, n_cfg, order, dtype
             assert np.isclose(out['mean_wavelength'][c], np.mean(1 / wvn[at]), rtol=1e-12, atol=0)
             assert np.isclose(out['mean_path_length'][c], rec['path_length'][at].astype(np.float64).mean(), rtol=1e-12, atol=0)
             assert out['mean_n_scat'][c] == rec['n_scat'][at].astype(np.int64).sum() / at.sum()
+
+
+def test_wavelengths_are_correctly_rounded_reciprocals(walker):
+    """One record a config: its mean wavelength is 1 / wvn to the last bit, also where the quotient
+    lies next to the middle between two doubles (2 - k 2^-52, k odd) and in the least and largest
+    binades."""
+    x = np.concatenate([(2.0 - np.arange(1, 4001, 2) * 2.0 ** -52) * s for s in (1.0, 0.25, 2.0 ** -20)] +
+                       [np.random.default_rng(3).uniform(0.3, 3.0, 4000), [1e-300, 2.0 ** -960, 2.0 ** 900, 0.5, 1.0, 3.0]])
+    rec = np.zeros(x.size, _abi.RECORD64)
+    rec['condition'], rec['wvn'], rec['config'] = 2, x, np.arange(x.size)
+    out = post.zenith_brf(walker, rec, 8, x.size)
+    assert np.array_equal(out['mean_wavelength'], 1 / x)
