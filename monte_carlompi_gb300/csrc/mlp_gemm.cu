@@ -45,6 +45,7 @@
 
 #include "../../include/mcw_mlp.h"
 #include "pdl.cuh"
+#include "rounded.cuh"
 #include "smem_limit.cuh"
 
 namespace mcw {
@@ -102,14 +103,8 @@ __device__ __forceinline__ unsigned long long now_ns() {
 }
 
 __device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.f + __expf(-z)); }
-// The sigmoid's quotient by a Newton step on the hardware's reciprocal (Markstein, IBM J. Res. Dev.
-// 34, 1990), which flushes divisors past 2^126.
 __device__ __forceinline__ float dsilu(float z) {
-    const float d = 1.f + __expf(-z);
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
-    float s = fmaf(fmaf(-d, y, 1.f), y, y);
-    if (d > 8.5e37f) s = 1.f / d;
+    const float s = reciprocal_rn(1.f + __expf(-z));
     return s * (1.f + z * (1.f - s));
 }
 

@@ -3,7 +3,7 @@
 // correctly rounded one, as sqrt() and / give it.  The correction misses it only where the exact value
 // lies within 2^-28 ulp of the middle between two doubles, which the residual of the result tells:
 // about one result in 500,000 is uncertain, and then taken from sqrt() or /.
-// Compiled with --fmad=false.
+// (Compiled with --fmad=false.)  And an FP32 reciprocal.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -82,6 +82,15 @@ __device__ __forceinline__ double sqrt_rn(double x) {
 __device__ __forceinline__ double quotient_rn(double a, double b, double rb) {
     const double q = quotient_res(a, b, rb);
     return moderate(b) && quotient_certain(q, a, b) ? q : a / b;
+}
+
+// 1 / d, d >= 1 (or NaN): a Newton step on the hardware's reciprocal, by the same author, which alone
+// is correctly rounded here (of every float from 1 to 2^126, which the hardware's flushes from there on).
+__device__ __forceinline__ float reciprocal_rn(float d) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    const float s = fmaf(fmaf(-d, y, 1.f), y, y);
+    return d > 8.5e37f ? 1.f / d : s;
 }
 
 }  // namespace mcw

@@ -1,7 +1,7 @@
-"""Square roots and quotients of the FP64 replay (csrc/rounded.cuh) against IEEE arithmetic, bit for
-bit: arguments whose exact result lies next to the middle between two doubles, where the kernels'
-correction alone rounds to the wrong side, arguments at random, and zeros, infinities, NaN, denormals
-and powers of two."""
+"""Square roots and quotients of the FP64 replay and the FP32 reciprocal of SiLU's derivative
+(csrc/rounded.cuh) against IEEE arithmetic, bit for bit: arguments whose exact result lies next to the
+middle between two doubles, where the kernels' correction alone rounds to the wrong side, arguments at
+random, zeros, infinities, NaN, denormals and powers of two; every float from 1 on."""
 import ctypes
 import subprocess
 
@@ -26,6 +26,23 @@ __global__ void probe(const double *a, const double *b, int n, double *q, double
     const bool pos = b[i] > 0 && moderate(b[i]);
     wrong[i] = (pos && sqrt_certain(g, b[i]) ? 1 : 0) | (moderate(b[i]) && quotient_certain(r, a[i], b[i]) ? 2 : 0) |
                (pos && g != sqrt(b[i]) ? 4 : 0) | (moderate(b[i]) && r != a[i] / b[i] ? 8 : 0);
+}
+__global__ void reciprocals(unsigned *bad) {
+    const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long i = 0x3f800000ull + blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i <= 0x7fc00000ull; i += step) {
+        const float d = __uint_as_float((unsigned)i), s = reciprocal_rn(d), want = 1.f / d;
+        if (s != want && !(s != s && want != want)) atomicAdd(bad, 1u);
+    }
+}
+// How many floats from 1 to infinity, and NaN, have another reciprocal than 1.f / d.
+extern "C" int reciprocals_off(unsigned *off) {
+    unsigned *d = nullptr;
+    if (cudaMalloc(&d, 4)) return 1;
+    cudaMemset(d, 0, 4);
+    reciprocals<<<1216, 256>>>(d);
+    cudaMemcpy(off, d, 4, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return (int)cudaGetLastError();
 }
 extern "C" int run(const double *a, const double *b, int n, double *q, double *s, unsigned char *wrong) {
     double *d = nullptr;
@@ -60,6 +77,7 @@ def probe(tmp_path_factory):
         assert lib.run(p(a), p(b), a.size, p(q), p(s), p(w)) == 0
         with np.errstate(all='ignore'):
             return a, b, q, a / b, s, np.sqrt(b), w
+    run.lib = lib
     return run
 
 
@@ -124,3 +142,8 @@ def test_at_random_and_at_the_ends(probe):
     ends = np.concatenate([ends, -ends])
     _, _, q, qw, s, sw, _ = probe(ends[:, None], ends[None, :])
     assert same(q, qw) and same(s, sw)
+
+
+def test_every_reciprocal_from_one_on(probe):
+    off = ctypes.c_uint32(1)
+    assert probe.lib.reciprocals_off(ctypes.byref(off)) == 0 and off.value == 0
