@@ -428,3 +428,61 @@ def test_grouped_adam_writes_no_padding_of_the_transposed_copies(rows, ld):
         at = off_t + c * ld
         want[:, at:at + rows] = w16[:, 8 + c:8 + rows * cols:cols]
     assert torch.equal(wt, want)
+
+
+@pytest.mark.parametrize('m,n,with32', [(128, 64, True), (31, 33, True), (640, 649, True), (640, 649, False), (256, 96, False)])
+def test_silu_derivative_bf16_output_is_the_rounded_f32(m, n, with32):
+    """The bf16 result of the SiLU' epilogue over its range, NaN and infinities among it, is its f32
+    result rounded, and the same without the f32 result (pairs of columns, whole and partial blocks)."""
+    a = torch.ones(1, m, 8, dtype=torch.bfloat16, device='cuda') / 8
+    b = torch.ones(1, n, 8, dtype=torch.bfloat16, device='cuda')
+    z = torch.linspace(-100, 100, m * n).reshape(m, n)
+    z[0, 0], z[0, 1], z[1, 0], z[1, 1] = float('nan'), float('inf'), float('-inf'), 0.0
+    zc = z.cuda()
+    out16, f32 = torch.zeros(2, m, n, dtype=torch.bfloat16, device='cuda'), torch.zeros(1, m, n, device='cuda')
+    for i, keep in enumerate((True, with32)):
+        more = dict(c2=f32.data_ptr(), ldc2=n, stride_c2=m * n) if keep else {}
+        q = _problem(_abi.EPI_DSILU, m, n, 8, a, b, out16[i:i + 1], 0, 0, aux=zc.data_ptr(), ldaux=n, stride_aux=m * n, **more)
+        assert _abi.load().mcw_mlp_gemm_batch(ctypes.byref(q), 1, _stream()) == 0
+    torch.cuda.synchronize()
+    want = f32[0].to(torch.bfloat16).float()
+    assert torch.isnan(want[0, 0]) and torch.isfinite(want).sum() >= m * n - 3
+    for i in range(2):
+        assert torch.allclose(out16[i].float(), want, rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize('G,B,rows,n_out', [(1, 1, 1, 1), (2, 33, 70, 649), (3, 64, 128, 40)])
+def test_gather_and_grouped_loss(G, B, rows, n_out):
+    """A step's batch with its transposed inputs, rows past the epoch's left alone, and the loss of
+    grouped outputs with its gradient in f32, bf16 and bf16 transposed."""
+    g = torch.Generator().manual_seed(B)
+    x_all = torch.randn(rows, 16, generator=g).to(torch.bfloat16).cuda()
+    t_all = torch.randn(rows, n_out, generator=g).cuda()
+    perm = torch.stack([torch.randperm(rows, generator=g) for _ in range(G)]).int().cuda()
+    L = _abi.load()
+    last = (rows - 1) // B                                    # the epoch's last batch, cut short
+    for c in (0, last):
+        x, t = torch.full((G, B, 16), 7.0, dtype=torch.bfloat16, device='cuda'), torch.full((G, B, n_out), 7.0, device='cuda')
+        xt = torch.full((G, 16, B), 7.0, dtype=torch.bfloat16, device='cuda')
+        counter = torch.tensor([c], dtype=torch.int32, device='cuda')
+        assert L.mcw_mlp_gather(x_all.data_ptr(), t_all.data_ptr(), n_out, n_out, perm.data_ptr(), rows, counter.data_ptr(),
+                                B, G, x.data_ptr(), B * 16, xt.data_ptr(), 16 * B, t.data_ptr(), n_out, B * n_out,
+                                _stream()) == 0
+        torch.cuda.synchronize()
+        for k in range(G):
+            at = perm[k, c * B:(c + 1) * B].long()
+            assert torch.equal(x[k, :at.numel()], x_all[at]) and torch.equal(t[k, :at.numel()], t_all[at])
+            assert torch.equal(xt[k], x[k].t()) and (x[k, at.numel():] == 7).all() and (t[k, at.numel():] == 7).all()
+    y, tt = torch.randn(G, B, n_out, generator=g).cuda(), torch.randn(G, B, n_out, generator=g).cuda()
+    w = torch.rand(n_out, generator=g).cuda()
+    g32, loss = torch.zeros(G, B, n_out, device='cuda'), torch.zeros(G, device='cuda')
+    g16, g16t = torch.zeros(G, B, n_out, dtype=torch.bfloat16, device='cuda'), torch.zeros(G, n_out, B, dtype=torch.bfloat16, device='cuda')
+    assert L.mcw_mlp_loss_grouped(y.data_ptr(), n_out, B * n_out, tt.data_ptr(), n_out, B * n_out, w.data_ptr(), G, B, n_out,
+                                  g32.data_ptr(), n_out, B * n_out, g16.data_ptr(), B * n_out, g16t.data_ptr(), B, n_out * B,
+                                  loss.data_ptr(), _stream()) == 0
+    torch.cuda.synchronize()
+    d = (y - tt).double()
+    # (FP32 sums of at most 2e4 terms: 1e-5 of the whole; a gradient has four roundings)
+    assert torch.allclose(loss.double(), (w.double() * d * d).mean((1, 2)), rtol=1e-5)
+    assert torch.allclose(g32.double(), 2 * w.double() * d / (B * n_out), rtol=1e-6, atol=0)
+    assert torch.equal(g16, g32.to(torch.bfloat16)) and torch.equal(g16t, g16.transpose(1, 2))
