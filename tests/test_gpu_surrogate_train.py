@@ -304,3 +304,23 @@ def test_costs_and_slopes_of_many_members(members):
     share = surrogate.bin_weights()
     assert np.allclose(cost.cpu(), (share * (rf - obs.numpy()) ** 2).sum(1), rtol=1e-10)
     assert np.allclose(sums[1].cpu(), (share * rj * rj).sum(1), rtol=1e-9)
+
+
+@pytest.mark.parametrize('lo,hi', [(-700.0, 700.0), (-12.0, 4.0), (-0.01, 0.01)])
+def test_members_exponential_to_half_an_ulp(lo, hi):
+    """exp of the members' outputs (floor 0, albedo 1) against extended precision: half an ulp, and 0.05
+    for the table's second part, the series (0.02), the reduced argument and three roundings of 2^-7 of
+    the result."""
+    from monte_carlompi_gb300 import _abi
+    n, bins = 200, surrogate.N_BRF
+    x = np.random.default_rng(8).uniform(lo, hi, (n, 649))
+    x[:, bins] = 0.0
+    ys = torch.zeros(n, 1, 656, dtype=torch.float16, device='cuda')            # n members, a row each
+    mean, std = torch.from_numpy(x).cuda(), torch.ones(n, 649, dtype=torch.float64, device='cuda')
+    brf, alb = torch.empty((n, bins), dtype=torch.float64, device='cuda'), torch.empty(n, dtype=torch.float64, device='cuda')
+    p = lambda t: t.data_ptr()  # noqa: E731
+    assert _abi.load().mcw_brf_members(p(ys), 656, n, 1, p(mean), p(std), 0.0, p(brf), p(alb), surrogate._stream(torch)) == 0
+    got, want = brf.cpu().numpy().astype(np.longdouble), np.exp(x[:, :bins].astype(np.longdouble))
+    ulp = np.ldexp(np.longdouble(1), np.frexp(want)[1] - 53)
+    assert (np.abs(got - want) / ulp).max() <= 0.55
+    assert (alb.cpu() == 1).all()
