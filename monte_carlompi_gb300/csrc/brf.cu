@@ -1,17 +1,19 @@
 // From the surrogate's standardised outputs to BRFs, in FP64: members' BRFs, their mean and
 // spread, a retrieval's costs and Gauss-Newton sums.  Compiled with --fmad=false: every product
 // and sum is rounded on its own, in the order of the array code these kernels took the place of
-// (surrogate.from_target, Ensemble.predict, inverse.surrogate_gn), but where one is written as fma.
+// (surrogate.from_target, Ensemble.predict, inverse.surrogate_gn), but where one is written as fma, means
+// over the members divided.
 //
 // Target space: y * std + mean = log(BRF / albedo + floor) for the 648 bins and log(albedo).
 //
 // What bounds them: FP64 (64 cycles a warp an operation on a sub-core), so every kernel takes each
-// exponential once, ten operations by table, divides once where it can, and keeps what it can in
+// exponential once, eleven operations by table, divides once where it can, and keeps what it can in
 // registers; a block per row, a thread per bin, sums by block reduction.  16 grid points of 128
-// observations, five members: 362 us with CUDA's exp and a division a weight a point, 254 now; a
-// Jacobian 46 and 40.  One retrieval of 128 observations with five members (16-point grid, six
+// observations, five members: 362 us with CUDA's exp and a division a weight a point, 285 now; a
+// Jacobian 46 now (259 and 44 with exponentials of 1.24 ulp, the floors taken off a sum and means by the
+// reciprocal, which lost digits).  One retrieval of 128 observations with five members (16-point grid, six
 // iterations, spreads): 92 ms on the host's cores and elementwise tensor kernels; 3.3 ms with these kernels and the steps and the encoding of log r on the host, a
-// wait for the device and two copies an iteration; 1.5 ms with the steps here too and the network
+// wait for the device and two copies an iteration; 1.6 ms with the steps here too and the network
 // laid out while the grid's costs are worked out.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -114,6 +116,14 @@ __device__ __forceinline__ double row_albedo(const __half *row, const double *st
     return exp(unscaled((double)__half2float(row[kBins]), std[kBins], mean[kBins]));
 }
 
+// t / members, correctly rounded, share = 1 / members: the residual's correction (Markstein, IBM J. Res.
+// Dev. 34, 1990).  With a whole number of at most 14 bits below the line the residual is exact, and the
+// quotient at least ulp / (2 members) from the middle between two doubles, or a double.
+__device__ __forceinline__ double mean_of(double t, int members, double share) {
+    const double q = t * share, s = fma(fma(-q, (double)members, t), share, q);
+    return (__double2hiint(q) & 0x7fffffff) < 0x7ff00000 ? s : q;
+}
+
 // The larger of x and lo; NaN stays NaN.
 __device__ __forceinline__ double at_least(double x, double lo) { return x < lo ? lo : x; }
 
@@ -209,8 +219,7 @@ __global__ void __launch_bounds__(kThreads) cost_kernel(const __half *ys, long l
     }
     for (int p = 0; p < np; ++p) {
         const int r = (p0 + p) * n_obs + o;
-        double c = 0.0, floors = 0.0;        // sum of (exp - floor) albedo = sum of exp albedo - these
-        for (int m = 0; m < members; ++m) floors += floor * albs[p * members + m];
+        double c = 0.0;
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             const int b = threadIdx.x + k * kThreads;
@@ -219,9 +228,9 @@ __global__ void __launch_bounds__(kThreads) cost_kernel(const __half *ys, long l
             for (int m = 0; m < members; ++m) {
                 const double *mu = mean + (size_t)m * (kBins + 1), *sd = std + (size_t)m * (kBins + 1);
                 const double y = (double)__half2float(ys[((size_t)m * rows + r) * pitch + b]);
-                t = fma(exp_by_table(fma(y, sd[b], mu[b]), tab), albs[p * members + m], t);
+                t = fma(exp_by_table(fma(y, sd[b], mu[b]), tab) - floor, albs[p * members + m], t);
             }
-            const double d = (t - floors) * share - x[k];
+            const double d = mean_of(t, members, share) - x[k];
             c += w[k] * (d * d);
         }
         c = block_sum(c, red);
@@ -263,9 +272,9 @@ __global__ void __launch_bounds__(kThreads) jacobian_kernel(const float *y, cons
             f2 += fm * fm;
             j += shape * dp * a + (shape - floor) * sh[2 * m + 1];
         }
-        f = f * each;
-        j = j * each;
-        const double v = at_least(f2 * each - f * f, 0.0);
+        f = mean_of(f, members, each);
+        j = mean_of(j, members, each);
+        const double v = at_least(mean_of(f2, members, each) - f * f, 0.0);
         if (f_out) f_out[(size_t)r * kBins + b] = f;
         if (j_out) j_out[(size_t)r * kBins + b] = j;
         if (v_out) v_out[(size_t)r * kBins + b] = v;

@@ -324,3 +324,44 @@ def test_members_exponential_to_half_an_ulp(lo, hi):
     ulp = np.ldexp(np.longdouble(1), np.frexp(want)[1] - 53)
     assert (np.abs(got - want) / ulp).max() <= 0.55
     assert (alb.cpu() == 1).all()
+
+
+@pytest.mark.parametrize('members', [1, 2, 3, 5, 7, 1000])
+def test_means_over_the_members_lose_nothing(members):
+    """Means over the members are the sums divided, to the last bit, infinities kept; and a grid cost of
+    BRFs next to 0 (exponentials next to the floor) keeps the digits of the members' own BRFs."""
+    from monte_carlompi_gb300 import _abi
+    n, bins, L, st = 6, surrogate.N_BRF, _abi.load(), surrogate._stream(torch)
+    rng, p = np.random.default_rng(members), lambda t: t.data_ptr()
+    new = lambda *shape: torch.empty(shape, dtype=torch.float64, device='cuda')  # noqa: E731
+    y = torch.from_numpy(rng.uniform(-3, 3, (1, n, 652)).astype(np.float32))
+    y[:, :, bins] = 0.0                                                        # albedo 1
+    y[0, 0, 0] = 800.0
+    yd = torch.ones(1, n, 652)
+    yd[:, :, bins] = 0.0
+
+    def slopes(k):
+        ys, yds = y.expand(k, n, 652).contiguous().cuda(), yd.expand(k, n, 652).contiguous().cuda()
+        mean, std, f, j, v = torch.zeros(k, 649, dtype=torch.float64, device='cuda'), \
+            torch.ones(k, 649, dtype=torch.float64, device='cuda'), new(n, bins), new(n, bins), new(n, bins)
+        assert L.mcw_brf_jacobian(p(ys), p(yds), 652, k, n, p(mean), p(std), 0.0, p(f), p(j), p(v), None, None, 0.0, 0.0,
+                                  None, None, st) == 0
+        return f.cpu().numpy(), j.cpu().numpy()
+    f1, j1 = slopes(1)
+    total = lambda t: np.add.accumulate(np.broadcast_to(t, (members, *t.shape)), 0)[-1]  # noqa: E731
+    f, j = slopes(members)
+    assert np.array_equal(f, total(f1) / members) and np.isinf(f[0, 0])
+    assert np.array_equal(j, total(j1) / members, equal_nan=True) and np.isnan(j).sum() == 1   # (infinity times 0)
+    # BRFs of 1e-11
+    fl = surrogate.BRF_FLOOR
+    mean = math.log(fl) + rng.uniform(-1e-9, 1e-9, (members, 649))
+    mean[:, bins] = -0.3
+    mean, std = torch.from_numpy(mean).cuda(), torch.ones(members, 649, dtype=torch.float64, device='cuda')
+    ys = torch.zeros(members, 1, 656, dtype=torch.float16, device='cuda')
+    brf, alb, cost = new(members, 1, bins), new(members, 1), new(1)
+    obs, share = torch.zeros(1, bins, dtype=torch.float64, device='cuda'), torch.from_numpy(surrogate.bin_weights()).cuda()
+    assert L.mcw_brf_members(p(ys), 656, members, 1, p(mean), p(std), fl, p(brf), p(alb), st) == 0
+    assert L.mcw_brf_cost(p(ys), 656, members, 1, 1, p(mean), p(std), fl, p(obs), p(share), 0.0, 0.0, p(cost), st) == 0
+    # (bins' means may cancel to a thousandth of their terms, each rounded once here and there)
+    want = (surrogate.bin_weights() * brf.cpu().numpy()[:, 0].mean(0) ** 2).sum()
+    assert abs(cost.item() / want - 1) < 1e-10
