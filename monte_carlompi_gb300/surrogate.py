@@ -207,7 +207,7 @@ def backward_cached(torch, gy, w16, cache, need_dx=True):
     down the layers, whose epilogues leave the column sums of every 128 rows, then the four weight
     gradients in one launch, which also adds up the bias gradients: the operands are read where
     they lie, transposed by the tensor core."""
-    zs, acts = cache
+    zs, acts = cache[0], [_rows16(torch, a) for a in cache[1]]
     m = gy.shape[0]
     dev = gy.device
     blocks = (m + 127) // 128
@@ -219,10 +219,10 @@ def backward_cached(torch, gy, w16, cache, need_dx=True):
     for layer in (3, 2, 1):
         # G_prev[b, i] = (sum_o G[b, o] W[o, i]) * silu'(Z_prev[b, i])
         n_out, k_in = w16[layer].shape
-        g = g16[layer]
+        g, w = g16[layer], _rows16(torch, w16[layer])
         prev = torch.empty((m, k_in), dtype=torch.bfloat16, device=dev)
         q = _abi.GemmProblemC(m=m, n=k_in, k=n_out, groups=1, splits=1, epilogue=_abi.EPI_DSILU, a=g.data_ptr(),
-                              lda=g.shape[1], b=w16[layer].data_ptr(), ldb=k_in, trans_b=1,
+                              lda=g.shape[1], b=w.data_ptr(), ldb=w.shape[1], trans_b=1,
                               aux=zs[layer - 1].data_ptr(), ldaux=k_in, c=prev.data_ptr(), ldc=k_in,
                               colsum=sums[layer - 1].data_ptr(), ld_colsum=k_in)
         rc = L.mcw_mlp_gemm_batch(ctypes.byref(q), 1, st)

@@ -341,3 +341,31 @@ def test_fused_forward_rows_do_not_depend_on_the_batch(n):
                                          y.data_ptr(), 664, surrogate._stream(torch))
     torch.cuda.synchronize()
     assert rc == 0 and torch.equal(y[:, :649], part) and (y[:, 649:] == 3).all()
+
+
+@pytest.mark.parametrize('offset', [1, 4, 8])
+def test_gradients_with_weights_off_16_byte_boundaries(offset):
+    """Forward and backward pass with every bf16 weight matrix, the inputs and what is kept of the forward
+    pass a view `offset` elements into a larger buffer: the gradients of the same matrices on boundaries."""
+    g = torch.Generator().manual_seed(3)
+    dims = surrogate.DIMS
+    w16 = [(torch.randn(n, k, generator=g) / k ** 0.5).to(torch.bfloat16).cuda() for k, n in zip(dims[:-1], dims[1:])]
+    bs = [torch.randn(n, generator=g).cuda() for n in dims[1:]]
+    x16, gy = torch.randn(77, dims[0], generator=g).to(torch.bfloat16).cuda(), torch.randn(77, dims[-1], generator=g).cuda()
+
+    def off(t):
+        flat = torch.zeros(t.numel() + offset, dtype=t.dtype, device='cuda')
+        flat[offset:] = t.flatten()
+        return flat[offset:].view(t.shape)
+
+    def run(x, ws, put=lambda t: t):
+        y, cache = surrogate.forward_cached(torch, x, ws, bs)
+        dx, dws, dbs = surrogate.backward_cached(torch, gy, ws, [[put(t) for t in part] for part in cache])
+        return [y, dx, *dws, *dbs]
+    got, want = run(off(x16), [off(w) for w in w16], off), run(x16, w16)
+    for a, b in zip(got[:-4], want):
+        assert torch.equal(a, b)
+    # (pre-activations off 8-byte boundaries take single columns, whose bias sums run row by row: 77 FP32
+    # additions in another order)
+    for a, b in zip(got[-4:], want[-4:]):
+        assert (a - b).abs().max() <= 77 * 2.0 ** -24 * 77 ** 0.5 * b.abs().max()
