@@ -687,7 +687,9 @@ template <int TN>
 cudaError_t launch_n(int epi, const GemmBatch &b, bool ta, bool tb, unsigned grid, size_t smem, cudaStream_t s) {
     switch (epi) {
         case MCW_EPI_F32:
-            if (ta && tb && b.sub == 2) return launch<MCW_EPI_F32, true, true, TN, 2>(b, grid, smem, s);
+            if constexpr (TN == 32) {              // (tiles of 64 columns: more than an SM's, the rule in launch_batch)
+                if (ta && tb && b.sub == 2) return launch<MCW_EPI_F32, true, true, TN, 2>(b, grid, smem, s);
+            }
             if (ta) return tb ? launch<MCW_EPI_F32, true, true, TN>(b, grid, smem, s)
                               : launch<MCW_EPI_F32, true, false, TN>(b, grid, smem, s);
             return tb ? launch<MCW_EPI_F32, false, true, TN>(b, grid, smem, s)

@@ -434,7 +434,6 @@ class SurrogateMLP:
 # ------------------------------------------------------------------ training engine
 
 IN_PAD = 16        # layer-1 inputs padded to 16: one 16-byte TMA row, one MMA K step
-OUT_PITCH = 656    # 649 outputs rounded up to 8 (16-byte bf16 rows)
 
 
 def _align8(n):
