@@ -752,10 +752,11 @@ int forward(const float *x, int32_t m, const float *b1, const float *b2, const f
     // two, each with its share of the output blocks; the hidden layers are computed by all of them),
     // in the instance with the deeper weight ring.  300 rows of one network, f32: 29.2 us with
     // three CTAs, 15.7 with eighteen; 2,048 rows of five members 23.9, now 20.7; 16,384 of one 29.7,
-    // now 27.4 (one CTA an SM); from 152 tiles on two CTAs share an SM.
+    // now 27.4 (one CTA an SM); with more tiles than SMs (152) two CTAs share one.
     const int work = tiles * members;
-    const int share = work * 6 <= 152 ? 6 : (work * 3 <= 152 ? 3 : (work * 2 <= 152 ? 2 : 1));
-    const bool one = work * share <= 152;
+    const long long sms = sm_count(), w = work;
+    const int share = w * 6 <= sms ? 6 : (w * 3 <= sms ? 3 : (w * 2 <= sms ? 2 : 1));
+    const bool one = w * share <= sms;
     const dim3 grid((unsigned)work, (unsigned)share);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned char *wb = static_cast<const unsigned char *>(blob);

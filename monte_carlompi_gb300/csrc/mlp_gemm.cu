@@ -723,19 +723,20 @@ int launch_batch(const McwGemmProblem *q, int np, cudaStream_t stream) {
         const int c = ((q[i].k + TK - 1) / TK + q[i].splits - 1) / q[i].splits;
         chunks = c > chunks ? c : chunks;
     }
+    const int sms = sm_count();
     // 64 columns a tile when that leaves two tiles per SM: at 65,536 rows with tiles of 32 / 64
     // columns the SiLU' product of 649 takes 92 / 69 us, of 256 62 / 51 (bias + SiLU 256 x 256 53 / 36,
     // the 256 x 649 output 84 / 72)
-    const int tn = t64 >= 304 ? 64 : 32;
+    const int tn = t64 >= 2 * sms ? 64 : 32;
     // two stages when the launch fills the SMs several times over (four CTAs of an SM overlap each
     // other), else up to eight, or as many as the chunks; five of two chunks each for a transposed
     // product with an SM to a CTA and a long chain, where a stage's handover (120 ns beside 20 ns an
     // MMA) is what is left: the weight gradients of 65,536 rows, 1,024 chunks a tile, take
     // 464 / 317 / 246 / 201 us with 2 / 3 / 4 / 8 stages, 176 with 5 of two
     const long long ctas = tn == 64 ? t64 : t32;
-    const int stages = ctas > 304 ? 2 : (ctas > 152 ? 4 : kMaxStages);
+    const int stages = ctas > 2 * sms ? 2 : (ctas > sms ? 4 : kMaxStages);
     b.stages = stages > chunks ? chunks : stages;
-    b.sub = q[0].epilogue == MCW_EPI_F32 && ta && tb && ctas <= 152 && chunks >= 4 * kMaxStages ? 2 : 1;
+    b.sub = q[0].epilogue == MCW_EPI_F32 && ta && tb && ctas <= sms && chunks >= 4 * kMaxStages ? 2 : 1;
     if (b.sub == 2) b.stages = 5;
     long long cta = 0;
     for (int i = 0; i < np; ++i) {

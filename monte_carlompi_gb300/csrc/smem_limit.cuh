@@ -1,4 +1,4 @@
-// Dynamic shared memory past 48 KB.
+// What the current device has: dynamic shared memory past 48 KB, SMs.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -23,6 +23,15 @@ inline cudaError_t allow_smem(const void *fn, size_t bytes) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e == cudaSuccess) have = bytes;
     return e;
+}
+
+// SMs of the current device (a GB300's 152 where it does not say).
+inline int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        n < 1)
+        return 152;
+    return n;
 }
 
 }  // namespace mcw
