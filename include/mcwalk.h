@@ -43,8 +43,10 @@ extern "C" {
 /* where mcw_walk writes per-photon records */
 #define MCW_RECORDS_NONE 0
 #define MCW_RECORDS_HOST 1   /* host pointer; pinned host memory (mcw_host_alloc, cudaHostAlloc,
-                                cudaHostRegister) is written by the walk directly, other host
-                                memory receives a device -> host copy after it */
+                                cudaHostRegister), and 16-byte aligned pageable memory where the GPU
+                                walks the host's page tables, is written by the walk directly (FP32
+                                records in pageable memory up to 4 MB), other host memory receives a
+                                device -> host copy after it */
 #define MCW_RECORDS_DEVICE 2 /* device pointer owned by the caller */
 
 /* exit-direction histogram: 18 zenith bins of 5 deg x 36 azimuth bins of 10 deg */

@@ -461,7 +461,11 @@ WalkArgs walk_args(const mcw_ctx *ctx, const Plan &plan, DevBuf &cfgs, DevBuf &l
 }
 
 constexpr int32_t kDrainSpread = 512;
-// FP32 records in pageable memory up to this size are written by the walk, more are copied
+// FP32 records in pageable memory up to this size are written by the walk, more are copied: what a photon
+// walks decides which is faster, and a call does not know it beforehand.  Calls with the copy / written by
+// the walk, us: walks of a few events 131,072 records 97 / 85, 200,000 114 / 108, 400,000 154 / 172,
+// 800,000 245 / 298; thin layers with soot 131,072 234 / 198, 800,000 711 / 564; deep snow 131,072 1,033 /
+// 1,009, 800,000 3,597 / 3,428.  Up to 4 MB (131,072) no walk loses by it.
 constexpr size_t kDirectBytes = 4u << 20;
 
 // Attach the drain queue (one slot per thread of the walk grid) when handover is on.
@@ -883,8 +887,7 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
         } else if ((mode != MCW_MODE_F32 || (size_t)plan.total * rec_size <= kDirectBytes) &&
                    reach_pageable(ctx, records, (size_t)plan.total * rec_size, 16, true)) {
             // pageable memory, where the GPU walks the host's page tables: written the same way, but
-            // for many records of the fastest walk (a call of 100,003 FP32 records 222 -> 197 us,
-            // 10,000 126 -> 118; 737,905 of short walks 262 by the copy, 318 without)
+            // for many FP32 records (kDirectBytes)
             dev_records = records;
             direct = true;
         } else {
