@@ -975,10 +975,9 @@ int mcw_walk(mcw_ctx *ctx, const mcw_config *cfgs, int32_t n_cfg, uint64_t seed,
         ra.budget_ns = (unsigned long long)(ctx->budget_s * 1e9);
         ra.seed = seed;
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev0, st));
-        CUDA_TRY(ctx, launch_walk_replay(ra, ctx->sm_count, st));
+        CUDA_TRY(ctx, launch_walk_replay(ra, ctx->sm_count, st, &shape.grid));
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev1, st));
         shape.block = 128;
-        shape.grid = (int)((plan.total + 127) / 128);
     }
     if (records_where == MCW_RECORDS_HOST && plan.total > 0 && !direct)
         CUDA_TRY(ctx, cudaMemcpyAsync(records, dev_records, (size_t)plan.total * rec_size, cudaMemcpyDeviceToHost, st));

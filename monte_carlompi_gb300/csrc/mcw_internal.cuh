@@ -236,7 +236,8 @@ constexpr int kDrainSlot = 6;
 // Launches the walk and, when a.drain_from > 0, the drain kernel after it
 // (sm_count SMs; a.drain must then hold grid * block slots).
 cudaError_t launch_walk_f32(const WalkArgs &a, bool impurity, int grid, int block, int sm_count, cudaStream_t s);
-cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s);
+// blocks: how many (of 128 threads) it launched.
+cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s, int *blocks);
 // The FP32 polarised walk (a.phase set, a.records holding mcw_record32p).  only: the one phase table
 // that every config uses, or null.
 cudaError_t launch_walk_pol32(const WalkArgs &a, const DevPhase32 *only, int sm_count, cudaStream_t s);

@@ -948,7 +948,8 @@ __global__ void __launch_bounds__(128, 3) walk_replay_pol_kernel(const ReplayArg
 
 }  // namespace
 
-cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s) {
+cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s, int *blocks) {
+    *blocks = 0;
     if (a.total <= 0) return cudaSuccess;
     if (a.pol) {
         // three blocks an SM (140 registers), and as many lanes a photon as let all photons walk at
@@ -958,17 +959,19 @@ cudaError_t launch_walk_replay(const ReplayArgs &a, int sm_count, cudaStream_t s
         while (glog > 0 && warps << (5 - glog) < a.total) --glog;
         const int64_t each = 4 << (5 - glog);                         // photons a block at a time
         const int64_t grid = std::min<int64_t>(3 * (int64_t)std::max(1, sm_count), (a.total + each - 1) / each);
+        *blocks = (int)grid;
         walk_replay_pol_kernel<<<(unsigned)grid, 128, 0, s>>>(a, glog);
         return cudaGetLastError();
     }
     // four blocks an SM (126 registers), a warp of each part on each of its four FP64 pipes; few
     // photons are spread over all of them
     ReplayArgs b = a;
-    const int64_t blocks = std::min<int64_t>(4 * (int64_t)std::max(1, sm_count), a.total);
-    const int64_t each = (a.total + blocks - 1) / blocks;
+    const int64_t grid = std::min<int64_t>(4 * (int64_t)std::max(1, sm_count), a.total);
+    const int64_t each = (a.total + grid - 1) / grid;
     b.slots = (int32_t)std::min<int64_t>(kSlots, each);
     b.claim = (int32_t)std::min<int64_t>(32, each);
-    walk_replay_kernel<<<(unsigned)blocks, 128, 0, s>>>(b);
+    *blocks = (int)grid;
+    walk_replay_kernel<<<(unsigned)grid, 128, 0, s>>>(b);
     return cudaGetLastError();
 }
 

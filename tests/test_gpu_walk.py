@@ -962,3 +962,20 @@ def test_replay_stopped_by_its_budget_leaves_every_record(walker, mode, n):
     assert np.isfinite(left['theta_n']).all() and (left['flags'] <= 1).all()
     again = walker.walk([cfg], 4, mode=mode).records
     assert again.tobytes() == whole.tobytes()
+
+
+@pytest.mark.parametrize('mode,n,per_sm,each', [('replay64', 5, 4, 1), ('replay64', 20000, 4, 1), ('pol64', 5, 3, 4),
+                                                ('pol64', 100000, 3, 128)])
+def test_replay_stats_tell_the_launch(walker, mode, n, per_sm, each):
+    """The blocks that a replay launched: as many as have photons (of `each` a block at this count), up
+    to the SMs' share."""
+    torch = pytest.importorskip('torch')
+    g = load_golden('pol' if mode == 'pol64' else 'thin')
+    ice, imp = golden_tables(g)
+    walker.set_tables([ice], imp)
+    if mode == 'pol64':
+        walker.set_phase_matrices([golden_phase(g)])
+    cfg = dataclasses.replace(golden_config(g), n_photon=n, tau_tot=1.0)
+    stats = walker.walk([cfg], 1, mode=mode, records=None).stats
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert stats['block_size'] == 128 and stats['grid'] == min(per_sm * sms, -(-n // each))
