@@ -13,7 +13,7 @@
 // Jacobian 46 now (259 and 44 with exponentials of 1.24 ulp, the floors taken off a sum and means by the
 // reciprocal, which lost digits).  One retrieval of 128 observations with five members (16-point grid, six
 // iterations, spreads): 92 ms on the host's cores and elementwise tensor kernels; 3.3 ms with these kernels and the steps and the encoding of log r on the host, a
-// wait for the device and two copies an iteration; 1.6 ms with the steps here too and the network
+// wait for the device and two copies an iteration; 1.55 ms with the steps here too and the network
 // laid out while the grid's costs are worked out.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -99,7 +99,7 @@ __device__ __forceinline__ double exp_by_table(double x, const double2 *tab) {
     const double y = T.x + fma(T.x, fma(q, r * r, r), T.y);
     return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
 }
-// The table in shared memory (the caller's barrier follows).
+// The table in shared memory (the caller's barrier follows); a row's one albedo takes it from kExp2.
 __device__ __forceinline__ void load_exp2(double2 *tab) {
     if (threadIdx.x < 64) tab[threadIdx.x] = kExp2[threadIdx.x];
 }
@@ -113,7 +113,7 @@ __device__ __forceinline__ double bin_brf(const __half *row, int b, const double
 }
 
 __device__ __forceinline__ double row_albedo(const __half *row, const double *std, const double *mean) {
-    return exp(unscaled((double)__half2float(row[kBins]), std[kBins], mean[kBins]));
+    return exp_by_table(unscaled((double)__half2float(row[kBins]), std[kBins], mean[kBins]), kExp2);
 }
 
 // t / members, correctly rounded, share = 1 / members: the residual's correction (Markstein, IBM J. Res.
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(kThreads) jacobian_kernel(const float *y, cons
     for (int m = threadIdx.x; m < members; m += kThreads) {
         const size_t at = ((size_t)m * n + r) * pitch + kBins;
         const double sd = std[(size_t)m * (kBins + 1) + kBins];
-        const double a = exp(unscaled((double)y[at], sd, mean[(size_t)m * (kBins + 1) + kBins]));
+        const double a = exp_by_table(unscaled((double)y[at], sd, mean[(size_t)m * (kBins + 1) + kBins]), kExp2);
         sh[2 * m] = a;
         sh[2 * m + 1] = a * ((double)ydot[at] * sd);
     }

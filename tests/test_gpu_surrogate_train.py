@@ -365,3 +365,21 @@ def test_means_over_the_members_lose_nothing(members):
     # (bins' means may cancel to a thousandth of their terms, each rounded once here and there)
     want = (surrogate.bin_weights() * brf.cpu().numpy()[:, 0].mean(0) ** 2).sum()
     assert abs(cost.item() / want - 1) < 1e-10
+
+
+def test_albedos_to_half_an_ulp():
+    """The members' albedos, as close to the exponential as the bins' (test_members_exponential_to_half_an_ulp)."""
+    from monte_carlompi_gb300 import _abi
+    n, bins = 20000, surrogate.N_BRF
+    x = np.random.default_rng(9).uniform(-9.0, 0.0, n)
+    mean = torch.zeros(n, 649, dtype=torch.float64, device='cuda')
+    mean[:, bins] = torch.from_numpy(x).cuda()
+    ys, std = torch.zeros(4000, 1, 656, dtype=torch.float16, device='cuda'), torch.ones(4000, 649, dtype=torch.float64, device='cuda')
+    alb, brf = torch.empty(n, dtype=torch.float64, device='cuda'), torch.empty((4000, bins), dtype=torch.float64, device='cuda')
+    p = lambda t: t.data_ptr()  # noqa: E731
+    for lo in range(0, n, 4000):
+        assert _abi.load().mcw_brf_members(p(ys), 656, 4000, 1, p(mean[lo:]), p(std), 0.0, p(brf), p(alb[lo:]),
+                                           surrogate._stream(torch)) == 0
+    got, want = alb.cpu().numpy().astype(np.longdouble), np.exp(x.astype(np.longdouble))
+    ulp = np.ldexp(np.longdouble(1), np.frexp(want)[1] - 53)
+    assert (np.abs(got - want) / ulp).max() <= 0.55
