@@ -657,7 +657,7 @@ __device__ __forceinline__ void mlp_fused_body(const float *x, int m, const floa
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n");
-                // this member's output rows (plain stores; the tensor map takes the member as a coordinate)
+                // this member's output rows
                 const int member = kEnsemble ? (int)blockIdx.x / tiles : 0;
                 const size_t yoff = kEnsemble ? (size_t)member * (size_t)m * (size_t)ldy : 0;
                 if (kHalf && wide)
