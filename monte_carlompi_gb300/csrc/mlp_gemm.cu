@@ -824,9 +824,10 @@ int mcw_mlp_gemm_batch(const McwGemmProblem *q, int32_t n, void *stream) {
     for (int i = 0; i < n; ++i) {
         const McwGemmProblem &s = q[i];
         if (s.m < 0 || s.n < 0 || s.k <= 0 || s.groups < 1 || s.splits < 1 || !s.a || !s.b || !s.c) return MCW_MLP_ERR_ARG;
+        if (s.m == 0 || s.n == 0) continue;                   // nothing to do, whatever the rest
         if (s.epilogue < MCW_EPI_F32 || s.epilogue > MCW_EPI_LOSS) return MCW_MLP_ERR_ARG;
-        if (s.epilogue != q[0].epilogue || (s.trans_a != 0) != (q[0].trans_a != 0) ||
-            (s.trans_b != 0) != (q[0].trans_b != 0))
+        if (np > 0 && (s.epilogue != kept[0].epilogue || (s.trans_a != 0) != (kept[0].trans_a != 0) ||
+                       (s.trans_b != 0) != (kept[0].trans_b != 0)))
             return MCW_MLP_ERR_ARG;
         if (!has_kernel(s.epilogue, s.trans_a != 0, s.trans_b != 0)) return MCW_MLP_ERR_ARG;
         if (s.splits > 1 && s.epilogue != MCW_EPI_F32) return MCW_MLP_ERR_ARG;
@@ -840,14 +841,14 @@ int mcw_mlp_gemm_batch(const McwGemmProblem *q, int32_t n, void *stream) {
         const int per = (chunks + s.splits - 1) / s.splits;
         if (s.splits > 1 && (chunks + per - 1) / per != s.splits) return MCW_MLP_ERR_ARG;   // the caller's partial layout
         if (!operands_ok(s)) return MCW_MLP_ERR_ARG;
-        if (s.m > 0 && s.n > 0) kept[np++] = s;
+        kept[np++] = s;
     }
     return np ? launch_batch(kept, np, static_cast<cudaStream_t>(stream)) : 0;
 }
 
 int mcw_mlp_gemm_grouped(const McwGemmGrouped *q, void *stream) {
     if (!q) return MCW_MLP_ERR_ARG;
-    if (q->epilogue > MCW_EPI_DSILU) return MCW_MLP_ERR_ARG;
+    if (q->epilogue > MCW_EPI_DSILU && q->m != 0 && q->n != 0) return MCW_MLP_ERR_ARG;
     McwGemmProblem s;
     memset(&s, 0, sizeof(s));
     s.m = q->m, s.n = q->n, s.k = q->k, s.groups = q->groups, s.splits = q->splits, s.epilogue = q->epilogue;

@@ -486,3 +486,20 @@ def test_gather_and_grouped_loss(G, B, rows, n_out):
     assert torch.allclose(loss.double(), (w.double() * d * d).mean((1, 2)), rtol=1e-5)
     assert torch.allclose(g32.double(), 2 * w.double() * d / (B * n_out), rtol=1e-6, atol=0)
     assert torch.equal(g16, g32.to(torch.bfloat16)) and torch.equal(g16t, g16.transpose(1, 2))
+
+
+def test_empty_products_are_nothing():
+    """A grouped product without rows or columns is nothing to do, whatever its operands' alignment and
+    pitches, alone and among others of a launch."""
+    a, b = torch.zeros(1, 128, 72, dtype=torch.bfloat16, device='cuda'), torch.ones(1, 64, 72, dtype=torch.bfloat16, device='cuda')
+    c = torch.full((1, 128, 64), 7.0, device='cuda')
+    for m, n, off, epi in ((0, 64, 0, _abi.EPI_F32), (128, 0, 2, _abi.EPI_F32), (0, 64, 2, _abi.EPI_BIAS_SILU)):
+        p = _abi.GemmGroupedC(m, n, 72, 1, 1, epi, a.data_ptr() + off, 71, 0, b.data_ptr(), 72, 0, None, 0, None, 0, 0,
+                              c.data_ptr(), 64, 0, 0, None, 0, 0, None, 0, 0)
+        assert _abi.load().mcw_mlp_gemm_grouped(ctypes.byref(p), _stream()) == 0
+    torch.cuda.synchronize()
+    assert (c == 7).all()
+    two = (_abi.GemmProblemC * 2)(_problem(_abi.EPI_LOSS, 0, 64, 72, a, b, c, 0, 0), _problem(_abi.EPI_F32, 128, 64, 72, a, b, c, 0, 0))
+    assert _abi.load().mcw_mlp_gemm_batch(two, 2, _stream()) == 0
+    torch.cuda.synchronize()
+    assert (c == 0).all()
