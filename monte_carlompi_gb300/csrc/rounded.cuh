@@ -73,15 +73,23 @@ __device__ __forceinline__ bool moderate(double x) {
     return h >= 0x30000000 && h < 0x43400000;
 }
 
+// Whether g = sqrt_res(x) and q = quotient_res(a, b, rcp_res(b)) are sqrt(x) and a / b, of any x, a, b.
+__device__ __forceinline__ bool sqrt_sure(double g, double x) {
+    return (to_bits(x) >> 63) == 0 & moderate(x) & sqrt_certain(g, x);
+}
+__device__ __forceinline__ bool quotient_sure(double q, double a, double b) {
+    return moderate(b) & quotient_certain(q, a, b);
+}
+
 // sqrt(x) and a / b, rb = rcp_res(b); any x, a, b.
 __device__ __forceinline__ double sqrt_rn(double x) {
     double h;
     const double g = sqrt_res(x, h);
-    return !(to_bits(x) >> 63) && moderate(x) && sqrt_certain(g, x) ? g : sqrt(x);
+    return sqrt_sure(g, x) ? g : sqrt(x);
 }
 __device__ __forceinline__ double quotient_rn(double a, double b, double rb) {
     const double q = quotient_res(a, b, rb);
-    return moderate(b) && quotient_certain(q, a, b) ? q : a / b;
+    return quotient_sure(q, a, b) ? q : a / b;
 }
 
 // 1 / d, d >= 1 (or NaN): a Newton step on the hardware's reciprocal, by the same author, which alone

@@ -27,10 +27,11 @@
 //    three each (rounded.cuh).
 // The draws assume that a step does nothing but scatter: a photon that ends, is reflected or is
 // replaced sits out the two rounds under way.  Every value is the one-thread walk's, in
-// its order of operations, every square root and quotient correctly rounded: the fourth warp looks
+// its order of operations, every square root and quotient correctly rounded: the third warp looks
 // at the residuals of all steps of a round side by side, and a step whose rounding they leave open (some
 // five in a million) is walked again with sqrt() and /, its photon's draws ahead dropped as at an
-// event.  10,000 photons of the reference's default run 18.7 ms without the look, 19.3 with it.
+// event.  10,000 photons of the reference's default run 14.4 to 16.3 ms without the look, 14.6 to 15.8
+// with it; 100,000 of a thin layer, which fill the FP64 pipe, 1.00 and 1.09.
 // 10,000 photons of the reference's default run: 193.7 ms on one thread each; 30.5 ms (0.94 us an
 // event of the longest walk) with one warp drawing and one walking, four lanes a photon, each
 // FP64 instruction serving all four through selects and shuffles; 16.0 ms now (0.47 us, 970
@@ -38,6 +39,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "mcw_internal.cuh"
 #include "rounded.cuh"
@@ -145,6 +147,7 @@ struct Ahead {
     double ct[32], st[32], cp[32], sp[32], dtau[32], inc[32];
     uint32_t fl[32];                         // 1 absorbed here, 2 by ice
     int32_t n, S, pole;                      // pole: a step about the vertical among them
+    uint32_t uncertain;                      // XY: steps to be walked again (uncertain_steps)
     int32_t slot[kSlots], steps[kSlots], lamb[kSlots], first[kSlots], shift[kSlots];
     uint32_t gen[kSlots];                    // the slot's count of events that the draws assume
     uint64_t k0[kSlots];                     // the photon's stream before the steps
@@ -197,9 +200,6 @@ __device__ __forceinline__ bool is_nan(double x) { return (to_bits(x) & 0x7fffff
 __device__ __forceinline__ bool is_unit(double x) { return (to_bits(x) & 0x7fffffffffffffffull) == 0x3ff0000000000000ull; }
 
 __device__ __forceinline__ double shfl_d(double x, int src) { return __shfl_sync(0xffffffffu, x, src); }
-
-// sqrt(1 - ct^2) as the reference writes it (ct = +-1: 0; past it, by rounding: NaN).
-__device__ __forceinline__ double sin_from(double ct) { return sqrt_rn(1 - ct * ct); }
 
 // The end of a step (:1390-1466) at depth z (z_prev before it): the path's exit correction, the
 // bottom's reflectance draw (uniform *k, taken when drawn), the end condition (0: walking on, or
@@ -340,26 +340,32 @@ __device__ void draw_ahead(const ReplayArgs &a, ReplayBlock &B, Ahead &next, int
         const double u0 = u01_bits(word(x0, odd)), u1 = u01_bits(odd ? word(x1, false) : word(x0, true)),
                      u2 = u01_bits(word(x1, odd)), u3 = u01_bits(odd ? word(x2, false) : word(x1, true)),
                      u4 = u01_bits(word(x2, odd));
-        double ct;
-        if (t == 0 && lamb) {
-            ct = ct_l;
-        } else if (s.flags & kIso) {                                  // Henyey_Greenstein2 (:790-800)
-            ct = 1 - 2 * u0;
-        } else {
-            const double den = s.hg_c + s.hg_d * u0;
-            const double q = quotient_rn(s.hg_b, den, rcp_res(den));
-            ct = s.hg_e * (s.hg_a - q * q);
-        }
         double sp, cp;
         sincos(u1 * kTwoPi, &sp, &cp);
         const double dtau = -log(u2);
+        // the step's cosine, sine (sqrt(1 - ct^2) as the reference writes it) and path, their roundings
+        // looked at together
+        const bool given = t == 0 && lamb, iso = (s.flags & kIso) != 0;
+        const double den = s.hg_c + s.hg_d * u0, q = quotient_res(s.hg_b, den, rcp_res(den));
+        double ct = given ? ct_l : (iso ? 1 - 2 * u0 : s.hg_e * (s.hg_a - q * q));   // Henyey_Greenstein2 (:790-800)
+        double h, inc = quotient_res(dtau, s.ext, s.rext);            // :1372
+        const double x = 1 - ct * ct;
+        double st = sqrt_res(x, h);
+        if (!((given | iso | quotient_sure(q, s.hg_b, den)) & sqrt_sure(st, x) & quotient_sure(inc, dtau, s.ext))) {
+            if (!(given | iso)) {
+                const double e = s.hg_b / den;
+                ct = s.hg_e * (s.hg_a - e * e);
+            }
+            st = sqrt(1 - ct * ct);
+            inc = dtau / s.ext;
+        }
         const bool ice = u4 > s.p_imp;                                // :1375-1383
         next.ct[lane] = ct;
-        next.st[lane] = sin_from(ct);
+        next.st[lane] = st;
         next.cp[lane] = cp;
         next.sp[lane] = sp;
         next.dtau[lane] = dtau;
-        next.inc[lane] = quotient_rn(dtau, s.ext, s.rext);            // :1372
+        next.inc[lane] = inc;
         next.fl[lane] = (u3 >= (ice ? s.ssa_ice : s.ssa_imp) ? 1u : 0u) | (ice ? 2u : 0u);
         if (t == 0) {
             next.slot[rank] = si;
@@ -461,6 +467,19 @@ __device__ __forceinline__ void xy_chain(Ahead &A, double va, double vb, const i
     }
 }
 
+// The steps of A, a bit each, whose square root or quotients the chains may have rounded otherwise than
+// sqrt() and / do (rounded.cuh).  A lane a step: six FP64 instructions for all of them, where a test in
+// the chains would take as many a step; in XY's warp, whose chain is shorter than Z's (between the
+// rounds, where the other warps wait for the states' commit, 14.4 -> 16.3 ms of 10,000 photons).
+__device__ unsigned uncertain_steps(const Ahead &A, int lane) {
+    const double mz = A.mzb[lane], sq = A.sq[lane];
+    // (about the vertical there is neither; past it, by rounding, all is NaN either way)
+    const bool sure = is_unit(mz) || is_nan(sq) ||
+                      (sqrt_certain(sq, 1.0 - mz * mz) && quotient_certain(A.quox[lane], A.numx[lane], sq) &&
+                       quotient_certain(A.quoy[lane], A.numy[lane], sq));
+    return __ballot_sync(0xffffffffu, !sure);
+}
+
 __device__ void walk_xy(ReplayBlock &B, Ahead &A, int lane) {
     const int rk = lane >> 1;
     const bool isX = !(lane & 1), held = holds(B, A, rk);
@@ -471,6 +490,9 @@ __device__ void walk_xy(ReplayBlock &B, Ahead &A, int lane) {
     const double va = lamb ? 0.0 : (isX ? slot.mux : slot.muy), vb = lamb ? 0.0 : (isX ? slot.muy : slot.mux);
     if (A.pole) xy_chain<true>(A, va, vb, base, steps, S, isX, lane);
     else xy_chain<false>(A, va, vb, base, steps, S, isX, lane);
+    __syncwarp();
+    const unsigned uncertain = uncertain_steps(A, lane);
+    if (lane == 0) A.uncertain = uncertain;
 }
 
 // M: depth and path over the same steps, two lanes a photon, and the first step with an end
@@ -509,18 +531,6 @@ __device__ int walk_m(ReplayBlock &B, Ahead &A, int lane) {
     return event ? -done : done;
 }
 
-// The steps of A, a bit each, whose square root or quotients the chains may have rounded otherwise than
-// sqrt() and / do (rounded.cuh).  A lane a step: six FP64 instructions for all of them, where a test in
-// the chains would take as many a step.
-__device__ unsigned uncertain_steps(const Ahead &A, int lane) {
-    const double mz = A.mzb[lane], sq = A.sq[lane];
-    // (about the vertical there is neither; past it, by rounding, all is NaN either way)
-    const bool sure = is_unit(mz) || is_nan(sq) ||
-                      (sqrt_certain(sq, 1.0 - mz * mz) && quotient_certain(A.quox[lane], A.numx[lane], sq) &&
-                       quotient_certain(A.quoy[lane], A.numy[lane], sq));
-    return __ballot_sync(0xffffffffu, !sure);
-}
-
 // Step e, the `t`-th of its photon's, again with sqrt() and /, from the state before it.
 __device__ __noinline__ void step_again(const Slot &slot, Ahead &A, int e, int t) {
     const double mux = t > 0 ? A.x[e - 1] : slot.mux, muy = t > 0 ? A.y[e - 1] : slot.muy, muz = A.mzb[e];
@@ -534,14 +544,14 @@ __device__ __noinline__ void step_again(const Slot &slot, Ahead &A, int e, int t
 }
 
 // The photons' states after the steps that XY and M walked: lane `rank` its photon's.  `walked`:
-// walk_m's result for it; `uncertain`: the steps to be walked again, where the photon's draws ahead
-// end as at an event.  Returns its end condition (-1: out of its stream).
-__device__ int commit(const ReplayArgs &a, ReplayBlock &B, Ahead &A, int rank, int walked, unsigned uncertain) {
+// walk_m's result for it.  At the first uncertain step, walked again, the photon's draws ahead end as
+// at an event.  Returns its end condition (-1: out of its stream).
+__device__ int commit(const ReplayArgs &a, ReplayBlock &B, Ahead &A, int rank, int walked) {
     bool event = walked < 0;
     int done = event ? -walked : walked;
     const int si = A.slot[rank];
     Slot &slot = B.slots[si];
-    const unsigned mine = (uncertain >> (rank * A.S)) & (0xffffffffu >> (32 - done));
+    const unsigned mine = (A.uncertain >> (rank * A.S)) & (0xffffffffu >> (32 - done));
     if (mine) {
         event = true;
         done = __ffs(mine);
@@ -620,8 +630,7 @@ __global__ void __launch_bounds__(128, 4) walk_replay_kernel(const ReplayArgs a)
             const bool mine = lane < kSlots && holds(B, now, lane & (kSlots - 1));
             const int w = __shfl_sync(0xffffffffu, walked, (2 * lane) & 31);
             const int si = mine ? now.slot[lane] : 0;
-            const unsigned uncertain = uncertain_steps(now, lane);
-            const int cond = mine ? commit(a, B, now, lane, w, uncertain) : 0;
+            const int cond = mine ? commit(a, B, now, lane, w) : 0;
             __syncwarp();
             // ---- finished photons leave their slots
             if (__any_sync(0xffffffffu, cond != 0)) {
@@ -695,13 +704,34 @@ __device__ __forceinline__ int64_t order_of(double x) {
     return b >= 0 ? b : ((int64_t)0x8000000000000000ull - b);
 }
 
+// sqrt(x) and a / b (rb: 1 / b nearly): by the corrections, `sure` kept where they are certain, or kExact
+// by CUDA's.  A test of a result costs its step the 110 to 290 cycles to the integer side; so what goes
+// into one decision is worked out by the corrections, looked at once, late, and, when not sure, worked
+// out again exactly.
+template <bool kExact>
+__device__ __forceinline__ double root(double x, bool &sure) {
+    if (kExact) return sqrt(x);
+    double h;
+    const double g = sqrt_res(x, h);
+    sure = sure & sqrt_sure(g, x);
+    return g;
+}
+template <bool kExact>
+__device__ __forceinline__ double quotient(double a, double b, double rb, bool &sure) {
+    if (kExact) return a / b;
+    const double q = quotient_res(a, b, rb);
+    sure = sure & quotient_sure(q, a, b);
+    return q;
+}
+
 // scipy interp1d (linear) on an ascending grid: searchsorted (left) clipped to [1, n - 1], then the
 // two-term form of interp1d._call_linear: the upper end's index and both weights.
 struct Segment {
     int k;
     double lo, hi;
 };
-__device__ __forceinline__ Segment segment_of(const DevPhase &ph, int e, double xn) {
+template <bool kExact>
+__device__ __forceinline__ Segment segment_of(const DevPhase &ph, int e, double xn, bool &sure) {
     const double *x = ph.cos_asc[e];
     const int n = ph.n_angle[e];
     const int64_t key = order_of(xn);
@@ -713,9 +743,9 @@ __device__ __forceinline__ Segment segment_of(const DevPhase &ph, int e, double 
     Segment s;
     s.k = lo < 1 ? 1 : (lo > n - 1 ? n - 1 : lo);
     const double xl = __ldg(x + s.k - 1), xh = __ldg(x + s.k), w = xh - xl;
-    const double rw = rcp_res(w);
-    s.hi = quotient_rn(xn - xl, w, rw);
-    s.lo = quotient_rn(xh - xn, w, rw);
+    const double rw = kExact ? 0.0 : rcp_res(w);
+    s.hi = quotient<kExact>(xn - xl, w, rw, sure);
+    s.lo = quotient<kExact>(xh - xn, w, rw, sure);
     return s;
 }
 __device__ __forceinline__ double element(const DevPhase &ph, int e, int row, const Segment &s) {
@@ -767,13 +797,89 @@ __device__ __forceinline__ bool pol_candidate(const DevPhase &ph, const Slot &s,
                     : -u1 * (ph.cos_cutoff - ph.cos_min) + ph.cos_cutoff;
     two_phi = 2 * (u2 * kTwoPi);
     const double r3 = 1.000001 * u3 * (one ? v.max1 : v.max2);        // :976-1001
-    const Segment g0 = segment_of(ph, 0, cos_theta);
-    const Segment g1 = ph.shared_grid ? g0 : segment_of(ph, 1, cos_theta);
-    const double S11 = element(ph, 0, s.row, g0), S12 = element(ph, 1, s.row, g1);
     double sp, cp;
     sincos(two_phi, &sp, &cp);
-    const double pf = st[0] * S11 + S12 * (st[1] * cp + st[2] * sp);
+    const double turn = st[1] * cp + st[2] * sp;
+    bool sure = true;
+    auto weight = [&](auto exact) {
+        const Segment g0 = segment_of<decltype(exact)::value>(ph, 0, cos_theta, sure);
+        const Segment g1 = ph.shared_grid ? g0 : segment_of<decltype(exact)::value>(ph, 1, cos_theta, sure);
+        return st[0] * element(ph, 0, s.row, g0) + element(ph, 1, s.row, g1) * turn;
+    };
+    double pf = weight(std::false_type{});
+    if (!sure) pf = weight(std::true_type{});
     return !(r3 > pf);
+}
+
+// Where a step of scattering cosine ct and azimuth phi takes a photon's direction and Stokes vector
+// (:1251-1342), and its path increment.
+struct PolMove {
+    double nx, ny, nz, st[4], inc;
+    bool sure;
+};
+template <bool kExact>
+__device__ __forceinline__ PolMove pol_move(const DevPhase &ph, int row, double mux, double muy, double muz, double ct,
+                                            double phi, double s0, double s1, double s2, double s3, bool reflected,
+                                            double dtau, double ext, double rext) {
+    PolMove m;
+    bool sure = true;
+    const double sint = root<kExact>(1 - ct * ct, sure);              // :1251-1253
+    double sinphi, cosphi;
+    sincos(phi, &sinphi, &cosphi);
+    if (is_unit(muz)) {                                               // :1262-1269
+        const bool up = !(to_bits(muz) >> 63);
+        m.nx = sint * cosphi;
+        m.ny = up ? sint * sinphi : -sint * sinphi;
+        m.nz = up ? ct : -ct;
+    } else {                                                          // :1270-1281
+        const double sq = root<kExact>(1 - muz * muz, sure), rq = kExact ? 0.0 : rcp_res(sq);
+        m.nx = quotient<kExact>(sint * (mux * muz * cosphi - muy * sinphi), sq, rq, sure) + mux * ct;
+        m.ny = quotient<kExact>(sint * (muy * muz * cosphi + mux * sinphi), sq, rq, sure) + muy * ct;
+        m.nz = -sq * sint * cosphi + muz * ct;
+    }
+    m.inc = quotient<kExact>(dtau, ext, rext, sure);                  // :1372
+    m.st[0] = 1, m.st[1] = m.st[2] = m.st[3] = 0;
+    if (!reflected) {                                                 // :1287-1342
+        const double phi_sca = acos(cosphi);
+        const double st[4] = {s0, s1, s2, s3};
+        double sp[4], sc[4], sm[4], P[6];
+        rotate_stokes(phi_sca, st, sp);
+        const Segment g = segment_of<kExact>(ph, 0, ct, sure);
+#pragma unroll
+        for (int e = 0; e < 6; ++e)
+            P[e] = element(ph, e, row, e == 0 || ph.shared_grid ? g : segment_of<kExact>(ph, e, ct, sure));
+        const double P11 = P[0], P12 = P[1], P22 = P[2], P33 = P[3], P43 = P[4], P44 = P[5];
+        sc[0] = sp[0] * P11 + sp[1] * P12;
+        sc[1] = sp[0] * P12 + sp[1] * P22;
+        sc[2] = sp[2] * P33 - sp[3] * P43;
+        sc[3] = sp[2] * P43 + sp[3] * P44;
+        // (by the corrections den is 0 or NaN only where it is not sure)
+        const double den = root<kExact>((1 - ct * ct) * (1 - m.nz * m.nz), sure), d = phi_sca >= kPi ? den : -den;
+        const double num = m.nz * ct - muz;
+        double cos_i = kExact && den == 0 ? 0 : quotient<kExact>(num, d, kExact ? 0.0 : rcp_res(d), sure);
+        if (cos_i < -1) cos_i = -1;
+        else if (cos_i > 1) cos_i = 1;
+        rotate_stokes(-acos(cos_i), sc, sm);
+        const double ri = kExact ? 0.0 : rcp_res(sm[0]);
+        if (kExact) m.st[0] = sm[0] / sm[0];
+        else sure = sure & moderate(sm[0]);
+#pragma unroll
+        for (int k = 1; k < 4; ++k) {
+            // (the scattering after a reflection leaves V at 0, of either sign)
+            const bool zero = !kExact && to_bits(sm[k]) << 1 == 0;
+            bool fine = true;
+            m.st[k] = quotient<kExact>(sm[k], sm[0], ri, fine);
+            if (zero) m.st[k] = sm[k] * ri;
+            sure = sure & (zero | fine);
+        }
+    }
+    m.sure = sure;
+    return m;
+}
+__device__ __noinline__ PolMove pol_move_exact(const DevPhase &ph, int row, double mux, double muy, double muz, double ct,
+                                               double phi, double s0, double s1, double s2, double s3, bool reflected,
+                                               double dtau, double ext) {
+    return pol_move<true>(ph, row, mux, muy, muz, ct, phi, s0, s1, s2, s3, reflected, dtau, ext, 0.0);
 }
 
 // A step of photon s past its first with its scattering angles (:1227-1466); returns its end
@@ -797,59 +903,19 @@ __device__ int pol_step(const DevPhase &ph, Slot &s, uint64_t seed, double st[4]
             if (r1 < 2 * sn * ct || tries >= 131072) break;           // no stream needs as many
         }
     }
-    const double sint = sin_from(ct);                                 // :1251-1253
-    const double phi = two_phi / 2.;
-    double sinphi, cosphi;
-    sincos(phi, &sinphi, &cosphi);
-    double nx, ny, nz;
-    if (is_unit(muz)) {                                               // :1262-1269
-        const bool up = !(to_bits(muz) >> 63);
-        nx = sint * cosphi;
-        ny = up ? sint * sinphi : -sint * sinphi;
-        nz = up ? ct : -ct;
-    } else {                                                          // :1270-1281
-        const double sq = sqrt_rn(1 - muz * muz), rq = rcp_res(sq);
-        const double tx = sint * (mux * muz * cosphi - muy * sinphi), ty = sint * (muy * muz * cosphi + mux * sinphi);
-        nx = quotient_rn(tx, sq, rq) + mux * ct;
-        ny = quotient_rn(ty, sq, rq) + muy * ct;
-        nz = -sq * sint * cosphi + muz * ct;
-    }
-    if (reflected) {                                                  // :1283-1285
-        st[0] = 1; st[1] = 0; st[2] = 0; st[3] = 0;
-    } else {                                                          // :1287-1342
-        const double phi_sca = acos(cosphi);
-        double sp[4], sc[4], sm[4], P[6];
-        rotate_stokes(phi_sca, st, sp);
-        const Segment g = segment_of(ph, 0, ct);
+    // (the reference's phi; a reflected photon starts again unpolarised, :1283-1285)
+    PolMove m = pol_move<false>(ph, s.row, mux, muy, muz, ct, two_phi / 2., st[0], st[1], st[2], st[3], reflected, dtau, s.ext,
+                                s.rext);
+    if (!m.sure) m = pol_move_exact(ph, s.row, mux, muy, muz, ct, two_phi / 2., st[0], st[1], st[2], st[3], reflected, dtau, s.ext);
 #pragma unroll
-        for (int e = 0; e < 6; ++e) P[e] = element(ph, e, s.row, e == 0 || ph.shared_grid ? g : segment_of(ph, e, ct));
-        const double P11 = P[0], P12 = P[1], P22 = P[2], P33 = P[3], P43 = P[4], P44 = P[5];
-        sc[0] = sp[0] * P11 + sp[1] * P12;
-        sc[1] = sp[0] * P12 + sp[1] * P22;
-        sc[2] = sp[2] * P33 - sp[3] * P43;
-        sc[3] = sp[2] * P43 + sp[3] * P44;
-        const double den = sqrt_rn((1 - ct * ct) * (1 - nz * nz));
-        double cos_i = 0;
-        if (!(den == 0)) {
-            const double sign = (phi_sca >= kPi) ? 1 : -1;
-            const double num = nz * ct - muz, d = sign * den;
-            cos_i = quotient_rn(num, d, rcp_res(d));
-            if (cos_i < -1) cos_i = -1;
-            else if (cos_i > 1) cos_i = 1;
-        }
-        rotate_stokes(-acos(cos_i), sc, sm);
-        const double ri = rcp_res(sm[0]);
-        st[0] = moderate(sm[0]) ? 1 : sm[0] / sm[0];
-#pragma unroll
-        for (int k = 1; k < 4; ++k) st[k] = quotient_rn(sm[k], sm[0], ri);
-    }
+    for (int k = 0; k < 4; ++k) st[k] = m.st[k];
     s.flags &= ~kRefl;
     const double zp = s.z;
-    s.z = zp + dtau * nz;                                             // :1352
-    s.mux = nx, s.muy = ny, s.muz = nz;                               // :1364-1369
-    s.path += quotient_rn(dtau, s.ext, s.rext);                       // :1372
+    s.z = zp + dtau * m.nz;                                           // :1352
+    s.mux = m.nx, s.muy = m.ny, s.muz = m.nz;                         // :1364-1369
+    s.path += m.inc;                                                  // :1372
     s.i += 1;
-    return step_end(s, seed, s.z, zp, dtau, nz, s.path, false, ssa_rand >= (ice ? s.ssa_ice : s.ssa_imp), ice, &s.k, &s.flags);
+    return step_end(s, seed, s.z, zp, dtau, m.nz, s.path, false, ssa_rand >= (ice ? s.ssa_ice : s.ssa_imp), ice, &s.k, &s.flags);
 }
 
 // 2^glog lanes a photon, the same state in each: they test candidates of the sampler side by side
@@ -860,7 +926,8 @@ __device__ int pol_step(const DevPhase &ph, Slot &s, uint64_t seed, double st[4]
 // one divisor its reciprocal, and sine and cosine come together: about 60 a candidate and 430 a
 // step's rest (145 and 650 with one thread a photon, whose warp also waited for the slowest of 32
 // samplers).  Hexagonal plates, 100 um, tau as below 40: 50 photons 40.4 -> 9.4 ms, 1,000
-// 80.8 -> 20.3, 10,000 95.6 -> 34.9, 40,000 153 -> 87; a lone photon's step 17 us.
+// 80.8 -> 20.3, 10,000 95.6 -> 34.9, 40,000 153 -> 87; a lone photon's step 17 us; with the look at the
+// roots' and quotients' roundings 7% more for 50, 1 to 2% for 10,000 and up.
 __global__ void __launch_bounds__(128, 3) walk_replay_pol_kernel(const ReplayArgs a, const int glog) {
     const int lane = threadIdx.x & 31, G = 1 << glog, gl = lane & (G - 1), g0 = lane - gl;
     const unsigned group = (G == 32 ? 0xffffffffu : ((1u << G) - 1u)) << g0;
