@@ -81,17 +81,6 @@ __device__ __forceinline__ bool quotient_sure(double q, double a, double b) {
     return moderate(b) & quotient_certain(q, a, b);
 }
 
-// sqrt(x) and a / b, rb = rcp_res(b); any x, a, b.
-__device__ __forceinline__ double sqrt_rn(double x) {
-    double h;
-    const double g = sqrt_res(x, h);
-    return sqrt_sure(g, x) ? g : sqrt(x);
-}
-__device__ __forceinline__ double quotient_rn(double a, double b, double rb) {
-    const double q = quotient_res(a, b, rb);
-    return quotient_sure(q, a, b) ? q : a / b;
-}
-
 // 1 / d, d >= 1 (or NaN): a Newton step on the hardware's reciprocal, by the same author, which alone
 // is correctly rounded here (of every float from 1 to 2^126, which the hardware's flushes from there on).
 __device__ __forceinline__ float reciprocal_rn(float d) {

@@ -20,8 +20,8 @@ __global__ void probe(const double *a, const double *b, int n, double *q, double
     if (i >= n) return;
     double h;
     const double rb = rcp_res(b[i]), g = sqrt_res(b[i], h), r = quotient_res(a[i], b[i], rb);
-    q[i] = quotient_rn(a[i], b[i], rb);
-    s[i] = sqrt_rn(b[i]);
+    q[i] = quotient_sure(r, a[i], b[i]) ? r : a[i] / b[i];
+    s[i] = sqrt_sure(g, b[i]) ? g : sqrt(b[i]);
     // 1, 2: the root, the quotient by its doubled reciprocal certain; 4: the corrections alone, not as sqrt or /
     const bool pos = b[i] > 0 && moderate(b[i]);
     wrong[i] = (pos && sqrt_certain(g, b[i]) ? 1 : 0) | (moderate(b[i]) && quotient_certain(r, a[i], b[i]) ? 2 : 0) |
